@@ -46,7 +46,7 @@ def build_oracle(force: bool = False) -> str:
 
 def build_reference(force: bool = False) -> bool:
     """Build oracle/_ref from the reference sources if they are present."""
-    if not os.path.isdir(REFERENCE_ROOT):
+    if not os.path.exists(os.path.join(REFERENCE_ROOT, "sun.cpp")):
         return False
     args = ["make", "-C", HERE, f"REF={REFERENCE_ROOT}"]
     if force:
