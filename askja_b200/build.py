@@ -30,12 +30,14 @@ CXX = "g++"
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVFLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden",
                   "--expt-relaxed-constexpr", "-ccbin", CXX]
-CU_SOURCES = ["kernels_fp64.cu", "kernels_fp32.cu", "kernels_split.cu", "engine.cu", "static_plaq.cu", "batch.cu"]
+CU_SOURCES = ["kernels_fp64.cu", "kernels_fp32.cu", "kernels_split.cu", "engine.cu", "static_plaq.cu", "batch.cu",
+              "mma64.cu", "mma64_full64.cu", "mma64_part64.cu", "mma64_full32.cu", "mma64_part32.cu"]
 # bench-only helper (compute-pipe peak probe for the roofline), not part of the product ABI
 PEAK_SRC = "peak.cu"
 PEAK_LIB = os.path.join(HERE, "libaskja_peak.so")
 CPP_SOURCES = ["hostio.cpp"]
-HEADERS = ["common.cuh", "small.cuh", "rows.cuh", "misc.cuh", "kernels.cuh", "launch.h", "batch.cuh", "tc.cuh", "eig.cuh", "pair.cuh", "tab.cuh", "split.cuh", "split.h"]
+HEADERS = ["common.cuh", "small.cuh", "rows.cuh", "misc.cuh", "kernels.cuh", "launch.h", "batch.cuh", "tc.cuh", "eig.cuh", "pair.cuh", "tab.cuh", "split.cuh", "split.h",
+           "mma64.cuh", "mma64.h", "mma64_launch.cuh"]
 
 
 def _newer(target: str, deps) -> bool:

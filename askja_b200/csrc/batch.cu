@@ -22,6 +22,8 @@
 #include "batch.cuh"
 #include "kernels.cuh"
 #include "launch.h"
+#include "mma64.cuh"
+#include "mma64.h"
 #include "split.h"
 
 using askja::Lat;
@@ -35,20 +37,23 @@ struct askja_batch {
   std::vector<askja_chain_params> params;
   std::vector<ChainDev> desc;
   ChainDev* d_desc = nullptr;
+  askja::m64::Job* d_jobs = nullptr;  // one per chain (NC >= 5 filled in), for the kernels of mma64.cuh
+  int* d_kin_item = nullptr;          // kinetic launch over the NC >= 5 chains
+  int n_kin_items = 0;
   std::vector<void*> allocs;
   cudaStream_t stream = nullptr;
   std::vector<cudaStream_t> side;
   std::vector<cudaEvent_t> ev;
   struct Group {
-    int N = 0;      // colour number (small path) or 0 for the row path
-    int nmax = 0;   // row path register bucket
-    int G = 1;      // row path groups per CTA
-    size_t smem = 0;
+    int N = 0;      // colour number
     std::vector<int> chains;
     int* d_start = nullptr;
     int* d_ids = nullptr;
     int* d_item = nullptr;  // per item: chain index (into the descriptors) and item within the chain, interleaved
     int nitems = 0;
+    // NC >= 5: the plaquette launch's list (d_item holds the link update's)
+    int* d_plaq_item = nullptr;
+    int n_plaq_items = 0;
   };
   std::vector<Group> groups;
   int* d_plaq_start = nullptr;
@@ -119,6 +124,13 @@ template <typename T>
 cudaError_t launch_force(askja_batch* b, const askja_batch::Group& g, cudaStream_t st, int mode, double ks) {
   using namespace askja::batch;
   const dim3 grid(g.nitems);
+  if (askja::m64_supported(g.N)) {
+    askja::m64::Grid mg;
+    mg.table = b->d_jobs;
+    mg.items = (const int2*)g.d_item;
+    mg.ctas = g.nitems;
+    return askja::m64::link(g.N, sizeof(T) == 8, askja::m64::Job{}, mg, b->cur, ks, mode, st);
+  }
   if (g.N == 2 || g.N == 3 || g.N == 4) {
     int maxd = 1;
     for (int c : g.chains) maxd = std::max(maxd, b->desc[c].lat.D);
@@ -158,18 +170,7 @@ cudaError_t launch_force(askja_batch* b, const askja_batch::Group& g, cudaStream
 #undef SMALL
     return cudaGetLastError();
   }
-  const dim3 blk(g.G * b->params[g.chains[0]].nc);
-#define ROWS(NM)                                                                                              \
-  if (g.nmax == NM) {                                                                                         \
-    auto k = mode ? kb_force_rows<NM, T, 1> : kb_force_rows<NM, T, 0>;                                        \
-    if constexpr (sizeof(T) == 4 && NM == 8)                                                                  \
-      if (mode) k = kb_force_rows8f;                                                                          \
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem);                        \
-    k<<<grid, blk, g.smem, st>>>(b->d_desc, (const int2*)g.d_item, b->cur, ks);                              \
-  }
-  ROWS(8) ROWS(16) ROWS(32) ROWS(64)
-#undef ROWS
-  return cudaGetLastError();
+  return cudaErrorInvalidValue;
 }
 
 // all groups' force launches for one MD step, forked onto side streams
@@ -196,8 +197,23 @@ template <typename T>
 int energies(askja_batch* b, int which) {
   using S2 = typename askja::Storage<T>::type;
   using namespace askja::batch;
-  kb_plaq<S2><<<b->n_plaq, askja::misc::RED_THREADS, 0, b->stream>>>(b->d_desc, b->d_plaq_start, b->nchains, b->cur);
-  kb_kinetic<S2><<<b->n_link, askja::misc::RED_THREADS, 0, b->stream>>>(b->d_desc, b->d_link_start, b->nchains);
+  if (b->n_plaq) {
+    kb_plaq<S2><<<b->n_plaq, askja::misc::RED_THREADS, 0, b->stream>>>(b->d_desc, b->d_plaq_start, b->nchains, b->cur);
+    kb_kinetic<S2><<<b->n_link, askja::misc::RED_THREADS, 0, b->stream>>>(b->d_desc, b->d_link_start, b->nchains);
+  }
+  askja::m64::Grid mg;
+  mg.table = b->d_jobs;
+  for (const auto& g : b->groups) {
+    if (!g.n_plaq_items) continue;
+    mg.items = (const int2*)g.d_plaq_item;
+    mg.ctas = g.n_plaq_items;
+    BCK(askja::m64::plaq(g.N, sizeof(T) == 8, askja::m64::Job{}, mg, b->cur, b->stream));
+  }
+  if (b->n_kin_items) {
+    mg.items = (const int2*)b->d_kin_item;
+    mg.ctas = b->n_kin_items;
+    BCK(askja::m64::kinetic(sizeof(T) == 8, askja::m64::Job{}, mg, 1, b->stream));
+  }
   kb_energy<<<b->nchains, askja::misc::RED_THREADS, 0, b->stream>>>(b->d_desc, which);
   BCK(cudaGetLastError());
   return ASKJA_OK;
@@ -308,7 +324,8 @@ int askja_batch_create(const askja_chain_params* chains, int nchains, int precis
   const size_t elem = precision == ASKJA_FP64 ? 16 : 8;
   b->desc.resize(nchains);
   size_t max_conf = 0;
-  std::vector<int> plaq_start(1, 0), link_start(1, 0), refresh_start(1, 0), copy_start(1, 0);
+  std::vector<int> plaq_start(1, 0), link_start(1, 0), refresh_start(1, 0), copy_start(1, 0), kin_item;
+  std::vector<askja::m64::Job> jobs(nchains);
   for (int c = 0; c < nchains; c++) {
     const askja_chain_params& p = chains[c];
     ChainDev& d = b->desc[c];
@@ -350,8 +367,7 @@ int askja_batch_create(const askja_chain_params* chains, int nchains, int precis
     d.beta = p.beta;
     d.scale = std::sqrt(2.0 * p.nc / p.beta);
     d.order = askja::taylor_order(p.level);
-    // FP32: reunitarise after each update; on the row kernels (NC > 4) by a
-    // Newton-Schulz step, with a full pass every FULL_REUNIT_EVERY
+    // FP32: reunitarise after each update; for NC > 4 by a Newton-Schulz step, with a full pass every FULL_REUNIT_EVERY
     // trajectories, as a single chain does
     d.reunit = precision == ASKJA_FP32 ? (p.nc > 4 ? 2 : 1) : 0;
     if (precision == ASKJA_FP32 && askja::splitk::supported(p.nc)) d.reunit = 0;  // residual planes: per trajectory
@@ -359,8 +375,11 @@ int askja_batch_create(const askja_chain_params* chains, int nchains, int precis
     if (int rc = dalloc(b, &d.st, sizeof(TrajState))) return fail(rc);
     if (cudaMemset(d.st, 0, sizeof(TrajState)) != cudaSuccess) return fail(berr(b, ASKJA_ERR_CUDA, "memset"));
     if (int rc = dalloc(b, &d.sums, 8 * sizeof(double))) return fail(rc);
-    d.plaq_blocks = (int)((V + askja::misc::RED_THREADS - 1) / askja::misc::RED_THREADS);
-    d.link_blocks = (int)((V * p.dim + askja::misc::RED_THREADS - 1) / askja::misc::RED_THREADS);
+    const bool m64 = askja::m64_supported(p.nc);
+    // the same partition as a single chain's reductions, so that the sums agree bit for bit
+    d.plaq_blocks = askja::m64::ctas_for(V, m64 ? askja::m64::links_per_cta(p.nc) : askja::misc::RED_THREADS);
+    d.link_blocks =
+        askja::m64::ctas_for(V * p.dim, m64 ? askja::m64::kinetic_links_per_cta() : askja::misc::RED_THREADS);
     if (int rc = dalloc(b, &d.partial, (2 * (size_t)d.plaq_blocks + d.link_blocks) * sizeof(double))) return fail(rc);
     d.n16 = (long)(fbytes / 16);
     if (precision == ASKJA_FP32 && askja::splitk::supported(p.nc)) {
@@ -376,8 +395,24 @@ int askja_batch_create(const askja_chain_params* chains, int nchains, int precis
       d.n16lo = (long)(lo_bytes / 16);
       b->any_split = true;
     }
-    plaq_start.push_back(plaq_start.back() + d.plaq_blocks);
-    link_start.push_back(link_start.back() + d.link_blocks);
+    plaq_start.push_back(plaq_start.back() + (m64 ? 0 : d.plaq_blocks));
+    link_start.push_back(link_start.back() + (m64 ? 0 : d.link_blocks));
+    if (m64) {
+      askja::m64::Job& j = jobs[c];
+      j = askja::detail::m64_job(L);
+      j.order = d.order;
+      j.project = d.reunit == 2;
+      j.U[0] = d.U[0];
+      j.U[1] = d.U[1];
+      j.Pin = j.Pout = d.P;
+      j.kick = j.dt = d.dt;
+      j.plaq_partial = d.partial;
+      j.kin_partial = d.partial + 2 * (size_t)d.plaq_blocks;
+      for (int t = 0; t < d.link_blocks; t++) {
+        kin_item.push_back(c);
+        kin_item.push_back(t);
+      }
+    }
     refresh_start.push_back(refresh_start.back() + (int)((V * p.dim + 127) / 128));
     copy_start.push_back(copy_start.back() + (int)((d.n16 + 4095) / 4096) + (int)((d.n16lo + 4095) / 4096));
     max_conf = std::max(max_conf, (size_t)V * p.dim * p.nc * p.nc * 16);
@@ -396,7 +431,14 @@ int askja_batch_create(const askja_chain_params* chains, int nchains, int precis
   b->n_refresh = refresh_start.back();
   b->n_copy = copy_start.back();
   if (int rc = dalloc(b, &b->staging, max_conf)) return fail(rc);
-  // force groups: one per small colour number, one per row-path bucket and colour number
+  b->n_kin_items = (int)(kin_item.size() / 2);
+  if (b->n_kin_items) {
+    if (int rc = upload_ints(b, &b->d_kin_item, kin_item)) return fail(rc);
+    if (int rc = dalloc(b, &b->d_jobs, jobs.size() * sizeof(jobs[0]))) return fail(rc);
+    if (cudaMemcpy(b->d_jobs, jobs.data(), jobs.size() * sizeof(jobs[0]), cudaMemcpyHostToDevice) != cudaSuccess)
+      return fail(berr(b, ASKJA_ERR_CUDA, "job upload"));
+  }
+  // force groups: one per colour number
   std::map<int, std::vector<int>> by_nc;
   for (int c = 0; c < nchains; c++) by_nc[chains[c].nc].push_back(c);
   for (auto& kv : by_nc) {
@@ -405,8 +447,8 @@ int askja_batch_create(const askja_chain_params* chains, int nchains, int precis
     const int N = kv.first;
     std::vector<int> start(1, 0);
     std::vector<int> item;
+    g.N = N;
     if (N <= 4) {
-      g.N = N;
       for (int c : g.chains) {
         start.push_back(start.back() + b->desc[c].lat.B);
         for (int t = 0; t < b->desc[c].lat.B; t++) {
@@ -415,21 +457,22 @@ int askja_batch_create(const askja_chain_params* chains, int nchains, int precis
         }
       }
     } else {
-      g.N = 0;
-      g.nmax = N <= 8 ? 8 : N <= 16 ? 16 : N <= 32 ? 32 : 64;
-      if (precision == ASKJA_FP64)
-        askja::detail::Rows<double>::shape(N, &g.G, &g.smem);
-      else
-        askja::detail::Rows<float>::shape(N, &g.G, &g.smem);
+      std::vector<int> plaq_item;
       for (int c : g.chains) {
         const Lat& L = b->desc[c].lat;
-        const int n = (int)((L.V + g.G - 1) / g.G) * L.D;
+        const int n = askja::m64::ctas_for((long)L.V * L.D, askja::m64::links_per_cta(N));
         start.push_back(start.back() + n);
         for (int t = 0; t < n; t++) {
           item.push_back(c);
           item.push_back(t);
         }
+        for (int t = 0; t < b->desc[c].plaq_blocks; t++) {
+          plaq_item.push_back(c);
+          plaq_item.push_back(t);
+        }
       }
+      g.n_plaq_items = (int)(plaq_item.size() / 2);
+      if (int rc = upload_ints(b, &g.d_plaq_item, plaq_item)) return fail(rc);
     }
     g.nitems = start.back();
     if (int rc = upload_ints(b, &g.d_start, start)) return fail(rc);

@@ -4,15 +4,15 @@
 // the chain c with item_start[c] <= i < item_start[c+1] (the force launches,
 // which run every MD step, read (chain, item within the chain) from a per-item
 // table instead); the CTA takes that chain's descriptor and runs the same
-// per-link / per-site code as the single-chain kernels (small.cuh, rows.cuh,
-// split.cuh, misc.cuh).  Chains of different sizes therefore share the GPU in
+// per-link / per-site code as the single-chain kernels (small.cuh, split.cuh,
+// misc.cuh).  Chains of NC >= 5 go through the single-chain kernels of
+// mma64.cuh themselves, which read a job table.  Chains of different sizes therefore share the GPU in
 // proportion to their work.
 #pragma once
 
 #include <type_traits>
 
 #include "misc.cuh"
-#include "rows.cuh"
 #include "small.cuh"
 #include "split.cuh"
 
@@ -74,20 +74,6 @@ __device__ __forceinline__ int load_chain(ChainDev& sd, const ChainDev* __restri
   for (int w = threadIdx.x; w < (int)(sizeof(ChainDev) / 4); w += blockDim.x) dst[w] = __ldg(src + w);
   __syncthreads();
   return blockIdx.x - __ldg(item_start + k);
-}
-
-// Copies the descriptor of the chain named by this CTA's entry (chain, item)
-// of the per-item table into shared memory; returns the item's index within
-// its chain (one load instead of load_chain's binary search).
-__device__ __forceinline__ int load_chain_at(ChainDev& sd, const ChainDev* __restrict__ descs,
-                                             const int2* __restrict__ item_chain) {
-  static_assert(sizeof(ChainDev) % 4 == 0, "descriptor copied in 4-byte words");
-  const int2 ct = __ldg(item_chain + blockIdx.x);
-  const uint32_t* src = reinterpret_cast<const uint32_t*>(descs + ct.x);
-  uint32_t* dst = reinterpret_cast<uint32_t*>(&sd);
-  for (int w = threadIdx.x; w < (int)(sizeof(ChainDev) / 4); w += blockDim.x) dst[w] = __ldg(src + w);
-  __syncthreads();
-  return ct.y;
 }
 
 // Force (+ link update) for the small-NC chains of one colour number: item =
@@ -167,40 +153,7 @@ __global__ void __launch_bounds__(128, 7) kb_force_small3f(const ChainDev* __res
   force_small_item<3, float, MODE, true>(descs, item_start, chain_ids, nchains, cur, kick_scale);
 }
 
-// Same for the row-per-thread path: item = G consecutive sites of one
-// direction (G = blockDim / NC), directions of a site block adjacent.
-template <int NMAX, typename T, int MODE>
-__global__ void kb_force_rows(const ChainDev* __restrict__ descs, const int2* __restrict__ item_chain, int cur,
-                              double kick_scale) {
-  using S2 = typename Storage<T>::type;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ int piv_s[64];
-  __shared__ cpx<T> det_s[64];
-  __shared__ ChainDev sd;
-  const int item = load_chain_at(sd, descs, item_chain);
-  const int G = blockDim.x / sd.lat.N;
-  rows::force_rows<NMAX, T, S2, MODE>(sd.lat, (const S2*)sd.U[cur], (const S2*)sd.P, (S2*)sd.P,
-                                      (S2*)sd.U[cur ^ 1], (T)(kick_scale * sd.dt), (T)sd.dt, sd.order, sd.reunit,
-                                      item % sd.lat.D, (item / sd.lat.D) * G, smem_raw, piv_s, det_s);
-}
-
-// FP32 with NMAX = 8, fused kick + drift: at most 128 registers (four
-// 128-thread CTAs per SM), as the single-chain rows::k_force8.
-static __global__ void __launch_bounds__(256, 2) kb_force_rows8f(const ChainDev* __restrict__ descs,
-                                                          const int2* __restrict__ item_chain, int cur,
-                                                          double kick_scale) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ int piv_s[64];
-  __shared__ cpx<float> det_s[64];
-  __shared__ ChainDev sd;
-  const int item = load_chain_at(sd, descs, item_chain);
-  const int G = blockDim.x / sd.lat.N;
-  rows::force_rows<8, float, float2, 1>(sd.lat, (const float2*)sd.U[cur], (const float2*)sd.P, (float2*)sd.P,
-                                        (float2*)sd.U[cur ^ 1], (float)(kick_scale * sd.dt), (float)sd.dt, sd.order,
-                                        sd.reunit, item % sd.lat.D, (item / sd.lat.D) * G, smem_raw, piv_s, det_s);
-}
-
-// Plaquette sums: item = RED_THREADS-site block; partial per chain block.
+// Plaquette sums of the NC <= 4 chains: item = RED_THREADS-site block; partial per chain block.
 template <typename S2>
 __global__ void __launch_bounds__(misc::RED_THREADS) kb_plaq(const ChainDev* __restrict__ descs,
                                                              const int* __restrict__ item_start, int nchains,
@@ -222,8 +175,7 @@ __global__ void __launch_bounds__(misc::RED_THREADS) kb_plaq(const ChainDev* __r
     switch (sd.lat.N) {
       case 2: misc::plaq_site<2, S2>(sd.lat, U, s, v); break;
       case 3: misc::plaq_site<3, S2>(sd.lat, U, s, v); break;
-      case 4: misc::plaq_site<4, S2>(sd.lat, U, s, v); break;
-      default: misc::plaq_site<0, S2>(sd.lat, U, s, v);
+      default: misc::plaq_site<4, S2>(sd.lat, U, s, v);
     }
   }
   misc::block_sum<2>(v);
@@ -233,7 +185,7 @@ __global__ void __launch_bounds__(misc::RED_THREADS) kb_plaq(const ChainDev* __r
   }
 }
 
-// Kinetic sums sum tr2(P): item = RED_THREADS-link block.
+// Kinetic sums sum tr2(P) of the NC <= 4 chains: item = RED_THREADS-link block.
 template <typename S2>
 __global__ void __launch_bounds__(misc::RED_THREADS) kb_kinetic(const ChainDev* __restrict__ descs,
                                                                 const int* __restrict__ item_start, int nchains) {
@@ -253,8 +205,7 @@ __global__ void __launch_bounds__(misc::RED_THREADS) kb_kinetic(const ChainDev* 
     switch (sd.lat.N) {
       case 2: misc::link_sums<2, S2>(sd.lat, (const S2*)sd.P, nullptr, nullptr, t, v); break;
       case 3: misc::link_sums<3, S2>(sd.lat, (const S2*)sd.P, nullptr, nullptr, t, v); break;
-      case 4: misc::link_sums<4, S2>(sd.lat, (const S2*)sd.P, nullptr, nullptr, t, v); break;
-      default: misc::link_sums<0, S2>(sd.lat, (const S2*)sd.P, nullptr, nullptr, t, v);
+      default: misc::link_sums<4, S2>(sd.lat, (const S2*)sd.P, nullptr, nullptr, t, v);
     }
   }
   misc::block_sum<3>(v);

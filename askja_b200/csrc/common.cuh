@@ -2,7 +2,7 @@
 // arithmetic on (re, im) pairs, the field layout, the periodic neighbour
 // table, Philox4x32-10 and Box-Muller.
 //
-// Field layout in HBM (all link and momentum fields), blocked by 32 sites:
+// Field layout in HBM, NC <= 4 (a thread owns a whole matrix): blocked by 32 sites,
 //   element e = r*NC + c of the matrix on link (site s, direction d) lives at
 //   f[((d * B + s/32) * NC*NC + e) * 32 + s%32],   B = ceil(V/32) site blocks,
 // as float2 (FP32 mode) or double2 (FP64 mode).  A warp that walks 32
@@ -10,8 +10,15 @@
 // element -- 256 B (FP32) / 512 B (FP64) per load instruction, coalesced --
 // and the NC*NC elements of one link are a fixed 32-element stride apart, so a
 // thread addresses a whole matrix from one base pointer with compile-time
-// offsets.  Sites V..32B-1 are padding.  Site numbering is the reference's
-// (structs.h:130-165): x0 slowest, x_{D-1} fastest.
+// offsets.  Sites V..32B-1 are padding.
+//
+// NC >= 5 (a warp or more owns a matrix): link-major, the row-major matrix of
+// link (s, d) contiguous at f[(d * V + s) * NC*NC + e], so that a warp's 8 x 8
+// tile loads (mma64.cuh) and the tensor-core path's operand loads (tc.cuh) read
+// whole sectors with no copy of the links into another order.
+//
+// Site numbering is the reference's (structs.h:130-165): x0 slowest, x_{D-1}
+// fastest.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -132,14 +139,51 @@ __device__ __forceinline__ int nb_minus(const Lat& L, int d, int s) {
   return __ldg(L.nbr + (size_t)(2 * d + 1) * L.V + s);
 }
 
-// Offset of element 0 of the link (d, s); element e is at + 32*e.
-__host__ __device__ __forceinline__ size_t mbase(const Lat& L, int d, int s) {
+// whether the fields of colour number N are link-major (else blocked by sites)
+__host__ __device__ __forceinline__ bool link_major(int N) { return N > 4; }
+
+// Offset of element 0 of the link (d, s) in the blocked layout; element e is at + 32*e.
+__host__ __device__ __forceinline__ size_t bbase(const Lat& L, int d, int s) {
   return ((size_t)d * L.B + (s >> 5)) * (size_t)(L.N * L.N) * 32 + (s & 31);
 }
 
+// Offset of element 0 of the link (d, s) and distance between its elements, either layout.
+__host__ __device__ __forceinline__ size_t mbase(const Lat& L, int d, int s) {
+  return link_major(L.N) ? ((size_t)d * L.V + s) * (size_t)(L.N * L.N) : bbase(L, d, s);
+}
+__host__ __device__ __forceinline__ int estride(const Lat& L) { return link_major(L.N) ? 1 : 32; }
+
 // Offset of element e of the link (d, s).
 __host__ __device__ __forceinline__ size_t eoff(const Lat& L, int d, int e, int s) {
-  return mbase(L, d, s) + (size_t)e * 32;
+  return mbase(L, d, s) + (size_t)e * estride(L);
+}
+
+// The same for a colour number known at compile time (NT 2..4: blocked, no
+// choice of layout at run time; NT 0: any).
+template <int NT>
+__host__ __device__ __forceinline__ size_t eoffn(const Lat& L, int d, int e, int s) {
+  if constexpr (NT > 0 && NT <= 4)
+    return ((size_t)d * L.B + (s >> 5)) * (size_t)(NT * NT * 32) + (s & 31) + (size_t)e * 32;
+  else
+    return eoff(L, d, e, s);
+}
+
+// Link and matrix element of the t-th complex number of a field; false for padding.
+__device__ __forceinline__ bool field_index(const Lat& L, long t, int* d, int* s, int* e) {
+  const int NN = L.N * L.N;
+  if (link_major(L.N)) {
+    const long l = t / NN;
+    *e = (int)(t - l * NN);
+    *d = (int)(l / L.V);
+    *s = (int)(l - (long)*d * L.V);
+    return *d < L.D;
+  }
+  const long rest = t >> 5;
+  *e = (int)(rest % NN);
+  const long db = rest / NN;
+  *d = (int)(db / L.B);
+  *s = (int)((db - (long)*d * L.B) * 32 + (t & 31));
+  return *s < L.V;
 }
 
 // Complex elements in one field (padding included).

@@ -193,9 +193,15 @@ cudaError_t force_launch(askja_ctx* c, int mode, int in, int out, double ek, dou
                       mode == 1 ? c->U[1 - c->cur] : nullptr, ek, ed);
 }
 
-// U <- exp(i eps Pi) U in place (updateUandcopyDown before its copy)
+// U <- exp(i eps Pi) U (updateUandcopyDown before its copy); the kernels of
+// link-major fields write the partner buffer, which becomes the current one
 cudaError_t drift_launch(askja_ctx* c, double eps) {
   if (c->split) return askja::splitk::drift(c->lc, cur_u(c), cur_ul(c), c->P2C, c->P2CL, eps);
+  if (askja::link_major(c->N) && c->lc.force_rows != 1) {
+    const cudaError_t e = c->ks->force(c->lc, 2, cur_u(c), c->P2, nullptr, c->U[1 - c->cur], 0.0, eps);
+    if (e == cudaSuccess) c->cur ^= 1;
+    return e;
+  }
   return c->ks->drift(c->lc, cur_u(c), c->P2, eps);
 }
 
@@ -243,10 +249,9 @@ int launch_ok(askja_ctx* c, cudaError_t e, const char* what) {
     if (rc_) return rc_;                          \
   } while (0)
 
-// whether the fused kick+drift runs on the row-per-thread kernels
-bool uses_rows(const askja_ctx* c) {
-  return c->lc.force_rows == 1 || (c->lc.force_rows == 0 && c->N > 4);
-}
+// whether the fused kick+drift projects each update without pinning the
+// determinant (row-per-thread and FP64-MMA kernels, with rows_ns)
+bool per_update_ns(const askja_ctx* c) { return c->lc.force_rows == 1 || c->N > 4; }
 
 bool paired(const askja_ctx* c) { return c->lc.force_rows == 3; }
 
@@ -280,12 +285,12 @@ int enqueue_trajectory(askja_ctx* c, int nsteps) {
     // trajectory starts from links projected onto SU(N) in FP64 (the saved
     // copy follows, so a rejected trajectory restores projected links)
     KL(askja::splitk::reunit(c->lc, cur_u(c), cur_ul(c), c->Uconf, c->ULconf), "reunitarise");
-  } else if (c->lc.reunit && (c->lc.force_rows == 2 || (c->lc.rows_ns && uses_rows(c)))) {
+  } else if (c->lc.reunit && (c->lc.force_rows == 2 || (c->lc.rows_ns && per_update_ns(c)))) {
     // the tensor-core link update keeps U' exactly as unitary as U (it
     // projects exp(i eps P), not U'); the rounding defect U accumulates (an
     // unbiased random walk, ~6e-8 sqrt(MD steps)) is removed here, before
     // every askja::FULL_REUNIT_EVERY-th trajectory, and the saved copy follows.  The
-    // FP32 row kernels project each update by a Newton-Schulz step, which
+    // other FP32 kernels of NC > 4 project each update by a Newton-Schulz step, which
     // leaves the determinant phase free; this pass pins it back to 1.
     askja::LaunchCtx lc = c->lc;
     lc.gate = &c->st->traj;
@@ -566,13 +571,13 @@ int askja_create(const askja_params* p, askja_ctx** out) {
   c->lc.rows_ns = p->precision == ASKJA_FP32;
   CKC(cudaMalloc(&c->tc_status, sizeof(unsigned)));
   CKC(cudaMemset(c->tc_status, 0, sizeof(unsigned)));
-  c->lc.scratch = c->staging;
   c->lc.status = c->tc_status;
-  // untuned default: tensor cores for NC = 32 and 64, else thread-per-link for NC <= 4 (rows above);
-  // NC = 16 on the tensor cores is an explicit path and an autotuner candidate
+  // untuned default: TF32 tensor cores for FP32 NC = 32 and 64, else thread-per-link for NC <= 4 and the
+  // FP64 MMA above; NC = 16 on the TF32 tensor cores is an explicit path and an autotuner candidate
   c->lc.force_rows = p->kernel_path != 0 ? p->kernel_path
                      : (p->nc >= 32 && askja::tc_supported(p->nc, p->dim, p->precision == ASKJA_FP64)) ? 2
-                                                                                                      : 0;
+                     : askja::m64_supported(p->nc)                                                            ? 4
+                                                                                                              : 0;
   c->lc.rows_groups = 0;
   c->lc.small_occ = 0;
   if (p->kernel_path == 0) {
@@ -1077,7 +1082,8 @@ int askja_run_trajectories(askja_ctx* c, int ntraj, int nsteps, int use_graph, a
 
 int askja_set_tuning(askja_ctx* c, const askja_tuning* t) {
   if (int rc = check_ctx(c)) return rc;
-  if (!t || t->path < 0 || t->path > 3 || (t->path == 0 && c->N > 4) || t->groups < 0 || (c->split && t->path != 0) ||
+  if (!t || t->path < 0 || t->path > 4 || (t->path == 0 && c->N > 4) ||
+      (t->path == 4 && !askja::m64_supported(c->N)) || t->groups < 0 || (c->split && t->path != 0) ||
       (t->path == 2 && !askja::tc_supported(c->N, c->D, c->p.precision == ASKJA_FP64)) ||
       (t->path == 3 && !askja::pair_supported(c->N, c->D, c->p.precision == ASKJA_FP64, c->lat.n[c->D - 1])))
     return set_err(c, ASKJA_ERR_ARG, "invalid tuning");
@@ -1104,6 +1110,7 @@ int askja_autotune(askja_ctx* c, int reps, askja_tuning* out) {
     cands.push_back({0, 0, 2});
   }
   if (askja::tc_supported(c->N, c->D, fp64)) cands.push_back({2, 0, 0});
+  if (askja::m64_supported(c->N)) cands.push_back({4, 0, 0});
 
   std::vector<int> seen;
   // the residual-plane mode has one mapping (thread per link); only its register budget is tuned

@@ -5,6 +5,8 @@
 #include <algorithm>
 
 #include "launch.h"
+#include "mma64.cuh"
+#include "mma64.h"
 #include "misc.cuh"
 #include "rows.cuh"
 #include "small.cuh"
@@ -129,23 +131,53 @@ cudaError_t small_drift(const LaunchCtx& c, void* U, const void* P, double eps) 
   return cudaGetLastError();
 }
 
-// Tensor-core link update (FP32 storage): per-link copy of U into the
-// scratch buffer, then one persistent launch over all links.
-// mode 0 kick, 1 kick + drift, 2 drift only (Uout may be U).
+// FP64-MMA kernels: this lattice's fields as their job
+inline m64::Job m64_job(const Lat& L) {
+  m64::Job j{};
+  j.nbr = L.nbr;
+  j.V = L.V;
+  j.D = L.D;
+  j.N = L.N;
+  j.r0 = L.r0;
+  j.r1 = L.r1;
+  return j;
+}
+
+template <typename T>
+cudaError_t reunit(const LaunchCtx& c, void* U);
+
+template <typename T>
+cudaError_t m64_link(const LaunchCtx& c, int mode, const void* U, const void* Pin, void* Pout, void* Uout, double ek,
+                     double ed) {
+  m64::Job j = m64_job(c.lat);
+  j.order = c.order;
+  // FP32 single chains: projected to first order in the kernel (as rows_ns); otherwise in full afterwards
+  const bool ns = sizeof(T) == 4 && c.rows_ns && mode == 1;
+  j.project = c.reunit && ns;
+  j.U[0] = const_cast<void*>(U);
+  j.U[1] = Uout;
+  j.Pin = Pin;
+  j.Pout = Pout;
+  j.kick = ek;
+  j.dt = ed;
+  cudaError_t e = m64::link(c.lat.N, sizeof(T) == 8, j, m64::Grid{}, 0, 1.0, mode, c.stream);
+  if (e != cudaSuccess || mode == 0 || !c.reunit || ns) return e;
+  LaunchCtx full = c;
+  full.gate = nullptr;
+  return reunit<T>(full, Uout);
+}
+
+// Tensor-core link update (FP32 storage): one persistent launch over all links.
+// mode 0 kick, 1 kick + drift, 2 drift only.
 template <int NC>
 cudaError_t tc_link(const LaunchCtx& c, int mode, const void* U, const void* Pin, void* Pout, void* Uout, double ek,
                     double ed) {
   const Lat& L = c.lat;
-  if (!c.scratch || !c.status) return cudaErrorInvalidValue;
-  float2* aos = static_cast<float2*>(c.scratch);
+  if (!c.status) return cudaErrorInvalidValue;
   int dev = 0, nsm = 0;
   cudaError_t e;
   if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
   if ((e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-  const int chunks = (NC * NC + 31) / 32;
-  const int z = std::max(1, std::min(chunks, (4 * nsm + L.B * L.D - 1) / (L.B * L.D)));
-  tc::k_to_aos<<<dim3(L.B, L.D, z), 256, 0, c.stream>>>(L, static_cast<const float2*>(U), aos);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
   auto k = mode == 0 ? tc::k_link<NC, 0> : mode == 1 ? tc::k_link<NC, 1> : tc::k_link<NC, 2>;
   const size_t smem = tc::Shape<NC>::SMEM;
   if ((e = set_smem(k, smem)) != cudaSuccess) return e;
@@ -169,7 +201,7 @@ cudaError_t tc_link(const LaunchCtx& c, int mode, const void* U, const void* Pin
   per = std::min(per, 2048 / tc::THREADS);
   per = std::max(1, std::min(per, 512 / tc::Shape<NC>::TMEM_COLS));
   const long grid = std::min(nlinks(L), (long)nsm * per);
-  k<<<(unsigned)grid, tc::THREADS, smem, c.stream>>>(L, aos, static_cast<const float2*>(Pin),
+  k<<<(unsigned)grid, tc::THREADS, smem, c.stream>>>(L, static_cast<const float2*>(U), static_cast<const float2*>(Pin),
                                                       static_cast<float2*>(Pout), static_cast<float2*>(Uout),
                                                       (float)ek, (float)ed, c.order, c.reunit, c.status);
   return cudaGetLastError();
@@ -220,7 +252,8 @@ cudaError_t force(const LaunchCtx& c, int mode, const void* U, const void* Pin, 
   if (c.force_rows == 2 && tc_supported(N, c.lat.D, sizeof(T) == 8))
     return tc_dispatch<T>(c, mode, U, Pin, Pout, Uout, ek, ed);
   if (c.force_rows == 3 && mode == 1) return pair_force<T>(c, U, Pin, Pout, Uout, ek, ed);
-  if (!c.force_rows || c.force_rows == 3) {
+  if (c.force_rows != 1) {
+    if (m64_supported(N)) return m64_link<T>(c, mode, U, Pin, Pout, Uout, ek, ed);
     if (N == 2) return small_force<2, T>(c, mode, U, Pin, Pout, Uout, ek, ed);
     if (N == 3) return small_force<3, T>(c, mode, U, Pin, Pout, Uout, ek, ed);
     if (N == 4) return small_force<4, T>(c, mode, U, Pin, Pout, Uout, ek, ed);
@@ -235,9 +268,7 @@ cudaError_t force(const LaunchCtx& c, int mode, const void* U, const void* Pin, 
 template <typename T>
 cudaError_t drift(const LaunchCtx& c, void* U, const void* P, double eps) {
   const int N = c.lat.N;
-  if (c.force_rows == 2 && tc_supported(N, c.lat.D, sizeof(T) == 8))
-    return tc_dispatch<T>(c, 2, U, P, nullptr, U, 0.0, eps);
-  if (!c.force_rows || c.force_rows == 3) {
+  if (c.force_rows != 1) {
     if (N == 2) return small_drift<2, T>(c, U, P, eps);
     if (N == 3) return small_drift<3, T>(c, U, P, eps);
     if (N == 4) return small_drift<4, T>(c, U, P, eps);
@@ -254,7 +285,7 @@ cudaError_t reunit(const LaunchCtx& c, void* U) {
   using S2 = typename Storage<T>::type;
   const int N = c.lat.N;
   const unsigned gsm = blocks_for(nlinks(c.lat), SMALL_THREADS);
-  if (!c.force_rows || c.force_rows == 3) {
+  if (c.force_rows != 1) {
     if (N == 2) {
       small::k_reunit<2, T, S2><<<gsm, SMALL_THREADS, 0, c.stream>>>(c.lat, (S2*)U);
       return cudaGetLastError();
@@ -282,13 +313,14 @@ template <typename T>
 cudaError_t plaq(const LaunchCtx& c, const void* U, double* partial, double* out) {
   using S2 = typename Storage<T>::type;
   const int N = c.lat.N;
-  if (N >= misc::BIG_NC) {
-    auto k = misc::k_plaq_big<S2>;
-    const size_t smem = 2 * (size_t)N * (N + 1) * sizeof(cpx<double>);
-    cudaError_t e;
-    if ((e = set_smem(k, smem)) != cudaSuccess) return e;
-    k<<<c.lat.V, misc::RED_THREADS, smem, c.stream>>>(c.lat, (const S2*)U, partial);
-    misc::k_finish<2><<<1, misc::RED_THREADS, 0, c.stream>>>(partial, c.lat.V, out);
+  if (m64_supported(N)) {
+    m64::Job j = m64_job(c.lat);
+    j.U[0] = const_cast<void*>(U);
+    j.plaq_partial = partial;
+    const cudaError_t e = m64::plaq(N, sizeof(T) == 8, j, m64::Grid{}, 0, c.stream);
+    if (e != cudaSuccess) return e;
+    misc::k_finish<2><<<1, misc::RED_THREADS, 0, c.stream>>>(partial, m64::ctas_for(c.lat.V, m64::links_per_cta(N)),
+                                                             out);
     return cudaGetLastError();
   }
   const unsigned nb = blocks_for(c.lat.V, misc::RED_THREADS);
@@ -296,10 +328,8 @@ cudaError_t plaq(const LaunchCtx& c, const void* U, double* partial, double* out
     misc::k_plaq<2, S2><<<nb, misc::RED_THREADS, 0, c.stream>>>(c.lat, (const S2*)U, partial);
   else if (N == 3)
     misc::k_plaq<3, S2><<<nb, misc::RED_THREADS, 0, c.stream>>>(c.lat, (const S2*)U, partial);
-  else if (N == 4)
-    misc::k_plaq<4, S2><<<nb, misc::RED_THREADS, 0, c.stream>>>(c.lat, (const S2*)U, partial);
   else
-    misc::k_plaq<0, S2><<<nb, misc::RED_THREADS, 0, c.stream>>>(c.lat, (const S2*)U, partial);
+    misc::k_plaq<4, S2><<<nb, misc::RED_THREADS, 0, c.stream>>>(c.lat, (const S2*)U, partial);
   misc::k_finish<2><<<1, misc::RED_THREADS, 0, c.stream>>>(partial, (int)nb, out);
   return cudaGetLastError();
 }
@@ -308,6 +338,16 @@ template <typename T>
 cudaError_t linksums(const LaunchCtx& c, const void* Pa, const void* Pb, const void* U, double* partial, double* out) {
   using S2 = typename Storage<T>::type;
   const int N = c.lat.N;
+  if (m64_supported(N) && Pa && !Pb && !U) {
+    m64::Job j = m64_job(c.lat);
+    j.Pin = Pa;
+    j.kin_partial = partial;
+    const cudaError_t e = m64::kinetic(sizeof(T) == 8, j, m64::Grid{}, 3, c.stream);
+    if (e != cudaSuccess) return e;
+    misc::k_finish<3><<<1, misc::RED_THREADS, 0, c.stream>>>(
+        partial, m64::ctas_for(nlinks(c.lat), m64::kinetic_links_per_cta()), out);
+    return cudaGetLastError();
+  }
   if (N >= misc::BIG_NC) {
     misc::k_linksums_big<S2><<<(unsigned)nlinks(c.lat), misc::RED_THREADS, 0, c.stream>>>(
         c.lat, (const S2*)Pa, (const S2*)Pb, (const S2*)U, partial);
@@ -383,6 +423,11 @@ cudaError_t refresh(const LaunchCtx& c, void* P, uint64_t seed, const unsigned l
   if (c.lat.N >= misc::BIG_NC) {
     misc::k_refresh_big<S2><<<(unsigned)nlinks(c.lat), misc::RED_THREADS, 0, c.stream>>>(c.lat, (S2*)P, seed, traj_dev,
                                                                                          traj_host, scale);
+    return cudaGetLastError();
+  }
+  if (link_major(c.lat.N)) {
+    misc::k_refresh_warp<S2><<<blocks_for(nlinks(c.lat), misc::RED_THREADS / 32), misc::RED_THREADS, 0, c.stream>>>(
+        c.lat, (S2*)P, seed, traj_dev, traj_host, scale);
     return cudaGetLastError();
   }
   misc::k_refresh<S2><<<blocks_for(nlinks(c.lat), 128), 128, 0, c.stream>>>(c.lat, (S2*)P, seed, traj_dev, traj_host,

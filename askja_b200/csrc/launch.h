@@ -34,13 +34,13 @@ struct LaunchCtx {
   int reunit;       // reunitarise after each link update
   int rows_ns;      // row kernels, FP32: project by one Newton-Schulz step per update (the engine
                     // re-orthonormalises with the determinant phase every few trajectories)
-  int force_rows;   // kernel mapping: 0 thread-per-link (NC <= 4), 1 row-per-thread,
+  int force_rows;   // kernel mapping: 0 automatic (thread-per-link for NC <= 4, FP64 MMA above),
+                    // 1 row-per-thread, 4 FP64 MMA (NC >= 5),
                     // 2 tensor cores (FP32, NC = 16, 32 or 64, DIM >= 2), 3 site pairs in
                     // packed FP32 (NC = 3, even n[DIM-1]; the fused kick+drift then
                     // expects the site-pair layout, see pair_swap)
   int rows_groups;  // row kernels: sites per CTA (0: default 128/NC)
   int small_occ;    // thread-per-link kernels: register budget for 0 default, 1 / 2 more resident CTAs
-  void* scratch;    // tensor-core path: per-link contiguous copy of U (V*D*NC*NC float2)
   unsigned* status; // tensor-core path: nonzero after a bounded wait gave up
   // row-kernel reunitarisation: run only when *gate % gate_every == 0 (null: always)
   const unsigned long long* gate;
@@ -55,6 +55,9 @@ constexpr int FULL_REUNIT_EVERY = 10;
 // whether the tensor-core mapping exists for this shape and precision
 inline bool tc_supported(int N, int D, bool fp64) { return !fp64 && (N == 16 || N == 32 || N == 64) && D >= 2; }
 
+// whether the FP64-MMA mapping exists for this colour number
+inline bool m64_supported(int N) { return link_major(N); }
+
 // whether the site-pair mapping exists (n_fast: extent of the fastest direction)
 inline bool pair_supported(int N, int D, bool fp64, int n_fast) {
   return !fp64 && N == 3 && D >= 2 && n_fast % 2 == 0;
@@ -65,7 +68,8 @@ inline bool pair_supported(int N, int D, bool fp64, int n_fast) {
 //   linksums -> out[0] sum tr2(Pa), out[1] sum 1/4 tr2(Pa+Pb), out[2] UViol
 //   gauss    -> out[0]
 struct KernelSet {
-  // mode 0: Pout = Pin - ek F(U); mode 1: also Uout = exp(i ed Pout) U
+  // mode 0: Pout = Pin - ek F(U); mode 1: also Uout = exp(i ed Pout) U;
+  // mode 2 (FP64 MMA and tensor cores): Uout = exp(i ed Pin) U
   cudaError_t (*force)(const LaunchCtx&, int mode, const void* U, const void* Pin, void* Pout, void* Uout, double ek,
                        double ed);
   cudaError_t (*drift)(const LaunchCtx&, void* U, const void* P, double eps);

@@ -74,8 +74,8 @@ __device__ __forceinline__ void plaq_site(const Lat& L, const S2* __restrict__ U
             cpx<double> ab = czero<double>(), dc = czero<double>();
 #pragma unroll(NT > 0 ? NT : 1)
             for (int k = 0; k < N; k++) {
-              cmac(ab, ldc<double>(U + eoff(L, mu, i * N + k, s)), ldc<double>(U + eoff(L, nu, k * N + j, xpmu)));
-              cmac(dc, ldc<double>(U + eoff(L, nu, i * N + k, s)), ldc<double>(U + eoff(L, mu, k * N + j, xpnu)));
+              cmac(ab, ldc<double>(U + eoffn<NT>(L, mu, i * N + k, s)), ldc<double>(U + eoffn<NT>(L, nu, k * N + j, xpmu)));
+              cmac(dc, ldc<double>(U + eoffn<NT>(L, nu, i * N + k, s)), ldc<double>(U + eoffn<NT>(L, mu, k * N + j, xpnu)));
             }
             // explicit fma: the same rounding in every kernel that inlines this
             tr = fma(ab.re, dc.re, tr);
@@ -114,13 +114,13 @@ __device__ __forceinline__ void link_sums(const Lat& L, const S2* __restrict__ P
       for (int i = 0; i < N; i++)
 #pragma unroll(NT > 0 ? NT : 1)
         for (int j = 0; j < N; j++) {
-          const cpx<double> x = ldc<double>(Pa + eoff(L, d, i * N + j, s));
-          const cpx<double> y = ldc<double>(Pa + eoff(L, d, j * N + i, s));
+          const cpx<double> x = ldc<double>(Pa + eoffn<NT>(L, d, i * N + j, s));
+          const cpx<double> y = ldc<double>(Pa + eoffn<NT>(L, d, j * N + i, s));
           a = fma(x.re, y.re, a);
           a = fma(-x.im, y.im, a);
           if (Pb) {
-            const cpx<double> x2 = ldc<double>(Pb + eoff(L, d, i * N + j, s));
-            const cpx<double> y2 = ldc<double>(Pb + eoff(L, d, j * N + i, s));
+            const cpx<double> x2 = ldc<double>(Pb + eoffn<NT>(L, d, i * N + j, s));
+            const cpx<double> y2 = ldc<double>(Pb + eoffn<NT>(L, d, j * N + i, s));
             b = fma(x.re + x2.re, y.re + y2.re, b);
             b = fma(-(x.im + x2.im), y.im + y2.im, b);
           }
@@ -137,8 +137,8 @@ __device__ __forceinline__ void link_sums(const Lat& L, const S2* __restrict__ P
           cpx<double> aij = czero<double>(), aji = czero<double>();
 #pragma unroll(NT > 0 ? NT : 1)
           for (int k = 0; k < N; k++) {
-            cmac_nc(aij, ldc<double>(U + eoff(L, d, i * N + k, s)), ldc<double>(U + eoff(L, d, j * N + k, s)));
-            cmac_nc(aji, ldc<double>(U + eoff(L, d, j * N + k, s)), ldc<double>(U + eoff(L, d, i * N + k, s)));
+            cmac_nc(aij, ldc<double>(U + eoffn<NT>(L, d, i * N + k, s)), ldc<double>(U + eoffn<NT>(L, d, j * N + k, s)));
+            cmac_nc(aji, ldc<double>(U + eoffn<NT>(L, d, j * N + k, s)), ldc<double>(U + eoffn<NT>(L, d, i * N + k, s)));
           }
           if (i == j) {
             aij.re -= 1.0;
@@ -171,6 +171,7 @@ template <typename S2>
 __global__ void __launch_bounds__(RED_THREADS) k_gauss(Lat L, const S2* __restrict__ U, const S2* __restrict__ Pi,
                                                        int links_per_block, double* __restrict__ partial) {
   const int N = L.N, NN = N * N;
+  const int es = estride(L);
   const long l0 = (long)blockIdx.x * links_per_block;
   const long l1 = min((long)L.V * L.D, l0 + links_per_block);
   for (int e = threadIdx.x; e < NN; e += blockDim.x) {
@@ -179,14 +180,15 @@ __global__ void __launch_bounds__(RED_THREADS) k_gauss(Lat L, const S2* __restri
     for (long l = l0; l < l1; l++) {
       const int d = (int)(l / L.V);
       const int s = (int)(l - (long)d * L.V);
-      cpx<double> g = ldc<double>(Pi + eoff(L, d, e, s));
+      const size_t b0 = mbase(L, d, s);
+      cpx<double> g = ldc<double>(Pi + b0 + e * es);
       // (U^dag Pi U)_ij = sum_ab conj(U_ai) Pi_ab U_bj
       cpx<double> t = czero<double>();
       for (int a = 0; a < N; a++) {
         cpx<double> pu = czero<double>();
         for (int b = 0; b < N; b++)
-          cmac(pu, ldc<double>(Pi + eoff(L, d, a * N + b, s)), ldc<double>(U + eoff(L, d, b * N + j, s)));
-        cmac_cn(t, ldc<double>(U + eoff(L, d, a * N + i, s)), pu);
+          cmac(pu, ldc<double>(Pi + b0 + (a * N + b) * es), ldc<double>(U + b0 + (b * N + j) * es));
+        cmac_cn(t, ldc<double>(U + b0 + (a * N + i) * es), pu);
       }
       sr += g.re - t.re;
       si += g.im - t.im;
@@ -342,8 +344,74 @@ __device__ __forceinline__ void refresh_link(const Lat& L, S2* __restrict__ P, u
   const int N = L.N;
   const int d = (int)(t / L.V);
   const int s = (int)(t - (long)d * L.V);
+  S2* p = P + mbase(L, d, s);
+  const int es = estride(L);
   refresh_entries(L, seed, traj, scale, d, s,
-                  [&](int i, int j, const cpx<double>& v) { stc(P + eoff(L, d, i * N + j, s), v); });
+                  [&](int i, int j, const cpx<double>& v) { stc(p + (i * N + j) * es, v); });
+}
+
+// refresh_link by cooperating threads (link-major fields; a warp or a CTA per link): thread per
+// matrix element of the upper triangle, the same draws and the same arithmetic
+// per entry, so the momenta are identical; both entries of a pair are written
+// within the link's contiguous matrix, where a thread per link strode by it.
+template <typename S2>
+__device__ __forceinline__ void refresh_link_coop(const Lat& L, S2* __restrict__ P, uint64_t seed, uint32_t traj,
+                                                  double scale, int d, int s, int lane, int lanes) {
+  const int N = L.N;
+  const unsigned long long lk = (unsigned long long)s * L.D + d;
+  const uint32_t k0 = (uint32_t)seed, k1 = (uint32_t)(seed >> 32);
+  S2* p = P + mbase(L, d, s);
+  auto block = [&](int blk, double (&g)[4]) {
+    u32x4 c;
+    c.x = (uint32_t)blk;
+    c.y = (uint32_t)lk;
+    c.z = (uint32_t)(lk >> 32);
+    c.w = traj;
+    normals4(philox4x32_10(c, k0, k1), g);
+  };
+  for (int e = lane; e < N * N; e += lanes) {
+    const int i = e / N, j = e - (e / N) * N;
+    if (j <= i) continue;
+    const int pr = i * (2 * N - i - 1) / 2 + (j - i - 1);
+    double g[4];
+    block((2 * pr) >> 2, g);
+    const double xs = pr & 1 ? g[2] : g[0], xa = pr & 1 ? g[3] : g[1];
+    stc(p + i * N + j, mkc<double>(0.5 * scale * xs, -0.5 * scale * xa));
+    stc(p + j * N + i, mkc<double>(0.5 * scale * xs, 0.5 * scale * xa));
+  }
+  if (lane == 0) {
+    const int a0 = N * (N - 1);
+    int cur = -1;
+    double g[4];
+    double suffix = 0.0;
+    for (int dd = N - 1; dd >= 0; dd--) {
+      double val = suffix;
+      if (dd >= 1) {
+        const int m = dd - 1;
+        const double nm = sqrt(0.5 / ((double)(m + 1) * (m + 2)));
+        const int a = a0 + m;
+        if ((a >> 2) != cur) {
+          block(a >> 2, g);
+          cur = a >> 2;
+        }
+        const double xm = g[a & 3];
+        val -= dd * nm * xm;
+        suffix += nm * xm;
+      }
+      stc(p + dd * N + dd, mkc<double>(scale * val, 0.0));
+    }
+  }
+}
+
+template <typename S2>
+__global__ void __launch_bounds__(RED_THREADS) k_refresh_warp(Lat L, S2* __restrict__ P, uint64_t seed,
+                                                              const unsigned long long* __restrict__ traj_dev,
+                                                              unsigned long long traj_host, double scale) {
+  const uint32_t traj = (uint32_t)(traj_dev ? *traj_dev : traj_host);
+  const long t = (long)blockIdx.x * (RED_THREADS / 32) + (threadIdx.x >> 5);
+  if (t >= (long)L.V * L.D) return;
+  const int d = (int)(t / L.V);
+  refresh_link_coop<S2>(L, P, seed, traj, scale, d, (int)(t - (long)d * L.V), threadIdx.x & 31, 32);
 }
 
 template <typename S2>
@@ -359,10 +427,9 @@ template <typename S2>
 __global__ void k_identity(Lat L, S2* __restrict__ U) {
   const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (long)field_elems(L)) return;
-  const int N = L.N;
-  const int e = (int)((t >> 5) % (N * N));
-  const int i = e / N, j = e - i * N;
-  stc(U + t, mkc<double>(i == j ? 1.0 : 0.0, 0.0));
+  int d, s, e;
+  field_index(L, t, &d, &s, &e);
+  stc(U + t, mkc<double>(e % (L.N + 1) == 0 ? 1.0 : 0.0, 0.0));
 }
 
 // Complex Gaussian matrices (unit variance per component pair) for the Haar
@@ -463,18 +530,13 @@ template <typename S2>
 __global__ void k_from_conf(Lat L, const double2* __restrict__ conf, S2* __restrict__ f) {
   const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (long)field_elems(L)) return;
-  // t indexes the device field: t = ((d*B + b)*NN + e)*32 + lane, site = 32b + lane
-  const int NN = L.N * L.N;
-  const long rest = t >> 5;
-  const int e = (int)(rest % NN);
-  const long db = rest / NN;
-  const int d = (int)(db / L.B);
-  const int s = (int)((db - (long)d * L.B) * 32 + (t & 31));
-  if (s >= L.V) {
+  // t indexes the device field
+  int d, s, e;
+  if (!field_index(L, t, &d, &s, &e)) {
     stc(f + t, mkc<double>(0.0, 0.0));
     return;
   }
-  const double2 v = conf[((size_t)s * L.D + d) * NN + e];
+  const double2 v = conf[((size_t)s * L.D + d) * (L.N * L.N) + e];
   stc(f + t, mkc<double>(v.x, v.y));
 }
 
@@ -622,59 +684,14 @@ __global__ void __launch_bounds__(RED_THREADS) k_linksums_big(Lat L, const S2* _
     for (int k = 0; k < 3; k++) partial[(size_t)t * 3 + k] = counted(L, s) ? v[k] : 0.0;
 }
 
-// refresh_link with one CTA per link: thread per off-diagonal pair (the pair's
-// two normals come from one Philox block), the diagonal by thread 0 in the
-// same order as refresh_link, so the momenta are identical.
+// refresh_link_coop with one CTA per link.
 template <typename S2>
 __global__ void k_refresh_big(Lat L, S2* __restrict__ P, uint64_t seed, const unsigned long long* __restrict__ traj_dev,
                               unsigned long long traj_host, double scale) {
   const uint32_t traj = (uint32_t)(traj_dev ? *traj_dev : traj_host);
-  const int N = L.N;
   const long t = blockIdx.x;
   const int d = (int)(t / L.V);
-  const int s = (int)(t - (long)d * L.V);
-  const unsigned long long lk = (unsigned long long)s * L.D + d;
-  const uint32_t k0 = (uint32_t)seed, k1 = (uint32_t)(seed >> 32);
-  auto block = [&](int blk, double (&g)[4]) {
-    u32x4 c;
-    c.x = (uint32_t)blk;
-    c.y = (uint32_t)lk;
-    c.z = (uint32_t)(lk >> 32);
-    c.w = traj;
-    normals4(philox4x32_10(c, k0, k1), g);
-  };
-  for (int e = threadIdx.x; e < N * N; e += blockDim.x) {
-    const int i = e / N, j = e - (e / N) * N;
-    if (j <= i) continue;
-    const int p = i * (2 * N - i - 1) / 2 + (j - i - 1);
-    double g[4];
-    block((2 * p) >> 2, g);
-    const double xs = g[(2 * p) & 3], xa = g[(2 * p + 1) & 3];
-    stc(P + eoff(L, d, i * N + j, s), mkc<double>(0.5 * scale * xs, -0.5 * scale * xa));
-    stc(P + eoff(L, d, j * N + i, s), mkc<double>(0.5 * scale * xs, 0.5 * scale * xa));
-  }
-  if (threadIdx.x == 0) {
-    const int a0 = N * (N - 1);
-    int cur = -1;
-    double g[4];
-    double suffix = 0.0;
-    for (int dd = N - 1; dd >= 0; dd--) {
-      double val = suffix;
-      if (dd >= 1) {
-        const int m = dd - 1;
-        const double nm = sqrt(0.5 / ((double)(m + 1) * (m + 2)));
-        const int a = a0 + m;
-        if ((a >> 2) != cur) {
-          block(a >> 2, g);
-          cur = a >> 2;
-        }
-        const double xm = g[a & 3];
-        val -= dd * nm * xm;
-        suffix += nm * xm;
-      }
-      stc(P + eoff(L, d, dd * N + dd, s), mkc<double>(scale * val, 0.0));
-    }
-  }
+  refresh_link_coop<S2>(L, P, seed, traj, scale, d, (int)(t - (long)d * L.V), threadIdx.x, blockDim.x);
 }
 
 }  // namespace misc

@@ -1,0 +1,624 @@
+// Link update, plaquette and kinetic sums for 5 <= NC <= 64 on the FP64 tensor
+// instruction (mma.sync m8n8k4 f64; tcgen05 has no FP64 kind), for FP64 and
+// FP32 storage.
+//
+// A matrix is cut into 8 x 8 tiles (NT = ceil(NC / 8) of them a side); one warp
+// owns the eight rows 8w .. 8w+7 of every left operand and result, NT warps
+// own a link.  A complex product is four real MMAs per 8 x 8 x 4 block.
+//
+// Register layout of a tile (the accumulator layout of the instruction): lane
+// holds row lane / 4, columns 2 (lane % 4) + {0, 1}.  The sum over k may run in
+// any order as long as both operands use the same one, so the k-steps take the
+// columns {0, 2, 4, 6} and {1, 3, 5, 7} of a tile: an accumulator tile is then
+// the left operand of the next product as it stands, with no exchange between
+// lanes.  A right operand Y^dag is a row-pattern load of Y (lane: row lane / 4,
+// columns 2 (lane % 4) + e), a right operand Y a column-pattern load (rows
+// 2 (lane % 4) + e, column lane / 4); both read whole sectors of the row-major
+// matrix of one link (link-major fields, common.cuh), straight from L1 / L2.
+// The adjoint of the staple sum is accumulated,
+//   G = sum_nu [U_nu(x) U_mu(x+nu)] U_nu(x+mu)^dag
+//             + [U_nu(x-nu)^dag U_mu(x-nu)] U_nu(x+mu-nu),
+// because then every product of the force, W^dag = G U^dag included, has a left
+// operand that is either a load or the accumulator before it.  Only three
+// matrices per link cross the warps' rows, through one shared-memory tile of
+// row stride 8 NT + 1 (conflict-free for rows and columns): W^dag (the kick
+// needs its transpose), X = i eps P and X^3 (right operands of the series).
+//
+// What bounds it: the FP64 pipe.  One 8 x 8 x 4 MMA takes 4 cycles of an SM
+// (36.8 TFLOP/s measured with independent accumulators); a link update of
+// LEVEL 8 in four dimensions is 18 products of NT^3 * 8 MMAs.  Operand loads
+// are 8 shared-bandwidth cycles per 32 cycles of MMA.
+#pragma once
+
+#include "launch.h"
+#include "misc.cuh"
+
+namespace askja {
+namespace m64 {
+
+// One lattice's fields, as the kernels read them: by value for a single chain,
+// from a table (with a per-CTA list of table index and block) for a batch.
+struct Job {
+  const int* nbr;
+  int V, D, N;
+  int order;    // Taylor order of the drift
+  int project;  // FP32 storage: project the links read onto U(N) to first order (see drift)
+  int r0, r1;   // sites counted by the reductions (Lat)
+  void* U[2];   // links in U[cur], updated links to U[cur ^ 1]
+  const void* Pin;
+  void* Pout;
+  double kick;  // kick step (times the launch's kick scale)
+  double dt;    // drift step
+  double* plaq_partial;
+  double* kin_partial;
+};
+
+// links per CTA: 8 warps, or one link where it takes more
+template <int NT>
+struct Cta {
+  static constexpr int LINKS = NT == 1 ? 8 : NT == 2 ? 4 : NT <= 4 ? 2 : 1;
+  static constexpr int THREADS = 32 * NT * LINKS;
+  static constexpr int LD = 8 * NT + 1;
+  static constexpr int TILE = 8 * NT * LD;  // double2 of one link's tile
+  // small matrices keep the rows of X and X^2 in registers; larger ones read X
+  // back from the momenta and keep X^2 in a second tile
+  static constexpr bool KEEP = NT <= 2;
+  static constexpr int TILES = KEEP ? 1 : 2;
+  static constexpr size_t SMEM = (size_t)LINKS * TILES * TILE * sizeof(double2);
+  // resident CTAs the register budget is set for
+  static constexpr int MIN_CTAS = NT == 1 ? 3 : NT == 2 ? 2 : NT <= 4 ? 2 : 1;
+};
+
+struct Acc {
+  double re[2], im[2];  // columns 2j, 2j + 1
+};
+struct Op {
+  double re, im;
+};
+
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+      : "+d"(c[0]), "+d"(c[1])
+      : "d"(a), "d"(b));
+}
+
+template <int NT>
+__device__ __forceinline__ void zero(Acc (&c)[NT]) {
+#pragma unroll
+  for (int t = 0; t < NT; t++) c[t].re[0] = c[t].re[1] = c[t].im[0] = c[t].im[1] = 0.0;
+}
+
+// two consecutive complex numbers of a row (c even)
+__device__ __forceinline__ void ld_pair(const double2* p, Op& a, Op& b) {
+  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(a.re), "=d"(a.im), "=d"(b.re), "=d"(b.im) : "l"(p));
+}
+__device__ __forceinline__ void ld_pair(const float2* p, Op& a, Op& b) {
+  const float4 v = __ldg(reinterpret_cast<const float4*>(p));
+  a.re = v.x;
+  a.im = v.y;
+  b.re = v.z;
+  b.im = v.w;
+}
+template <typename S2>
+__device__ __forceinline__ Op ld_one(const S2* p) {
+  const S2 v = __ldg(p);
+  Op o;
+  o.re = v.x;
+  o.im = v.y;
+  return o;
+}
+__device__ __forceinline__ Op op0() {
+  Op o;
+  o.re = o.im = 0.0;
+  return o;
+}
+
+// Who this thread is within its link, and the two load patterns.  FULL: NC = 8 NT.
+template <int NT, bool FULL>
+struct Who {
+  int w, q, j, n;  // row block, lane / 4, lane % 4, NC (when not FULL)
+  __device__ __forceinline__ int N() const { return FULL ? 8 * NT : n; }
+  // row 8 rb + q, columns 8 cb + 2 j + {0, 1}
+  template <typename S2>
+  __device__ __forceinline__ void rows(const S2* m, int rb, int cb, Op (&o)[2]) const {
+    const int r = 8 * rb + q, c = 8 * cb + 2 * j;
+    if constexpr (FULL) {
+      ld_pair(m + r * N() + c, o[0], o[1]);
+    } else {
+      o[0] = r < n && c < n ? ld_one(m + r * n + c) : op0();
+      o[1] = r < n && c + 1 < n ? ld_one(m + r * n + c + 1) : op0();
+    }
+  }
+  // rows 8 rb + 2 j + {0, 1}, column 8 cb + q
+  template <typename S2>
+  __device__ __forceinline__ void cols(const S2* m, int rb, int cb, Op (&o)[2]) const {
+    const int r = 8 * rb + 2 * j, c = 8 * cb + q;
+    if constexpr (FULL) {
+      o[0] = ld_one(m + r * N() + c);
+      o[1] = ld_one(m + (r + 1) * N() + c);
+    } else {
+      o[0] = r < n && c < n ? ld_one(m + r * n + c) : op0();
+      o[1] = r + 1 < n && c < n ? ld_one(m + (r + 1) * n + c) : op0();
+    }
+  }
+};
+
+// c += A B (CONJ false) or A conj(B) (CONJ true: the right operand is given as
+// the elements of Y for the product with Y^dag).  fa(kb, a): the left operand's
+// own-row elements of tile column kb, fb(kb, t, b): the right operand's.
+template <int NT, bool CONJ, int KU, typename FA, typename FB>
+__device__ __forceinline__ void prod(Acc (&c)[NT], FA&& fa, FB&& fb) {
+#pragma unroll KU
+  for (int kb = 0; kb < NT; kb++) {
+    Op a[2];
+    fa(kb, a);
+    const double n0 = CONJ ? -a[0].re : -a[0].im, n1 = CONJ ? -a[1].re : -a[1].im;
+#pragma unroll
+    for (int t = 0; t < NT; t++) {
+      Op b[2];
+      fb(kb, t, b);
+      dmma(c[t].re, a[0].re, b[0].re);
+      dmma(c[t].im, CONJ ? a[0].im : a[0].re, CONJ ? b[0].re : b[0].im);
+      dmma(c[t].re, CONJ ? a[0].im : n0, b[0].im);
+      dmma(c[t].im, CONJ ? n0 : a[0].im, CONJ ? b[0].im : b[0].re);
+      dmma(c[t].re, a[1].re, b[1].re);
+      dmma(c[t].im, CONJ ? a[1].im : a[1].re, CONJ ? b[1].re : b[1].im);
+      dmma(c[t].re, CONJ ? a[1].im : n1, b[1].im);
+      dmma(c[t].im, CONJ ? n1 : a[1].im, CONJ ? b[1].im : b[1].re);
+    }
+  }
+}
+
+// the rows of an accumulator as left operand
+template <int NT>
+__device__ __forceinline__ void from_acc(const Acc (&c)[NT], int kb, Op (&a)[2]) {
+  a[0].re = c[kb].re[0];
+  a[0].im = c[kb].im[0];
+  a[1].re = c[kb].re[1];
+  a[1].im = c[kb].im[1];
+}
+
+// Barrier over the NT warps of link slot `slot` (a warp's own tile: NT = 1).
+template <int NT>
+__device__ __forceinline__ void link_sync(int slot) {
+  if constexpr (NT == 1)
+    __syncwarp();
+  else
+    asm volatile("bar.sync %0, %1;" ::"r"(slot + 1), "r"(32 * NT) : "memory");
+}
+
+__device__ __forceinline__ double round_to(const double2*, double v) { return v; }
+__device__ __forceinline__ double round_to(const float2*, double v) { return (double)(float)v; }
+__device__ __forceinline__ double2 pack(const double2*, double re, double im) { return make_double2(re, im); }
+__device__ __forceinline__ float2 pack(const float2*, double re, double im) {
+  return make_float2((float)re, (float)im);
+}
+
+// own rows of an accumulator to a field matrix
+template <int NT, bool FULL, typename S2>
+__device__ __forceinline__ void store_rows(S2* m, const Who<NT, FULL>& me, const Acc (&c)[NT]) {
+  const int r = 8 * me.w + me.q;
+#pragma unroll
+  for (int t = 0; t < NT; t++) {
+    const int col = 8 * t + 2 * me.j;
+#pragma unroll
+    for (int e = 0; e < 2; e++)
+      if (FULL || (r < me.n && col + e < me.n)) m[r * me.N() + col + e] = pack(m, c[t].re[e], c[t].im[e]);
+  }
+}
+
+// own rows of an accumulator to the link's shared tile
+template <int NT, bool FULL>
+__device__ __forceinline__ void tile_rows(double2* S, const Who<NT, FULL>& me, const Acc (&c)[NT]) {
+  double2* p = S + (8 * me.w + me.q) * Cta<NT>::LD + 2 * me.j;
+#pragma unroll
+  for (int t = 0; t < NT; t++)
+#pragma unroll
+    for (int e = 0; e < 2; e++) p[8 * t + e] = make_double2(c[t].re[e], c[t].im[e]);
+}
+
+// column-pattern read of the shared tile (right operand)
+template <int NT, bool FULL>
+__device__ __forceinline__ void tile_cols(const double2* S, const Who<NT, FULL>& me, int rb, int cb, Op (&o)[2]) {
+  const double2* p = S + (8 * rb + 2 * me.j) * Cta<NT>::LD + 8 * cb + me.q;
+#pragma unroll
+  for (int e = 0; e < 2; e++) {
+    const double2 v = p[e * Cta<NT>::LD];
+    o[e].re = v.x;
+    o[e].im = v.y;
+  }
+}
+
+__device__ __forceinline__ double inv_factorial(int k, int order) {
+  constexpr double f[9] = {1.0,       1.0,       1.0 / 2,   1.0 / 6,   1.0 / 24,
+                           1.0 / 120, 1.0 / 720, 1.0 / 5040, 1.0 / 40320};
+  double v = 0.0;
+#pragma unroll
+  for (int i = 0; i < 9; i++)
+    if (i == k && i <= order) v = f[i];
+  return v;
+}
+
+// mode 0: Pout = Pin - kick F(U);  1: the same, and Uout = exp(i dt Pout) U;
+// 2: Uout = exp(i dt Pin) U.
+//
+// The exponential is the Taylor sum by Paterson-Stockmeyer in blocks of three
+// terms (X^2, X^3, then Horner in X^3: 5 products for order 8, 4 for order 6,
+// U included, instead of 8 and 6 by Horner), formed without its identity term:
+// U' = U + (E - 1) U.  P is not assumed Hermitian.
+// FP32 storage with `project`: U' = U + (E - 1 - (U U^dag - 1) / 2) U, the
+// Newton-Schulz step on the links as read; it differs from projecting first by
+// |E - 1| times the defect that the FP32 store left, which the next update
+// removes in turn.
+template <int NT, bool FULL, typename S2>
+__global__ void __launch_bounds__(Cta<NT>::THREADS, Cta<NT>::MIN_CTAS)
+    k_link(const __grid_constant__ Job one, const Job* __restrict__ table, const int2* __restrict__ items, int cur,
+           double kick_scale, int mode) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  using CT = Cta<NT>;
+  constexpr int KU = NT <= 4 ? NT : 1;  // left operands from memory: the k loop stays rolled for large NC
+  const Job* __restrict__ jp = &one;
+  int blk = blockIdx.x;
+  if (table) {
+    const int2 it = __ldg(items + blk);
+    jp = table + it.x;
+    blk = it.y;
+  }
+  const Job& job = *jp;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int slot = wid / NT;
+  const int V = job.V, D = job.D;
+  Who<NT, FULL> me;
+  me.w = wid - slot * NT;
+  me.q = lane >> 2;
+  me.j = lane & 3;
+  me.n = job.N;
+  const int idx = blk * CT::LINKS + slot;
+  if (idx >= V * D) return;  // whole links: no barrier is left waiting
+  const int x = idx / D, mu = idx - x * D;
+  const size_t NN = FULL ? (size_t)64 * NT * NT : (size_t)me.n * me.n;
+  const S2* __restrict__ U = static_cast<const S2*>(job.U[cur]);
+  const int* __restrict__ nbr = job.nbr;
+  auto link = [&](int d, int s) { return U + ((size_t)d * V + s) * NN; };
+  const size_t own = ((size_t)mu * V + x) * NN;
+  const S2* Ux = U + own;
+  double2* S = reinterpret_cast<double2*>(smem_raw) + slot * (CT::TILES * CT::TILE);
+  const int r = 8 * me.w + me.q;
+  Acc X[NT];  // rows of X = i dt P
+
+  if (mode != 2) {
+    Acc G[NT];
+    zero(G);
+    const int xpmu = __ldg(nbr + (size_t)(2 * mu) * V + x);
+#pragma unroll 1
+    for (int nu = 0; nu < D; nu++) {
+      if (nu == mu) continue;
+      const int xpnu = __ldg(nbr + (size_t)(2 * nu) * V + x);
+      const int xmnu = __ldg(nbr + (size_t)(2 * nu + 1) * V + x);
+      const int xpmu_mnu = __ldg(nbr + (size_t)(2 * nu + 1) * V + xpmu);
+      Acc T[NT];
+      {
+        const S2 *a = link(nu, x), *b = link(mu, xpnu), *y = link(nu, xpmu);
+        zero(T);
+        prod<NT, false, KU>(
+            T, [&](int kb, Op(&o)[2]) { me.rows(a, me.w, kb, o); },
+            [&](int kb, int t, Op(&o)[2]) { me.cols(b, kb, t, o); });
+        prod<NT, true, NT>(
+            G, [&](int kb, Op(&o)[2]) { from_acc(T, kb, o); },
+            [&](int kb, int t, Op(&o)[2]) { me.rows(y, t, kb, o); });
+      }
+      {
+        const S2 *a = link(nu, xmnu), *b = link(mu, xmnu), *y = link(nu, xpmu_mnu);
+        zero(T);
+        prod<NT, false, KU>(
+            T,
+            [&](int kb, Op(&o)[2]) {
+              me.cols(a, kb, me.w, o);
+              o[0].im = -o[0].im;
+              o[1].im = -o[1].im;
+            },
+            [&](int kb, int t, Op(&o)[2]) { me.cols(b, kb, t, o); });
+        prod<NT, false, NT>(
+            G, [&](int kb, Op(&o)[2]) { from_acc(T, kb, o); },
+            [&](int kb, int t, Op(&o)[2]) { me.cols(y, kb, t, o); });
+      }
+    }
+    Acc Wd[NT];  // W^dag
+    zero(Wd);
+    prod<NT, true, NT>(
+        Wd, [&](int kb, Op(&o)[2]) { from_acc(G, kb, o); },
+        [&](int kb, int t, Op(&o)[2]) { me.rows(Ux, t, kb, o); });
+    tile_rows(S, me, Wd);
+    link_sync<NT>(slot);
+    // kick with the traceless anti-hermitian part of W: z = (W^dag)_cr = conj(W_rc)
+    const int N = me.N();
+    double trim = 0.0;
+    for (int k = 0; k < N; k++) trim -= S[k * (CT::LD + 1)].y;
+    trim /= N;
+    const double ek = kick_scale * job.kick, ed = job.dt;
+    const S2* P = static_cast<const S2*>(job.Pin) + own;
+    S2* Po = static_cast<S2*>(job.Pout) + own;
+#pragma unroll
+    for (int t = 0; t < NT; t++) {
+      Op z[2];
+      tile_cols(S, me, t, me.w, z);
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const int c = 8 * t + 2 * me.j + e;
+        const bool in = FULL || (r < N && c < N);
+        const double fr = r == c ? -z[e].im - trim : -0.5 * (z[e].im + Wd[t].im[e]);
+        const double fi = r == c ? 0.0 : -0.5 * (z[e].re - Wd[t].re[e]);
+        double pr = 0.0, pi = 0.0;
+        if (in) {
+          const S2 p = P[r * N + c];
+          pr = round_to(P, fma(-ek, fr, (double)p.x));
+          pi = round_to(P, fma(-ek, fi, (double)p.y));
+          Po[r * N + c] = pack(P, pr, pi);
+        }
+        X[t].re[e] = -ed * pi;
+        X[t].im[e] = ed * pr;
+      }
+    }
+    if (mode == 0) return;
+    link_sync<NT>(slot);
+  } else {
+    const S2* P = static_cast<const S2*>(job.Pin) + own;
+    const double ed = job.dt;
+#pragma unroll
+    for (int t = 0; t < NT; t++) {
+      Op p[2];
+      me.rows(P, me.w, t, p);
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        X[t].re[e] = -ed * p[e].im;
+        X[t].im[e] = ed * p[e].re;
+      }
+    }
+  }
+  const int order = job.order;
+  // rows of X again where keeping them costs registers: from the momenta just
+  // written (or read), which this thread owns
+  auto x_rows = [&](int t, Op(&o)[2]) {
+    if constexpr (CT::KEEP) {
+      from_acc(X, t, o);
+    } else {
+      const S2* P = (mode == 2 ? static_cast<const S2*>(job.Pin) : static_cast<const S2*>(job.Pout)) + own;
+      const double ed = job.dt;
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const int c = 8 * t + 2 * me.j + e;
+        S2 p = {};
+        if (FULL || (r < me.n && c < me.n)) p = P[r * me.N() + c];
+        o[e].re = -ed * p.y;
+        o[e].im = ed * p.x;
+      }
+    }
+  };
+  tile_rows(S, me, X);
+  link_sync<NT>(slot);
+  Acc E[NT], X2[NT];
+  double2* S2t = S + CT::TILE;  // X^2, own rows only (not KEEP)
+  auto tile_row = [&](const double2* tile, int kb, Op(&o)[2]) {
+    const double2* p = tile + r * CT::LD + 8 * kb + 2 * me.j;
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+      const double2 v = p[e];
+      o[e].re = v.x;
+      o[e].im = v.y;
+    }
+  };
+  zero(X2);
+  prod<NT, false, KU>(
+      X2,
+      [&](int kb, Op(&o)[2]) {
+        if constexpr (CT::KEEP)
+          from_acc(X, kb, o);
+        else
+          tile_row(S, kb, o);
+      },
+      [&](int kb, int t, Op(&o)[2]) { tile_cols(S, me, kb, t, o); });
+  if constexpr (!CT::KEEP) tile_rows(S2t, me, X2);
+  auto x2_rows = [&](int kb, Op(&o)[2]) {
+    if constexpr (CT::KEEP)
+      from_acc(X2, kb, o);
+    else
+      tile_row(S2t, kb, o);
+  };
+  auto block = [&](Acc(&c)[NT], int k) {  // sum_{i<3} X^i / (k + i)!, the identity of k = 0 left out
+    const double a0 = k ? inv_factorial(k, order) : 0.0, a1 = inv_factorial(k + 1, order),
+                 a2 = inv_factorial(k + 2, order);
+#pragma unroll
+    for (int t = 0; t < NT; t++) {
+      Op o[2], o2[2];
+      x_rows(t, o);
+      x2_rows(t, o2);
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        c[t].re[e] = fma(a2, o2[e].re, fma(a1, o[e].re, r == 8 * t + 2 * me.j + e ? a0 : 0.0));
+        c[t].im[e] = fma(a2, o2[e].im, a1 * o[e].im);
+      }
+    }
+  };
+  int k = order - order % 3;
+  if (k == 0) {
+    block(E, 0);
+  } else {
+    {
+      Acc X3[NT];
+      zero(X3);
+      prod<NT, false, KU>(
+          X3, [&](int kb, Op(&o)[2]) { x2_rows(kb, o); },
+          [&](int kb, int t, Op(&o)[2]) { tile_cols(S, me, kb, t, o); });
+      link_sync<NT>(slot);
+      tile_rows(S, me, X3);
+      if (k == order) {  // the top block is the single term X^k / k!: joined to the next one down
+        k -= 3;
+        block(E, k);
+        const double a = inv_factorial(order, order);
+#pragma unroll
+        for (int t = 0; t < NT; t++)
+#pragma unroll
+          for (int e = 0; e < 2; e++) {
+            E[t].re[e] = fma(a, X3[t].re[e], E[t].re[e]);
+            E[t].im[e] = fma(a, X3[t].im[e], E[t].im[e]);
+          }
+      } else {
+        block(E, k);
+      }
+    }
+    link_sync<NT>(slot);
+#pragma unroll 1
+    while (k > 0) {
+      k -= 3;
+      Acc H[NT];
+      block(H, k);
+      prod<NT, false, NT>(
+          H, [&](int kb, Op(&o)[2]) { from_acc(E, kb, o); },
+          [&](int kb, int t, Op(&o)[2]) { tile_cols(S, me, kb, t, o); });
+#pragma unroll
+      for (int t = 0; t < NT; t++) E[t] = H[t];
+    }
+  }
+  if (sizeof(S2) == 8 && job.project) {
+    Acc M[NT];
+    zero(M);
+    prod<NT, true, KU>(
+        M, [&](int kb, Op(&o)[2]) { me.rows(Ux, me.w, kb, o); },
+        [&](int kb, int t, Op(&o)[2]) { me.rows(Ux, t, kb, o); });
+#pragma unroll
+    for (int t = 0; t < NT; t++)
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const bool diag = r == 8 * t + 2 * me.j + e && (FULL || r < me.n);
+        E[t].re[e] -= 0.5 * (M[t].re[e] - (diag ? 1.0 : 0.0));
+        E[t].im[e] -= 0.5 * M[t].im[e];
+      }
+  }
+  Acc Y[NT];
+#pragma unroll
+  for (int t = 0; t < NT; t++) {
+    Op o[2];
+    me.rows(Ux, me.w, t, o);
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+      Y[t].re[e] = o[e].re;
+      Y[t].im[e] = o[e].im;
+    }
+  }
+  prod<NT, false, NT>(
+      Y, [&](int kb, Op(&o)[2]) { from_acc(E, kb, o); },
+      [&](int kb, int t, Op(&o)[2]) { me.cols(Ux, kb, t, o); });
+  store_rows(static_cast<S2*>(job.U[cur ^ 1]) + own, me, Y);
+}
+
+// Plaquette sums, NT warps per site: Re sum_ij (AB)_ij conj((DC)_ij) of every
+// plane, A = U_mu(x), B = U_nu(x+mu), D = U_nu(x), C = U_mu(x+nu); the block's
+// temporal and spatial sums go to plaq_partial[2 blk], [2 blk + 1].
+// Two products a plane at the FP64 MMA rate, where a thread per site (NC < 16)
+// or four threads per row (above) did them on the FMA pipe from uncoalesced
+// loads.
+template <int NT, bool FULL, typename S2>
+__global__ void __launch_bounds__(Cta<NT>::THREADS)
+    k_plaq(const __grid_constant__ Job one, const Job* __restrict__ table, const int2* __restrict__ items, int cur) {
+  constexpr int KU = NT <= 4 ? NT : 1;
+  const Job* __restrict__ jp = &one;
+  int blk = blockIdx.x;
+  if (table) {
+    const int2 it = __ldg(items + blk);
+    jp = table + it.x;
+    blk = it.y;
+  }
+  const Job& job = *jp;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int slot = wid / NT;
+  const int V = job.V, D = job.D;
+  Who<NT, FULL> me;
+  me.w = wid - slot * NT;
+  me.q = lane >> 2;
+  me.j = lane & 3;
+  me.n = job.N;
+  const int x = blk * Cta<NT>::LINKS + slot;
+  const size_t NN = FULL ? (size_t)64 * NT * NT : (size_t)me.n * me.n;
+  const S2* __restrict__ U = static_cast<const S2*>(job.U[cur]);
+  const int* __restrict__ nbr = job.nbr;
+  auto link = [&](int d, int s) { return U + ((size_t)d * V + s) * NN; };
+  double v[2] = {0.0, 0.0};
+  if (x < V && x >= job.r0 && (job.r1 == 0 || x < job.r1)) {
+#pragma unroll 1
+    for (int mu = 0; mu < D; mu++) {
+      const int xpmu = __ldg(nbr + (size_t)(2 * mu) * V + x);
+#pragma unroll 1
+      for (int nu = mu + 1; nu < D; nu++) {
+        const int xpnu = __ldg(nbr + (size_t)(2 * nu) * V + x);
+        const S2 *a = link(mu, x), *b = link(nu, xpmu), *d = link(nu, x), *c = link(mu, xpnu);
+        Acc AB[NT], DC[NT];
+        zero(AB);
+        zero(DC);
+        prod<NT, false, KU>(
+            AB, [&](int kb, Op(&o)[2]) { me.rows(a, me.w, kb, o); },
+            [&](int kb, int t, Op(&o)[2]) { me.cols(b, kb, t, o); });
+        prod<NT, false, KU>(
+            DC, [&](int kb, Op(&o)[2]) { me.rows(d, me.w, kb, o); },
+            [&](int kb, int t, Op(&o)[2]) { me.cols(c, kb, t, o); });
+        double tr = 0.0;
+#pragma unroll
+        for (int t = 0; t < NT; t++)
+#pragma unroll
+          for (int e = 0; e < 2; e++) {
+            tr = fma(AB[t].re[e], DC[t].re[e], tr);
+            tr = fma(AB[t].im[e], DC[t].im[e], tr);
+          }
+        v[mu == 0 ? 0 : 1] += (me.w == 0 && lane == 0 ? 1.0 : 0.0) - tr / me.N();
+      }
+    }
+  }
+  misc::block_sum<2>(v);
+  if (threadIdx.x == 0) {
+    job.plaq_partial[2 * (size_t)blk + 0] = v[0];
+    job.plaq_partial[2 * (size_t)blk + 1] = v[1];
+  }
+}
+
+// Kinetic sums sum ReTr(P P) of KIN_LINKS links per CTA, a warp per link at a
+// time, both elements of a pair read from the same contiguous matrix;
+// kin_partial[stride * blk].
+constexpr int KIN_LINKS = 64;
+template <typename S2>
+__global__ void __launch_bounds__(misc::RED_THREADS)
+    k_kinetic(const __grid_constant__ Job one, const Job* __restrict__ table, const int2* __restrict__ items,
+              int stride) {
+  const Job* __restrict__ jp = &one;
+  int blk = blockIdx.x;
+  if (table) {
+    const int2 it = __ldg(items + blk);
+    jp = table + it.x;
+    blk = it.y;
+  }
+  const Job& job = *jp;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int N = job.N, NN = N * N;
+  const long nl = (long)job.V * job.D;
+  const long l0 = (long)blk * KIN_LINKS, l1 = min(nl, l0 + KIN_LINKS);
+  double v[1] = {0.0};
+  for (long l = l0 + wid; l < l1; l += misc::RED_THREADS / 32) {
+    const int s = (int)(l % job.V);
+    if (!(s >= job.r0 && (job.r1 == 0 || s < job.r1))) continue;
+    const S2* P = static_cast<const S2*>(job.Pin) + (size_t)l * NN;
+    double a = 0.0;
+    for (int e = lane; e < NN; e += 32) {
+      const int i = e / N, j = e - i * N;
+      const Op p = ld_one(P + e), q = ld_one(P + j * N + i);
+      a = fma(p.re, q.re, a);
+      a = fma(-p.im, q.im, a);
+    }
+    v[0] += a;
+  }
+  misc::block_sum<1>(v);
+  if (threadIdx.x == 0) {
+    job.kin_partial[(size_t)stride * blk] = v[0];
+    for (int k = 1; k < stride; k++) job.kin_partial[(size_t)stride * blk + k] = 0.0;
+  }
+}
+
+}  // namespace m64
+}  // namespace askja

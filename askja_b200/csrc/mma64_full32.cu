@@ -1,0 +1,8 @@
+// FP64-MMA kernels, FP32 storage, NC a multiple of 8 (a translation unit of its own: build time).
+#include "mma64_launch.cuh"
+
+namespace askja {
+namespace m64 {
+ASKJA_M64_ENTRIES(full32, true, float2)
+}  // namespace m64
+}  // namespace askja

@@ -42,12 +42,13 @@ template <int NMAX, typename T, typename S2>
 __device__ __forceinline__ void stage_row(cpx<T>* tile, int NP, const S2* __restrict__ f, const Lat& L, int d,
                                           int s, int r) {
   const int N = L.N;
-  const S2* p = f + mbase(L, d, s) + (size_t)r * N * 32;
+  const int es = estride(L);
+  const S2* p = f + mbase(L, d, s) + (size_t)r * N * es;
 #pragma unroll
   for (int c = 0; c < NMAX; c += 2) {
     if (c >= N) continue;
-    const cpx<T> v0 = ldc<T>(p + c * 32);
-    const cpx<T> v1 = c + 1 < N ? ldc<T>(p + (c + 1) * 32) : czero<T>();
+    const cpx<T> v0 = ldc<T>(p + c * es);
+    const cpx<T> v1 = c + 1 < N ? ldc<T>(p + (c + 1) * es) : czero<T>();
     if constexpr (sizeof(T) == 4) {
       *reinterpret_cast<float4*>(tile + r * NP + c) = make_float4(v0.re, v0.im, v1.re, v1.im);
     } else {

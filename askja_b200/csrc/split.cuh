@@ -211,7 +211,7 @@ __device__ __forceinline__ void force_coefs(float (&f)[Dims<N>::NCOEF], const sm
 template <int N>
 __device__ __forceinline__ void load_lo(small::Mat<N, float>& M, const uint32_t* __restrict__ UL, const Lat& L, int d,
                                         int s) {
-  const uint32_t* p = UL + mbase(L, d, s);
+  const uint32_t* p = UL + bbase(L, d, s);
 #pragma unroll
   for (int i = 0; i < N; i++)
 #pragma unroll
@@ -224,7 +224,7 @@ __device__ __forceinline__ void load_lo(small::Mat<N, float>& M, const uint32_t*
 template <int N>
 __device__ __forceinline__ void store_lo(uint32_t* __restrict__ UL, const small::Mat<N, float>& M, const Lat& L,
                                          int d, int s) {
-  uint32_t* p = UL + mbase(L, d, s);
+  uint32_t* p = UL + bbase(L, d, s);
 #pragma unroll
   for (int i = 0; i < N; i++)
 #pragma unroll
@@ -235,7 +235,7 @@ __device__ __forceinline__ void store_lo(uint32_t* __restrict__ UL, const small:
 template <int N>
 __device__ __forceinline__ void load_exact(small::Mat<N, double>& M, const float2* __restrict__ U,
                                            const uint32_t* __restrict__ UL, const Lat& L, int d, int s) {
-  const size_t b = mbase(L, d, s);
+  const size_t b = bbase(L, d, s);
 #pragma unroll
   for (int i = 0; i < N; i++)
 #pragma unroll
@@ -250,7 +250,7 @@ __device__ __forceinline__ void load_exact(small::Mat<N, double>& M, const float
 template <int N>
 __device__ __forceinline__ void load_exact_row(cpx<double> (&r)[N], const float2* __restrict__ U,
                                                const uint32_t* __restrict__ UL, const Lat& L, int d, int s, int i) {
-  const size_t b = mbase(L, d, s) + (size_t)i * N * 32;
+  const size_t b = bbase(L, d, s) + (size_t)i * N * 32;
 #pragma unroll
   for (int j = 0; j < N; j++) {
     const float2 h = U[b + j * 32];
@@ -262,7 +262,7 @@ __device__ __forceinline__ void load_exact_row(cpx<double> (&r)[N], const float2
 template <int N>
 __device__ __forceinline__ void store_exact(float2* __restrict__ U, uint32_t* __restrict__ UL,
                                             const small::Mat<N, double>& M, const Lat& L, int d, int s) {
-  const size_t b = mbase(L, d, s);
+  const size_t b = bbase(L, d, s);
 #pragma unroll
   for (int i = 0; i < N; i++)
 #pragma unroll

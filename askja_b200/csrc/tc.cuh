@@ -36,9 +36,9 @@
 // the CTA barrier (bounded: after about a second the kernel records an error
 // in *status and stops), then all threads read the
 // accumulator with tcgen05.ld (warp w reads TMEM lanes 32(w%4).., columns
-// (w/4)*NC/2 ..), and write the next operand.  Neighbour links are read from
-// a per-link contiguous copy of U (k_to_aos), P and the outputs use the
-// blocked field layout of common.cuh.
+// (w/4)*NC/2 ..), and write the next operand.  U, P and the outputs are the
+// link-major fields of common.cuh (reading U in place instead of a per-launch
+// contiguous copy saved the copy's 56 us of 2.26 ms at SU(32) 8^4).
 //
 // The link update is carried as U' = U + (E - 1) U with E = exp(i eps P) to
 // order LEVEL, so the tensor cores only form products of small matrices and
@@ -506,11 +506,11 @@ struct Term {
 };
 
 template <int NC>
-__device__ __forceinline__ Term staple_term(const Lat& L, const float2* __restrict__ aos, int mu, int x, int i) {
+__device__ __forceinline__ Term staple_term(const Lat& L, const float2* __restrict__ U, int mu, int x, int i) {
   const size_t NN = (size_t)NC * NC;
   const int j = i >> 1;
   const int nu = j < mu ? j : j + 1;
-  auto link = [&](int d, int site) { return aos + ((size_t)d * L.V + site) * NN; };
+  auto link = [&](int d, int site) { return U + ((size_t)d * L.V + site) * NN; };
   const int xpmu = nb_plus(L, mu, x);
   Term t;
   if ((i & 1) == 0) {  // upper: U_nu(x+mu) U_mu^dag(x+nu) U_nu^dag(x)
@@ -535,7 +535,7 @@ __device__ __forceinline__ Term staple_term(const Lat& L, const float2* __restri
 // MODE 0: Pout = Pin - eps_k F(U)
 // MODE 1: also Uout = exp(i eps_d Pout) U (reunitarised when reunit)
 // MODE 2: Uout = exp(i eps_d Pin) U only
-// U is read from `aos` (per-link contiguous copy); Uout may be U itself.
+// Uout is another buffer than U.
 // Register budget: NC = 64 one CTA per SM (its shared memory allows no
 // second); NC = 16 and 32 at most 64 registers, four CTAs per SM, whose
 // products and epilogues overlap (SU(32) 8^4 2.31 -> 2.23 ms, SU(16) 6^4
@@ -543,7 +543,7 @@ __device__ __forceinline__ Term staple_term(const Lat& L, const float2* __restri
 // spill).
 template <int NC, int MODE>
 __global__ void __launch_bounds__(THREADS, NC == 64 ? 1 : 4)
-    k_link(Lat L, const float2* __restrict__ aos, const float2* Pin, float2* Pout, float2* Uout, float eps_k,
+    k_link(Lat L, const float2* __restrict__ U, const float2* Pin, float2* Pout, float2* Uout, float eps_k,
            float eps_d, int order, int reunit, unsigned* status) {
   using SH = Shape<NC>;
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -571,13 +571,13 @@ __global__ void __launch_bounds__(THREADS, NC == 64 ? 1 : 4)
   for (long l = blockIdx.x; l < nl && ok; l += gridDim.x) {
     const int mu = (int)(l / L.V);
     const int x = (int)(l - (long)mu * L.V);
-    const float2* ulink = aos + ((size_t)mu * L.V + x) * NN;
-    const size_t fb = mbase(L, mu, x);
+    const float2* ulink = U + ((size_t)mu * L.V + x) * NN;
+    const size_t fb = (size_t)l * NN;
     Frag<NC> fa, fb1;
     if (MODE != 2) {
       // ---- staple sum S (TMEM columns NC..2NC-1)
       const int nterms = 2 * (L.D - 1);
-      Term t = staple_term<NC>(L, aos, mu, x, 0);
+      Term t = staple_term<NC>(L, U, mu, x, 0);
       fetch<NC>(fa, t.a, kind_rowwise(t.ka));
       fetch<NC>(fb1, t.b1, kind_rowwise(t.kb1));
       for (int i = 0; i < nterms && ok; i++) {
@@ -592,7 +592,7 @@ __global__ void __launch_bounds__(THREADS, NC == 64 ? 1 : 4)
         put<NC>(s, fb1, t.kb2);
         go<NC>(s, tS, i > 0 ? 1u : 0u);
         if (i + 1 < nterms) {
-          t = staple_term<NC>(L, aos, mu, x, i + 1);
+          t = staple_term<NC>(L, U, mu, x, i + 1);
           fetch<NC>(fa, t.a, kind_rowwise(t.ka));
           fetch<NC>(fb1, t.b1, kind_rowwise(t.kb1));
         } else {
@@ -608,7 +608,7 @@ __global__ void __launch_bounds__(THREADS, NC == 64 ? 1 : 4)
       go<NC>(s, tT, 0);
       float2 pn[SH::EPT];
 #pragma unroll
-      for (int q = 0; q < SH::EPT; q++) pn[q] = Pin[fb + 32 * (size_t)(tid + THREADS * q)];
+      for (int q = 0; q < SH::EPT; q++) pn[q] = Pin[fb + tid + THREADS * q];
       ok = done(s, phase);
       if (!ok) break;
       acc_row<NC>(tT + ro.lane + ro.c0, v);
@@ -632,7 +632,7 @@ __global__ void __launch_bounds__(THREADS, NC == 64 ? 1 : 4)
         }
         pn[q].x = fmaf(-eps_k, fr, pn[q].x);
         pn[q].y = fmaf(-eps_k, fi, pn[q].y);
-        Pout[fb + 32 * (size_t)e] = pn[q];
+        Pout[fb + e] = pn[q];
       }
       if (MODE == 0) continue;
       __syncthreads();
@@ -647,7 +647,7 @@ __global__ void __launch_bounds__(THREADS, NC == 64 ? 1 : 4)
 #pragma unroll
       for (int q = 0; q < SH::EPT; q++) {
         const int e = tid + THREADS * q;
-        const float2 p = Pin[fb + 32 * (size_t)e];
+        const float2 p = Pin[fb + e];
         s.plain[(e / NC) * SH::PS + e % NC] = p.x;
         s.plain[(NC + e / NC) * SH::PS + e % NC] = p.y;
       }
@@ -794,7 +794,7 @@ __global__ void __launch_bounds__(THREADS, NC == 64 ? 1 : 4)
         const float2 u = __ldg(ur + j);
         const float wr = fmaf(g, u.x, s.plain[row * SH::PS + j]);
         const float wi = fmaf(g, u.y, s.plain[(NC + row) * SH::PS + j]);
-        Uout[fb + 32 * (size_t)(row * NC + j)] = make_float2(u.x + wr, u.y + wi);
+        Uout[fb + row * NC + j] = make_float2(u.x + wr, u.y + wi);
       }
     }
     __syncthreads();
@@ -842,29 +842,6 @@ __global__ void __launch_bounds__(THREADS) k_wait_probe(unsigned* status, long l
   if (tid < 32) {
     fence_after();
     tmem_dealloc(tbase, SH::TMEM_COLS);
-  }
-}
-
-// blocked field layout -> per-link contiguous row-major copy (32 sites x 32
-// elements per tile, both sides coalesced)
-static __global__ void k_to_aos(Lat L, const float2* __restrict__ f, float2* __restrict__ aos) {
-  __shared__ float2 tile[32][33];
-  const int b = blockIdx.x, d = blockIdx.y;
-  const int nn = L.N * L.N;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int chunks = (nn + 31) / 32;
-  for (int ch = blockIdx.z; ch < chunks; ch += gridDim.z) {
-    const int e0 = ch * 32;
-    for (int r = w; r < 32; r += 8) {
-      const int e = e0 + r;
-      if (e < nn) tile[r][lane] = f[(((size_t)d * L.B + b) * nn + e) * 32 + lane];
-    }
-    __syncthreads();
-    for (int r = w; r < 32; r += 8) {
-      const int site = b * 32 + r, e = e0 + lane;
-      if (site < L.V && e < nn) aos[((size_t)d * L.V + site) * nn + e] = tile[lane][r];
-    }
-    __syncthreads();
   }
 }
 
