@@ -379,7 +379,7 @@ int askja_batch_create(const askja_chain_params* chains, int nchains, int precis
     // the same partition as a single chain's reductions, so that the sums agree bit for bit
     d.plaq_blocks = askja::m64::ctas_for(V, m64 ? askja::m64::links_per_cta(p.nc) : askja::misc::RED_THREADS);
     d.link_blocks =
-        askja::m64::ctas_for(V * p.dim, m64 ? askja::m64::kinetic_links_per_cta() : askja::misc::RED_THREADS);
+        askja::m64::ctas_for(V * p.dim, m64 ? askja::m64::kinetic_links_per_cta(p.nc) : askja::misc::RED_THREADS);
     if (int rc = dalloc(b, &d.partial, (2 * (size_t)d.plaq_blocks + d.link_blocks) * sizeof(double))) return fail(rc);
     d.n16 = (long)(fbytes / 16);
     if (precision == ASKJA_FP32 && askja::splitk::supported(p.nc)) {
@@ -413,7 +413,8 @@ int askja_batch_create(const askja_chain_params* chains, int nchains, int precis
         kin_item.push_back(t);
       }
     }
-    refresh_start.push_back(refresh_start.back() + (int)((V * p.dim + 127) / 128));
+    refresh_start.push_back(refresh_start.back() +
+                            (int)(((m64 ? askja::misc::refresh_threads(L) : V * p.dim) + 127) / 128));
     copy_start.push_back(copy_start.back() + (int)((d.n16 + 4095) / 4096) + (int)((d.n16lo + 4095) / 4096));
     max_conf = std::max(max_conf, (size_t)V * p.dim * p.nc * p.nc * 16);
     // cold start

@@ -241,7 +241,7 @@ static __global__ void kb_metropolis(const ChainDev* __restrict__ descs, int nch
   if (c < nchains) misc::metropolis(descs[c].st, descs[c].seed, nullptr, 0);
 }
 
-// Momentum refresh: item = 128-link block.
+// Momentum refresh: item = 128 links, or 128 threads of misc::refresh_block for link-major fields.
 template <typename S2>
 __global__ void __launch_bounds__(128) kb_refresh(const ChainDev* __restrict__ descs, const int* __restrict__ item_start,
                                                   int nchains) {
@@ -257,6 +257,8 @@ __global__ void __launch_bounds__(128) kb_refresh(const ChainDev* __restrict__ d
       case 3: split::refresh_link<3>(sd.lat, P, PL, sd.seed, traj, sd.scale, t); break;
       default: split::refresh_link<4>(sd.lat, P, PL, sd.seed, traj, sd.scale, t);
     }
+  } else if (link_major(sd.lat.N)) {
+    misc::refresh_block<S2>(sd.lat, (S2*)sd.P, sd.seed, traj, sd.scale, t);
   } else {
     misc::refresh_link<S2>(sd.lat, (S2*)sd.P, sd.seed, traj, sd.scale, t);
   }
@@ -264,7 +266,7 @@ __global__ void __launch_bounds__(128) kb_refresh(const ChainDev* __restrict__ d
 
 // Residual-plane chains: projection onto SU(N) in FP64 before each
 // trajectory, into the links and the saved copy (split::reunit_link); the
-// other chains' items return at once.  Item = 128-link block (the refresh list).
+// other chains' items return at once.  Item: the refresh list.
 static __global__ void __launch_bounds__(128) kb_reunit_split(const ChainDev* __restrict__ descs,
                                                               const int* __restrict__ item_start, int nchains,
                                                               int cur) {

@@ -345,7 +345,7 @@ cudaError_t linksums(const LaunchCtx& c, const void* Pa, const void* Pb, const v
     const cudaError_t e = m64::kinetic(sizeof(T) == 8, j, m64::Grid{}, 3, c.stream);
     if (e != cudaSuccess) return e;
     misc::k_finish<3><<<1, misc::RED_THREADS, 0, c.stream>>>(
-        partial, m64::ctas_for(nlinks(c.lat), m64::kinetic_links_per_cta()), out);
+        partial, m64::ctas_for(nlinks(c.lat), m64::kinetic_links_per_cta(N)), out);
     return cudaGetLastError();
   }
   if (N >= misc::BIG_NC) {
@@ -420,13 +420,8 @@ template <typename T>
 cudaError_t refresh(const LaunchCtx& c, void* P, uint64_t seed, const unsigned long long* traj_dev,
                     unsigned long long traj_host, double scale) {
   using S2 = typename Storage<T>::type;
-  if (c.lat.N >= misc::BIG_NC) {
-    misc::k_refresh_big<S2><<<(unsigned)nlinks(c.lat), misc::RED_THREADS, 0, c.stream>>>(c.lat, (S2*)P, seed, traj_dev,
-                                                                                         traj_host, scale);
-    return cudaGetLastError();
-  }
   if (link_major(c.lat.N)) {
-    misc::k_refresh_warp<S2><<<blocks_for(nlinks(c.lat), misc::RED_THREADS / 32), misc::RED_THREADS, 0, c.stream>>>(
+    misc::k_refresh_blocks<S2><<<blocks_for(misc::refresh_threads(c.lat), 128), 128, 0, c.stream>>>(
         c.lat, (S2*)P, seed, traj_dev, traj_host, scale);
     return cudaGetLastError();
   }

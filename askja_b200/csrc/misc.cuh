@@ -350,17 +350,29 @@ __device__ __forceinline__ void refresh_link(const Lat& L, S2* __restrict__ P, u
                   [&](int i, int j, const cpx<double>& v) { stc(p + (i * N + j) * es, v); });
 }
 
-// refresh_link by cooperating threads (link-major fields; a warp or a CTA per link): thread per
-// matrix element of the upper triangle, the same draws and the same arithmetic
-// per entry, so the momenta are identical; both entries of a pair are written
-// within the link's contiguous matrix, where a thread per link strode by it.
+// refresh_link for link-major fields, a thread per Philox block: block b of a
+// link holds the normals of the off-diagonal pairs 2b and 2b + 1, and one more
+// thread per link (in warps of their own, after all pairs) draws the diagonal.
+// The same draws and arithmetic per entry, so the momenta are identical.  What
+// bounds it is the FP64 log / sqrt / sincospi of each block; a CTA per link left
+// most threads on the empty lower triangle and all of them behind the serial
+// diagonal (SU(64) 4x8x16 138 us, SU(32) 8^4 414 us).
+__host__ __device__ inline int refresh_pair_blocks(int N) { return (N * (N - 1) / 2 + 1) / 2; }
+inline long refresh_threads(const Lat& L) { return (long)L.V * L.D * (refresh_pair_blocks(L.N) + 1); }
+
 template <typename S2>
-__device__ __forceinline__ void refresh_link_coop(const Lat& L, S2* __restrict__ P, uint64_t seed, uint32_t traj,
-                                                  double scale, int d, int s, int lane, int lanes) {
-  const int N = L.N;
+__device__ __forceinline__ void refresh_block(const Lat& L, S2* __restrict__ P, uint64_t seed, uint32_t traj,
+                                              double scale, long t) {
+  const int N = L.N, nb = refresh_pair_blocks(N);
+  const long nl = (long)L.V * L.D;
+  if (t >= nl * (nb + 1)) return;
+  const bool diag = t >= nl * nb;
+  const long l = diag ? t - nl * nb : t / nb;
+  const int d = (int)(l / L.V);
+  const int s = (int)(l - (long)d * L.V);
   const unsigned long long lk = (unsigned long long)s * L.D + d;
   const uint32_t k0 = (uint32_t)seed, k1 = (uint32_t)(seed >> 32);
-  S2* p = P + mbase(L, d, s);
+  S2* p = P + (size_t)l * (N * N);
   auto block = [&](int blk, double (&g)[4]) {
     u32x4 c;
     c.x = (uint32_t)blk;
@@ -369,49 +381,58 @@ __device__ __forceinline__ void refresh_link_coop(const Lat& L, S2* __restrict__
     c.w = traj;
     normals4(philox4x32_10(c, k0, k1), g);
   };
-  for (int e = lane; e < N * N; e += lanes) {
-    const int i = e / N, j = e - (e / N) * N;
-    if (j <= i) continue;
-    const int pr = i * (2 * N - i - 1) / 2 + (j - i - 1);
-    double g[4];
-    block((2 * pr) >> 2, g);
-    const double xs = pr & 1 ? g[2] : g[0], xa = pr & 1 ? g[3] : g[1];
-    stc(p + i * N + j, mkc<double>(0.5 * scale * xs, -0.5 * scale * xa));
-    stc(p + j * N + i, mkc<double>(0.5 * scale * xs, 0.5 * scale * xa));
-  }
-  if (lane == 0) {
-    const int a0 = N * (N - 1);
-    int cur = -1;
-    double g[4];
-    double suffix = 0.0;
-    for (int dd = N - 1; dd >= 0; dd--) {
-      double val = suffix;
-      if (dd >= 1) {
-        const int m = dd - 1;
-        const double nm = sqrt(0.5 / ((double)(m + 1) * (m + 2)));
-        const int a = a0 + m;
-        if ((a >> 2) != cur) {
-          block(a >> 2, g);
-          cur = a >> 2;
-        }
-        const double xm = g[a & 3];
-        val -= dd * nm * xm;
-        suffix += nm * xm;
+  double g[4];
+  if (!diag) {
+    const int b = (int)(t - l * nb);
+    block(b, g);
+    // row i of pair q (row-major upper triangle): the first row whose end lies beyond q
+    const int q = 2 * b;
+    const float m = N - 0.5f;
+    int i = (int)(m - sqrtf(fmaxf(m * m - 2.0f * q, 0.0f)));
+    while (i > 0 && i * (2 * N - i - 1) / 2 > q) i--;
+    while ((i + 1) * (2 * N - i - 2) / 2 <= q) i++;
+    int j = i + 1 + q - i * (2 * N - i - 1) / 2;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      if (i >= N - 1) break;  // an odd pair count: the block's second half is the diagonal's
+      const double xs = g[2 * h], xa = g[2 * h + 1];
+      stc(p + i * N + j, mkc<double>(0.5 * scale * xs, -0.5 * scale * xa));
+      stc(p + j * N + i, mkc<double>(0.5 * scale * xs, 0.5 * scale * xa));
+      if (++j == N) {
+        i++;
+        j = i + 1;
       }
-      stc(p + dd * N + dd, mkc<double>(scale * val, 0.0));
     }
+    return;
+  }
+  const int a0 = N * (N - 1);
+  int cur = -1;
+  double suffix = 0.0;
+  for (int dd = N - 1; dd >= 0; dd--) {
+    double val = suffix;
+    if (dd >= 1) {
+      const int m = dd - 1;
+      const double nm = sqrt(0.5 / ((double)(m + 1) * (m + 2)));
+      const int a = a0 + m;
+      if ((a >> 2) != cur) {
+        block(a >> 2, g);
+        cur = a >> 2;
+      }
+      const int r = a & 3;
+      const double xm = r == 0 ? g[0] : r == 1 ? g[1] : r == 2 ? g[2] : g[3];
+      val -= dd * nm * xm;
+      suffix += nm * xm;
+    }
+    stc(p + dd * N + dd, mkc<double>(scale * val, 0.0));
   }
 }
 
 template <typename S2>
-__global__ void __launch_bounds__(RED_THREADS) k_refresh_warp(Lat L, S2* __restrict__ P, uint64_t seed,
-                                                              const unsigned long long* __restrict__ traj_dev,
-                                                              unsigned long long traj_host, double scale) {
+__global__ void __launch_bounds__(128) k_refresh_blocks(Lat L, S2* __restrict__ P, uint64_t seed,
+                                                        const unsigned long long* __restrict__ traj_dev,
+                                                        unsigned long long traj_host, double scale) {
   const uint32_t traj = (uint32_t)(traj_dev ? *traj_dev : traj_host);
-  const long t = (long)blockIdx.x * (RED_THREADS / 32) + (threadIdx.x >> 5);
-  if (t >= (long)L.V * L.D) return;
-  const int d = (int)(t / L.V);
-  refresh_link_coop<S2>(L, P, seed, traj, scale, d, (int)(t - (long)d * L.V), threadIdx.x & 31, 32);
+  refresh_block<S2>(L, P, seed, traj, scale, (long)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 template <typename S2>
@@ -682,16 +703,6 @@ __global__ void __launch_bounds__(RED_THREADS) k_linksums_big(Lat L, const S2* _
   if (threadIdx.x == 0)
 #pragma unroll
     for (int k = 0; k < 3; k++) partial[(size_t)t * 3 + k] = counted(L, s) ? v[k] : 0.0;
-}
-
-// refresh_link_coop with one CTA per link.
-template <typename S2>
-__global__ void k_refresh_big(Lat L, S2* __restrict__ P, uint64_t seed, const unsigned long long* __restrict__ traj_dev,
-                              unsigned long long traj_host, double scale) {
-  const uint32_t traj = (uint32_t)(traj_dev ? *traj_dev : traj_host);
-  const long t = blockIdx.x;
-  const int d = (int)(t / L.V);
-  refresh_link_coop<S2>(L, P, seed, traj, scale, d, (int)(t - (long)d * L.V), threadIdx.x, blockDim.x);
 }
 
 }  // namespace misc

@@ -14,7 +14,7 @@ int links_per_cta(int N) {
   }
 }
 
-int kinetic_links_per_cta() { return KIN_LINKS; }
+int kinetic_links_per_cta(int N) { return kin_links(N); }
 
 cudaError_t link(int N, bool fp64, const Job& one, const Grid& g, int cur, double ks, int mode, cudaStream_t st) {
   const int NT = (N + 7) / 8;
@@ -29,7 +29,7 @@ cudaError_t plaq(int N, bool fp64, const Job& one, const Grid& g, int cur, cudaS
 }
 
 cudaError_t kinetic(bool fp64, const Job& one, const Grid& g, int stride, cudaStream_t st) {
-  const int ctas = g.table ? g.ctas : ctas_for((long)one.V * one.D, KIN_LINKS);
+  const int ctas = g.table ? g.ctas : ctas_for((long)one.V * one.D, kin_links(one.N));
   if (fp64)
     k_kinetic<double2><<<ctas, misc::RED_THREADS, 0, st>>>(one, g.table, g.items, stride);
   else

@@ -15,14 +15,18 @@
 // columns 2 (lane % 4) + e), a right operand Y a column-pattern load (rows
 // 2 (lane % 4) + e, column lane / 4); both read whole sectors of the row-major
 // matrix of one link (link-major fields, common.cuh), straight from L1 / L2.
-// The adjoint of the staple sum is accumulated,
-//   G = sum_nu [U_nu(x) U_mu(x+nu)] U_nu(x+mu)^dag
-//             + [U_nu(x-nu)^dag U_mu(x-nu)] U_nu(x+mu-nu),
-// because then every product of the force, W^dag = G U^dag included, has a left
-// operand that is either a load or the accumulator before it.  Only three
-// matrices per link cross the warps' rows, through one shared-memory tile of
-// row stride 8 NT + 1 (conflict-free for rows and columns): W^dag (the kick
-// needs its transpose), X = i eps P and X^3 (right operands of the series).
+// The staple sum
+//   S = sum_nu [U_nu(x+mu) U_mu(x+nu)^dag] U_nu(x)^dag
+//             + [U_nu(x+mu-nu)^dag U_mu(x-nu)^dag] U_nu(x-nu)
+// has a load or the accumulator before it as every left operand, and two of its
+// six links per plane as column-pattern loads.  A column load touches four
+// lines per quarter-warp, 32 L1 wavefronts a matrix against 8 for a row load:
+// accumulating S^dag instead spares S its way through shared memory but makes
+// four of the six links column loads (SU(8) 10^4: 573 wavefronts a link, L1
+// 80 % busy, 117 us an update).  Four matrices per link cross the warps' rows,
+// through one shared-memory tile of row stride 8 NT + 1 (conflict-free for rows
+// and columns): S, W = U S (the kick needs its transpose), X = i eps P and X^3
+// (right operands of the series).
 //
 // What bounds it: the FP64 pipe.  One 8 x 8 x 4 MMA takes 4 cycles of an SM
 // (36.8 TFLOP/s measured with independent accumulators); a link update of
@@ -99,6 +103,33 @@ __device__ __forceinline__ void ld_pair(const float2* p, Op& a, Op& b) {
   b.re = v.z;
   b.im = v.w;
 }
+// the same from memory that this launch may write, and to memory
+__device__ __forceinline__ void ld_pair_rw(const double2* p, Op& a, Op& b) {
+  asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+               : "=d"(a.re), "=d"(a.im), "=d"(b.re), "=d"(b.im)
+               : "l"(p)
+               : "memory");
+}
+__device__ __forceinline__ void ld_pair_rw(const float2* p, Op& a, Op& b) {
+  const float4 v = *reinterpret_cast<const float4*>(p);
+  a.re = v.x;
+  a.im = v.y;
+  b.re = v.z;
+  b.im = v.w;
+}
+__device__ __forceinline__ void st_pair(double2* p, const Op& a, const Op& b) {
+  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(a.re), "d"(a.im), "d"(b.re), "d"(b.im)
+               : "memory");
+}
+__device__ __forceinline__ void st_pair(float2* p, const Op& a, const Op& b) {
+  *reinterpret_cast<float4*>(p) = make_float4((float)a.re, (float)a.im, (float)b.re, (float)b.im);
+}
+__device__ __forceinline__ double round_to(const double2*, double v) { return v; }
+__device__ __forceinline__ double round_to(const float2*, double v) { return (double)(float)v; }
+__device__ __forceinline__ double2 pack(const double2*, double re, double im) { return make_double2(re, im); }
+__device__ __forceinline__ float2 pack(const float2*, double re, double im) {
+  return make_float2((float)re, (float)im);
+}
 template <typename S2>
 __device__ __forceinline__ Op ld_one(const S2* p) {
   const S2 v = __ldg(p);
@@ -127,6 +158,36 @@ struct Who {
     } else {
       o[0] = r < n && c < n ? ld_one(m + r * n + c) : op0();
       o[1] = r < n && c + 1 < n ? ld_one(m + r * n + c + 1) : op0();
+    }
+  }
+  // own rows, columns 8 t + 2 j + {0, 1}, of a matrix this launch also writes
+  template <typename S2>
+  __device__ __forceinline__ void own(const S2* m, int t, Op (&o)[2]) const {
+    const int r = 8 * w + q, c = 8 * t + 2 * j;
+    if constexpr (FULL) {
+      ld_pair_rw(m + r * N() + c, o[0], o[1]);
+    } else {
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        o[e] = op0();
+        if (r < n && c + e < n) {
+          const S2 v = m[r * n + c + e];
+          o[e].re = v.x;
+          o[e].im = v.y;
+        }
+      }
+    }
+  }
+  // the same elements to a matrix
+  template <typename S2>
+  __device__ __forceinline__ void put(S2* m, int t, const Op (&o)[2]) const {
+    const int r = 8 * w + q, c = 8 * t + 2 * j;
+    if constexpr (FULL) {
+      st_pair(m + r * N() + c, o[0], o[1]);
+    } else {
+#pragma unroll
+      for (int e = 0; e < 2; e++)
+        if (r < n && c + e < n) m[r * n + c + e] = pack(m, o[e].re, o[e].im);
     }
   }
   // rows 8 rb + 2 j + {0, 1}, column 8 cb + q
@@ -187,23 +248,14 @@ __device__ __forceinline__ void link_sync(int slot) {
     asm volatile("bar.sync %0, %1;" ::"r"(slot + 1), "r"(32 * NT) : "memory");
 }
 
-__device__ __forceinline__ double round_to(const double2*, double v) { return v; }
-__device__ __forceinline__ double round_to(const float2*, double v) { return (double)(float)v; }
-__device__ __forceinline__ double2 pack(const double2*, double re, double im) { return make_double2(re, im); }
-__device__ __forceinline__ float2 pack(const float2*, double re, double im) {
-  return make_float2((float)re, (float)im);
-}
-
 // own rows of an accumulator to a field matrix
 template <int NT, bool FULL, typename S2>
 __device__ __forceinline__ void store_rows(S2* m, const Who<NT, FULL>& me, const Acc (&c)[NT]) {
-  const int r = 8 * me.w + me.q;
 #pragma unroll
   for (int t = 0; t < NT; t++) {
-    const int col = 8 * t + 2 * me.j;
-#pragma unroll
-    for (int e = 0; e < 2; e++)
-      if (FULL || (r < me.n && col + e < me.n)) m[r * me.N() + col + e] = pack(m, c[t].re[e], c[t].im[e]);
+    Op o[2];
+    from_acc(c, t, o);
+    me.put(m, t, o);
   }
 }
 
@@ -287,8 +339,8 @@ __global__ void __launch_bounds__(Cta<NT>::THREADS, Cta<NT>::MIN_CTAS)
   Acc X[NT];  // rows of X = i dt P
 
   if (mode != 2) {
-    Acc G[NT];
-    zero(G);
+    Acc W[NT];  // the staple sum S first
+    zero(W);
     const int xpmu = __ldg(nbr + (size_t)(2 * mu) * V + x);
 #pragma unroll 1
     for (int nu = 0; nu < D; nu++) {
@@ -298,42 +350,44 @@ __global__ void __launch_bounds__(Cta<NT>::THREADS, Cta<NT>::MIN_CTAS)
       const int xpmu_mnu = __ldg(nbr + (size_t)(2 * nu + 1) * V + xpmu);
       Acc T[NT];
       {
-        const S2 *a = link(nu, x), *b = link(mu, xpnu), *y = link(nu, xpmu);
+        const S2 *a = link(nu, xpmu), *b = link(mu, xpnu), *y = link(nu, x);
         zero(T);
-        prod<NT, false, KU>(
+        prod<NT, true, KU>(
             T, [&](int kb, Op(&o)[2]) { me.rows(a, me.w, kb, o); },
-            [&](int kb, int t, Op(&o)[2]) { me.cols(b, kb, t, o); });
+            [&](int kb, int t, Op(&o)[2]) { me.rows(b, t, kb, o); });
         prod<NT, true, NT>(
-            G, [&](int kb, Op(&o)[2]) { from_acc(T, kb, o); },
+            W, [&](int kb, Op(&o)[2]) { from_acc(T, kb, o); },
             [&](int kb, int t, Op(&o)[2]) { me.rows(y, t, kb, o); });
       }
       {
-        const S2 *a = link(nu, xmnu), *b = link(mu, xmnu), *y = link(nu, xpmu_mnu);
+        const S2 *a = link(nu, xpmu_mnu), *b = link(mu, xmnu), *y = link(nu, xmnu);
         zero(T);
-        prod<NT, false, KU>(
+        prod<NT, true, KU>(
             T,
             [&](int kb, Op(&o)[2]) {
               me.cols(a, kb, me.w, o);
               o[0].im = -o[0].im;
               o[1].im = -o[1].im;
             },
-            [&](int kb, int t, Op(&o)[2]) { me.cols(b, kb, t, o); });
+            [&](int kb, int t, Op(&o)[2]) { me.rows(b, t, kb, o); });
         prod<NT, false, NT>(
-            G, [&](int kb, Op(&o)[2]) { from_acc(T, kb, o); },
+            W, [&](int kb, Op(&o)[2]) { from_acc(T, kb, o); },
             [&](int kb, int t, Op(&o)[2]) { me.cols(y, kb, t, o); });
       }
     }
-    Acc Wd[NT];  // W^dag
-    zero(Wd);
-    prod<NT, true, NT>(
-        Wd, [&](int kb, Op(&o)[2]) { from_acc(G, kb, o); },
-        [&](int kb, int t, Op(&o)[2]) { me.rows(Ux, t, kb, o); });
-    tile_rows(S, me, Wd);
+    tile_rows(S, me, W);
     link_sync<NT>(slot);
-    // kick with the traceless anti-hermitian part of W: z = (W^dag)_cr = conj(W_rc)
+    zero(W);
+    prod<NT, false, KU>(
+        W, [&](int kb, Op(&o)[2]) { me.rows(Ux, me.w, kb, o); },
+        [&](int kb, int t, Op(&o)[2]) { tile_cols(S, me, kb, t, o); });
+    link_sync<NT>(slot);
+    tile_rows(S, me, W);
+    link_sync<NT>(slot);
+    // kick with the traceless anti-hermitian part of W: z = W_cr
     const int N = me.N();
     double trim = 0.0;
-    for (int k = 0; k < N; k++) trim -= S[k * (CT::LD + 1)].y;
+    for (int k = 0; k < N; k++) trim += S[k * (CT::LD + 1)].y;
     trim /= N;
     const double ek = kick_scale * job.kick, ed = job.dt;
     const S2* P = static_cast<const S2*>(job.Pin) + own;
@@ -342,22 +396,19 @@ __global__ void __launch_bounds__(Cta<NT>::THREADS, Cta<NT>::MIN_CTAS)
     for (int t = 0; t < NT; t++) {
       Op z[2];
       tile_cols(S, me, t, me.w, z);
+      Op p[2];
+      me.own(P, t, p);
 #pragma unroll
       for (int e = 0; e < 2; e++) {
         const int c = 8 * t + 2 * me.j + e;
-        const bool in = FULL || (r < N && c < N);
-        const double fr = r == c ? -z[e].im - trim : -0.5 * (z[e].im + Wd[t].im[e]);
-        const double fi = r == c ? 0.0 : -0.5 * (z[e].re - Wd[t].re[e]);
-        double pr = 0.0, pi = 0.0;
-        if (in) {
-          const S2 p = P[r * N + c];
-          pr = round_to(P, fma(-ek, fr, (double)p.x));
-          pi = round_to(P, fma(-ek, fi, (double)p.y));
-          Po[r * N + c] = pack(P, pr, pi);
-        }
-        X[t].re[e] = -ed * pi;
-        X[t].im[e] = ed * pr;
+        const double fr = r == c ? W[t].im[e] - trim : 0.5 * (W[t].im[e] + z[e].im);
+        const double fi = r == c ? 0.0 : -0.5 * (W[t].re[e] - z[e].re);
+        p[e].re = round_to(P, fma(-ek, fr, p[e].re));
+        p[e].im = round_to(P, fma(-ek, fi, p[e].im));
+        X[t].re[e] = -ed * p[e].im;
+        X[t].im[e] = ed * p[e].re;
       }
+      me.put(Po, t, p);
     }
     if (mode == 0) return;
     link_sync<NT>(slot);
@@ -384,13 +435,12 @@ __global__ void __launch_bounds__(Cta<NT>::THREADS, Cta<NT>::MIN_CTAS)
     } else {
       const S2* P = (mode == 2 ? static_cast<const S2*>(job.Pin) : static_cast<const S2*>(job.Pout)) + own;
       const double ed = job.dt;
+      Op p[2];
+      me.own(P, t, p);
 #pragma unroll
       for (int e = 0; e < 2; e++) {
-        const int c = 8 * t + 2 * me.j + e;
-        S2 p = {};
-        if (FULL || (r < me.n && c < me.n)) p = P[r * me.N() + c];
-        o[e].re = -ed * p.y;
-        o[e].im = ed * p.x;
+        o[e].re = -ed * p[e].im;
+        o[e].im = ed * p[e].re;
       }
     }
   };
@@ -579,10 +629,15 @@ __global__ void __launch_bounds__(Cta<NT>::THREADS)
   }
 }
 
-// Kinetic sums sum ReTr(P P) of KIN_LINKS links per CTA, a warp per link at a
-// time, both elements of a pair read from the same contiguous matrix;
-// kin_partial[stride * blk].
-constexpr int KIN_LINKS = 64;
+// Kinetic sums sum ReTr(P P): a warp takes 8 x 8 tiles of a link's matrix, each
+// with its mirror tile in the column pattern (whole sectors, where element pairs
+// read a row length apart took 365 us for SU(64) 4x8x16 on 24 CTAs);
+// KIN_TILES tiles per CTA, whole links; kin_partial[stride * blk].
+constexpr int KIN_TILES = 64;
+__host__ __device__ inline int kin_links(int N) {
+  const int nt = (N + 7) / 8;
+  return KIN_TILES / (nt * nt) > 0 ? KIN_TILES / (nt * nt) : 1;
+}
 template <typename S2>
 __global__ void __launch_bounds__(misc::RED_THREADS)
     k_kinetic(const __grid_constant__ Job one, const Job* __restrict__ table, const int2* __restrict__ items,
@@ -596,22 +651,30 @@ __global__ void __launch_bounds__(misc::RED_THREADS)
   }
   const Job& job = *jp;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int N = job.N, NN = N * N;
+  const int N = job.N, nt = (N + 7) / 8;
   const long nl = (long)job.V * job.D;
-  const long l0 = (long)blk * KIN_LINKS, l1 = min(nl, l0 + KIN_LINKS);
+  const long l0 = (long)blk * kin_links(N);
+  const int links = (int)min((long)kin_links(N), nl - l0);
+  Who<8, false> me;
+  me.w = 0;
+  me.q = lane >> 2;
+  me.j = lane & 3;
+  me.n = N;
   double v[1] = {0.0};
-  for (long l = l0 + wid; l < l1; l += misc::RED_THREADS / 32) {
+  for (int f = wid; f < links * nt * nt; f += misc::RED_THREADS / 32) {
+    const long l = l0 + f / (nt * nt);
+    const int t = f % (nt * nt), ti = t / nt, tj = t - ti * nt;
     const int s = (int)(l % job.V);
     if (!(s >= job.r0 && (job.r1 == 0 || s < job.r1))) continue;
-    const S2* P = static_cast<const S2*>(job.Pin) + (size_t)l * NN;
-    double a = 0.0;
-    for (int e = lane; e < NN; e += 32) {
-      const int i = e / N, j = e - i * N;
-      const Op p = ld_one(P + e), q = ld_one(P + j * N + i);
-      a = fma(p.re, q.re, a);
-      a = fma(-p.im, q.im, a);
+    const S2* P = static_cast<const S2*>(job.Pin) + (size_t)l * N * N;
+    Op p[2], q[2];
+    me.rows(P, ti, tj, p);
+    me.cols(P, tj, ti, q);
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+      v[0] = fma(p[e].re, q[e].re, v[0]);
+      v[0] = fma(-p[e].im, q[e].im, v[0]);
     }
-    v[0] += a;
   }
   misc::block_sum<1>(v);
   if (threadIdx.x == 0) {

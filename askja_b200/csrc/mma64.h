@@ -18,7 +18,7 @@ struct Grid {
 
 // links (k_link) or sites (k_plaq) and links (k_kinetic) per CTA
 int links_per_cta(int N);
-int kinetic_links_per_cta();
+int kinetic_links_per_cta(int N);
 inline int ctas_for(long n, int per) { return (int)((n + per - 1) / per); }
 
 // mode 0 kick, 1 kick + drift, 2 drift (mma64.cuh); fp64: storage
