@@ -377,7 +377,7 @@ int askja_batch_create(const askja_chain_params* chains, int nchains, int precis
     if (int rc = dalloc(b, &d.sums, 8 * sizeof(double))) return fail(rc);
     const bool m64 = askja::m64_supported(p.nc);
     // the same partition as a single chain's reductions, so that the sums agree bit for bit
-    d.plaq_blocks = askja::m64::ctas_for(V, m64 ? askja::m64::links_per_cta(p.nc) : askja::misc::RED_THREADS);
+    d.plaq_blocks = askja::m64::ctas_for(V, m64 ? askja::m64::sites_per_cta(p.nc) : askja::misc::RED_THREADS);
     d.link_blocks =
         askja::m64::ctas_for(V * p.dim, m64 ? askja::m64::kinetic_links_per_cta(p.nc) : askja::misc::RED_THREADS);
     if (int rc = dalloc(b, &d.partial, (2 * (size_t)d.plaq_blocks + d.link_blocks) * sizeof(double))) return fail(rc);

@@ -2,9 +2,8 @@
 // eigenphase distributions of measurements4d.cpp:185-309 (getevs), which the
 // reference computes with Eigen's ComplexEigenSolver on the host.
 //
-// One CTA per line: the line product W is formed in FP64 as in k_lines (row
-// per thread, running product in shared memory), then warp 0 computes the
-// eigenvalues of W: Householder reduction to upper Hessenberg form, then the
+// The line products W are formed in FP64 by lines.cuh (NC <= 4) and mma64.cuh;
+// one warp computes the eigenvalues of each W: Householder reduction to upper Hessenberg form, then the
 // implicitly shifted complex QR iteration (single Wilkinson shift, an
 // exceptional shift every 11th iteration without deflation) on the active
 // window only, deflating from the bottom.  Rotations and reflections are
@@ -173,41 +172,6 @@ static __device__ void hessenberg_qr(cpx<double>* H, int N, cpx<double>* v, cpx<
     }
   }
   __syncwarp();
-}
-
-// Line q starts at q * start_stride and runs along `dir` through all
-// n[dir] links (the lines of k_lines); ev[q*N + i] = eigenvalue i of W_q.
-template <typename S2>
-__global__ void k_line_eigs(Lat L, const S2* __restrict__ U, int dir, int start_stride, double2* __restrict__ ev,
-                            int* __restrict__ fail) {
-  extern __shared__ __align__(16) unsigned char esm[];
-  const int N = L.N;
-  cpx<double>* W = reinterpret_cast<cpx<double>*>(esm);
-  cpx<double>* tmp = W + N * N;  // product scratch, later Householder vector and eigenvalues
-  const int r = threadIdx.x;
-  int pos = blockIdx.x * start_stride;
-  if (r < N)
-    for (int c = 0; c < N; c++) W[r * N + c] = ldc<double>(U + eoff(L, dir, r * N + c, pos));
-  __syncthreads();
-  for (int st = 0; st < L.n[dir] - 1; st++) {
-    pos = nb_plus(L, dir, pos);
-    if (r < N)
-      for (int c = 0; c < N; c++) {
-        cpx<double> s = czero<double>();
-        for (int k = 0; k < N; k++) cmac(s, W[r * N + k], ldc<double>(U + eoff(L, dir, k * N + c, pos)));
-        tmp[r * N + c] = s;
-      }
-    __syncthreads();
-    if (r < N)
-      for (int c = 0; c < N; c++) W[r * N + c] = tmp[r * N + c];
-    __syncthreads();
-  }
-  if (r < 32) {
-    cpx<double>* vsc = tmp;
-    cpx<double>* e = tmp + N;
-    hessenberg_qr(W, N, vsc, e, fail);
-    for (int i = r; i < N; i += 32) ev[(size_t)blockIdx.x * N + i] = make_double2(e[i].re, e[i].im);
-  }
 }
 
 }  // namespace eig

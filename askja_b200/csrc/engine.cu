@@ -26,6 +26,7 @@
 
 #include "../../include/askja_gpu.h"
 #include "launch.h"
+#include "lines.cuh"
 #include "misc.cuh"
 #include "split.h"
 
@@ -52,6 +53,9 @@ static thread_local std::string g_last_error;
 static std::mutex g_tune_mutex;
 static std::map<std::tuple<int, int, int>, askja_tuning> g_tune_cache;
 
+// doubles of scalar results in front of the per-line results
+constexpr int SUMS = 8;
+
 struct askja_ctx {
   askja_params p{};
   Lat lat{};
@@ -67,10 +71,10 @@ struct askja_ctx {
   void* Uconf = nullptr;
   int* nbr = nullptr;
   double* partial = nullptr;
-  double* sums = nullptr;   // [0..1] plaq t/s, [2..4] link sums, [5] gauss, [6..] line results
-  double* lines = nullptr;  // per-line results
-  double2* eigs = nullptr;  // eigenvalues of the N0 + N1 lines of askja_eigenphases
-  int* eigfail = nullptr;
+  double* sums = nullptr;   // [0..1] plaq t/s, [2..4] link sums, [5] gauss
+  double* lines = nullptr;  // per-line results, behind the sums in the same allocation (SUMS doubles on)
+  double2* eigs = nullptr;  // eigenvalues of the N0 + N1 lines of askja_eigenphases, then
+  int* eigfail = nullptr;   // their convergence flag, in the same allocation
   TrajState* st = nullptr;
   double* logbuf = nullptr;
   int logcap = 0;
@@ -455,7 +459,7 @@ void askja_destroy(askja_ctx* c) {
   if (c->up_bad) cudaFree(c->up_bad);
   if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
   void* bufs[] = {c->U[0], c->U[1], c->P,      c->P2,      c->Uconf,     c->nbr,       c->partial, c->sums,
-                  c->lines, c->st,  c->logbuf, c->staging, c->nonfinite, c->tc_status, c->eigs,    c->eigfail,
+                  c->st,    c->logbuf, c->staging, c->nonfinite, c->tc_status, c->eigs,
                   c->UL[0], c->UL[1], c->ULconf, c->PC, c->PCL, c->P2C, c->P2CL};
   for (void* b : bufs)
     if (b) cudaFree(b);
@@ -532,13 +536,14 @@ int askja_create(const askja_params* p, askja_ctx** out) {
   CKC(cudaMemcpy(c->nbr, nbr.data(), nbr.size() * sizeof(int), cudaMemcpyHostToDevice));
   L.nbr = c->nbr;
   CKC(cudaMalloc(&c->partial, askja::partial_doubles(L) * sizeof(double)));
-  CKC(cudaMalloc(&c->sums, 64 * sizeof(double)));
   long maxlines = 1;
   for (int i = 0; i < p->dim; i++) maxlines = std::max(maxlines, (long)p->n[i]);
-  CKC(cudaMalloc(&c->lines, (maxlines + 8) * sizeof(double)));
+  CKC(cudaMalloc(&c->sums, (SUMS + p->dim * maxlines + 8) * sizeof(double)));
+  c->lines = c->sums + SUMS;
   if (p->dim >= 2) {
-    CKC(cudaMalloc(&c->eigs, (size_t)(p->n[0] + p->n[1]) * p->nc * sizeof(double2)));
-    CKC(cudaMalloc(&c->eigfail, sizeof(int)));
+    const size_t neig = (size_t)(p->n[0] + p->n[1]) * p->nc;
+    CKC(cudaMalloc(&c->eigs, (neig + 1) * sizeof(double2)));
+    c->eigfail = reinterpret_cast<int*>(c->eigs + neig);
   }
   CKC(cudaMalloc(&c->st, sizeof(TrajState)));
   CKC(cudaMemset(c->st, 0, sizeof(TrajState)));
@@ -832,14 +837,20 @@ int askja_GaussLaw(askja_ctx* c, double* out) {
   return scal(c, c->sums + 5, out, 1);
 }
 
+static double mean_of(const double* v, int n) {
+  double s = 0;
+  for (int i = 0; i < n; i++) s += v[i];
+  return s / n;
+}
+
 static int line_mean(askja_ctx* c, int dir, int nlines, int start_stride, double* out) {
   DevGuard g(c->p.device);
-  KL(c->ks->lines(c->lc, cur_u(c), dir, nlines, start_stride, c->lines), "lines");
+  askja::LineSet ls{};
+  ls.add(dir, nlines, start_stride);
+  KL(c->ks->lines(c->lc, cur_u(c), ls, c->lines), "lines");
   std::vector<double> h(nlines);
   if (int rc = scal(c, c->lines, h.data(), nlines)) return rc;
-  double s = 0;
-  for (double v : h) s += v;
-  *out = s / nlines;
+  *out = mean_of(h.data(), nlines);
   return ASKJA_OK;
 }
 
@@ -870,14 +881,15 @@ int askja_eigenphases(askja_ctx* c, double* w, double* p) {
   const int N = c->N, n0 = c->lat.n[0], n1 = c->lat.n[1];
   CK(cudaMemsetAsync(c->eigfail, 0, sizeof(int), c->stream));
   // Wilson lines along direction 1 through (x0, 0, ..), Polyakov lines along 0 through (0, x1, 0, ..)
-  KL(c->ks->line_eigs(c->lc, cur_u(c), 1, n0, c->lat.stride[0], c->eigs, c->eigfail), "line eigenvalues");
-  KL(c->ks->line_eigs(c->lc, cur_u(c), 0, n1, c->lat.stride[1], c->eigs + (size_t)n0 * N, c->eigfail),
-     "line eigenvalues");
-  std::vector<double2> ev((size_t)(n0 + n1) * N);
-  int fail = 0;
+  askja::LineSet ls{};
+  ls.add(1, n0, c->lat.stride[0]);
+  ls.add(0, n1, c->lat.stride[1]);
+  KL(c->ks->line_eigs(c->lc, cur_u(c), ls, c->eigs, c->eigfail), "line eigenvalues");
+  std::vector<double2> ev((size_t)(n0 + n1) * N + 1);  // the flag behind the eigenvalues
   CK(cudaMemcpyAsync(ev.data(), c->eigs, ev.size() * sizeof(double2), cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaMemcpyAsync(&fail, c->eigfail, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
+  int fail = 0;
+  memcpy(&fail, &ev.back(), sizeof fail);
   if (fail) return set_err(c, ASKJA_ERR_CUDA, "line eigenvalues did not converge");
   // per line: phases, re-centred by the winding when |winding| > 0.1, sorted, summed; then averaged
   const double pi = 3.14159265358979323846;
@@ -924,12 +936,24 @@ int askja_measure(askja_ctx* c, double* out) {
   if (int rc = check_ctx(c)) return rc;
   if (!out) return set_err(c, ASKJA_ERR_ARG, "null output");
   if (c->D < 2) return set_err(c, ASKJA_ERR_ARG, "askja_measure needs DIM >= 2");
-  if (int rc = askja_PlaqExp(c, out, out + 1)) return rc;
-  if (int rc = askja_PolyakovLoop(c, out + 2)) return rc;
-  for (int d = 1; d < c->D; d++)
-    if (int rc = askja_WilsonLoopDir(c, d, out + 2 + d)) return rc;
-  if (int rc = askja_GaussLaw(c, out + c->D + 2)) return rc;
-  return askja_UViol(c, out + c->D + 3);
+  // the observables of the single calls, enqueued together and read back once
+  DevGuard g(c->p.device);
+  askja::LineSet ls{};
+  ls.add(0, c->lat.n[1], c->lat.stride[1]);
+  for (int d = 1; d < c->D; d++) ls.add(d, c->lat.n[0], c->lat.stride[0]);
+  KL(plaq_launch(c), "plaq");
+  KL(linksums_launch(c, -1, -1, true), "linksums");
+  KL(momenta_views(c), "momentum matrices");
+  KL(c->ks->gauss(c->lc, cur_u(c), c->P2, c->partial, c->sums + 5), "gauss");
+  KL(c->ks->lines(c->lc, cur_u(c), ls, c->lines), "lines");
+  std::vector<double> h(SUMS + ls.lines());
+  if (int rc = scal(c, c->sums, h.data(), (int)h.size())) return rc;
+  out[0] = h[0];
+  out[1] = h[1];
+  for (int i = 0; i < ls.sets; i++) out[2 + i] = mean_of(h.data() + SUMS + ls.first[i], ls.first[i + 1] - ls.first[i]);
+  out[c->D + 2] = h[5];
+  out[c->D + 3] = h[4];
+  return ASKJA_OK;
 }
 
 int askja_FourierTrafo(askja_ctx* c, double* coefficients) {

@@ -12,7 +12,7 @@
 #include "small.cuh"
 #include "pair.cuh"
 #include "tab.cuh"
-#include "eig.cuh"
+#include "lines.cuh"
 #include "tc.cuh"
 
 namespace askja {
@@ -319,7 +319,7 @@ cudaError_t plaq(const LaunchCtx& c, const void* U, double* partial, double* out
     j.plaq_partial = partial;
     const cudaError_t e = m64::plaq(N, sizeof(T) == 8, j, m64::Grid{}, 0, c.stream);
     if (e != cudaSuccess) return e;
-    misc::k_finish<2><<<1, misc::RED_THREADS, 0, c.stream>>>(partial, m64::ctas_for(c.lat.V, m64::links_per_cta(N)),
+    misc::k_finish<2><<<1, misc::RED_THREADS, 0, c.stream>>>(partial, m64::ctas_for(c.lat.V, m64::sites_per_cta(N)),
                                                              out);
     return cudaGetLastError();
   }
@@ -338,20 +338,24 @@ template <typename T>
 cudaError_t linksums(const LaunchCtx& c, const void* Pa, const void* Pb, const void* U, double* partial, double* out) {
   using S2 = typename Storage<T>::type;
   const int N = c.lat.N;
-  if (m64_supported(N) && Pa && !Pb && !U) {
+  if (m64_supported(N)) {
     m64::Job j = m64_job(c.lat);
+    j.U[0] = const_cast<void*>(U);
     j.Pin = Pa;
+    j.Pin2 = Pb;
     j.kin_partial = partial;
-    const cudaError_t e = m64::kinetic(sizeof(T) == 8, j, m64::Grid{}, 3, c.stream);
+    const bool fp64 = sizeof(T) == 8;
+    int n = m64::ctas_for(nlinks(c.lat), m64::sites_per_cta(N));
+    if (U && Pa) return cudaErrorInvalidValue;  // one sum per call
+    cudaError_t e = cudaSuccess;
+    if (U) {
+      e = m64::uviol(N, fp64, j, c.stream);
+    } else {
+      n = m64::ctas_for(nlinks(c.lat), m64::kinetic_links_per_cta(N));
+      e = m64::kinetic(fp64, j, m64::Grid{}, 3, c.stream);
+    }
     if (e != cudaSuccess) return e;
-    misc::k_finish<3><<<1, misc::RED_THREADS, 0, c.stream>>>(
-        partial, m64::ctas_for(nlinks(c.lat), m64::kinetic_links_per_cta(N)), out);
-    return cudaGetLastError();
-  }
-  if (N >= misc::BIG_NC) {
-    misc::k_linksums_big<S2><<<(unsigned)nlinks(c.lat), misc::RED_THREADS, 0, c.stream>>>(
-        c.lat, (const S2*)Pa, (const S2*)Pb, (const S2*)U, partial);
-    misc::k_finish<3><<<1, misc::RED_THREADS, 0, c.stream>>>(partial, (int)nlinks(c.lat), out);
+    misc::k_finish<3><<<1, misc::RED_THREADS, 0, c.stream>>>(partial, n, out);
     return cudaGetLastError();
   }
   const unsigned nb = blocks_for(nlinks(c.lat), misc::RED_THREADS);
@@ -361,58 +365,79 @@ cudaError_t linksums(const LaunchCtx& c, const void* Pa, const void* Pb, const v
   else if (N == 3)
     misc::k_linksums<3, S2><<<nb, misc::RED_THREADS, 0, c.stream>>>(c.lat, (const S2*)Pa, (const S2*)Pb,
                                                                     (const S2*)U, partial);
-  else if (N == 4)
-    misc::k_linksums<4, S2><<<nb, misc::RED_THREADS, 0, c.stream>>>(c.lat, (const S2*)Pa, (const S2*)Pb,
-                                                                    (const S2*)U, partial);
   else
-    misc::k_linksums<0, S2><<<nb, misc::RED_THREADS, 0, c.stream>>>(c.lat, (const S2*)Pa, (const S2*)Pb,
+    misc::k_linksums<4, S2><<<nb, misc::RED_THREADS, 0, c.stream>>>(c.lat, (const S2*)Pa, (const S2*)Pb,
                                                                     (const S2*)U, partial);
   misc::k_finish<3><<<1, misc::RED_THREADS, 0, c.stream>>>(partial, (int)nb, out);
   return cudaGetLastError();
 }
 
-constexpr int GAUSS_LINKS_PER_BLOCK = 256;
+// groups (NC >= 5) or CTAs whose partial matrices the Gauss law sums
+inline int gauss_partials(const Lat& L) {
+  if (m64_supported(L.N)) return m64::gauss_groups(L.N, nlinks(L));
+  return (int)std::min<long>(blocks_for(nlinks(L), 128), 4 * 148);
+}
 
+// partial: gauss_partials matrices and their sum
 template <typename T>
 cudaError_t gauss(const LaunchCtx& c, const void* U, const void* Pi, double* partial, double* out) {
   using S2 = typename Storage<T>::type;
-  const unsigned nb = blocks_for(nlinks(c.lat), GAUSS_LINKS_PER_BLOCK);
-  const int NN = c.lat.N * c.lat.N;
-  const int thr = std::min(misc::RED_THREADS, ((NN + 31) / 32) * 32);
-  misc::k_gauss<S2><<<nb, thr, 0, c.stream>>>(c.lat, (const S2*)U, (const S2*)Pi, GAUSS_LINKS_PER_BLOCK, partial);
-  misc::k_gauss_finish<<<1, thr, 2 * NN * sizeof(double), c.stream>>>(partial, (int)nb, c.lat.N, out);
+  const int N = c.lat.N, n2 = 2 * N * N, np = gauss_partials(c.lat);
+  const S2 *u = (const S2*)U, *p = (const S2*)Pi;
+  if (m64_supported(N)) {
+    m64::Job j = m64_job(c.lat);
+    j.U[0] = const_cast<void*>(U);
+    j.Pin = Pi;
+    j.kin_partial = partial;
+    const cudaError_t e = m64::gauss(N, sizeof(T) == 8, j, c.stream);
+    if (e != cudaSuccess) return e;
+  } else if (N == 2) {
+    lines::k_gauss<2, S2><<<np, 128, 0, c.stream>>>(c.lat, u, p, partial);
+  } else if (N == 3) {
+    lines::k_gauss<3, S2><<<np, 128, 0, c.stream>>>(c.lat, u, p, partial);
+  } else {
+    lines::k_gauss<4, S2><<<np, 128, 0, c.stream>>>(c.lat, u, p, partial);
+  }
+  double* sum = partial + (size_t)np * n2;
+  lines::k_gauss_sum<<<(n2 + 7) / 8, 256, 0, c.stream>>>(partial, np, n2, sum);
+  lines::k_gauss_finish<<<1, misc::RED_THREADS, 0, c.stream>>>(sum, N, out);
   return cudaGetLastError();
 }
 
 template <typename T>
-cudaError_t lines(const LaunchCtx& c, const void* U, int dir, int nlines, int start_stride, double* out) {
+cudaError_t line_traces(const LaunchCtx& c, const void* U, const LineSet& ls, double* out) {
   using S2 = typename Storage<T>::type;
-  const int N = c.lat.N;
-  const size_t smem = 2 * (size_t)N * N * sizeof(cpx<double>);
-  auto k = misc::k_lines<S2>;
-  cudaError_t e;
-  if ((e = set_smem(k, smem)) != cudaSuccess) return e;
-  k<<<nlines, ((N + 31) / 32) * 32, smem, c.stream>>>(c.lat, (const S2*)U, dir, start_stride, out);
+  const int N = c.lat.N, n = ls.lines();
+  if (m64_supported(N)) return m64::lines(sizeof(T) == 8, c.lat, U, ls, out, nullptr, nullptr, c.stream);
+  const S2* u = (const S2*)U;
+  if (N == 2)
+    lines::k_lines<2, S2><<<blocks_for(n, 4), 128, 0, c.stream>>>(c.lat, u, ls, n, out);
+  else if (N == 3)
+    lines::k_lines<3, S2><<<blocks_for(n, 4), 128, 0, c.stream>>>(c.lat, u, ls, n, out);
+  else
+    lines::k_lines<4, S2><<<blocks_for(n, 4), 128, 0, c.stream>>>(c.lat, u, ls, n, out);
   return cudaGetLastError();
 }
 
 template <typename T>
 cudaError_t slice_trace(const LaunchCtx& c, const void* U, double* out) {
   using S2 = typename Storage<T>::type;
-  misc::k_slice_trace<S2><<<c.lat.n[0], misc::RED_THREADS, 0, c.stream>>>(c.lat, (const S2*)U, out);
+  misc::k_slice_trace<S2><<<c.lat.n[0], misc::SLICE_THREADS, 0, c.stream>>>(c.lat, (const S2*)U, out);
   return cudaGetLastError();
 }
 
 template <typename T>
-cudaError_t line_eigs(const LaunchCtx& c, const void* U, int dir, int nlines, int start_stride, double2* ev,
-                      int* fail) {
+cudaError_t line_eigs(const LaunchCtx& c, const void* U, const LineSet& ls, double2* ev, int* fail) {
   using S2 = typename Storage<T>::type;
-  const int N = c.lat.N;
-  const size_t smem = 2 * (size_t)N * N * sizeof(cpx<double>);
-  auto k = eig::k_line_eigs<S2>;
-  cudaError_t e;
-  if ((e = set_smem(k, smem)) != cudaSuccess) return e;
-  k<<<nlines, std::max(32, (N + 31) / 32 * 32), smem, c.stream>>>(c.lat, (const S2*)U, dir, start_stride, ev, fail);
+  const int N = c.lat.N, n = ls.lines();
+  if (m64_supported(N)) return m64::lines(sizeof(T) == 8, c.lat, U, ls, nullptr, ev, fail, c.stream);
+  const S2* u = (const S2*)U;
+  if (N == 2)
+    lines::k_line_eigs<2, S2><<<n, 32, 0, c.stream>>>(c.lat, u, ls, ev, fail);
+  else if (N == 3)
+    lines::k_line_eigs<3, S2><<<n, 32, 0, c.stream>>>(c.lat, u, ls, ev, fail);
+  else
+    lines::k_line_eigs<4, S2><<<n, 32, 0, c.stream>>>(c.lat, u, ls, ev, fail);
   return cudaGetLastError();
 }
 
@@ -508,7 +533,7 @@ cudaError_t wait_probe(const LaunchCtx& c, long long cycles) {
 
 template <typename T>
 constexpr KernelSet make_set() {
-  return KernelSet{&force<T>,   &drift<T>,   &reunit<T>,  &plaq<T>,           &linksums<T>,  &gauss<T>, &lines<T>,
+  return KernelSet{&force<T>,   &drift<T>,   &reunit<T>,  &plaq<T>,           &linksums<T>,  &gauss<T>, &line_traces<T>,
                    &slice_trace<T>, &line_eigs<T>, &refresh<T>, &identity<T>, &gauss_matrices<T>, &from_conf<T>, &to_conf<T>, &pair_swap<T>, &fourier<T>, &tab_sites<T>,
                    &wait_probe<T>};
 }

@@ -27,6 +27,8 @@ struct DevGuard {
   DevGuard& operator=(const DevGuard&) = delete;
 };
 
+struct LineSet;  // lines.cuh
+
 struct LaunchCtx {
   Lat lat;
   cudaStream_t stream;
@@ -78,11 +80,11 @@ struct KernelSet {
   cudaError_t (*linksums)(const LaunchCtx&, const void* Pa, const void* Pb, const void* U, double* partial,
                           double* out);
   cudaError_t (*gauss)(const LaunchCtx&, const void* U, const void* Pi, double* partial, double* out);
-  cudaError_t (*lines)(const LaunchCtx&, const void* U, int dir, int nlines, int start_stride, double* out);
+  // |Tr W| / NC of every line of the set
+  cudaError_t (*lines)(const LaunchCtx&, const void* U, const LineSet&, double* out);
   cudaError_t (*slice_trace)(const LaunchCtx&, const void* U, double* out);
   // eigenvalues of closed line matrices: ev[q*NC + i] (complex), *fail set on no convergence
-  cudaError_t (*line_eigs)(const LaunchCtx&, const void* U, int dir, int nlines, int start_stride, double2* ev,
-                           int* fail);
+  cudaError_t (*line_eigs)(const LaunchCtx&, const void* U, const LineSet&, double2* ev, int* fail);
   cudaError_t (*refresh)(const LaunchCtx&, void* P, uint64_t seed, const unsigned long long* traj_dev,
                          unsigned long long traj_host, double scale);
   cudaError_t (*identity)(const LaunchCtx&, void* U);

@@ -163,122 +163,34 @@ __global__ void __launch_bounds__(RED_THREADS) k_linksums(Lat L, const S2* __res
     for (int k = 0; k < 3; k++) partial[blockIdx.x * 3 + k] = v[k];
 }
 
-// Gauss law (sun.cpp:415-438): the lattice sum of Pi_j(x) - U_j^dag(x-j) Pi_j(x-j) U_j(x-j)
-// over all sites and directions.  Re-indexing x -> x+j turns every term into a
-// function of one link l: Pi_l - U_l^dag Pi_l U_l.  One block accumulates its
-// links' matrices element by element; partial[b*2*N*N + 2e + {0,1}].
-template <typename S2>
-__global__ void __launch_bounds__(RED_THREADS) k_gauss(Lat L, const S2* __restrict__ U, const S2* __restrict__ Pi,
-                                                       int links_per_block, double* __restrict__ partial) {
-  const int N = L.N, NN = N * N;
-  const int es = estride(L);
-  const long l0 = (long)blockIdx.x * links_per_block;
-  const long l1 = min((long)L.V * L.D, l0 + links_per_block);
-  for (int e = threadIdx.x; e < NN; e += blockDim.x) {
-    const int i = e / N, j = e - i * N;
-    double sr = 0.0, si = 0.0;
-    for (long l = l0; l < l1; l++) {
-      const int d = (int)(l / L.V);
-      const int s = (int)(l - (long)d * L.V);
-      const size_t b0 = mbase(L, d, s);
-      cpx<double> g = ldc<double>(Pi + b0 + e * es);
-      // (U^dag Pi U)_ij = sum_ab conj(U_ai) Pi_ab U_bj
-      cpx<double> t = czero<double>();
-      for (int a = 0; a < N; a++) {
-        cpx<double> pu = czero<double>();
-        for (int b = 0; b < N; b++)
-          cmac(pu, ldc<double>(Pi + b0 + (a * N + b) * es), ldc<double>(U + b0 + (b * N + j) * es));
-        cmac_cn(t, ldc<double>(U + b0 + (a * N + i) * es), pu);
-      }
-      sr += g.re - t.re;
-      si += g.im - t.im;
-    }
-    partial[(size_t)blockIdx.x * 2 * NN + 2 * e] = sr;
-    partial[(size_t)blockIdx.x * 2 * NN + 2 * e + 1] = si;
-  }
-}
-
-// Sum the Gauss-law partials and return tr2 of the summed matrix.
-static __global__ void k_gauss_finish(const double* __restrict__ partial, int nblocks, int N, double* __restrict__ out) {
-  extern __shared__ double gsum[];
-  const int NN = N * N;
-  for (int e = threadIdx.x; e < NN; e += blockDim.x) {
-    double sr = 0.0, si = 0.0;
-    for (int b = 0; b < nblocks; b++) {
-      sr += partial[(size_t)b * 2 * NN + 2 * e];
-      si += partial[(size_t)b * 2 * NN + 2 * e + 1];
-    }
-    gsum[2 * e] = sr;
-    gsum[2 * e + 1] = si;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double r = 0.0;
-    for (int i = 0; i < N; i++)
-      for (int j = 0; j < N; j++) {
-        const double ar = gsum[2 * (i * N + j)], ai = gsum[2 * (i * N + j) + 1];
-        const double br = gsum[2 * (j * N + i)], bi = gsum[2 * (j * N + i) + 1];
-        r += ar * br - ai * bi;
-      }
-    *out = r;
-  }
-}
-
-// Closed Wilson lines: line q starts at site q*start_stride and runs along
-// direction `dir` through all n[dir] links; out[q] = |Tr W| / NC.
-// One block (NC threads, thread r owns row r of W) per line; the running
-// product is kept in shared memory.
-// sun.cpp:307-362 (one line, dir 0 from site 0), measurements4d.cpp:410-466
-// (Polyakov: dir 0 through (0,x1,0..)), measurements4d.cpp:311-355 (dir >= 1
-// through (x0,0,..)).
-template <typename S2>
-__global__ void k_lines(Lat L, const S2* __restrict__ U, int dir, int start_stride, double* __restrict__ out) {
-  extern __shared__ __align__(16) unsigned char lsm[];
-  cpx<double>* W = reinterpret_cast<cpx<double>*>(lsm);
-  cpx<double>* tmp = W + L.N * L.N;
-  const int N = L.N;
-  const int r = threadIdx.x;
-  int pos = blockIdx.x * start_stride;
-  if (r < N)
-    for (int c = 0; c < N; c++) W[r * N + c] = ldc<double>(U + eoff(L, dir, r * N + c, pos));
-  __syncthreads();
-  for (int st = 0; st < L.n[dir] - 1; st++) {
-    pos = nb_plus(L, dir, pos);
-    if (r < N)
-      for (int c = 0; c < N; c++) {
-        cpx<double> s = czero<double>();
-        for (int k = 0; k < N; k++) cmac(s, W[r * N + k], ldc<double>(U + eoff(L, dir, k * N + c, pos)));
-        tmp[r * N + c] = s;
-      }
-    __syncthreads();
-    if (r < N)
-      for (int c = 0; c < N; c++) W[r * N + c] = tmp[r * N + c];
-    __syncthreads();
-  }
-  if (r == 0) {
-    double tr = 0.0, ti = 0.0;
-    for (int k = 0; k < N; k++) {
-      tr += W[k * N + k].re;
-      ti += W[k * N + k].im;
-    }
-    out[blockIdx.x] = hypot(tr, ti) / N;
-  }
-}
-
 // Slice averages for measurements4d.cpp:357-408 scalarLoopcorr:
-// out[x0] = mean over the x0-slice of ReTr U_{D-1} / NC.  One block per slice.
+// out[x0] = mean over the x0-slice of ReTr U_{D-1} / NC.  One CTA per slice, of
+// as many threads as there may be: the slices are few and their loads are all
+// the kernel does (SU(3) 16^4: 22 us with 256 threads).
+constexpr int SLICE_THREADS = 1024;
 template <typename S2>
-__global__ void __launch_bounds__(RED_THREADS) k_slice_trace(Lat L, const S2* __restrict__ U, double* __restrict__ out) {
-  const int N = L.N;
+__global__ void __launch_bounds__(SLICE_THREADS) k_slice_trace(Lat L, const S2* __restrict__ U,
+                                                               double* __restrict__ out) {
+  __shared__ double sh[SLICE_THREADS / 32];
+  const int N = L.N, es = estride(L);
   const int slice = L.stride[0];
-  double v[1] = {0.0};
-  for (int s = blockIdx.x * slice + threadIdx.x; s < (blockIdx.x + 1) * slice; s += blockDim.x) {
+  double v = 0.0;
+  for (int s = blockIdx.x * slice + threadIdx.x; s < (blockIdx.x + 1) * slice; s += SLICE_THREADS) {
+    const S2* p = U + mbase(L, L.D - 1, s);
     double t = 0.0;
-    for (int k = 0; k < N; k++) t += ldc<double>(U + eoff(L, L.D - 1, k * N + k, s)).re;
-    v[0] += t / N;
+    for (int k = 0; k < N; k++) t += (double)p[(size_t)k * (N + 1) * es].x;
+    v += t / N;
   }
-  block_sum<1>(v);
-  if (threadIdx.x == 0) out[blockIdx.x] = v[0] / slice;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    v = sh[threadIdx.x];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if (threadIdx.x == 0) out[blockIdx.x] = v / slice;
+  }
 }
 
 // Momentum refresh (sun.cpp:209-252 initializeE with the reference's
@@ -658,51 +570,6 @@ __global__ void __launch_bounds__(RED_THREADS) k_plaq_big(Lat L, const S2* __res
     partial[(size_t)s * 2 + 0] = in ? nt - v[0] / N : 0.0;
     partial[(size_t)s * 2 + 1] = in ? ns - v[1] / N : 0.0;
   }
-}
-
-// link_sums of one link per CTA; partial[t*3 + k]
-template <typename S2>
-__global__ void __launch_bounds__(RED_THREADS) k_linksums_big(Lat L, const S2* __restrict__ Pa,
-                                                              const S2* __restrict__ Pb, const S2* __restrict__ U,
-                                                              double* __restrict__ partial) {
-  const int N = L.N;
-  const long t = blockIdx.x;
-  const int d = (int)(t / L.V);
-  const int s = (int)(t - (long)d * L.V);
-  double a = 0.0, b = 0.0, c = 0.0;
-  for (int e = threadIdx.x; e < N * N; e += RED_THREADS) {
-    const int i = e / N, j = e - (e / N) * N;
-    if (Pa) {
-      const cpx<double> x = ldc<double>(Pa + eoff(L, d, i * N + j, s));
-      const cpx<double> y = ldc<double>(Pa + eoff(L, d, j * N + i, s));
-      a = fma(x.re, y.re, a);
-      a = fma(-x.im, y.im, a);
-      if (Pb) {
-        const cpx<double> x2 = ldc<double>(Pb + eoff(L, d, i * N + j, s));
-        const cpx<double> y2 = ldc<double>(Pb + eoff(L, d, j * N + i, s));
-        b = fma(x.re + x2.re, y.re + y2.re, b);
-        b = fma(-(x.im + x2.im), y.im + y2.im, b);
-      }
-    }
-    if (U) {
-      cpx<double> aij = czero<double>(), aji = czero<double>();
-      for (int k = 0; k < N; k++) {
-        cmac_nc(aij, ldc<double>(U + eoff(L, d, i * N + k, s)), ldc<double>(U + eoff(L, d, j * N + k, s)));
-        cmac_nc(aji, ldc<double>(U + eoff(L, d, j * N + k, s)), ldc<double>(U + eoff(L, d, i * N + k, s)));
-      }
-      if (i == j) {
-        aij.re -= 1.0;
-        aji.re -= 1.0;
-      }
-      c = fma(aij.re, aji.re, c);
-      c = fma(-aij.im, aji.im, c);
-    }
-  }
-  double v[3] = {a, 0.25 * b, c};
-  block_sum<3>(v);
-  if (threadIdx.x == 0)
-#pragma unroll
-    for (int k = 0; k < 3; k++) partial[(size_t)t * 3 + k] = counted(L, s) ? v[k] : 0.0;
 }
 
 }  // namespace misc

@@ -35,6 +35,7 @@
 #pragma once
 
 #include "launch.h"
+#include "lines.cuh"
 #include "misc.cuh"
 
 namespace askja {
@@ -50,6 +51,7 @@ struct Job {
   int r0, r1;   // sites counted by the reductions (Lat)
   void* U[2];   // links in U[cur], updated links to U[cur ^ 1]
   const void* Pin;
+  const void* Pin2;  // second momenta of k_kinetic, or null
   void* Pout;
   double kick;  // kick step (times the launch's kick scale)
   double dt;    // drift step
@@ -57,11 +59,18 @@ struct Job {
   double* kin_partial;
 };
 
-// links per CTA: 8 warps, or one link where it takes more
+// CTA shapes.  Link update: four warps a CTA (one link from NT = 3 on) at the
+// tightest register budget that does not spill much.  Small CTAs fill the last
+// wave better and cost nothing, the warps of different links being independent:
+// us per fused step against eight-warp CTAs of 2-3 a SM, SU(8) 10^4 112 -> 105,
+// SU(16) 6^4 102 -> 99, SU(24) 6^3 51 -> 43, SU(32) 6^4 751 -> 722 (94 % of the
+// MMA rate).  Plaquette: about eight warps, a site each NT.
 template <int NT>
 struct Cta {
-  static constexpr int LINKS = NT == 1 ? 8 : NT == 2 ? 4 : NT <= 4 ? 2 : 1;
+  static constexpr int LINKS = NT == 1 ? 4 : NT == 2 ? 2 : 1;
+  static constexpr int SITES = NT == 1 ? 8 : NT == 2 ? 4 : NT <= 4 ? 2 : 1;
   static constexpr int THREADS = 32 * NT * LINKS;
+  static constexpr int PLAQ_THREADS = 32 * NT * SITES;
   static constexpr int LD = 8 * NT + 1;
   static constexpr int TILE = 8 * NT * LD;  // double2 of one link's tile
   // small matrices keep the rows of X and X^2 in registers; larger ones read X
@@ -70,7 +79,7 @@ struct Cta {
   static constexpr int TILES = KEEP ? 1 : 2;
   static constexpr size_t SMEM = (size_t)LINKS * TILES * TILE * sizeof(double2);
   // resident CTAs the register budget is set for
-  static constexpr int MIN_CTAS = NT == 1 ? 3 : NT == 2 ? 2 : NT <= 4 ? 2 : 1;
+  static constexpr int MIN_CTAS = NT == 1 ? 8 : NT == 2 ? 4 : NT == 3 ? 5 : NT == 4 ? 4 : 1;
 };
 
 struct Acc {
@@ -341,13 +350,16 @@ __global__ void __launch_bounds__(Cta<NT>::THREADS, Cta<NT>::MIN_CTAS)
   if (mode != 2) {
     Acc W[NT];  // the staple sum S first
     zero(W);
+    // lane nu fetches the neighbours of plane nu, all planes at once (D <= 16)
     const int xpmu = __ldg(nbr + (size_t)(2 * mu) * V + x);
+    const int ln = min(lane, D - 1);
+    const int xp = __ldg(nbr + (size_t)(2 * ln) * V + x), xm = __ldg(nbr + (size_t)(2 * ln + 1) * V + x),
+              xpm = __ldg(nbr + (size_t)(2 * ln + 1) * V + xpmu);
 #pragma unroll 1
     for (int nu = 0; nu < D; nu++) {
       if (nu == mu) continue;
-      const int xpnu = __ldg(nbr + (size_t)(2 * nu) * V + x);
-      const int xmnu = __ldg(nbr + (size_t)(2 * nu + 1) * V + x);
-      const int xpmu_mnu = __ldg(nbr + (size_t)(2 * nu + 1) * V + xpmu);
+      const int xpnu = __shfl_sync(0xffffffffu, xp, nu), xmnu = __shfl_sync(0xffffffffu, xm, nu),
+                xpmu_mnu = __shfl_sync(0xffffffffu, xpm, nu);
       Acc T[NT];
       {
         const S2 *a = link(nu, xpmu), *b = link(mu, xpnu), *y = link(nu, x);
@@ -568,7 +580,7 @@ __global__ void __launch_bounds__(Cta<NT>::THREADS, Cta<NT>::MIN_CTAS)
 // or four threads per row (above) did them on the FMA pipe from uncoalesced
 // loads.
 template <int NT, bool FULL, typename S2>
-__global__ void __launch_bounds__(Cta<NT>::THREADS)
+__global__ void __launch_bounds__(Cta<NT>::PLAQ_THREADS)
     k_plaq(const __grid_constant__ Job one, const Job* __restrict__ table, const int2* __restrict__ items, int cur) {
   constexpr int KU = NT <= 4 ? NT : 1;
   const Job* __restrict__ jp = &one;
@@ -587,7 +599,7 @@ __global__ void __launch_bounds__(Cta<NT>::THREADS)
   me.q = lane >> 2;
   me.j = lane & 3;
   me.n = job.N;
-  const int x = blk * Cta<NT>::LINKS + slot;
+  const int x = blk * Cta<NT>::SITES + slot;
   const size_t NN = FULL ? (size_t)64 * NT * NT : (size_t)me.n * me.n;
   const S2* __restrict__ U = static_cast<const S2*>(job.U[cur]);
   const int* __restrict__ nbr = job.nbr;
@@ -629,7 +641,7 @@ __global__ void __launch_bounds__(Cta<NT>::THREADS)
   }
 }
 
-// Kinetic sums sum ReTr(P P): a warp takes 8 x 8 tiles of a link's matrix, each
+// Kinetic sums sum ReTr(P P) and, with Pin2, sum ReTr((P + P2)^2) / 4: a warp takes 8 x 8 tiles of a link's matrix, each
 // with its mirror tile in the column pattern (whole sectors, where element pairs
 // read a row length apart took 365 us for SU(64) 4x8x16 on 24 CTAs);
 // KIN_TILES tiles per CTA, whole links; kin_partial[stride * blk].
@@ -660,7 +672,7 @@ __global__ void __launch_bounds__(misc::RED_THREADS)
   me.q = lane >> 2;
   me.j = lane & 3;
   me.n = N;
-  double v[1] = {0.0};
+  double v[2] = {0.0, 0.0};
   for (int f = wid; f < links * nt * nt; f += misc::RED_THREADS / 32) {
     const long l = l0 + f / (nt * nt);
     const int t = f % (nt * nt), ti = t / nt, tj = t - ti * nt;
@@ -675,12 +687,194 @@ __global__ void __launch_bounds__(misc::RED_THREADS)
       v[0] = fma(p[e].re, q[e].re, v[0]);
       v[0] = fma(-p[e].im, q[e].im, v[0]);
     }
+    if (job.Pin2) {
+      const S2* P2 = static_cast<const S2*>(job.Pin2) + (size_t)l * N * N;
+      Op p2[2], q2[2];
+      me.rows(P2, ti, tj, p2);
+      me.cols(P2, tj, ti, q2);
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        v[1] = fma(p[e].re + p2[e].re, q[e].re + q2[e].re, v[1]);
+        v[1] = fma(-(p[e].im + p2[e].im), q[e].im + q2[e].im, v[1]);
+      }
+    }
+  }
+  misc::block_sum<2>(v);
+  if (threadIdx.x == 0) {  // stride 3: [P P, (P + P2)^2 / 4, no unitarity sum]
+    job.kin_partial[(size_t)stride * blk] = v[0];
+    if (stride == 3) {
+      job.kin_partial[(size_t)stride * blk + 1] = 0.25 * v[1];
+      job.kin_partial[(size_t)stride * blk + 2] = 0.0;
+    }
+  }
+}
+
+// UViol (sun.cpp:441-471): sum ReTr((U U^dag - 1)^2), the matrix Hermitian, so
+// the sum of its squared moduli; SITES links per CTA, partial[3 blk + 2].
+template <int NT, bool FULL, typename S2>
+__global__ void __launch_bounds__(Cta<NT>::PLAQ_THREADS) k_uviol(const __grid_constant__ Job job) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int slot = wid / NT;
+  Who<NT, FULL> me;
+  me.w = wid - slot * NT;
+  me.q = lane >> 2;
+  me.j = lane & 3;
+  me.n = job.N;
+  const long l = (long)blockIdx.x * Cta<NT>::SITES + slot;
+  const int s = (int)(l % job.V);
+  double v[1] = {0.0};
+  if (l < (long)job.V * job.D && s >= job.r0 && (job.r1 == 0 || s < job.r1)) {
+    const S2* u = static_cast<const S2*>(job.U[0]) + (size_t)l * me.N() * me.N();
+    Acc M[NT];
+    zero(M);
+    prod<NT, true, (NT <= 4 ? NT : 1)>(
+        M, [&](int kb, Op(&o)[2]) { me.rows(u, me.w, kb, o); },
+        [&](int kb, int t, Op(&o)[2]) { me.rows(u, t, kb, o); });
+    const int r = 8 * me.w + me.q;
+#pragma unroll
+    for (int t = 0; t < NT; t++)
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const double re = M[t].re[e] - (r == 8 * t + 2 * me.j + e && r < me.N() ? 1.0 : 0.0);
+        v[0] = fma(re, re, v[0]);
+        v[0] = fma(M[t].im[e], M[t].im[e], v[0]);
+      }
   }
   misc::block_sum<1>(v);
   if (threadIdx.x == 0) {
-    job.kin_partial[(size_t)stride * blk] = v[0];
-    for (int k = 1; k < stride; k++) job.kin_partial[(size_t)stride * blk + k] = 0.0;
+    double* p = job.kin_partial + 3 * (size_t)blockIdx.x;
+    p[0] = p[1] = 0.0;
+    p[2] = v[0];
   }
+}
+
+// Gauss law: sum over the links of Pi - U^dag Pi U (lines.cuh), NT warps per
+// group, each group's links accumulated in its warps' registers with a grid
+// stride; the group's matrix goes to kin_partial[g * 2 NC^2 + 2 e + {0, 1}].
+template <int NT, bool FULL, typename S2>
+__global__ void __launch_bounds__(Cta<NT>::PLAQ_THREADS) k_gauss(const __grid_constant__ Job job, int ngroups) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int slot = wid / NT;
+  Who<NT, FULL> me;
+  me.w = wid - slot * NT;
+  me.q = lane >> 2;
+  me.j = lane & 3;
+  me.n = job.N;
+  const int g = blockIdx.x * Cta<NT>::SITES + slot;
+  if (g >= ngroups) return;
+  const int N = me.N();
+  const long nl = (long)job.V * job.D;
+  Acc G[NT];
+  zero(G);
+  for (long l = g; l < nl; l += ngroups) {
+    const S2* u = static_cast<const S2*>(job.U[0]) + (size_t)l * N * N;
+    const S2* p = static_cast<const S2*>(job.Pin) + (size_t)l * N * N;
+    Acc T[NT];
+    zero(T);
+    prod<NT, false, (NT <= 4 ? NT : 1)>(
+        T,
+        [&](int kb, Op(&o)[2]) {  // -U^dag
+          me.cols(u, kb, me.w, o);
+          o[0].re = -o[0].re;
+          o[1].re = -o[1].re;
+        },
+        [&](int kb, int t, Op(&o)[2]) { me.cols(p, kb, t, o); });
+    prod<NT, false, NT>(
+        G, [&](int kb, Op(&o)[2]) { from_acc(T, kb, o); },
+        [&](int kb, int t, Op(&o)[2]) { me.cols(u, kb, t, o); });
+#pragma unroll
+    for (int t = 0; t < NT; t++) {
+      Op o[2];
+      me.rows(p, me.w, t, o);
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        G[t].re[e] += o[e].re;
+        G[t].im[e] += o[e].im;
+      }
+    }
+  }
+  double2* out = reinterpret_cast<double2*>(job.kin_partial) + (size_t)g * N * N;
+#pragma unroll
+  for (int t = 0; t < NT; t++) {
+    const int r = 8 * me.w + me.q, c = 8 * t + 2 * me.j;
+#pragma unroll
+    for (int e = 0; e < 2; e++)
+      if (FULL || (r < N && c + e < N)) out[r * N + c + e] = make_double2(G[t].re[e], G[t].im[e]);
+  }
+}
+
+// Closed lines (LineSet of lines.cuh), NT warps per line: the running product
+// is each warp's accumulator rows, so a link of the line is one product with no
+// barrier.  ev null: out[q] = |Tr W_q| / NC; else the eigenvalues of W_q by one
+// warp from shared memory (eig.cuh).
+template <int NT, bool FULL, typename S2>
+__global__ void __launch_bounds__(32 * NT) k_lines(const __grid_constant__ Lat L, const S2* __restrict__ U,
+                                                   const __grid_constant__ LineSet ls, double* __restrict__ out,
+                                                   double2* __restrict__ ev, int* __restrict__ fail) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int lane = threadIdx.x & 31;
+  Who<NT, FULL> me;
+  me.w = threadIdx.x >> 5;
+  me.q = lane >> 2;
+  me.j = lane & 3;
+  me.n = L.N;
+  const int N = me.N();
+  int start;
+  const int dir = line_of(ls, blockIdx.x, &start);
+  const S2* u = U + ((size_t)dir * L.V + start) * N * N;
+  const size_t step = (size_t)L.stride[dir] * N * N;
+  Acc W[NT];
+#pragma unroll
+  for (int t = 0; t < NT; t++) {
+    Op o[2];
+    me.rows(u, me.w, t, o);
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+      W[t].re[e] = o[e].re;
+      W[t].im[e] = o[e].im;
+    }
+  }
+  for (int k = 1; k < L.n[dir]; k++) {
+    u += step;
+    Acc T[NT];
+    zero(T);
+    prod<NT, false, NT>(
+        T, [&](int kb, Op(&o)[2]) { from_acc(W, kb, o); },
+        [&](int kb, int t, Op(&o)[2]) { me.cols(u, kb, t, o); });
+#pragma unroll
+    for (int t = 0; t < NT; t++) W[t] = T[t];
+  }
+  const int r = 8 * me.w + me.q;
+  if (ev) {
+    cpx<double>* H = reinterpret_cast<cpx<double>*>(smem_raw);
+#pragma unroll
+    for (int t = 0; t < NT; t++)
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const int c = 8 * t + 2 * me.j + e;
+        if (r < N && c < N) H[r * N + c] = mkc<double>(W[t].re[e], W[t].im[e]);
+      }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      cpx<double>* v = H + N * N;
+      cpx<double>* e = v + N;
+      eig::hessenberg_qr(H, N, v, e, fail);
+      __syncwarp();
+      for (int i = lane; i < N; i += 32) ev[(size_t)blockIdx.x * N + i] = make_double2(e[i].re, e[i].im);
+    }
+    return;
+  }
+  double v[2] = {0.0, 0.0};
+#pragma unroll
+  for (int t = 0; t < NT; t++)
+#pragma unroll
+    for (int e = 0; e < 2; e++)
+      if (r == 8 * t + 2 * me.j + e && r < N) {
+        v[0] += W[t].re[e];
+        v[1] += W[t].im[e];
+      }
+  misc::block_sum<2>(v);
+  if (threadIdx.x == 0) out[blockIdx.x] = hypot(v[0], v[1]) / N;
 }
 
 }  // namespace m64

@@ -111,6 +111,35 @@ def test_batch_equals_single_chains(precision):
             np.testing.assert_array_equal(ends[c], e.get_links())
 
 
+@pytest.mark.parametrize("nc,dims", [(2, [40, 3]), (3, [33, 2, 2]), (3, [65]), (4, [1, 5, 4]), (4, [97, 2]), (5, [4, 3]),
+                                     (8, [3, 2, 3]), (13, [2, 4]), (24, [2, 3]), (33, [3, 2]), (64, [2, 2])])
+def test_lines_gauss_and_unitarity_vs_oracle(nc, dims):
+    """Line products shared between lanes (NC <= 4: extents around 32 and 64
+    links) or walked by the MMA, the Gauss law's grouped sums, UViol of links
+    that are not unitary, and the one-read-back measure()."""
+    O, u, pi, rng = start(nc, dims, 3 * nc)
+    u = u * (1.0 + 0.01 * rng.standard_normal(u.shape))
+    with ab.Engine(nc, dims, beta=2.0 * nc, precision="fp64") as e:
+        e.set_links(u)
+        e.set_momenta(pi, 0)
+        e.updateE(0.05)
+        Pi = O.updateE(u, pi, 0.05)
+        one = {"WilsonLoop": (e.WilsonLoop(), O.WilsonLoop_sun(u)), "GaussLaw": (e.GaussLaw(), O.GaussLaw(u, Pi)),
+               "UViol": (e.UViol(), O.UViol(u)), "EnergyEl": (e.EnergyEl(), O.EnergyEl(pi, Pi))}
+        if len(dims) > 1:
+            one["Polyakov"] = (e.PolyakovLoop(), O.PolyakovLoop(u))
+            one["slices"] = (e.scalarLoopcorr(), O.scalarLoopcorr(u))
+            for d in range(1, len(dims)):
+                one[f"Wilson{d}"] = (e.WilsonLoopDir(d), O.WilsonLoopDir(u, d))
+            t, s = e.PlaqExp()
+            want = [t, s, e.PolyakovLoop()] + [e.WilsonLoopDir(d) for d in range(1, len(dims))]
+            want += [e.GaussLaw(), e.UViol()]
+            np.testing.assert_array_equal(e.measure(), want)
+        for name, (got, ref) in one.items():
+            # a line of n links multiplies the rounding of n products; the links' norms stray by 1 %
+            np.testing.assert_allclose(got, ref, rtol=1e-11, atol=1e-12, err_msg=name)
+
+
 @pytest.mark.parametrize("nc", [6, 16, 40])
 def test_counted_ranges_add_up(nc):
     O, u, pi, _ = start(nc, [5, 3], nc)
