@@ -584,7 +584,8 @@ int askja_create(const askja_params* p, askja_ctx** out) {
                      : askja::m64_supported(p->nc)                                                            ? 4
                                                                                                               : 0;
   c->lc.rows_groups = 0;
-  c->lc.small_occ = 0;
+  c->lc.small_occ =
+      p->kernel_path == 0 ? askja::default_occupancy(p->nc, p->precision == ASKJA_FP64, c->split, V) : 0;
   if (p->kernel_path == 0) {
     std::lock_guard<std::mutex> lock(g_tune_mutex);
     auto it = g_tune_cache.find(std::make_tuple(p->nc, p->dim, p->precision));

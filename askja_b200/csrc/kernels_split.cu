@@ -47,10 +47,9 @@ cudaError_t force(const LaunchCtx& c, int mode, const void* U, const void* UL, c
   return by_nc(c.lat.N, [&](auto n) {
     constexpr int N = decltype(n)::value;
     auto launch = [&](auto kern) {
-      kern<<<grid, threads, 0, c.stream>>>(c.lat, (const float2*)U, (const uint32_t*)UL, (const float*)Pin,
-                                           (const uint32_t*)PLin, (float*)Pout, (uint32_t*)PLout, (float2*)Uout,
-                                           (uint32_t*)ULout, (float)ek, (float)ed, c.order);
-      return cudaGetLastError();
+      return launch_overlapped(kern, grid, threads, 0, c.stream, c.lat, (const float2*)U, (const uint32_t*)UL,
+                               (const float*)Pin, (const uint32_t*)PLin, (float*)Pout, (uint32_t*)PLout, (float2*)Uout,
+                               (uint32_t*)ULout, (float)ek, (float)ed, c.order);
     };
     if (mode == 0) {
       if (c.small_occ == 2) return launch(split::k_force<N, 0, 2>);

@@ -29,6 +29,28 @@ struct DevGuard {
 
 struct LineSet;  // lines.cuh
 
+// Launches a kernel that begins with grid_wait() (common.cuh) so that its CTAs
+// may be placed while the kernel before it in the stream drains (programmatic
+// dependent launch): the start of one MD step hides behind the end of the one
+// before.  Everything the kernel reads or writes comes after its grid_wait().
+// Graph-replayed us per step: SU(3) 8^4 FP64 6.81 -> 6.56, SU(2) 10^4 FP64
+// 6.76 -> 6.01, SU(8) 4^4 FP64 6.62 -> 6.29; nothing to gain on large lattices.
+template <typename... P, typename... A>
+cudaError_t launch_overlapped(void (*k)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t stream,
+                              A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k, static_cast<P>(args)...);
+}
+
 struct LaunchCtx {
   Lat lat;
   cudaStream_t stream;
@@ -59,6 +81,20 @@ inline bool tc_supported(int N, int D, bool fp64) { return !fp64 && (N == 16 || 
 
 // whether the FP64-MMA mapping exists for this colour number
 inline bool m64_supported(int N) { return link_major(N); }
+
+// Untuned register budget (LaunchCtx::small_occ) of the thread-per-link kernels,
+// by 32-site tiles.  Measured us per step at budget 0 and 2:
+//  FP32 (residual planes), NC = 2, 3: with more tiles than four CTAs per SM
+//   hold, the tight budget's seven CTAs hide more latency (SU(3) 32^4 469 / 443,
+//   SU(2) 16^4 15.5 / 12.9); below, the loose one's extra loads in flight win
+//   (SU(3) 12^4 11.3 / 11.1, 10^4 7.4 / 8.4, 8^4 4.5 / 6.5).  NC = 4 spills at 2.
+//  FP64, NC = 2: the budgets are the other way round (80 and 126 registers):
+//   10^4 6.8 / 5.6, 16^4 19.5 / 19.0, 32^4 308 / 326.  NC = 3: no difference.
+inline int default_occupancy(int N, bool fp64, bool residual, long V) {
+  const long tiles = (V + 31) / 32;
+  if (fp64) return N == 2 && tiles <= 2048 ? 2 : 0;
+  return residual && N <= 3 && tiles > 4 * 148 ? 2 : 0;
+}
 
 // whether the site-pair mapping exists (n_fast: extent of the fastest direction)
 inline bool pair_supported(int N, int D, bool fp64, int n_fast) {

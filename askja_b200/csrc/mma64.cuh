@@ -315,6 +315,7 @@ template <int NT, bool FULL, typename S2>
 __global__ void __launch_bounds__(Cta<NT>::THREADS, Cta<NT>::MIN_CTAS)
     k_link(const __grid_constant__ Job one, const Job* __restrict__ table, const int2* __restrict__ items, int cur,
            double kick_scale, int mode) {
+  grid_wait();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   using CT = Cta<NT>;
   constexpr int KU = NT <= 4 ? NT : 1;  // left operands from memory: the k loop stays rolled for large NC
@@ -570,6 +571,7 @@ __global__ void __launch_bounds__(Cta<NT>::THREADS, Cta<NT>::MIN_CTAS)
   prod<NT, false, NT>(
       Y, [&](int kb, Op(&o)[2]) { from_acc(E, kb, o); },
       [&](int kb, int t, Op(&o)[2]) { me.cols(Ux, kb, t, o); });
+  grid_done();
   store_rows(static_cast<S2*>(job.U[cur ^ 1]) + own, me, Y);
 }
 

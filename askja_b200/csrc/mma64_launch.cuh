@@ -20,8 +20,11 @@ cudaError_t launch_link(const Job& one, const Grid& g, int cur, double ks, int m
     if (e != cudaSuccess) return e;
   }
   const int ctas = g.table ? g.ctas : ctas_for((long)one.V * one.D, Cta<NT>::LINKS);
-  k<<<ctas, Cta<NT>::THREADS, smem, st>>>(one, g.table, g.items, cur, ks, mode);
-  return cudaGetLastError();
+  if (g.table) {  // a batch's launches depend on other streams' work: ordinary order
+    k<<<ctas, Cta<NT>::THREADS, smem, st>>>(one, g.table, g.items, cur, ks, mode);
+    return cudaGetLastError();
+  }
+  return launch_overlapped(k, ctas, Cta<NT>::THREADS, smem, st, one, g.table, g.items, cur, ks, mode);
 }
 
 template <int NT, bool FULL, typename S2>

@@ -285,6 +285,21 @@ __device__ __forceinline__ void expi_times(Mat<N, T>& Tm, const Mat<N, T>& P, co
   }
 }
 
+// Tm = U + Em U, the small product summed on its own so that every entry has
+// one rounding at U's size (as Horner's last step has), not one per term
+template <int N, typename T>
+__device__ __forceinline__ void add_update(Mat<N, T>& Tm, const Mat<N, T>& Em, const Mat<N, T>& U) {
+#pragma unroll
+  for (int i = 0; i < N; i++)
+#pragma unroll
+    for (int j = 0; j < N; j++) {
+      cpx<T> s = czero<T>();
+#pragma unroll
+      for (int k = 0; k < N; k++) cmac(s, Em.a[i][k], U.a[k][j]);
+      Tm.a[i][j] = mkc<T>(U.a[i][j].re + s.re, U.a[i][j].im + s.im);
+    }
+}
+
 template <typename T>
 __device__ __forceinline__ cpx<T> cmul(const cpx<T>& a, const cpx<T>& b) {
   cpx<T> z = czero<T>();
@@ -304,6 +319,7 @@ template <int N, typename T>
 __device__ __forceinline__ void expi_times_ch(Mat<N, T>& Tm, const Mat<N, T>& P, const Mat<N, T>& Ux, T eps,
                                               int order) {
   static_assert(N == 2 || N == 3, "Cayley-Hamilton form for N = 2, 3");
+  constexpr bool MINUS_ONE = sizeof(T) == 8;  // FP64 forms E - 1
   Mat<N, T> X;
 #pragma unroll
   for (int i = 0; i < N; i++)
@@ -321,7 +337,7 @@ __device__ __forceinline__ void expi_times_ch(Mat<N, T>& Tm, const Mat<N, T>& P,
     cpx<T> d = cmul(X.a[0][0], X.a[1][1]);
     cmsub(d, X.a[0][1], X.a[1][0]);
     cpx<T> al = mkc<T>(T(1), T(0)), be = czero<T>();  // X^0
-    cpx<T> sa = al, sb = be;
+    cpx<T> sa = MINUS_ONE ? czero<T>() : al, sb = be;
     T f = T(1);
 #pragma unroll
     for (int k = 1; k <= 8; k++) {  // order <= 8; unrolled so that 1/k is a constant
@@ -367,7 +383,7 @@ __device__ __forceinline__ void expi_times_ch(Mat<N, T>& Tm, const Mat<N, T>& P,
     cmsub(c0, X.a[0][1], m1);
     cmac(c0, X.a[0][2], m2);
     cpx<T> al = mkc<T>(T(1), T(0)), be = czero<T>(), ga = czero<T>();  // X^0
-    cpx<T> sa = al, sb = be, sc = ga;
+    cpx<T> sa = MINUS_ONE ? czero<T>() : al, sb = be, sc = ga;
     T f = T(1);
 #pragma unroll
     for (int k = 1; k <= 8; k++) {  // order <= 8; unrolled so that 1/k is a constant
@@ -398,7 +414,10 @@ __device__ __forceinline__ void expi_times_ch(Mat<N, T>& Tm, const Mat<N, T>& P,
         E.a[i][j] = e;
       }
   }
-  mul_nn(Tm, E, Ux);
+  if constexpr (MINUS_ONE)
+    add_update(Tm, E, Ux);
+  else
+    mul_nn(Tm, E, Ux);
 }
 
 // The same series for N = 3 written in P, for Hermitian P (every momentum
@@ -508,8 +527,12 @@ __device__ __forceinline__ void expi_times_herm3(Mat<3, T>& Tm, const Mat<3, T>&
     m = fma(B.im, pl.re, m);
     E.a[j][i] = mkc<T>(r, m);
   }
-  Tm = Ux;
-  mac_nn(Tm, E, Ux);
+  if constexpr (sizeof(T) == 8) {
+    add_update(Tm, E, Ux);
+  } else {
+    Tm = Ux;
+    mac_nn(Tm, E, Ux);
+  }
 }
 
 // The same for N = 4, any X = i eps P: X^4 = e1 X^3 - e2 X^2 + e3 X - e4 with
@@ -593,10 +616,10 @@ __device__ __forceinline__ void expi_times_ch4(Mat<4, T>& Tm, const Mat<4, T>& P
     }
 #pragma unroll
     for (int j = 0; j < 4; j++) {
-      cpx<T> s = Ux.a[i][j];
+      cpx<T> s = czero<T>();
 #pragma unroll
       for (int k = 0; k < 4; k++) cmac(s, e[k], Ux.a[k][j]);
-      Tm.a[i][j] = s;
+      Tm.a[i][j] = mkc<T>(Ux.a[i][j].re + s.re, Ux.a[i][j].im + s.im);
     }
   }
 }
@@ -730,6 +753,7 @@ __device__ __forceinline__ void force_link(const Lat& L, const S2* __restrict__ 
     Mat<N, T> Tm;
     expi_update(Tm, P, Ux, eps_d, order);
     if (reunit) reunitarise(Tm);
+    if (L.D <= 4) grid_done();
     store(Uout, Tm, L, mu, x);
   }
 }
@@ -738,6 +762,7 @@ template <int N, typename T, typename S2, int MODE>
 __global__ void __launch_bounds__(128) k_force(Lat L, const S2* __restrict__ U, const S2* Pin,
                                                S2* Pout, S2* __restrict__ Uout, T eps_k, T eps_d,
                                                int order, int reunit) {
+  grid_wait();
   const int x = blockIdx.x * 32 + (threadIdx.x & 31);
   if (x >= L.V) return;
   for (int mu = threadIdx.x >> 5; mu < L.D; mu += (blockDim.x >> 5)) force_link<N, T, S2, MODE>(
@@ -751,6 +776,7 @@ template <int N, typename T, typename S2, int MODE, int OCC = 1>
 __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 5 + OCC : 2 + OCC)
     k_force_occ(Lat L, const S2* __restrict__ U, const S2* Pin, S2* Pout, S2* __restrict__ Uout, T eps_k, T eps_d,
                 int order, int reunit) {
+  grid_wait();
   const int x = blockIdx.x * 32 + (threadIdx.x & 31);
   if (x >= L.V) return;
   for (int mu = threadIdx.x >> 5; mu < L.D; mu += (blockDim.x >> 5))

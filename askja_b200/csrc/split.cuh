@@ -489,6 +489,7 @@ __device__ __forceinline__ void link_update(const Lat& L, const float2* __restri
       for (int j = 0; j < N; j++) {
         add_split2(Ux.a[i][j].re, Ux.a[i][j].im, Ul.a[i][j].re, Ul.a[i][j].im, Dm.a[i][j].re, Dm.a[i][j].im);
       }
+    if (L.D <= 4) grid_done();
     small::store(Uout, Ux, L, mu, x);
     store_lo<N>(ULout, Ul, L, mu, x);
   }
@@ -501,6 +502,7 @@ __global__ void __launch_bounds__(128, OCC == 0 ? 4 : 5 + OCC)
     k_force(Lat L, const float2* __restrict__ U, const uint32_t* __restrict__ UL, const float* Pin,
             const uint32_t* PLin, float* Pout, uint32_t* PLout, float2* __restrict__ Uout,
             uint32_t* __restrict__ ULout, float eps_k, float eps_d, int order) {
+  grid_wait();
   const int x = blockIdx.x * 32 + (threadIdx.x & 31);
   if (x >= L.V) return;
   for (int mu = threadIdx.x >> 5; mu < L.D; mu += (blockDim.x >> 5))
