@@ -124,6 +124,7 @@ template <typename T>
 cudaError_t launch_force(askja_batch* b, const askja_batch::Group& g, cudaStream_t st, int mode, double ks) {
   using namespace askja::batch;
   const dim3 grid(g.nitems);
+  const int flags = mode & ~3;  // energy sums: every chain but those of the residual-plane mode
   if (askja::m64_supported(g.N)) {
     askja::m64::Grid mg;
     mg.table = b->d_jobs;
@@ -131,6 +132,7 @@ cudaError_t launch_force(askja_batch* b, const askja_batch::Group& g, cudaStream
     mg.ctas = g.nitems;
     return askja::m64::link(g.N, sizeof(T) == 8, askja::m64::Job{}, mg, b->cur, ks, mode, st);
   }
+  mode &= 3;
   if (g.N == 2 || g.N == 3 || g.N == 4) {
     int maxd = 1;
     for (int c : g.chains) maxd = std::max(maxd, b->desc[c].lat.D);
@@ -154,6 +156,15 @@ cudaError_t launch_force(askja_batch* b, const askja_batch::Group& g, cudaStream
           kb_force_small3f<1><<<grid, blk, 0, st>>>(b->d_desc, g.d_start, g.d_ids, (int)g.chains.size(), b->cur, ks);
         else
           kb_force_small3f<0><<<grid, blk, 0, st>>>(b->d_desc, g.d_start, g.d_ids, (int)g.chains.size(), b->cur, ks);
+        return cudaGetLastError();
+      }
+    }
+    if constexpr (sizeof(T) == 8) {
+      if (flags) {
+        auto k = g.N == 2 ? (mode ? kb_force_sums<2, 1> : kb_force_sums<2, 0>)
+                 : g.N == 3 ? (mode ? kb_force_sums<3, 1> : kb_force_sums<3, 0>)
+                            : (mode ? kb_force_sums<4, 1> : kb_force_sums<4, 0>);
+        k<<<grid, blk, 0, st>>>(b->d_desc, g.d_start, g.d_ids, (int)g.chains.size(), b->cur, ks);
         return cudaGetLastError();
       }
     }
@@ -197,24 +208,27 @@ template <typename T>
 int energies(askja_batch* b, int which) {
   using S2 = typename askja::Storage<T>::type;
   using namespace askja::batch;
-  if (b->n_plaq) {
+  // the two ends of a trajectory: only the chains whose force launches do not sum their energies
+  const bool all = which == 2;
+  if (b->n_plaq && (all || b->any_split)) {
     kb_plaq<S2><<<b->n_plaq, askja::misc::RED_THREADS, 0, b->stream>>>(b->d_desc, b->d_plaq_start, b->nchains, b->cur);
     kb_kinetic<S2><<<b->n_link, askja::misc::RED_THREADS, 0, b->stream>>>(b->d_desc, b->d_link_start, b->nchains);
   }
   askja::m64::Grid mg;
   mg.table = b->d_jobs;
   for (const auto& g : b->groups) {
-    if (!g.n_plaq_items) continue;
+    if (!g.n_plaq_items || !all) continue;
     mg.items = (const int2*)g.d_plaq_item;
     mg.ctas = g.n_plaq_items;
     BCK(askja::m64::plaq(g.N, sizeof(T) == 8, askja::m64::Job{}, mg, b->cur, b->stream));
   }
-  if (b->n_kin_items) {
+  if (b->n_kin_items && all) {
     mg.items = (const int2*)b->d_kin_item;
     mg.ctas = b->n_kin_items;
     BCK(askja::m64::kinetic(sizeof(T) == 8, askja::m64::Job{}, mg, 1, b->stream));
   }
-  kb_energy<<<b->nchains, askja::misc::RED_THREADS, 0, b->stream>>>(b->d_desc, which);
+  if (all || b->any_split)
+    kb_energy<<<b->nchains, askja::misc::RED_THREADS, 0, b->stream>>>(b->d_desc, which);
   BCK(cudaGetLastError());
   return ASKJA_OK;
 }
@@ -239,12 +253,12 @@ int enqueue_trajectory(askja_batch* b, int nsteps) {
   BCK(cudaGetLastError());
   if (int rc = energies<T>(b, 0)) return rc;
   for (int i = 0; i < nsteps; i++) {
-    if (int rc = md_step<T>(b, 1, i == 0 ? 0.5 : 1.0)) return rc;
+    if (int rc = md_step<T>(b, i == 0 ? 1 | askja::SUMS_OLD : 1, i == 0 ? 0.5 : 1.0)) return rc;
     b->cur ^= 1;
   }
-  if (int rc = md_step<T>(b, 0, 0.5)) return rc;
+  if (int rc = md_step<T>(b, askja::SUMS_NEW, 0.5)) return rc;
   if (int rc = energies<T>(b, 1)) return rc;
-  kb_metropolis<<<(b->nchains + 127) / 128, 128, 0, b->stream>>>(b->d_desc, b->nchains);
+  kb_metropolis<<<b->nchains, askja::misc::ENERGY_THREADS, 0, b->stream>>>(b->d_desc);
   kb_accept_copy<<<b->n_copy, 256, 0, b->stream>>>(b->d_desc, b->d_copy_start, b->nchains, b->cur);
   BCK(cudaGetLastError());
   return ASKJA_OK;
@@ -397,6 +411,10 @@ int askja_batch_create(const askja_chain_params* chains, int nchains, int precis
     }
     plaq_start.push_back(plaq_start.back() + (m64 ? 0 : d.plaq_blocks));
     link_start.push_back(link_start.back() + (m64 ? 0 : d.link_blocks));
+    if (m64 || precision == ASKJA_FP64) {
+      d.ctas = askja::sum_ctas(L);
+      if (int rc = dalloc(b, &d.pairs, 4 * (size_t)d.ctas * sizeof(double))) return fail(rc);
+    }
     if (m64) {
       askja::m64::Job& j = jobs[c];
       j = askja::detail::m64_job(L);
@@ -406,6 +424,8 @@ int askja_batch_create(const askja_chain_params* chains, int nchains, int precis
       j.U[1] = d.U[1];
       j.Pin = j.Pout = d.P;
       j.kick = j.dt = d.dt;
+      j.pairs = d.pairs;
+      j.ctas = d.ctas;
       j.plaq_partial = d.partial;
       j.kin_partial = d.partial + 2 * (size_t)d.plaq_blocks;
       for (int t = 0; t < d.link_blocks; t++) {

@@ -33,6 +33,8 @@ struct ChainDev {
   misc::TrajState* st;
   double* sums;     // 8 doubles: [0,1] plaquette t/s, [2..4] link sums
   double* partial;  // this chain's reduction partials
+  double* pairs;    // energy sums of the force CTAs at the two ends of a trajectory, or null
+  int ctas;         // force CTAs of this chain
   int plaq_blocks;  // RED_THREADS-site blocks
   int link_blocks;  // RED_THREADS-link blocks
   long n16;         // field size in 16-byte units
@@ -92,12 +94,12 @@ __device__ __forceinline__ void force_small_item(const ChainDev* __restrict__ de
   using LatRef = typename std::conditional<BYVAL, const Lat, const Lat&>::type;
   LatRef L = sd.lat;
   const int x = tile * 32 + (threadIdx.x & 31);
-  if (x >= L.V) return;
   const S2* U = (const S2*)sd.U[cur];
   S2* P = (S2*)sd.P;
   S2* Uo = (S2*)sd.U[cur ^ 1];
   const T ek = (T)(kick_scale * sd.dt), ed = (T)sd.dt;
   const int order = sd.order, reunit = sd.reunit;
+  if (x >= L.V) return;
   for (int mu = threadIdx.x >> 5; mu < L.D; mu += (blockDim.x >> 5))
     small::force_link<N, T, S2, MODE>(L, U, P, P, Uo, ek, ed, order, reunit, mu, x);
 }
@@ -213,10 +215,26 @@ __global__ void __launch_bounds__(misc::RED_THREADS) kb_kinetic(const ChainDev* 
   if (threadIdx.x == 0) sd.partial[2 * sd.plaq_blocks + blk] = v[0];
 }
 
+// FP64 thread-per-link chains at the two ends of a trajectory: the force launch with its CTA's energy sums.
+template <int N, int MODE>
+__global__ void __launch_bounds__(128) kb_force_sums(const ChainDev* __restrict__ descs,
+                                                     const int* __restrict__ item_start,
+                                                     const int* __restrict__ chain_ids, int nchains, int cur,
+                                                     double kick_scale) {
+  __shared__ ChainDev sd;
+  const int tile = load_chain(sd, descs, item_start, chain_ids, nchains);
+  double2* P = (double2*)sd.P;
+  small::force_tile_sums<N, double, double2, MODE>(sd.lat, (const double2*)sd.U[cur], P, P, (double2*)sd.U[cur ^ 1],
+                                                   kick_scale * sd.dt, sd.dt, sd.order, sd.reunit, tile,
+                                                   sd.pairs + 2 * ((size_t)tile + (MODE == 0 ? sd.ctas : 0)));
+}
+
 // One block per chain: sums its partials and, with `which` = 0 / 1, writes
-// H = beta (S + K / (2 NC)) to st->h_old / st->h_new.
+// H = beta (S + K / (2 NC)) to st->h_old / st->h_new (chains whose force
+// launches sum their energies: only which = 2).
 static __global__ void kb_energy(const ChainDev* __restrict__ descs, int which) {
   const ChainDev& d = descs[blockIdx.x];
+  if (which < 2 && d.pairs) return;
   double v[3] = {0.0, 0.0, 0.0};
   for (int b = threadIdx.x; b < d.plaq_blocks; b += blockDim.x) {
     v[0] += d.partial[2 * b];
@@ -236,9 +254,13 @@ static __global__ void kb_energy(const ChainDev* __restrict__ descs, int which) 
   }
 }
 
-static __global__ void kb_metropolis(const ChainDev* __restrict__ descs, int nchains) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c < nchains) misc::metropolis(descs[c].st, descs[c].seed, nullptr, 0);
+// One block per chain: the Metropolis test, with H from the force launches' sums where they have them.
+static __global__ void __launch_bounds__(misc::ENERGY_THREADS) kb_metropolis(const ChainDev* __restrict__ descs) {
+  const ChainDev& d = descs[blockIdx.x];
+  if (d.pairs)
+    misc::energies_and_test(d.pairs, d.ctas, d.lat, d.beta, d.st, d.seed, nullptr, 0);
+  else if (threadIdx.x == 0)
+    misc::metropolis(d.st, d.seed, nullptr, 0);
 }
 
 // Momentum refresh: item = 128 links, or 128 threads of misc::refresh_block for link-major fields.

@@ -194,7 +194,7 @@ cudaError_t force_launch(askja_ctx* c, int mode, int in, int out, double ek, dou
                                 out ? c->P2C : c->PC, out ? c->P2CL : c->PCL, Uo, ULo, ek, ed);
   }
   return c->ks->force(c->lc, mode, cur_u(c), in ? c->P2 : c->P, out ? c->P2 : c->P,
-                      mode == 1 ? c->U[1 - c->cur] : nullptr, ek, ed);
+                      (mode & 3) == 1 ? c->U[1 - c->cur] : nullptr, ek, ed);
 }
 
 // U <- exp(i eps Pi) U (updateUandcopyDown before its copy); the kernels of
@@ -257,6 +257,15 @@ int launch_ok(askja_ctx* c, cudaError_t e, const char* what) {
 // determinant (row-per-thread and FP64-MMA kernels, with rows_ns)
 bool per_update_ns(const askja_ctx* c) { return c->lc.force_rows == 1 || c->N > 4; }
 
+// whether the force kernels at the two ends of a trajectory also sum the
+// energies: FP64 arithmetic (W of the FP32 kernels is too coarse for dH) on all
+// sites (a counted range is a range of plaquette corners, not of links)
+bool sums_energies(const askja_ctx* c) {
+  if (c->split || c->lat.r0 != 0 || (c->lat.r1 != 0 && c->lat.r1 != (int)c->V)) return false;
+  if (askja::m64_supported(c->N)) return c->lc.force_rows == 0 || c->lc.force_rows == 4;
+  return c->p.precision == ASKJA_FP64 && c->lc.force_rows == 0;
+}
+
 bool paired(const askja_ctx* c) { return c->lc.force_rows == 3; }
 
 // Site-pair mapping: the fused kick+drift launches run on the site-pair
@@ -269,12 +278,13 @@ int pair_layout(askja_ctx* c, void* P) {
   return ASKJA_OK;
 }
 
-// n fused kick+drift launches: the first kicks by first_kick, the others by dt
-int fused_steps(askja_ctx* c, int n, double first_kick, double dt) {
+// n fused kick+drift launches: the first kicks by first_kick (with the given
+// mode flags), the others by dt
+int fused_steps(askja_ctx* c, int n, double first_kick, double dt, int first_flags = 0) {
   if (n <= 0) return ASKJA_OK;
   if (int rc = pair_layout(c, c->P)) return rc;
   for (int i = 0; i < n; i++) {
-    KL(force_launch(c, 1, 0, 0, i == 0 ? first_kick : dt, dt), "kick+drift");
+    KL(force_launch(c, i == 0 ? 1 | first_flags : 1, 0, 0, i == 0 ? first_kick : dt, dt), "kick+drift");
     c->cur ^= 1;
   }
   return pair_layout(c, c->P);
@@ -302,24 +312,32 @@ int enqueue_trajectory(askja_ctx* c, int nsteps) {
     KL(c->ks->reunit(lc, cur_u(c)), "reunitarise");
     KL(cudaMemcpyAsync(c->Uconf, cur_u(c), c->field_bytes, cudaMemcpyDeviceToDevice, c->stream), "save links");
   }
+  const bool sums = sums_energies(c);
   {
     Range rh("askja: refresh + H_old");
     KL(refresh_launch(c, c->p.seed, &c->st->traj, 0), "refresh");
-    KL(plaq_launch(c), "plaq");
-    KL(linksums_launch(c, 0, -1, false), "kinetic");
-    askja::misc::k_energy<<<1, 1, 0, c->stream>>>(c->sums, c->p.beta, c->N, &c->st->h_old);
-    KL(cudaGetLastError(), "energy");
+    if (!sums) {
+      KL(plaq_launch(c), "plaq");
+      KL(linksums_launch(c, 0, -1, false), "kinetic");
+      askja::misc::k_energy<<<1, 1, 0, c->stream>>>(c->sums, c->p.beta, c->N, &c->st->h_old);
+      KL(cudaGetLastError(), "energy");
+    }
   }
   {
     Range rl("askja: leapfrog");
-    if (int rc = fused_steps(c, nsteps, 0.5 * dt, dt)) return rc;
+    if (int rc = fused_steps(c, nsteps, 0.5 * dt, dt, sums ? askja::SUMS_OLD : 0)) return rc;
   }
   Range rm("askja: H_new + Metropolis");
-  KL(force_launch(c, 0, 0, 0, 0.5 * dt, 0.0), "kick");
-  KL(plaq_launch(c), "plaq");
-  KL(linksums_launch(c, 0, -1, false), "kinetic");
-  askja::misc::k_energy<<<1, 1, 0, c->stream>>>(c->sums, c->p.beta, c->N, &c->st->h_new);
-  askja::misc::k_metropolis<<<1, 1, 0, c->stream>>>(c->st, c->p.seed, c->logbuf, c->logcap);
+  KL(force_launch(c, sums ? askja::SUMS_NEW : 0, 0, 0, 0.5 * dt, 0.0), "kick");
+  if (sums) {
+    askja::misc::k_energies_metropolis<<<1, askja::misc::ENERGY_THREADS, 0, c->stream>>>(
+        c->partial, askja::sum_ctas(c->lat), c->lat, c->p.beta, c->st, c->p.seed, c->logbuf, c->logcap);
+  } else {
+    KL(plaq_launch(c), "plaq");
+    KL(linksums_launch(c, 0, -1, false), "kinetic");
+    askja::misc::k_energy<<<1, 1, 0, c->stream>>>(c->sums, c->p.beta, c->N, &c->st->h_new);
+    askja::misc::k_metropolis<<<1, 1, 0, c->stream>>>(c->st, c->p.seed, c->logbuf, c->logcap);
+  }
   askja::misc::k_accept_copy<<<4 * 148, 256, 0, c->stream>>>(c->st, (uint4*)cur_u(c), (uint4*)c->Uconf,
                                                              (long)(c->field_bytes / 16));
   if (c->split)
@@ -577,6 +595,7 @@ int askja_create(const askja_params* p, askja_ctx** out) {
   CKC(cudaMalloc(&c->tc_status, sizeof(unsigned)));
   CKC(cudaMemset(c->tc_status, 0, sizeof(unsigned)));
   c->lc.status = c->tc_status;
+  c->lc.pairs = c->partial;
   // untuned default: TF32 tensor cores for FP32 NC = 32 and 64, else thread-per-link for NC <= 4 and the
   // FP64 MMA above; NC = 16 on the TF32 tensor cores is an explicit path and an autotuner candidate
   c->lc.force_rows = p->kernel_path != 0 ? p->kernel_path

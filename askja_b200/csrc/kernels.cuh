@@ -99,6 +99,14 @@ cudaError_t small_force(const LaunchCtx& c, int mode, const void* U, const void*
   const int threads = 32 * std::min(c.lat.D, 4);
   const S2* u = (const S2*)U;
   const S2* pi = (const S2*)Pin;
+  if constexpr (sizeof(T) == 8) {
+    if (mode & (SUMS_OLD | SUMS_NEW)) {
+      auto ks = mode & SUMS_NEW ? small::k_force_sums<N, T, S2, 0> : small::k_force_sums<N, T, S2, 1>;
+      return launch_overlapped(ks, grid, threads, 0, c.stream, c.lat, u, pi, (S2*)Pout, (S2*)Uout, ek, ed, c.order,
+                               c.reunit, c.pairs + (mode & SUMS_NEW ? 2 * (size_t)grid : 0));
+    }
+  }
+  if (mode > 1) return cudaErrorInvalidValue;
   auto k = c.small_occ == 2
                ? (mode == 0 ? small::k_force_occ<N, T, S2, 0, 2> : small::k_force_occ<N, T, S2, 1, 2>)
            : c.small_occ == 1
@@ -137,7 +145,7 @@ cudaError_t m64_link(const LaunchCtx& c, int mode, const void* U, const void* Pi
   m64::Job j = m64_job(c.lat);
   j.order = c.order;
   // FP32 single chains: projected to first order in the kernel (as rows_ns); otherwise in full afterwards
-  const bool ns = sizeof(T) == 4 && c.rows_ns && mode == 1;
+  const bool ns = sizeof(T) == 4 && c.rows_ns && (mode & 3) == 1;
   j.project = c.reunit && ns;
   j.U[0] = const_cast<void*>(U);
   j.U[1] = Uout;
@@ -145,8 +153,10 @@ cudaError_t m64_link(const LaunchCtx& c, int mode, const void* U, const void* Pi
   j.Pout = Pout;
   j.kick = ek;
   j.dt = ed;
+  j.pairs = c.pairs;
+  j.ctas = sum_ctas(c.lat);
   cudaError_t e = m64::link(c.lat.N, sizeof(T) == 8, j, m64::Grid{}, 0, 1.0, mode, c.stream);
-  if (e != cudaSuccess || mode == 0 || !c.reunit || ns) return e;
+  if (e != cudaSuccess || (mode & 3) == 0 || !c.reunit || ns) return e;
   LaunchCtx full = c;
   full.gate = nullptr;
   return reunit<T>(full, Uout);

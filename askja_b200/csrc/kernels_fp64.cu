@@ -17,7 +17,12 @@ size_t partial_doubles(const Lat& L) {
                                          : std::max(2 * (size_t)m64::ctas_for(L.V, m64::sites_per_cta(L.N)),
                                                     3 * (size_t)m64::ctas_for(nl, m64::sites_per_cta(L.N)));
   const size_t fourier = 2 * (size_t)L.n[0];  // FourierTrafo: one plaquette partial per site 0..N0-1
-  return std::max(std::max(std::max(plaq, big), std::max(links, gauss)), fourier) + 64;
+  const size_t pairs = 4 * (size_t)sum_ctas(L);  // energy sums at the two ends of a trajectory
+  return std::max({plaq, big, links, gauss, fourier, pairs}) + 64;
+}
+
+int sum_ctas(const Lat& L) {
+  return m64_supported(L.N) ? m64::ctas_for((long)L.V * L.D, m64::links_per_cta(L.N)) : L.B;
 }
 
 int rows_effective_groups(int N, bool fp64, int want) {

@@ -42,21 +42,20 @@ size_t coef_words(const Lat& L) {
 
 cudaError_t force(const LaunchCtx& c, int mode, const void* U, const void* UL, const void* Pin, const void* PLin,
                   void* Pout, void* PLout, void* Uout, void* ULout, double ek, double ed) {
-  const unsigned grid = blocks_for(c.lat.V, 32);
   const int threads = 32 * std::min(c.lat.D, 4);
   return by_nc(c.lat.N, [&](auto n) {
     constexpr int N = decltype(n)::value;
-    auto launch = [&](auto kern) {
-      return launch_overlapped(kern, grid, threads, 0, c.stream, c.lat, (const float2*)U, (const uint32_t*)UL,
+    auto launch = [&](auto kern, int tiles = 1) {
+      return launch_overlapped(kern, blocks_for(c.lat.V, 32 * tiles), threads * tiles, 0, c.stream, c.lat, (const float2*)U, (const uint32_t*)UL,
                                (const float*)Pin, (const uint32_t*)PLin, (float*)Pout, (uint32_t*)PLout, (float2*)Uout,
                                (uint32_t*)ULout, (float)ek, (float)ed, c.order);
     };
     if (mode == 0) {
-      if (c.small_occ == 2) return launch(split::k_force<N, 0, 2>);
+      if (c.small_occ == 2) return launch(split::k_force<N, 0, 2>, split::Tiles<N, 2>::PER_CTA);
       if (c.small_occ == 1) return launch(split::k_force<N, 0, 1>);
       return launch(split::k_force<N, 0, 0>);
     }
-    if (c.small_occ == 2) return launch(split::k_force<N, 1, 2>);
+    if (c.small_occ == 2) return launch(split::k_force<N, 1, 2>, split::Tiles<N, 2>::PER_CTA);
     if (c.small_occ == 1) return launch(split::k_force<N, 1, 1>);
     return launch(split::k_force<N, 1, 0>);
   });

@@ -51,6 +51,13 @@ cudaError_t launch_overlapped(void (*k)(P...), unsigned grid, unsigned block, si
   return cudaLaunchKernelEx(&cfg, k, static_cast<P>(args)...);
 }
 
+// Flags on the mode of a force launch: each CTA also writes (sum ReTr W, sum
+// tr2 P) of its links -- P before the kick with SUMS_OLD, after it with SUMS_NEW
+// -- to LaunchCtx::pairs, the old pairs first.  W = U S sums every plaquette
+// four times, so the two ends of a trajectory give H without passes of their own
+// over the fields.
+constexpr int SUMS_OLD = 4, SUMS_NEW = 8;
+
 struct LaunchCtx {
   Lat lat;
   cudaStream_t stream;
@@ -65,6 +72,7 @@ struct LaunchCtx {
                     // expects the site-pair layout, see pair_swap)
   int rows_groups;  // row kernels: sites per CTA (0: default 128/NC)
   int small_occ;    // thread-per-link kernels: register budget for 0 default, 1 / 2 more resident CTAs
+  double* pairs;    // energy sums of the CTAs (SUMS_OLD / SUMS_NEW)
   unsigned* status; // tensor-core path: nonzero after a bounded wait gave up
   // row-kernel reunitarisation: run only when *gate % gate_every == 0 (null: always)
   const unsigned long long* gate;
@@ -140,6 +148,9 @@ struct KernelSet {
 
 // size (in doubles) of the partial buffer the reductions need
 size_t partial_doubles(const Lat& L);
+
+// CTAs of a force launch of the kernels that take SUMS_OLD / SUMS_NEW
+int sum_ctas(const Lat& L);
 
 // sites per CTA the row-per-thread kernels actually use for a requested value
 // (0: default), after the thread-count and shared-memory limits

@@ -442,6 +442,73 @@ __device__ __forceinline__ void metropolis(TrajState* st, uint64_t seed, double*
   st->traj++;
 }
 
+// Sums of n pairs by a CTA of ENERGY_THREADS, the same order for a chain alone
+// and in a batch; four running sums a thread keep the loads of the long lists
+// (a pair per CTA of the force launch) in flight.
+constexpr int ENERGY_THREADS = 1024;
+__device__ __forceinline__ void sum_pairs(const double2* __restrict__ p, int n, double (&v)[2]) {
+  __shared__ double2 sh[ENERGY_THREADS / 32];
+  double2 a[4] = {};
+  int i = threadIdx.x;
+  for (; i + 3 * ENERGY_THREADS < n; i += 4 * ENERGY_THREADS)
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const double2 z = p[i + u * ENERGY_THREADS];
+      a[u].x += z.x;
+      a[u].y += z.y;
+    }
+  for (; i < n; i += ENERGY_THREADS) {
+    a[0].x += p[i].x;
+    a[0].y += p[i].y;
+  }
+  double x = (a[0].x + a[1].x) + (a[2].x + a[3].x), y = (a[0].y + a[1].y) + (a[2].y + a[3].y);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    x += __shfl_down_sync(0xffffffffu, x, o);
+    y += __shfl_down_sync(0xffffffffu, y, o);
+  }
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = make_double2(x, y);
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    x = sh[threadIdx.x].x;
+    y = sh[threadIdx.x].y;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      x += __shfl_down_sync(0xffffffffu, x, o);
+      y += __shfl_down_sync(0xffffffffu, y, o);
+    }
+  }
+  v[0] = x;
+  v[1] = y;
+  __syncthreads();
+}
+
+// H from the pairs of a force launch: W = sum ReTr(U S) counts each of the
+// D (D-1) / 2 plaquettes per site four times, K = sum tr2 P.
+__device__ __forceinline__ double energy_of(const double (&v)[2], double beta, const Lat& L) {
+  const double np = 0.5 * L.D * (L.D - 1) * (double)L.V;
+  return beta * ((np - v[0] / (4.0 * L.N)) + v[1] / (2.0 * L.N));
+}
+
+__device__ __forceinline__ void energies_and_test(const double* __restrict__ pairs, int ctas, const Lat& L, double beta,
+                                                  TrajState* st, uint64_t seed, double* __restrict__ log_out,
+                                                  int log_cap) {
+  double a[2], b[2];
+  sum_pairs(reinterpret_cast<const double2*>(pairs), ctas, a);
+  sum_pairs(reinterpret_cast<const double2*>(pairs) + ctas, ctas, b);
+  if (threadIdx.x == 0) {
+    st->h_old = energy_of(a, beta, L);
+    st->h_new = energy_of(b, beta, L);
+    metropolis(st, seed, log_out, log_cap);
+  }
+}
+
+static __global__ void __launch_bounds__(ENERGY_THREADS)
+    k_energies_metropolis(const double* __restrict__ pairs, int ctas, Lat L, double beta, TrajState* st, uint64_t seed,
+                          double* __restrict__ log_out, int log_cap) {
+  energies_and_test(pairs, ctas, L, beta, st, seed, log_out, log_cap);
+}
+
 static __global__ void k_metropolis(TrajState* st, uint64_t seed, double* __restrict__ log_out, int log_cap) {
   metropolis(st, seed, log_out, log_cap);
 }

@@ -55,6 +55,8 @@ struct Job {
   void* Pout;
   double kick;  // kick step (times the launch's kick scale)
   double dt;    // drift step
+  double* pairs;  // energy sums of the CTAs (SUMS_OLD, then SUMS_NEW)
+  int ctas;       // CTAs of this job's link launch
   double* plaq_partial;
   double* kin_partial;
 };
@@ -301,7 +303,9 @@ __device__ __forceinline__ double inv_factorial(int k, int order) {
 }
 
 // mode 0: Pout = Pin - kick F(U);  1: the same, and Uout = exp(i dt Pout) U;
-// 2: Uout = exp(i dt Pin) U.
+// 2: Uout = exp(i dt Pin) U.  SUMS (mode 0, 1): v += (ReTr W, ReTr P P) of own
+// rows, P after a kick alone (the end of a trajectory), before a kick and drift
+// (its start).
 //
 // The exponential is the Taylor sum by Paterson-Stockmeyer in blocks of three
 // terms (X^2, X^3, then Horner in X^3: 5 products for order 8, 4 for order 6,
@@ -311,32 +315,13 @@ __device__ __forceinline__ double inv_factorial(int k, int order) {
 // Newton-Schulz step on the links as read; it differs from projecting first by
 // |E - 1| times the defect that the FP32 store left, which the next update
 // removes in turn.
-template <int NT, bool FULL, typename S2>
-__global__ void __launch_bounds__(Cta<NT>::THREADS, Cta<NT>::MIN_CTAS)
-    k_link(const __grid_constant__ Job one, const Job* __restrict__ table, const int2* __restrict__ items, int cur,
-           double kick_scale, int mode) {
-  grid_wait();
-  extern __shared__ __align__(16) unsigned char smem_raw[];
+template <int NT, bool FULL, typename S2, bool SUMS>
+__device__ __forceinline__ void update_link(const Job& job, int idx, const Who<NT, FULL>& me, int slot, int cur,
+                                            double kick_scale, int mode, double2* S, double (&v)[2]) {
   using CT = Cta<NT>;
   constexpr int KU = NT <= 4 ? NT : 1;  // left operands from memory: the k loop stays rolled for large NC
-  const Job* __restrict__ jp = &one;
-  int blk = blockIdx.x;
-  if (table) {
-    const int2 it = __ldg(items + blk);
-    jp = table + it.x;
-    blk = it.y;
-  }
-  const Job& job = *jp;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int slot = wid / NT;
+  const int lane = threadIdx.x & 31;
   const int V = job.V, D = job.D;
-  Who<NT, FULL> me;
-  me.w = wid - slot * NT;
-  me.q = lane >> 2;
-  me.j = lane & 3;
-  me.n = job.N;
-  const int idx = blk * CT::LINKS + slot;
-  if (idx >= V * D) return;  // whole links: no barrier is left waiting
   const int x = idx / D, mu = idx - x * D;
   const size_t NN = FULL ? (size_t)64 * NT * NT : (size_t)me.n * me.n;
   const S2* __restrict__ U = static_cast<const S2*>(job.U[cur]);
@@ -344,11 +329,34 @@ __global__ void __launch_bounds__(Cta<NT>::THREADS, Cta<NT>::MIN_CTAS)
   auto link = [&](int d, int s) { return U + ((size_t)d * V + s) * NN; };
   const size_t own = ((size_t)mu * V + x) * NN;
   const S2* Ux = U + own;
-  double2* S = reinterpret_cast<double2*>(smem_raw) + slot * (CT::TILES * CT::TILE);
   const int r = 8 * me.w + me.q;
   Acc X[NT];  // rows of X = i dt P
 
+  // ReTr(P P) of own rows, through the tile
+  auto kinetic = [&](const S2* P) {
+    Op p[2], q[2];
+#pragma unroll
+    for (int t = 0; t < NT; t++) {
+      me.own(P, t, p);
+#pragma unroll
+      for (int e = 0; e < 2; e++) S[r * CT::LD + 8 * t + 2 * me.j + e] = make_double2(p[e].re, p[e].im);
+    }
+    link_sync<NT>(slot);
+#pragma unroll
+    for (int t = 0; t < NT; t++) {
+      me.own(P, t, p);
+      tile_cols(S, me, t, me.w, q);
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        v[1] = fma(p[e].re, q[e].re, v[1]);
+        v[1] = fma(-p[e].im, q[e].im, v[1]);
+      }
+    }
+    link_sync<NT>(slot);
+  };
+
   if (mode != 2) {
+    if (SUMS && mode == 1) kinetic(static_cast<const S2*>(job.Pin) + own);
     Acc W[NT];  // the staple sum S first
     zero(W);
     // lane nu fetches the neighbours of plane nu, all planes at once (D <= 16)
@@ -423,8 +431,15 @@ __global__ void __launch_bounds__(Cta<NT>::THREADS, Cta<NT>::MIN_CTAS)
       }
       me.put(Po, t, p);
     }
-    if (mode == 0) return;
+    if (SUMS) {
+#pragma unroll
+      for (int t = 0; t < NT; t++)
+#pragma unroll
+        for (int e = 0; e < 2; e++) v[0] += r == 8 * t + 2 * me.j + e ? W[t].re[e] : 0.0;
+    }
     link_sync<NT>(slot);
+    if (SUMS && mode == 0) kinetic(Po);
+    if (mode == 0) return;
   } else {
     const S2* P = static_cast<const S2*>(job.Pin) + own;
     const double ed = job.dt;
@@ -573,6 +588,42 @@ __global__ void __launch_bounds__(Cta<NT>::THREADS, Cta<NT>::MIN_CTAS)
       [&](int kb, int t, Op(&o)[2]) { me.cols(Ux, kb, t, o); });
   grid_done();
   store_rows(static_cast<S2*>(job.U[cur ^ 1]) + own, me, Y);
+}
+
+template <int NT, bool FULL, typename S2, bool SUMS>
+__global__ void __launch_bounds__(Cta<NT>::THREADS, Cta<NT>::MIN_CTAS)
+    k_link(const __grid_constant__ Job one, const Job* __restrict__ table, const int2* __restrict__ items, int cur,
+           double kick_scale, int mode) {
+  grid_wait();
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const Job* __restrict__ jp = &one;
+  int blk = blockIdx.x;
+  if (table) {
+    const int2 it = __ldg(items + blk);
+    jp = table + it.x;
+    blk = it.y;
+  }
+  const Job& job = *jp;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int slot = wid / NT;
+  Who<NT, FULL> me;
+  me.w = wid - slot * NT;
+  me.q = lane >> 2;
+  me.j = lane & 3;
+  me.n = job.N;
+  const int idx = blk * Cta<NT>::LINKS + slot;
+  double2* S = reinterpret_cast<double2*>(smem_raw) + slot * (Cta<NT>::TILES * Cta<NT>::TILE);
+  double v[2] = {0.0, 0.0};
+  // whole links: no barrier of a link is left waiting
+  if (idx < job.V * job.D) update_link<NT, FULL, S2, SUMS>(job, idx, me, slot, cur, kick_scale, mode, S, v);
+  if constexpr (SUMS) {
+    misc::block_sum<2>(v);
+    if (threadIdx.x == 0) {
+      double* p = job.pairs + 2 * ((size_t)blk + (mode == 0 ? job.ctas : 0));
+      p[0] = v[0];
+      p[1] = v[1];
+    }
+  }
 }
 
 // Plaquette sums, NT warps per site: Re sum_ij (AB)_ij conj((DC)_ij) of every

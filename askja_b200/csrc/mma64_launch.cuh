@@ -13,7 +13,9 @@ namespace m64 {
 
 template <int NT, bool FULL, typename S2>
 cudaError_t launch_link(const Job& one, const Grid& g, int cur, double ks, int mode, cudaStream_t st) {
-  auto k = k_link<NT, FULL, S2>;
+  const bool sums = mode & (SUMS_OLD | SUMS_NEW);
+  mode &= 3;
+  auto k = sums ? k_link<NT, FULL, S2, true> : k_link<NT, FULL, S2, false>;
   const size_t smem = Cta<NT>::SMEM;
   if (smem > 48 * 1024) {
     const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

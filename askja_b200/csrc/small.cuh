@@ -17,6 +17,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "misc.cuh"
 
 namespace askja {
 namespace small {
@@ -231,6 +232,20 @@ __device__ __forceinline__ void staple_sum(Mat<N, T>& acc, const S2* __restrict_
       mac_nn(acc, T1, A);
     }
   }
+}
+
+// ReTr(P P)
+template <int N, typename T>
+__device__ __forceinline__ double tr2(const Mat<N, T>& P) {
+  double a = 0.0;
+#pragma unroll
+  for (int i = 0; i < N; i++)
+#pragma unroll
+    for (int j = 0; j < N; j++) {
+      a = fma((double)P.a[i][j].re, (double)P.a[j][i].re, a);
+      a = fma(-(double)P.a[i][j].im, (double)P.a[j][i].im, a);
+    }
+  return a;
 }
 
 // P <- P - eps * Adjoint(W), Adjoint(W) = -i/2 [(W - W^dag) - Tr(W - W^dag)/N]
@@ -740,14 +755,20 @@ __device__ __forceinline__ void reunitarise(Mat<N, T>& M) {
 template <int N, typename T, typename S2, int MODE>
 __device__ __forceinline__ void force_link(const Lat& L, const S2* __restrict__ U, const S2* Pin, S2* Pout,
                                            S2* __restrict__ Uout, T eps_k, T eps_d, int order, int reunit, int mu,
-                                           int x) {
+                                           int x, double* sums = nullptr) {
   Mat<N, T> acc, Ux, W;
   staple_sum<N, T, S2>(acc, U, L, mu, x);
   load(Ux, U, L, mu, x);
   mul_nn(W, Ux, acc);
   Mat<N, T> P;
   load(P, Pin, L, mu, x);
+  if (sums && MODE == 1) sums[1] += tr2(P);
   kick_ta(P, W, eps_k);
+  if (sums) {
+    if (MODE == 0) sums[1] += tr2(P);
+#pragma unroll
+    for (int k = 0; k < N; k++) sums[0] += W.a[k][k].re;
+  }
   store(Pout, P, L, mu, x);
   if (MODE == 1) {
     Mat<N, T> Tm;
@@ -767,6 +788,32 @@ __global__ void __launch_bounds__(128) k_force(Lat L, const S2* __restrict__ U, 
   if (x >= L.V) return;
   for (int mu = threadIdx.x >> 5; mu < L.D; mu += (blockDim.x >> 5)) force_link<N, T, S2, MODE>(
       L, U, Pin, Pout, Uout, eps_k, eps_d, order, reunit, mu, x);
+}
+
+// The same with the energy sums of the CTA's links (launch.h): the two ends of an FP64 trajectory.
+template <int N, typename T, typename S2, int MODE>
+__device__ __forceinline__ void force_tile_sums(const Lat& L, const S2* __restrict__ U, const S2* Pin, S2* Pout,
+                                                S2* __restrict__ Uout, T eps_k, T eps_d, int order, int reunit,
+                                                int tile, double* pair) {
+  const int x = tile * 32 + (threadIdx.x & 31);
+  double v[2] = {0.0, 0.0};
+  if (x < L.V)
+    for (int mu = threadIdx.x >> 5; mu < L.D; mu += (blockDim.x >> 5))
+      force_link<N, T, S2, MODE>(L, U, Pin, Pout, Uout, eps_k, eps_d, order, reunit, mu, x, v);
+  misc::block_sum<2>(v);
+  if (threadIdx.x == 0) {
+    pair[0] = v[0];
+    pair[1] = v[1];
+  }
+}
+
+template <int N, typename T, typename S2, int MODE>
+__global__ void __launch_bounds__(128) k_force_sums(Lat L, const S2* __restrict__ U, const S2* Pin, S2* Pout,
+                                                    S2* __restrict__ Uout, T eps_k, T eps_d, int order, int reunit,
+                                                    double* __restrict__ pairs) {
+  grid_wait();
+  force_tile_sums<N, T, S2, MODE>(L, U, Pin, Pout, Uout, eps_k, eps_d, order, reunit, blockIdx.x,
+                                  pairs + 2 * (size_t)blockIdx.x);
 }
 
 // The same kernel with a tighter register budget for more resident CTAs

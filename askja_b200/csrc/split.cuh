@@ -496,16 +496,28 @@ __device__ __forceinline__ void link_update(const Lat& L, const float2* __restri
 }
 
 // Register budget: at most 128 registers (4 resident CTAs of 128 threads per
-// SM) for OCC 0, bounded for 6 / 7 resident CTAs for OCC 1 / 2.
+// SM) for OCC 0, bounded for 6 / 7 resident CTAs for OCC 1 / 2.  SU(3) at OCC 2
+// takes two neighbouring tiles in one CTA, three CTAs per SM: 24 warps of 80
+// registers instead of 28 of 72, but links of the two tiles' common
+// neighbourhood hit L1 (32^4 491 -> 480 us per step under the power cap, 24^4
+// 156 -> 147; three tiles and two CTAs the same, seven tiles in one CTA no gain).
+template <int N, int OCC>
+struct Tiles {
+  static constexpr int PER_CTA = N == 3 && OCC == 2 ? 2 : 1;
+  static constexpr int MIN_CTAS = OCC == 0 ? 4 : PER_CTA == 2 ? 3 : 5 + OCC;
+};
 template <int N, int MODE, int OCC>
-__global__ void __launch_bounds__(128, OCC == 0 ? 4 : 5 + OCC)
+__global__ void __launch_bounds__(128 * Tiles<N, OCC>::PER_CTA, Tiles<N, OCC>::MIN_CTAS)
     k_force(Lat L, const float2* __restrict__ U, const uint32_t* __restrict__ UL, const float* Pin,
             const uint32_t* PLin, float* Pout, uint32_t* PLout, float2* __restrict__ Uout,
             uint32_t* __restrict__ ULout, float eps_k, float eps_d, int order) {
   grid_wait();
-  const int x = blockIdx.x * 32 + (threadIdx.x & 31);
+  constexpr int TPC = Tiles<N, OCC>::PER_CTA;
+  const int warps = (blockDim.x >> 5) / TPC, w = threadIdx.x >> 5;  // warps per tile
+  const int t = TPC == 1 ? 0 : w / warps;
+  const int x = (blockIdx.x * TPC + t) * 32 + (threadIdx.x & 31);
   if (x >= L.V) return;
-  for (int mu = threadIdx.x >> 5; mu < L.D; mu += (blockDim.x >> 5))
+  for (int mu = w - t * warps; mu < L.D; mu += warps)
     link_update<N, MODE>(L, U, UL, Pin, PLin, Pout, PLout, Uout, ULout, eps_k, eps_d, order, mu, x);
 }
 
