@@ -225,7 +225,7 @@ int energies(askja_batch* b, int which) {
   if (b->n_kin_items && all) {
     mg.items = (const int2*)b->d_kin_item;
     mg.ctas = b->n_kin_items;
-    BCK(askja::m64::kinetic(sizeof(T) == 8, askja::m64::Job{}, mg, 1, b->stream));
+    BCK(askja::m64::kinetic(sizeof(T) == 8, askja::m64::Job{}, mg, b->stream));
   }
   if (all || b->any_split)
     kb_energy<<<b->nchains, askja::misc::RED_THREADS, 0, b->stream>>>(b->d_desc, which);

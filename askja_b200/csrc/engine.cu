@@ -71,7 +71,7 @@ struct askja_ctx {
   void* Uconf = nullptr;
   int* nbr = nullptr;
   double* partial = nullptr;
-  double* sums = nullptr;   // [0..1] plaq t/s, [2..4] link sums, [5] gauss
+  double* sums = nullptr;   // [0..1] plaq t/s, [2..4] link sums, [5] gauss; last: ticket
   double* lines = nullptr;  // per-line results, behind the sums in the same allocation (SUMS doubles on)
   double2* eigs = nullptr;  // eigenvalues of the N0 + N1 lines of askja_eigenphases, then
   int* eigfail = nullptr;   // their convergence flag, in the same allocation
@@ -197,16 +197,17 @@ cudaError_t force_launch(askja_ctx* c, int mode, int in, int out, double ek, dou
                       (mode & 3) == 1 ? c->U[1 - c->cur] : nullptr, ek, ed);
 }
 
-// U <- exp(i eps Pi) U (updateUandcopyDown before its copy); the kernels of
+// U <- exp(i eps Pi) U and pi <- Pi (updateUandcopyDown); the kernels of
 // link-major fields write the partner buffer, which becomes the current one
 cudaError_t drift_launch(askja_ctx* c, double eps) {
-  if (c->split) return askja::splitk::drift(c->lc, cur_u(c), cur_ul(c), c->P2C, c->P2CL, eps);
+  if (c->split)
+    return askja::splitk::drift(c->lc, cur_u(c), cur_ul(c), c->P2C, c->P2CL, c->PC, c->PCL, eps);
   if (askja::link_major(c->N) && c->lc.force_rows != 1) {
     const cudaError_t e = c->ks->force(c->lc, 2, cur_u(c), c->P2, nullptr, c->U[1 - c->cur], 0.0, eps);
     if (e == cudaSuccess) c->cur ^= 1;
-    return e;
+    return e == cudaSuccess ? copy_down(c) : e;
   }
-  return c->ks->drift(c->lc, cur_u(c), c->P2, eps);
+  return c->ks->drift(c->lc, cur_u(c), c->P2, c->P, eps);
 }
 
 cudaError_t plaq_launch(askja_ctx* c) {
@@ -596,6 +597,8 @@ int askja_create(const askja_params* p, askja_ctx** out) {
   CKC(cudaMemset(c->tc_status, 0, sizeof(unsigned)));
   c->lc.status = c->tc_status;
   c->lc.pairs = c->partial;
+  CKC(cudaMemset(c->sums, 0, SUMS * sizeof(double)));
+  c->lc.ticket = reinterpret_cast<unsigned*>(c->sums + SUMS - 1);
   // untuned default: TF32 tensor cores for FP32 NC = 32 and 64, else thread-per-link for NC <= 4 and the
   // FP64 MMA above; NC = 16 on the TF32 tensor cores is an explicit path and an autotuner candidate
   c->lc.force_rows = p->kernel_path != 0 ? p->kernel_path
@@ -746,7 +749,6 @@ int askja_updateUandcopyDown(askja_ctx* c, double eps) {
   if (int rc = check_ctx(c)) return rc;
   DevGuard g(c->p.device);
   KL(drift_launch(c, eps), "drift");
-  CK(copy_down(c));
   CK(cudaStreamSynchronize(c->stream));
   return ASKJA_OK;
 }
@@ -1037,7 +1039,6 @@ int askja_md_steps(askja_ctx* c, int nsteps, double eps) {
   DevGuard g(c->p.device);
   // D(eps) with Pi, pi = Pi ...
   KL(drift_launch(c, eps), "drift");
-  CK(copy_down(c));
   // ... then (K D) fused, in place on pi ...
   if (int rc = fused_steps(c, nsteps - 1, eps, eps)) return rc;
   // ... and the last kick out of place: Pi = pi - eps F(u)

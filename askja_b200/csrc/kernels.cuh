@@ -107,6 +107,13 @@ cudaError_t small_force(const LaunchCtx& c, int mode, const void* U, const void*
     }
   }
   if (mode > 1) return cudaErrorInvalidValue;
+  if constexpr (sizeof(T) == 8 && N <= 3) {
+    if (c.small_occ == 0 && small::force_ahead(N, c.lat.V)) {
+      auto ka = mode == 0 ? small::k_force_ahead<N, T, S2, 0> : small::k_force_ahead<N, T, S2, 1>;
+      return launch_overlapped(ka, grid, threads, 0, c.stream, c.lat, u, pi, (S2*)Pout, (S2*)Uout, ek, ed, c.order,
+                               c.reunit);
+    }
+  }
   auto k = c.small_occ == 2
                ? (mode == 0 ? small::k_force_occ<N, T, S2, 0, 2> : small::k_force_occ<N, T, S2, 1, 2>)
            : c.small_occ == 1
@@ -117,10 +124,10 @@ cudaError_t small_force(const LaunchCtx& c, int mode, const void* U, const void*
 }
 
 template <int N, typename T>
-cudaError_t small_drift(const LaunchCtx& c, void* U, const void* P, double eps) {
+cudaError_t small_drift(const LaunchCtx& c, void* U, const void* P, void* Pcopy, double eps) {
   using S2 = typename Storage<T>::type;
   small::k_drift<N, T, S2><<<blocks_for(nlinks(c.lat), SMALL_THREADS), SMALL_THREADS, 0, c.stream>>>(
-      c.lat, (S2*)U, (const S2*)P, (T)eps, c.order, c.reunit);
+      c.lat, (S2*)U, (const S2*)P, (S2*)Pcopy, (T)eps, c.order, c.reunit);
   return cudaGetLastError();
 }
 
@@ -261,13 +268,15 @@ cudaError_t force(const LaunchCtx& c, int mode, const void* U, const void* Pin, 
 }
 
 template <typename T>
-cudaError_t drift(const LaunchCtx& c, void* U, const void* P, double eps) {
+cudaError_t drift(const LaunchCtx& c, void* U, const void* P, void* Pcopy, double eps) {
   const int N = c.lat.N;
   if (c.force_rows != 1) {
-    if (N == 2) return small_drift<2, T>(c, U, P, eps);
-    if (N == 3) return small_drift<3, T>(c, U, P, eps);
-    if (N == 4) return small_drift<4, T>(c, U, P, eps);
+    if (N == 2) return small_drift<2, T>(c, U, P, Pcopy, eps);
+    if (N == 3) return small_drift<3, T>(c, U, P, Pcopy, eps);
+    if (N == 4) return small_drift<4, T>(c, U, P, Pcopy, eps);
   }
+  const cudaError_t e = cudaMemcpyAsync(Pcopy, P, field_elems(c.lat) * sizeof(cpx<T>), cudaMemcpyDeviceToDevice, c.stream);
+  if (e != cudaSuccess) return e;
   if (N <= 8) return rows_drift<8, T>(c, U, P, eps);
   if (N <= 16) return rows_drift<16, T>(c, U, P, eps);
   if (N <= 32) return rows_drift<32, T>(c, U, P, eps);
@@ -312,20 +321,17 @@ cudaError_t plaq(const LaunchCtx& c, const void* U, double* partial, double* out
     m64::Job j = m64_job(c.lat);
     j.U[0] = const_cast<void*>(U);
     j.plaq_partial = partial;
-    const cudaError_t e = m64::plaq(N, sizeof(T) == 8, j, m64::Grid{}, 0, c.stream);
-    if (e != cudaSuccess) return e;
-    misc::k_finish<2><<<1, misc::RED_THREADS, 0, c.stream>>>(partial, m64::ctas_for(c.lat.V, m64::sites_per_cta(N)),
-                                                             out);
-    return cudaGetLastError();
+    j.out = out;
+    j.ticket = c.ticket;
+    return m64::plaq(N, sizeof(T) == 8, j, m64::Grid{}, 0, c.stream);
   }
   const unsigned nb = blocks_for(c.lat.V, misc::RED_THREADS);
   if (N == 2)
-    misc::k_plaq<2, S2><<<nb, misc::RED_THREADS, 0, c.stream>>>(c.lat, (const S2*)U, partial);
+    misc::k_plaq<2, S2><<<nb, misc::RED_THREADS, 0, c.stream>>>(c.lat, (const S2*)U, partial, out, c.ticket);
   else if (N == 3)
-    misc::k_plaq<3, S2><<<nb, misc::RED_THREADS, 0, c.stream>>>(c.lat, (const S2*)U, partial);
+    misc::k_plaq<3, S2><<<nb, misc::RED_THREADS, 0, c.stream>>>(c.lat, (const S2*)U, partial, out, c.ticket);
   else
-    misc::k_plaq<4, S2><<<nb, misc::RED_THREADS, 0, c.stream>>>(c.lat, (const S2*)U, partial);
-  misc::k_finish<2><<<1, misc::RED_THREADS, 0, c.stream>>>(partial, (int)nb, out);
+    misc::k_plaq<4, S2><<<nb, misc::RED_THREADS, 0, c.stream>>>(c.lat, (const S2*)U, partial, out, c.ticket);
   return cudaGetLastError();
 }
 
@@ -339,31 +345,22 @@ cudaError_t linksums(const LaunchCtx& c, const void* Pa, const void* Pb, const v
     j.Pin = Pa;
     j.Pin2 = Pb;
     j.kin_partial = partial;
+    j.out = out;
+    j.ticket = c.ticket;
     const bool fp64 = sizeof(T) == 8;
-    int n = m64::ctas_for(nlinks(c.lat), m64::sites_per_cta(N));
     if (U && Pa) return cudaErrorInvalidValue;  // one sum per call
-    cudaError_t e = cudaSuccess;
-    if (U) {
-      e = m64::uviol(N, fp64, j, c.stream);
-    } else {
-      n = m64::ctas_for(nlinks(c.lat), m64::kinetic_links_per_cta(N));
-      e = m64::kinetic(fp64, j, m64::Grid{}, 3, c.stream);
-    }
-    if (e != cudaSuccess) return e;
-    misc::k_finish<3><<<1, misc::RED_THREADS, 0, c.stream>>>(partial, n, out);
-    return cudaGetLastError();
+    return U ? m64::uviol(N, fp64, j, c.stream) : m64::kinetic(fp64, j, m64::Grid{}, c.stream);
   }
   const unsigned nb = blocks_for(nlinks(c.lat), misc::RED_THREADS);
   if (N == 2)
     misc::k_linksums<2, S2><<<nb, misc::RED_THREADS, 0, c.stream>>>(c.lat, (const S2*)Pa, (const S2*)Pb,
-                                                                    (const S2*)U, partial);
+                                                                    (const S2*)U, partial, out, c.ticket);
   else if (N == 3)
     misc::k_linksums<3, S2><<<nb, misc::RED_THREADS, 0, c.stream>>>(c.lat, (const S2*)Pa, (const S2*)Pb,
-                                                                    (const S2*)U, partial);
+                                                                    (const S2*)U, partial, out, c.ticket);
   else
     misc::k_linksums<4, S2><<<nb, misc::RED_THREADS, 0, c.stream>>>(c.lat, (const S2*)Pa, (const S2*)Pb,
-                                                                    (const S2*)U, partial);
-  misc::k_finish<3><<<1, misc::RED_THREADS, 0, c.stream>>>(partial, (int)nb, out);
+                                                                    (const S2*)U, partial, out, c.ticket);
   return cudaGetLastError();
 }
 

@@ -61,11 +61,13 @@ cudaError_t force(const LaunchCtx& c, int mode, const void* U, const void* UL, c
   });
 }
 
-cudaError_t drift(const LaunchCtx& c, void* U, void* UL, const void* P, const void* PL, double eps) {
+cudaError_t drift(const LaunchCtx& c, void* U, void* UL, const void* P, const void* PL, void* Pcopy, void* PLcopy,
+                  double eps) {
   return by_nc(c.lat.N, [&](auto n) {
     constexpr int N = decltype(n)::value;
     split::k_drift<N><<<blocks_for(nlinks(c.lat), THREADS), THREADS, 0, c.stream>>>(
-        c.lat, (float2*)U, (uint32_t*)UL, (const float*)P, (const uint32_t*)PL, (float)eps, c.order);
+        c.lat, (float2*)U, (uint32_t*)UL, (const float*)P, (const uint32_t*)PL, (float*)Pcopy, (uint32_t*)PLcopy,
+        (float)eps, c.order);
     return cudaGetLastError();
   });
 }
@@ -83,8 +85,8 @@ cudaError_t plaq(const LaunchCtx& c, const void* U, const void* UL, double* part
   const unsigned nb = blocks_for(c.lat.V, misc::RED_THREADS);
   return by_nc(c.lat.N, [&](auto n) {
     constexpr int N = decltype(n)::value;
-    split::k_plaq<N><<<nb, misc::RED_THREADS, 0, c.stream>>>(c.lat, (const float2*)U, (const uint32_t*)UL, partial);
-    misc::k_finish<2><<<1, misc::RED_THREADS, 0, c.stream>>>(partial, (int)nb, out);
+    split::k_plaq<N><<<nb, misc::RED_THREADS, 0, c.stream>>>(c.lat, (const float2*)U, (const uint32_t*)UL, partial,
+                                                                 out, c.ticket);
     return cudaGetLastError();
   });
 }
@@ -96,8 +98,7 @@ cudaError_t linksums(const LaunchCtx& c, const void* Pa, const void* PLa, const 
     constexpr int N = decltype(n)::value;
     split::k_linksums<N><<<nb, misc::RED_THREADS, 0, c.stream>>>(
         c.lat, (const float*)Pa, (const uint32_t*)PLa, (const float*)Pb, (const uint32_t*)PLb, (const float2*)U,
-        (const uint32_t*)UL, partial);
-    misc::k_finish<3><<<1, misc::RED_THREADS, 0, c.stream>>>(partial, (int)nb, out);
+        (const uint32_t*)UL, partial, out, c.ticket);
     return cudaGetLastError();
   });
 }

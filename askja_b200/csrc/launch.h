@@ -72,6 +72,7 @@ struct LaunchCtx {
                     // expects the site-pair layout, see pair_swap)
   int rows_groups;  // row kernels: sites per CTA (0: default 128/NC)
   int small_occ;    // thread-per-link kernels: register budget for 0 default, 1 / 2 more resident CTAs
+  unsigned* ticket; // zero between reductions (misc::publish)
   double* pairs;    // energy sums of the CTAs (SUMS_OLD / SUMS_NEW)
   unsigned* status; // tensor-core path: nonzero after a bounded wait gave up
   // row-kernel reunitarisation: run only when *gate % gate_every == 0 (null: always)
@@ -118,7 +119,8 @@ struct KernelSet {
   // mode 2 (FP64 MMA and tensor cores): Uout = exp(i ed Pin) U
   cudaError_t (*force)(const LaunchCtx&, int mode, const void* U, const void* Pin, void* Pout, void* Uout, double ek,
                        double ed);
-  cudaError_t (*drift)(const LaunchCtx&, void* U, const void* P, double eps);
+  // U = exp(i eps P) U in place and Pcopy = P
+  cudaError_t (*drift)(const LaunchCtx&, void* U, const void* P, void* Pcopy, double eps);
   cudaError_t (*reunit)(const LaunchCtx&, void* U);
   cudaError_t (*plaq)(const LaunchCtx&, const void* U, double* partial, double* out);
   cudaError_t (*linksums)(const LaunchCtx&, const void* Pa, const void* Pb, const void* U, double* partial,

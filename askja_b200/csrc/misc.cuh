@@ -55,6 +55,38 @@ __global__ void k_finish(const double* __restrict__ partial, int nblocks, double
     for (int k = 0; k < K; k++) out[k] = v[k];
 }
 
+// Writes this block's K sums (in thread 0) to the partials and lets the last
+// block to do so add them up, in block order whatever the finishing order, into
+// out (not null): no launch of its own for the total.  *ticket counts the
+// blocks, zero before and after.
+template <int K>
+__device__ __forceinline__ void publish(const double (&v)[K], double* __restrict__ partial, double* __restrict__ out,
+                                        unsigned* ticket) {
+  __shared__ bool last;
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int k = 0; k < K; k++) partial[(size_t)blockIdx.x * K + k] = v[k];
+    __threadfence();
+    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  double s[K];
+#pragma unroll
+  for (int k = 0; k < K; k++) s[k] = 0.0;
+#pragma unroll 8
+  for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x)
+#pragma unroll
+    for (int k = 0; k < K; k++) s[k] += __ldcg(partial + (size_t)b * K + k);
+  block_sum<K>(s);
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int k = 0; k < K; k++) out[k] = s[k];
+    *ticket = 0;
+  }
+}
+
 // Plaquette sums per site (sun.cpp:507-537 EnergyMag; measurements4d.cpp:885-927
 // PlaqExp).  partial[b*2 + 0] = temporal planes (0,k), [b*2+1] = spatial (j,k), j>=1.
 // ReTr(A B C^dag D^dag) is evaluated as Re sum_ij (AB)_ij conj((DC)_ij).
@@ -88,14 +120,12 @@ __device__ __forceinline__ void plaq_site(const Lat& L, const S2* __restrict__ U
 }
 
 template <int NT, typename S2>
-__global__ void __launch_bounds__(RED_THREADS) k_plaq(Lat L, const S2* __restrict__ U, double* __restrict__ partial) {
+__global__ void __launch_bounds__(RED_THREADS) k_plaq(Lat L, const S2* __restrict__ U, double* __restrict__ partial,
+                                                      double* __restrict__ out, unsigned* ticket) {
   double v[2] = {0.0, 0.0};
   plaq_site<NT, S2>(L, U, blockIdx.x * blockDim.x + threadIdx.x, v);
   block_sum<2>(v);
-  if (threadIdx.x == 0) {
-    partial[blockIdx.x * 2 + 0] = v[0];
-    partial[blockIdx.x * 2 + 1] = v[1];
-  }
+  publish<2>(v, partial, out, ticket);
 }
 
 // Per-link sums: [0] = sum ReTr(A A) for A = Pa (sun.cpp:540-548 simpleenergyEl),
@@ -154,13 +184,12 @@ __device__ __forceinline__ void link_sums(const Lat& L, const S2* __restrict__ P
 
 template <int NT, typename S2>
 __global__ void __launch_bounds__(RED_THREADS) k_linksums(Lat L, const S2* __restrict__ Pa, const S2* __restrict__ Pb,
-                                                          const S2* __restrict__ U, double* __restrict__ partial) {
+                                                          const S2* __restrict__ U, double* __restrict__ partial,
+                                                          double* __restrict__ out, unsigned* ticket) {
   double v[3] = {0.0, 0.0, 0.0};
   link_sums<NT, S2>(L, Pa, Pb, U, (long)blockIdx.x * blockDim.x + threadIdx.x, v);
   block_sum<3>(v);
-  if (threadIdx.x == 0)
-#pragma unroll
-    for (int k = 0; k < 3; k++) partial[blockIdx.x * 3 + k] = v[k];
+  publish<3>(v, partial, out, ticket);
 }
 
 // Slice averages for measurements4d.cpp:357-408 scalarLoopcorr:

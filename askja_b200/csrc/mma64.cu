@@ -59,12 +59,12 @@ cudaError_t lines(bool fp64, const Lat& L, const void* U, const LineSet& ls, dou
   return (fp64 ? lines_part64 : lines_part32)(NT, L, U, ls, out, ev, fail, st);
 }
 
-cudaError_t kinetic(bool fp64, const Job& one, const Grid& g, int stride, cudaStream_t st) {
+cudaError_t kinetic(bool fp64, const Job& one, const Grid& g, cudaStream_t st) {
   const int ctas = g.table ? g.ctas : ctas_for((long)one.V * one.D, kin_links(one.N));
   if (fp64)
-    k_kinetic<double2><<<ctas, misc::RED_THREADS, 0, st>>>(one, g.table, g.items, stride);
+    k_kinetic<double2><<<ctas, misc::RED_THREADS, 0, st>>>(one, g.table, g.items);
   else
-    k_kinetic<float2><<<ctas, misc::RED_THREADS, 0, st>>>(one, g.table, g.items, stride);
+    k_kinetic<float2><<<ctas, misc::RED_THREADS, 0, st>>>(one, g.table, g.items);
   return cudaGetLastError();
 }
 

@@ -59,6 +59,8 @@ struct Job {
   int ctas;       // CTAs of this job's link launch
   double* plaq_partial;
   double* kin_partial;
+  double* out;       // totals of a reduction launched for one lattice (misc::publish)
+  unsigned* ticket;
 };
 
 // CTA shapes.  Link update: four warps a CTA (one link from NT = 3 on) at the
@@ -688,7 +690,9 @@ __global__ void __launch_bounds__(Cta<NT>::PLAQ_THREADS)
     }
   }
   misc::block_sum<2>(v);
-  if (threadIdx.x == 0) {
+  if (!table) {
+    misc::publish<2>(v, job.plaq_partial, job.out, job.ticket);
+  } else if (threadIdx.x == 0) {
     job.plaq_partial[2 * (size_t)blk + 0] = v[0];
     job.plaq_partial[2 * (size_t)blk + 1] = v[1];
   }
@@ -697,7 +701,8 @@ __global__ void __launch_bounds__(Cta<NT>::PLAQ_THREADS)
 // Kinetic sums sum ReTr(P P) and, with Pin2, sum ReTr((P + P2)^2) / 4: a warp takes 8 x 8 tiles of a link's matrix, each
 // with its mirror tile in the column pattern (whole sectors, where element pairs
 // read a row length apart took 365 us for SU(64) 4x8x16 on 24 CTAs);
-// KIN_TILES tiles per CTA, whole links; kin_partial[stride * blk].
+// KIN_TILES tiles per CTA, whole links; three sums per CTA and their totals for
+// one lattice, kin_partial[blk] in a batch.
 constexpr int KIN_TILES = 64;
 __host__ __device__ inline int kin_links(int N) {
   const int nt = (N + 7) / 8;
@@ -705,8 +710,7 @@ __host__ __device__ inline int kin_links(int N) {
 }
 template <typename S2>
 __global__ void __launch_bounds__(misc::RED_THREADS)
-    k_kinetic(const __grid_constant__ Job one, const Job* __restrict__ table, const int2* __restrict__ items,
-              int stride) {
+    k_kinetic(const __grid_constant__ Job one, const Job* __restrict__ table, const int2* __restrict__ items) {
   const Job* __restrict__ jp = &one;
   int blk = blockIdx.x;
   if (table) {
@@ -753,17 +757,16 @@ __global__ void __launch_bounds__(misc::RED_THREADS)
     }
   }
   misc::block_sum<2>(v);
-  if (threadIdx.x == 0) {  // stride 3: [P P, (P + P2)^2 / 4, no unitarity sum]
-    job.kin_partial[(size_t)stride * blk] = v[0];
-    if (stride == 3) {
-      job.kin_partial[(size_t)stride * blk + 1] = 0.25 * v[1];
-      job.kin_partial[(size_t)stride * blk + 2] = 0.0;
-    }
+  if (!table) {
+    const double w[3] = {v[0], 0.25 * v[1], 0.0};
+    misc::publish<3>(w, job.kin_partial, job.out, job.ticket);
+  } else if (threadIdx.x == 0) {
+    job.kin_partial[blk] = v[0];
   }
 }
 
 // UViol (sun.cpp:441-471): sum ReTr((U U^dag - 1)^2), the matrix Hermitian, so
-// the sum of its squared moduli; SITES links per CTA, partial[3 blk + 2].
+// the sum of its squared moduli; SITES links per CTA.
 template <int NT, bool FULL, typename S2>
 __global__ void __launch_bounds__(Cta<NT>::PLAQ_THREADS) k_uviol(const __grid_constant__ Job job) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -794,11 +797,8 @@ __global__ void __launch_bounds__(Cta<NT>::PLAQ_THREADS) k_uviol(const __grid_co
       }
   }
   misc::block_sum<1>(v);
-  if (threadIdx.x == 0) {
-    double* p = job.kin_partial + 3 * (size_t)blockIdx.x;
-    p[0] = p[1] = 0.0;
-    p[2] = v[0];
-  }
+  const double w[3] = {0.0, 0.0, v[0]};
+  misc::publish<3>(w, job.kin_partial, job.out, job.ticket);
 }
 
 // Gauss law: sum over the links of Pi - U^dag Pi U (lines.cuh), NT warps per

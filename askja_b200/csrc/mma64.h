@@ -33,7 +33,7 @@ inline int ctas_for(long n, int per) { return (int)((n + per - 1) / per); }
 cudaError_t link(int N, bool fp64, const Job& one, const Grid& g, int cur, double kick_scale, int mode,
                  cudaStream_t stream);
 cudaError_t plaq(int N, bool fp64, const Job& one, const Grid& g, int cur, cudaStream_t stream);
-// unitarity sums of U[0] at kin_partial[3 * block + 2] (sites_per_cta links a block)
+// unitarity sum of U[0]
 cudaError_t uviol(int N, bool fp64, const Job& one, cudaStream_t stream);
 // Gauss-law matrices of `groups` groups of links of U[0] and Pin, at kin_partial
 int gauss_groups(int N, long nlinks);
@@ -41,8 +41,8 @@ cudaError_t gauss(int N, bool fp64, const Job& one, cudaStream_t stream);
 // |Tr| / NC of the lines (out) or their eigenvalues (ev, fail)
 cudaError_t lines(bool fp64, const Lat& L, const void* U, const LineSet& ls, double* out, double2* ev, int* fail,
                   cudaStream_t stream);
-// kinetic sums of Pin (and Pin2) at kin_partial[stride * block]; every colour number in one launch
-cudaError_t kinetic(bool fp64, const Job& one, const Grid& g, int stride, cudaStream_t stream);
+// kinetic sums of Pin (and Pin2); every colour number in one launch
+cudaError_t kinetic(bool fp64, const Job& one, const Grid& g, cudaStream_t stream);
 
 }  // namespace m64
 }  // namespace askja

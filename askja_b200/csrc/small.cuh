@@ -203,11 +203,45 @@ __device__ __forceinline__ void su3_third_row(Mat<3, T>& M) {
 // SU(3), so its third row is taken as conj(r0 x r1) (24 instead of 36 real
 // multiply-adds; exact for links in SU(3), which the FP32 path keeps by
 // reunitarising every update).
-template <int N, typename T, typename S2>
+// AHEAD: the next staple's links are loaded while this one is multiplied (the
+// same operations in the same order), for FP64 kernels with registers to spare
+// (see force_ahead).
+template <int N, typename T, typename S2, bool AHEAD = false>
 __device__ __forceinline__ void staple_sum(Mat<N, T>& acc, const S2* __restrict__ U, const Lat& L, int mu, int x) {
   constexpr bool R2 = N == 3 && sizeof(T) == 4;
   zero(acc);
   const int xpmu = nb_plus(L, mu, x);
+  if constexpr (AHEAD) {
+    if (L.D < 2) return;
+    int nu = mu == 0 ? 1 : 0;
+    int xmnu = nb_minus(L, nu, x), xpmu_mnu = nb_minus(L, nu, xpmu);
+    Mat<N, T> A, B, C, T1;
+    load(A, U, L, nu, xpmu);
+    load(B, U, L, mu, nb_plus(L, nu, x));
+    load(C, U, L, nu, x);
+    for (;;) {
+      const int next = nu + 1 + (nu + 1 == mu);
+      const bool more = next < L.D;
+      const int ni = more ? next : nu;
+      const int xpnu2 = nb_plus(L, ni, x), xmnu2 = nb_minus(L, ni, x), xpmu_mnu2 = nb_minus(L, ni, xpmu);
+      mul_nd(T1, A, B);
+      load(A, U, L, nu, xpmu_mnu);
+      load(B, U, L, mu, xmnu);
+      mac_nd(acc, T1, C);
+      load(C, U, L, nu, xmnu);
+      mul_dd(T1, A, B);
+      if (more) {
+        load(A, U, L, next, xpmu);
+        load(B, U, L, mu, xpnu2);
+      }
+      mac_nn(acc, T1, C);
+      if (!more) return;
+      load(C, U, L, next, x);
+      nu = next;
+      xmnu = xmnu2;
+      xpmu_mnu = xpmu_mnu2;
+    }
+  }
   for (int nu = 0; nu < L.D; nu++) {
     if (nu == mu) continue;
     const int xpnu = nb_plus(L, nu, x);
@@ -752,12 +786,12 @@ __device__ __forceinline__ void reunitarise(Mat<N, T>& M) {
 // once and then served from L1/L2 to the other warps, instead of being
 // re-fetched in D separate direction sweeps.  Each warp still reads 32
 // consecutive sites per element.
-template <int N, typename T, typename S2, int MODE>
+template <int N, typename T, typename S2, int MODE, bool AHEAD = false>
 __device__ __forceinline__ void force_link(const Lat& L, const S2* __restrict__ U, const S2* Pin, S2* Pout,
                                            S2* __restrict__ Uout, T eps_k, T eps_d, int order, int reunit, int mu,
                                            int x, double* sums = nullptr) {
   Mat<N, T> acc, Ux, W;
-  staple_sum<N, T, S2>(acc, U, L, mu, x);
+  staple_sum<N, T, S2, AHEAD>(acc, U, L, mu, x);
   load(Ux, U, L, mu, x);
   mul_nn(W, Ux, acc);
   Mat<N, T> P;
@@ -788,6 +822,24 @@ __global__ void __launch_bounds__(128) k_force(Lat L, const S2* __restrict__ U, 
   if (x >= L.V) return;
   for (int mu = threadIdx.x >> 5; mu < L.D; mu += (blockDim.x >> 5)) force_link<N, T, S2, MODE>(
       L, U, Pin, Pout, Uout, eps_k, eps_d, order, reunit, mu, x);
+}
+
+// FP64 with the links of the next staple in flight: at most two CTAs per SM (234
+// registers for N = 3), which is all a lattice of force_ahead's size has.  us
+// per graph-replayed step, SU(3) 8^4 6.3 -> 5.6, 16^3 5.2 -> 4.3; with three
+// resident CTAs to hide the loads the plain kernel wins (10^4 11.0 / 12.2, 32^4
+// 909 / 954).  N = 2 has the registers at any size (32^4 389 -> 376).
+inline bool force_ahead(int N, long V) { return N == 2 || (N == 3 && (V + 31) / 32 <= 2 * 148); }
+
+template <int N, typename T, typename S2, int MODE>
+__global__ void __launch_bounds__(128, 2) k_force_ahead(Lat L, const S2* __restrict__ U, const S2* Pin, S2* Pout,
+                                                        S2* __restrict__ Uout, T eps_k, T eps_d, int order,
+                                                        int reunit) {
+  grid_wait();
+  const int x = blockIdx.x * 32 + (threadIdx.x & 31);
+  if (x >= L.V) return;
+  for (int mu = threadIdx.x >> 5; mu < L.D; mu += (blockDim.x >> 5))
+    force_link<N, T, S2, MODE, true>(L, U, Pin, Pout, Uout, eps_k, eps_d, order, reunit, mu, x);
 }
 
 // The same with the energy sums of the CTA's links (launch.h): the two ends of an FP64 trajectory.
@@ -830,11 +882,11 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 5 + OCC : 2 + OCC)
     force_link<N, T, S2, MODE>(L, U, Pin, Pout, Uout, eps_k, eps_d, order, reunit, mu, x);
 }
 
-// In-place drift: U <- exp(i eps P) U (updateUandcopyDown; the copy pi = Pi is
-// done by the caller).  Optionally reunitarises.
+// In-place drift U <- exp(i eps P) U and the copy pi = Pi of updateUandcopyDown
+// (to Pcopy, the momenta being in registers).  Optionally reunitarises.
 template <int N, typename T, typename S2>
-__global__ void __launch_bounds__(128) k_drift(Lat L, S2* __restrict__ U, const S2* __restrict__ P, T eps, int order,
-                                               int reunit) {
+__global__ void __launch_bounds__(128) k_drift(Lat L, S2* __restrict__ U, const S2* __restrict__ P,
+                                               S2* __restrict__ Pcopy, T eps, int order, int reunit) {
   const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (long)L.V * L.D) return;
   const int mu = (int)(t / L.V);
@@ -842,6 +894,7 @@ __global__ void __launch_bounds__(128) k_drift(Lat L, S2* __restrict__ U, const 
   Mat<N, T> Ux, Pm, Tm;
   load(Ux, U, L, mu, x);
   load(Pm, P, L, mu, x);
+  store(Pcopy, Pm, L, mu, x);
   expi_update(Tm, Pm, Ux, eps, order);
   if (reunit) reunitarise(Tm);
   store(U, Tm, L, mu, x);

@@ -522,10 +522,11 @@ __global__ void __launch_bounds__(128 * Tiles<N, OCC>::PER_CTA, Tiles<N, OCC>::M
 }
 
 // In-place link update without a kick: U <- U + (E - 1) U, E = exp(i eps P)
-// (updateUandcopyDown on the momenta P).
+// (updateUandcopyDown on the momenta P, its copy pi = Pi included).
 template <int N>
 __global__ void __launch_bounds__(128) k_drift(Lat L, float2* __restrict__ U, uint32_t* __restrict__ UL,
-                                               const float* __restrict__ P, const uint32_t* __restrict__ PL, float eps,
+                                               const float* __restrict__ P, const uint32_t* __restrict__ PL,
+                                               float* __restrict__ Pcopy, uint32_t* __restrict__ PLcopy, float eps,
                                                int order) {
   using small::Mat;
   const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -534,6 +535,7 @@ __global__ void __launch_bounds__(128) k_drift(Lat L, float2* __restrict__ U, ui
   const int x = (int)(t - (long)mu * L.V);
   float ph[Dims<N>::NCOEF], pl[Dims<N>::NCOEF];
   load_coefs<N>(ph, pl, P, PL, L, mu, x);
+  store_coefs<N>(Pcopy, PLcopy, ph, pl, L, mu, x);
   Mat<N, float> Pm, E, Dm, Ux, Ul;
   coefs_to_mat<N, float>(Pm, ph);
   small::load(Ux, U, L, mu, x);
@@ -617,14 +619,12 @@ __device__ __forceinline__ void plaq_site(const Lat& L, const float2* __restrict
 template <int N>
 __global__ void __launch_bounds__(misc::RED_THREADS, N <= 3 ? 2 : 1) k_plaq(Lat L, const float2* __restrict__ U,
                                                             const uint32_t* __restrict__ UL,
-                                                            double* __restrict__ partial) {
+                                                            double* __restrict__ partial,
+                                                            double* __restrict__ out, unsigned* ticket) {
   double v[2] = {0.0, 0.0};
   plaq_site<N>(L, U, UL, blockIdx.x * blockDim.x + threadIdx.x, v);
   misc::block_sum<2>(v);
-  if (threadIdx.x == 0) {
-    partial[blockIdx.x * 2 + 0] = v[0];
-    partial[blockIdx.x * 2 + 1] = v[1];
-  }
+  misc::publish<2>(v, partial, out, ticket);
 }
 
 // tr(P^2) of link t (t = d V + s) from coordinates hi + lo, 0 past the end
@@ -652,7 +652,8 @@ __global__ void __launch_bounds__(misc::RED_THREADS) k_linksums(Lat L, const flo
                                                                 const uint32_t* __restrict__ PLb,
                                                                 const float2* __restrict__ U,
                                                                 const uint32_t* __restrict__ UL,
-                                                                double* __restrict__ partial) {
+                                                                double* __restrict__ partial,
+                                                                double* __restrict__ out, unsigned* ticket) {
   constexpr int NC = Dims<N>::NCOEF;
   double v[3] = {0.0, 0.0, 0.0};
   const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -698,9 +699,7 @@ __global__ void __launch_bounds__(misc::RED_THREADS) k_linksums(Lat L, const flo
     }
   }
   misc::block_sum<3>(v);
-  if (threadIdx.x == 0)
-#pragma unroll
-    for (int k = 0; k < 3; k++) partial[blockIdx.x * 3 + k] = v[k];
+  misc::publish<3>(v, partial, out, ticket);
 }
 
 // Momentum refresh into coordinates: the entries misc::refresh_link draws

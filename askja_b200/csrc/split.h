@@ -24,8 +24,9 @@ size_t coef_words(const Lat& L);
 // mode 0: Pout = Pin - ek F(U);  mode 1: also U' = U + (exp(i ed Pout) - 1) U into (Uout, ULout)
 cudaError_t force(const LaunchCtx& c, int mode, const void* U, const void* UL, const void* Pin, const void* PLin,
                   void* Pout, void* PLout, void* Uout, void* ULout, double ek, double ed);
-// U <- U + (exp(i eps P) - 1) U in place
-cudaError_t drift(const LaunchCtx& c, void* U, void* UL, const void* P, const void* PL, double eps);
+// U <- U + (exp(i eps P) - 1) U in place, and (Pcopy, PLcopy) = (P, PL)
+cudaError_t drift(const LaunchCtx& c, void* U, void* UL, const void* P, const void* PL, void* Pcopy, void* PLcopy,
+                  double eps);
 // projection onto SU(N) in FP64, in place and (Usave non-null) also into (Usave, ULsave)
 cudaError_t reunit(const LaunchCtx& c, void* U, void* UL, void* Usave = nullptr, void* ULsave = nullptr);
 // out[0] temporal, out[1] spatial plaquette sums

@@ -40,10 +40,10 @@ def test_fp64_exponential_every_order(nc, hermitian):
             assert rel(e.get_links(), want) < 1e-12, level
 
 
-# lattices on either side of the rules of default_occupancy
+# lattices on either side of the rules of default_occupancy and force_ahead
 @pytest.mark.parametrize("nc,dims,precision", [(2, [24, 32, 26], "fp32"), (2, [23, 32, 25], "fp32"),
                                                (3, [24, 32, 26], "fp32"), (2, [64, 32, 32], "fp64"),
-                                               (2, [65, 32, 32], "fp64"), (4, [24, 32, 26], "fp32")])
+                                               (2, [65, 32, 32], "fp64"), (3, [16, 32, 18], "fp64"), (3, [17, 32, 18], "fp64"), (4, [24, 32, 26], "fp32")])
 def test_register_budgets_give_the_same_fields(nc, dims, precision):
     out = []
     for occ in (None, 0, 1, 2):
