@@ -66,7 +66,7 @@ struct LaunchCtx {
   int rows_ns;      // row kernels, FP32: project by one Newton-Schulz step per update (the engine
                     // re-orthonormalises with the determinant phase every few trajectories)
   int force_rows;   // kernel mapping: 0 automatic (thread-per-link for NC <= 4, FP64 MMA above),
-                    // 1 row-per-thread, 4 FP64 MMA (NC >= 5),
+                    // 1 row-per-thread, 4 warp MMA (NC >= 5: FP64, split TF32 for FP32 storage),
                     // 2 tensor cores (FP32, NC = 16, 32 or 64, DIM >= 2), 3 site pairs in
                     // packed FP32 (NC = 3, even n[DIM-1]; the fused kick+drift then
                     // expects the site-pair layout, see pair_swap)

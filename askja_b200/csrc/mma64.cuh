@@ -1,6 +1,7 @@
 // Link update, plaquette and kinetic sums for 5 <= NC <= 64 on the FP64 tensor
 // instruction (mma.sync m8n8k4 f64; tcgen05 has no FP64 kind), for FP64 and
-// FP32 storage.
+// FP32 storage; the kicks and fused updates of FP32 storage in TF32 split in two
+// (see prod).
 //
 // A matrix is cut into 8 x 8 tiles (NT = ceil(NC / 8) of them a side); one warp
 // owns the eight rows 8w .. 8w+7 of every left operand and result, NT warps
@@ -69,29 +70,37 @@ struct Job {
 // us per fused step against eight-warp CTAs of 2-3 a SM, SU(8) 10^4 112 -> 105,
 // SU(16) 6^4 102 -> 99, SU(24) 6^3 51 -> 43, SU(32) 6^4 751 -> 722 (94 % of the
 // MMA rate).  Plaquette: about eight warps, a site each NT.
-template <int NT>
+// R: the arithmetic (double: FP64 MMA; float: split TF32 MMA, see prod).
+template <int NT, typename R = double>
 struct Cta {
   static constexpr int LINKS = NT == 1 ? 4 : NT == 2 ? 2 : 1;
   static constexpr int SITES = NT == 1 ? 8 : NT == 2 ? 4 : NT <= 4 ? 2 : 1;
   static constexpr int THREADS = 32 * NT * LINKS;
   static constexpr int PLAQ_THREADS = 32 * NT * SITES;
-  static constexpr int LD = 8 * NT + 1;
-  static constexpr int TILE = 8 * NT * LD;  // double2 of one link's tile
+  using V2 = typename Storage<R>::type;
+  static constexpr int LD = 8 * NT + (sizeof(R) == 8 ? 1 : 2);  // conflict-free column reads
+  static constexpr int TILE = 8 * NT * LD;  // complex numbers of one link's tile
   // small matrices keep the rows of X and X^2 in registers; larger ones read X
   // back from the momenta and keep X^2 in a second tile
-  static constexpr bool KEEP = NT <= 2;
+  static constexpr bool KEEP = NT <= (sizeof(R) == 8 ? 2 : 4);
   static constexpr int TILES = KEEP ? 1 : 2;
-  static constexpr size_t SMEM = (size_t)LINKS * TILES * TILE * sizeof(double2);
-  // resident CTAs the register budget is set for
-  static constexpr int MIN_CTAS = NT == 1 ? 8 : NT == 2 ? 4 : NT == 3 ? 5 : NT == 4 ? 4 : 1;
+  static constexpr size_t SMEM = (size_t)LINKS * TILES * TILE * sizeof(V2);
+  // resident CTAs the register budget is set for; float at 6 / 8 and 4 / 5 / 3 CTAs
+  // (NT = 1, 2): SU(8) 10^4 90 / 93 us a step, SU(16) 6^4 74 / 80 / 76
+  static constexpr int MIN_CTAS = sizeof(R) == 8 ? (NT == 1 ? 8 : NT == 2 ? 4 : NT == 3 ? 5 : NT == 4 ? 4 : 1)
+                                                 : (NT == 1 ? 6 : NT == 2 ? 4 : NT == 3 ? 5 : NT == 4 ? 3 : 1);
 };
 
-struct Acc {
-  double re[2], im[2];  // columns 2j, 2j + 1
+template <typename R>
+struct AccT {
+  R re[2], im[2];  // columns 2j, 2j + 1
 };
-struct Op {
-  double re, im;
+template <typename R>
+struct OpT {
+  R re, im;
 };
+using Acc = AccT<double>;
+using Op = OpT<double>;
 
 __device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
   asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
@@ -99,17 +108,18 @@ __device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
       : "d"(a), "d"(b));
 }
 
-template <int NT>
-__device__ __forceinline__ void zero(Acc (&c)[NT]) {
+template <int NT, typename R>
+__device__ __forceinline__ void zero(AccT<R> (&c)[NT]) {
 #pragma unroll
-  for (int t = 0; t < NT; t++) c[t].re[0] = c[t].re[1] = c[t].im[0] = c[t].im[1] = 0.0;
+  for (int t = 0; t < NT; t++) c[t].re[0] = c[t].re[1] = c[t].im[0] = c[t].im[1] = R(0);
 }
 
 // two consecutive complex numbers of a row (c even)
 __device__ __forceinline__ void ld_pair(const double2* p, Op& a, Op& b) {
   asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(a.re), "=d"(a.im), "=d"(b.re), "=d"(b.im) : "l"(p));
 }
-__device__ __forceinline__ void ld_pair(const float2* p, Op& a, Op& b) {
+template <typename R>
+__device__ __forceinline__ void ld_pair(const float2* p, OpT<R>& a, OpT<R>& b) {
   const float4 v = __ldg(reinterpret_cast<const float4*>(p));
   a.re = v.x;
   a.im = v.y;
@@ -123,7 +133,8 @@ __device__ __forceinline__ void ld_pair_rw(const double2* p, Op& a, Op& b) {
                : "l"(p)
                : "memory");
 }
-__device__ __forceinline__ void ld_pair_rw(const float2* p, Op& a, Op& b) {
+template <typename R>
+__device__ __forceinline__ void ld_pair_rw(const float2* p, OpT<R>& a, OpT<R>& b) {
   const float4 v = *reinterpret_cast<const float4*>(p);
   a.re = v.x;
   a.im = v.y;
@@ -134,26 +145,29 @@ __device__ __forceinline__ void st_pair(double2* p, const Op& a, const Op& b) {
   asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(a.re), "d"(a.im), "d"(b.re), "d"(b.im)
                : "memory");
 }
-__device__ __forceinline__ void st_pair(float2* p, const Op& a, const Op& b) {
+template <typename R>
+__device__ __forceinline__ void st_pair(float2* p, const OpT<R>& a, const OpT<R>& b) {
   *reinterpret_cast<float4*>(p) = make_float4((float)a.re, (float)a.im, (float)b.re, (float)b.im);
 }
 __device__ __forceinline__ double round_to(const double2*, double v) { return v; }
 __device__ __forceinline__ double round_to(const float2*, double v) { return (double)(float)v; }
+__device__ __forceinline__ float round_to(const float2*, float v) { return v; }
 __device__ __forceinline__ double2 pack(const double2*, double re, double im) { return make_double2(re, im); }
 __device__ __forceinline__ float2 pack(const float2*, double re, double im) {
   return make_float2((float)re, (float)im);
 }
-template <typename S2>
-__device__ __forceinline__ Op ld_one(const S2* p) {
+template <typename R = double, typename S2>
+__device__ __forceinline__ OpT<R> ld_one(const S2* p) {
   const S2 v = __ldg(p);
-  Op o;
-  o.re = v.x;
-  o.im = v.y;
+  OpT<R> o;
+  o.re = (R)v.x;
+  o.im = (R)v.y;
   return o;
 }
-__device__ __forceinline__ Op op0() {
-  Op o;
-  o.re = o.im = 0.0;
+template <typename R = double>
+__device__ __forceinline__ OpT<R> op0() {
+  OpT<R> o;
+  o.re = o.im = R(0);
   return o;
 }
 
@@ -163,37 +177,37 @@ struct Who {
   int w, q, j, n;  // row block, lane / 4, lane % 4, NC (when not FULL)
   __device__ __forceinline__ int N() const { return FULL ? 8 * NT : n; }
   // row 8 rb + q, columns 8 cb + 2 j + {0, 1}
-  template <typename S2>
-  __device__ __forceinline__ void rows(const S2* m, int rb, int cb, Op (&o)[2]) const {
+  template <typename R, typename S2>
+  __device__ __forceinline__ void rows(const S2* m, int rb, int cb, OpT<R> (&o)[2]) const {
     const int r = 8 * rb + q, c = 8 * cb + 2 * j;
     if constexpr (FULL) {
       ld_pair(m + r * N() + c, o[0], o[1]);
     } else {
-      o[0] = r < n && c < n ? ld_one(m + r * n + c) : op0();
-      o[1] = r < n && c + 1 < n ? ld_one(m + r * n + c + 1) : op0();
+      o[0] = r < n && c < n ? ld_one<R>(m + r * n + c) : op0<R>();
+      o[1] = r < n && c + 1 < n ? ld_one<R>(m + r * n + c + 1) : op0<R>();
     }
   }
   // own rows, columns 8 t + 2 j + {0, 1}, of a matrix this launch also writes
-  template <typename S2>
-  __device__ __forceinline__ void own(const S2* m, int t, Op (&o)[2]) const {
+  template <typename R, typename S2>
+  __device__ __forceinline__ void own(const S2* m, int t, OpT<R> (&o)[2]) const {
     const int r = 8 * w + q, c = 8 * t + 2 * j;
     if constexpr (FULL) {
       ld_pair_rw(m + r * N() + c, o[0], o[1]);
     } else {
 #pragma unroll
       for (int e = 0; e < 2; e++) {
-        o[e] = op0();
+        o[e] = op0<R>();
         if (r < n && c + e < n) {
           const S2 v = m[r * n + c + e];
-          o[e].re = v.x;
-          o[e].im = v.y;
+          o[e].re = (R)v.x;
+          o[e].im = (R)v.y;
         }
       }
     }
   }
   // the same elements to a matrix
-  template <typename S2>
-  __device__ __forceinline__ void put(S2* m, int t, const Op (&o)[2]) const {
+  template <typename R, typename S2>
+  __device__ __forceinline__ void put(S2* m, int t, const OpT<R> (&o)[2]) const {
     const int r = 8 * w + q, c = 8 * t + 2 * j;
     if constexpr (FULL) {
       st_pair(m + r * N() + c, o[0], o[1]);
@@ -204,15 +218,15 @@ struct Who {
     }
   }
   // rows 8 rb + 2 j + {0, 1}, column 8 cb + q
-  template <typename S2>
-  __device__ __forceinline__ void cols(const S2* m, int rb, int cb, Op (&o)[2]) const {
+  template <typename R, typename S2>
+  __device__ __forceinline__ void cols(const S2* m, int rb, int cb, OpT<R> (&o)[2]) const {
     const int r = 8 * rb + 2 * j, c = 8 * cb + q;
     if constexpr (FULL) {
-      o[0] = ld_one(m + r * N() + c);
-      o[1] = ld_one(m + (r + 1) * N() + c);
+      o[0] = ld_one<R>(m + r * N() + c);
+      o[1] = ld_one<R>(m + (r + 1) * N() + c);
     } else {
-      o[0] = r < n && c < n ? ld_one(m + r * n + c) : op0();
-      o[1] = r + 1 < n && c < n ? ld_one(m + (r + 1) * n + c) : op0();
+      o[0] = r < n && c < n ? ld_one<R>(m + r * n + c) : op0<R>();
+      o[1] = r + 1 < n && c < n ? ld_one<R>(m + (r + 1) * n + c) : op0<R>();
     }
   }
 };
@@ -220,6 +234,24 @@ struct Who {
 // c += A B (CONJ false) or A conj(B) (CONJ true: the right operand is given as
 // the elements of Y for the product with Y^dag).  fa(kb, a): the left operand's
 // own-row elements of tile column kb, fb(kb, t, b): the right operand's.
+//
+// FP32 arithmetic (R = float): m16n8k8 TF32 MMAs on the 16 x 8 stack [Re A; Im A],
+//   [Re; Im] C += [Re A; Im A] Re B + [-Im A; Re A] Im B,
+// whose accumulator rows q and q + 8 are the real and imaginary parts of the
+// same elements as the FP64 layout's (k slots j and j + 4 take the columns 2j and
+// 2j + 1).  Every operand is split x = hi + lo, hi rounded to TF32's 11 bits; hi hi
+// starts each 8-column step from a zero accumulator and is added to c in FP32
+// with round to nearest (the tensor cores' own accumulation rounds toward zero:
+// chained, it would scale the staple sum by 1 - 1e-6), lo hi + hi lo, 2^-11
+// smaller, is chained.  Six MMAs of 2.1 SM cycles per 8 x 8 x 8 complex block
+// against 32 cycles for the eight FP64 ones (measured 276 TFLOP/s TF32, 36.8
+// FP64); what bounds it is the wait for operands and their splitting.  us per
+// fused step, FP64 MMA on FP32 storage -> split TF32: SU(8) 10^4 106 -> 90,
+// SU(5) 17x15x13 25.7 -> 23, SU(16) 6^4 102 -> 74, SU(24) 6^3 44 -> 31, SU(48)
+// 6^3 431 -> 293.  Links after 20 updates are 5.8e-8 from 64 bits at SU(8) 10^4
+// (FP64 MMA 5.4e-8, the FP32 row kernels 2.1e-7), dH 1.4e-3 (3e-4, 1.7e-2).
+// Two row blocks a warp, sharing a right operand's split, gained nothing (SU(16)
+// 73, SU(32) 8^4 2112 against 2041).
 template <int NT, bool CONJ, int KU, typename FA, typename FB>
 __device__ __forceinline__ void prod(Acc (&c)[NT], FA&& fa, FB&& fb) {
 #pragma unroll KU
@@ -243,9 +275,72 @@ __device__ __forceinline__ void prod(Acc (&c)[NT], FA&& fa, FB&& fb) {
   }
 }
 
+__device__ __forceinline__ void tmma(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
+  asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+// x = hi + lo, hi with TF32's mantissa (rounded to nearest in magnitude)
+__device__ __forceinline__ void split_tf32(float x, uint32_t& hi, uint32_t& lo) {
+  hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
+  lo = __float_as_uint(x - __uint_as_float(hi));
+}
+
+template <int NT, bool CONJ, int KU, typename FA, typename FB>
+__device__ __forceinline__ void prod(AccT<float> (&c)[NT], FA&& fa, FB&& fb) {
+  float cor[NT][4];
+#pragma unroll
+  for (int t = 0; t < NT; t++) cor[t][0] = cor[t][1] = cor[t][2] = cor[t][3] = 0.f;
+#pragma unroll KU
+  for (int kb = 0; kb < NT; kb++) {
+    OpT<float> a[2];
+    fa(kb, a);
+    constexpr uint32_t SIGN = 0x80000000u;
+    uint32_t h1[4], l1[4], h2[4], l2[4];  // [Re; Im] and [-Im; Re] (CONJ: [Im; -Re])
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+      split_tf32(a[e].re, h1[2 * e], l1[2 * e]);
+      split_tf32(a[e].im, h1[2 * e + 1], l1[2 * e + 1]);
+      h2[2 * e] = CONJ ? h1[2 * e + 1] : h1[2 * e + 1] ^ SIGN;
+      l2[2 * e] = CONJ ? l1[2 * e + 1] : l1[2 * e + 1] ^ SIGN;
+      h2[2 * e + 1] = CONJ ? h1[2 * e] ^ SIGN : h1[2 * e];
+      l2[2 * e + 1] = CONJ ? l1[2 * e] ^ SIGN : l1[2 * e];
+    }
+#pragma unroll
+    for (int t = 0; t < NT; t++) {
+      OpT<float> b[2];
+      fb(kb, t, b);
+      uint32_t rh[2], rl[2], ih[2], il[2];
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        split_tf32(b[e].re, rh[e], rl[e]);
+        split_tf32(b[e].im, ih[e], il[e]);
+      }
+      float m[4] = {0.f, 0.f, 0.f, 0.f};
+      tmma(m, h1, rh);
+      tmma(m, h2, ih);
+      tmma(cor[t], l1, rh);
+      tmma(cor[t], l2, ih);
+      tmma(cor[t], h1, rl);
+      tmma(cor[t], h2, il);
+      c[t].re[0] += m[0];
+      c[t].re[1] += m[1];
+      c[t].im[0] += m[2];
+      c[t].im[1] += m[3];
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < NT; t++) {
+    c[t].re[0] += cor[t][0];
+    c[t].re[1] += cor[t][1];
+    c[t].im[0] += cor[t][2];
+    c[t].im[1] += cor[t][3];
+  }
+}
+
 // the rows of an accumulator as left operand
-template <int NT>
-__device__ __forceinline__ void from_acc(const Acc (&c)[NT], int kb, Op (&a)[2]) {
+template <int NT, typename R>
+__device__ __forceinline__ void from_acc(const AccT<R> (&c)[NT], int kb, OpT<R> (&a)[2]) {
   a[0].re = c[kb].re[0];
   a[0].im = c[kb].im[0];
   a[1].re = c[kb].re[1];
@@ -262,33 +357,33 @@ __device__ __forceinline__ void link_sync(int slot) {
 }
 
 // own rows of an accumulator to a field matrix
-template <int NT, bool FULL, typename S2>
-__device__ __forceinline__ void store_rows(S2* m, const Who<NT, FULL>& me, const Acc (&c)[NT]) {
+template <int NT, bool FULL, typename R, typename S2>
+__device__ __forceinline__ void store_rows(S2* m, const Who<NT, FULL>& me, const AccT<R> (&c)[NT]) {
 #pragma unroll
   for (int t = 0; t < NT; t++) {
-    Op o[2];
+    OpT<R> o[2];
     from_acc(c, t, o);
     me.put(m, t, o);
   }
 }
 
 // own rows of an accumulator to the link's shared tile
-template <int NT, bool FULL>
-__device__ __forceinline__ void tile_rows(double2* S, const Who<NT, FULL>& me, const Acc (&c)[NT]) {
-  double2* p = S + (8 * me.w + me.q) * Cta<NT>::LD + 2 * me.j;
+template <int NT, bool FULL, typename R, typename V2>
+__device__ __forceinline__ void tile_rows(V2* S, const Who<NT, FULL>& me, const AccT<R> (&c)[NT]) {
+  V2* p = S + (8 * me.w + me.q) * Cta<NT, R>::LD + 2 * me.j;
 #pragma unroll
   for (int t = 0; t < NT; t++)
 #pragma unroll
-    for (int e = 0; e < 2; e++) p[8 * t + e] = make_double2(c[t].re[e], c[t].im[e]);
+    for (int e = 0; e < 2; e++) p[8 * t + e] = pack(S, c[t].re[e], c[t].im[e]);
 }
 
 // column-pattern read of the shared tile (right operand)
-template <int NT, bool FULL>
-__device__ __forceinline__ void tile_cols(const double2* S, const Who<NT, FULL>& me, int rb, int cb, Op (&o)[2]) {
-  const double2* p = S + (8 * rb + 2 * me.j) * Cta<NT>::LD + 8 * cb + me.q;
+template <int NT, bool FULL, typename R, typename V2>
+__device__ __forceinline__ void tile_cols(const V2* S, const Who<NT, FULL>& me, int rb, int cb, OpT<R> (&o)[2]) {
+  const V2* p = S + (8 * rb + 2 * me.j) * Cta<NT, R>::LD + 8 * cb + me.q;
 #pragma unroll
   for (int e = 0; e < 2; e++) {
-    const double2 v = p[e * Cta<NT>::LD];
+    const V2 v = p[e * Cta<NT, R>::LD];
     o[e].re = v.x;
     o[e].im = v.y;
   }
@@ -317,10 +412,13 @@ __device__ __forceinline__ double inv_factorial(int k, int order) {
 // Newton-Schulz step on the links as read; it differs from projecting first by
 // |E - 1| times the defect that the FP32 store left, which the next update
 // removes in turn.
-template <int NT, bool FULL, typename S2, bool SUMS>
+template <int NT, bool FULL, typename S2, bool SUMS, typename R>
 __device__ __forceinline__ void update_link(const Job& job, int idx, const Who<NT, FULL>& me, int slot, int cur,
-                                            double kick_scale, int mode, double2* S, double (&v)[2]) {
-  using CT = Cta<NT>;
+                                            double kick_scale, int mode, typename Cta<NT, R>::V2* S, double (&v)[2]) {
+  using CT = Cta<NT, R>;
+  using V2 = typename CT::V2;
+  using Acc = AccT<R>;
+  using Op = OpT<R>;
   constexpr int KU = NT <= 4 ? NT : 1;  // left operands from memory: the k loop stays rolled for large NC
   const int lane = threadIdx.x & 31;
   const int V = job.V, D = job.D;
@@ -341,7 +439,7 @@ __device__ __forceinline__ void update_link(const Job& job, int idx, const Who<N
     for (int t = 0; t < NT; t++) {
       me.own(P, t, p);
 #pragma unroll
-      for (int e = 0; e < 2; e++) S[r * CT::LD + 8 * t + 2 * me.j + e] = make_double2(p[e].re, p[e].im);
+      for (int e = 0; e < 2; e++) S[r * CT::LD + 8 * t + 2 * me.j + e] = pack(S, p[e].re, p[e].im);
     }
     link_sync<NT>(slot);
 #pragma unroll
@@ -350,8 +448,8 @@ __device__ __forceinline__ void update_link(const Job& job, int idx, const Who<N
       tile_cols(S, me, t, me.w, q);
 #pragma unroll
       for (int e = 0; e < 2; e++) {
-        v[1] = fma(p[e].re, q[e].re, v[1]);
-        v[1] = fma(-p[e].im, q[e].im, v[1]);
+        v[1] = fma((double)p[e].re, (double)q[e].re, v[1]);
+        v[1] = fma(-(double)p[e].im, (double)q[e].im, v[1]);
       }
     }
     link_sync<NT>(slot);
@@ -409,10 +507,10 @@ __device__ __forceinline__ void update_link(const Job& job, int idx, const Who<N
     link_sync<NT>(slot);
     // kick with the traceless anti-hermitian part of W: z = W_cr
     const int N = me.N();
-    double trim = 0.0;
+    R trim = R(0);
     for (int k = 0; k < N; k++) trim += S[k * (CT::LD + 1)].y;
-    trim /= N;
-    const double ek = kick_scale * job.kick, ed = job.dt;
+    trim = trim / R(N);
+    const R ek = (R)(kick_scale * job.kick), ed = (R)job.dt;
     const S2* P = static_cast<const S2*>(job.Pin) + own;
     S2* Po = static_cast<S2*>(job.Pout) + own;
 #pragma unroll
@@ -424,8 +522,8 @@ __device__ __forceinline__ void update_link(const Job& job, int idx, const Who<N
 #pragma unroll
       for (int e = 0; e < 2; e++) {
         const int c = 8 * t + 2 * me.j + e;
-        const double fr = r == c ? W[t].im[e] - trim : 0.5 * (W[t].im[e] + z[e].im);
-        const double fi = r == c ? 0.0 : -0.5 * (W[t].re[e] - z[e].re);
+        const R fr = r == c ? W[t].im[e] - trim : R(0.5) * (W[t].im[e] + z[e].im);
+        const R fi = r == c ? R(0) : R(-0.5) * (W[t].re[e] - z[e].re);
         p[e].re = round_to(P, fma(-ek, fr, p[e].re));
         p[e].im = round_to(P, fma(-ek, fi, p[e].im));
         X[t].re[e] = -ed * p[e].im;
@@ -437,14 +535,14 @@ __device__ __forceinline__ void update_link(const Job& job, int idx, const Who<N
 #pragma unroll
       for (int t = 0; t < NT; t++)
 #pragma unroll
-        for (int e = 0; e < 2; e++) v[0] += r == 8 * t + 2 * me.j + e ? W[t].re[e] : 0.0;
+        for (int e = 0; e < 2; e++) v[0] += r == 8 * t + 2 * me.j + e ? (double)W[t].re[e] : 0.0;
     }
     link_sync<NT>(slot);
     if (SUMS && mode == 0) kinetic(Po);
     if (mode == 0) return;
   } else {
     const S2* P = static_cast<const S2*>(job.Pin) + own;
-    const double ed = job.dt;
+    const R ed = (R)job.dt;
 #pragma unroll
     for (int t = 0; t < NT; t++) {
       Op p[2];
@@ -464,7 +562,7 @@ __device__ __forceinline__ void update_link(const Job& job, int idx, const Who<N
       from_acc(X, t, o);
     } else {
       const S2* P = (mode == 2 ? static_cast<const S2*>(job.Pin) : static_cast<const S2*>(job.Pout)) + own;
-      const double ed = job.dt;
+      const R ed = (R)job.dt;
       Op p[2];
       me.own(P, t, p);
 #pragma unroll
@@ -477,12 +575,12 @@ __device__ __forceinline__ void update_link(const Job& job, int idx, const Who<N
   tile_rows(S, me, X);
   link_sync<NT>(slot);
   Acc E[NT], X2[NT];
-  double2* S2t = S + CT::TILE;  // X^2, own rows only (not KEEP)
-  auto tile_row = [&](const double2* tile, int kb, Op(&o)[2]) {
-    const double2* p = tile + r * CT::LD + 8 * kb + 2 * me.j;
+  V2* S2t = S + CT::TILE;  // X^2, own rows only (not KEEP)
+  auto tile_row = [&](const V2* tile, int kb, Op(&o)[2]) {
+    const V2* p = tile + r * CT::LD + 8 * kb + 2 * me.j;
 #pragma unroll
     for (int e = 0; e < 2; e++) {
-      const double2 v = p[e];
+      const V2 v = p[e];
       o[e].re = v.x;
       o[e].im = v.y;
     }
@@ -505,8 +603,8 @@ __device__ __forceinline__ void update_link(const Job& job, int idx, const Who<N
       tile_row(S2t, kb, o);
   };
   auto block = [&](Acc(&c)[NT], int k) {  // sum_{i<3} X^i / (k + i)!, the identity of k = 0 left out
-    const double a0 = k ? inv_factorial(k, order) : 0.0, a1 = inv_factorial(k + 1, order),
-                 a2 = inv_factorial(k + 2, order);
+    const R a0 = k ? (R)inv_factorial(k, order) : R(0), a1 = (R)inv_factorial(k + 1, order),
+            a2 = (R)inv_factorial(k + 2, order);
 #pragma unroll
     for (int t = 0; t < NT; t++) {
       Op o[2], o2[2];
@@ -514,7 +612,7 @@ __device__ __forceinline__ void update_link(const Job& job, int idx, const Who<N
       x2_rows(t, o2);
 #pragma unroll
       for (int e = 0; e < 2; e++) {
-        c[t].re[e] = fma(a2, o2[e].re, fma(a1, o[e].re, r == 8 * t + 2 * me.j + e ? a0 : 0.0));
+        c[t].re[e] = fma(a2, o2[e].re, fma(a1, o[e].re, r == 8 * t + 2 * me.j + e ? a0 : R(0)));
         c[t].im[e] = fma(a2, o2[e].im, a1 * o[e].im);
       }
     }
@@ -534,7 +632,7 @@ __device__ __forceinline__ void update_link(const Job& job, int idx, const Who<N
       if (k == order) {  // the top block is the single term X^k / k!: joined to the next one down
         k -= 3;
         block(E, k);
-        const double a = inv_factorial(order, order);
+        const R a = (R)inv_factorial(order, order);
 #pragma unroll
         for (int t = 0; t < NT; t++)
 #pragma unroll
@@ -549,6 +647,8 @@ __device__ __forceinline__ void update_link(const Job& job, int idx, const Who<N
     link_sync<NT>(slot);
 #pragma unroll 1
     while (k > 0) {
+      // large matrices read the tile anew: its loads hoisted out of the loop would all spill
+      if (NT > 2) asm volatile("" ::: "memory");
       k -= 3;
       Acc H[NT];
       block(H, k);
@@ -560,40 +660,46 @@ __device__ __forceinline__ void update_link(const Job& job, int idx, const Who<N
     }
   }
   if (sizeof(S2) == 8 && job.project) {
-    Acc M[NT];
+    AccT<double> M[NT];  // always in FP64: what counts is its distance from 1
     zero(M);
     prod<NT, true, KU>(
-        M, [&](int kb, Op(&o)[2]) { me.rows(Ux, me.w, kb, o); },
-        [&](int kb, int t, Op(&o)[2]) { me.rows(Ux, t, kb, o); });
+        M, [&](int kb, OpT<double>(&o)[2]) { me.rows(Ux, me.w, kb, o); },
+        [&](int kb, int t, OpT<double>(&o)[2]) { me.rows(Ux, t, kb, o); });
 #pragma unroll
     for (int t = 0; t < NT; t++)
 #pragma unroll
       for (int e = 0; e < 2; e++) {
         const bool diag = r == 8 * t + 2 * me.j + e && (FULL || r < me.n);
-        E[t].re[e] -= 0.5 * (M[t].re[e] - (diag ? 1.0 : 0.0));
-        E[t].im[e] -= 0.5 * M[t].im[e];
+        E[t].re[e] -= (R)(0.5 * (M[t].re[e] - (diag ? 1.0 : 0.0)));
+        E[t].im[e] -= (R)(0.5 * M[t].im[e]);
       }
   }
+  // U' = U + (E - 1) U; FP32 sums the small product on its own
   Acc Y[NT];
+  auto add_u = [&]() {
 #pragma unroll
-  for (int t = 0; t < NT; t++) {
-    Op o[2];
-    me.rows(Ux, me.w, t, o);
+    for (int t = 0; t < NT; t++) {
+      Op o[2];
+      me.rows(Ux, me.w, t, o);
 #pragma unroll
-    for (int e = 0; e < 2; e++) {
-      Y[t].re[e] = o[e].re;
-      Y[t].im[e] = o[e].im;
+      for (int e = 0; e < 2; e++) {
+        Y[t].re[e] += o[e].re;
+        Y[t].im[e] += o[e].im;
+      }
     }
-  }
+  };
+  zero(Y);
+  if constexpr (sizeof(R) == 8) add_u();
   prod<NT, false, NT>(
       Y, [&](int kb, Op(&o)[2]) { from_acc(E, kb, o); },
       [&](int kb, int t, Op(&o)[2]) { me.cols(Ux, kb, t, o); });
+  if constexpr (sizeof(R) == 4) add_u();
   grid_done();
   store_rows(static_cast<S2*>(job.U[cur ^ 1]) + own, me, Y);
 }
 
-template <int NT, bool FULL, typename S2, bool SUMS>
-__global__ void __launch_bounds__(Cta<NT>::THREADS, Cta<NT>::MIN_CTAS)
+template <int NT, bool FULL, typename S2, bool SUMS, typename R>
+__global__ void __launch_bounds__(Cta<NT, R>::THREADS, Cta<NT, R>::MIN_CTAS)
     k_link(const __grid_constant__ Job one, const Job* __restrict__ table, const int2* __restrict__ items, int cur,
            double kick_scale, int mode) {
   grid_wait();
@@ -614,10 +720,11 @@ __global__ void __launch_bounds__(Cta<NT>::THREADS, Cta<NT>::MIN_CTAS)
   me.j = lane & 3;
   me.n = job.N;
   const int idx = blk * Cta<NT>::LINKS + slot;
-  double2* S = reinterpret_cast<double2*>(smem_raw) + slot * (Cta<NT>::TILES * Cta<NT>::TILE);
+  using CT = Cta<NT, R>;
+  auto* S = reinterpret_cast<typename CT::V2*>(smem_raw) + slot * (CT::TILES * CT::TILE);
   double v[2] = {0.0, 0.0};
   // whole links: no barrier of a link is left waiting
-  if (idx < job.V * job.D) update_link<NT, FULL, S2, SUMS>(job, idx, me, slot, cur, kick_scale, mode, S, v);
+  if (idx < job.V * job.D) update_link<NT, FULL, S2, SUMS, R>(job, idx, me, slot, cur, kick_scale, mode, S, v);
   if constexpr (SUMS) {
     misc::block_sum<2>(v);
     if (threadIdx.x == 0) {

@@ -1,4 +1,4 @@
-// Instantiations of the FP64-MMA kernels for one storage type; included by the
+// Instantiations of the MMA kernels for one storage type; included by the
 // translation units mma64_*.cu, each of which defines a pair of entry points
 // for NC a multiple of 8 (FULL) or not.
 #pragma once
@@ -13,10 +13,19 @@ namespace m64 {
 
 template <int NT, bool FULL, typename S2>
 cudaError_t launch_link(const Job& one, const Grid& g, int cur, double ks, int mode, cudaStream_t st) {
+  // FP32 storage: the kicks and fused updates in split TF32, unless the launch
+  // also sums the energies (two a trajectory: the sums take FP64 products of the
+  // stored links) or only drifts (once a trajectory).  Figures beside prod.
   const bool sums = mode & (SUMS_OLD | SUMS_NEW);
   mode &= 3;
-  auto k = sums ? k_link<NT, FULL, S2, true> : k_link<NT, FULL, S2, false>;
-  const size_t smem = Cta<NT>::SMEM;
+  auto k = sums ? k_link<NT, FULL, S2, true, double> : k_link<NT, FULL, S2, false, double>;
+  size_t smem = Cta<NT>::SMEM;
+  if constexpr (sizeof(S2) == 8) {
+    if (!sums && mode != 2) {
+      k = k_link<NT, FULL, S2, false, float>;
+      smem = Cta<NT, float>::SMEM;
+    }
+  }
   if (smem > 48 * 1024) {
     const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;

@@ -90,6 +90,32 @@ def test_reunitarise_after_each_update_fp64(nc):
         assert rel(e.get_links(), want) < 1e-11
 
 
+@pytest.mark.parametrize("nc", [5, 8, 11, 16, 23, 31, 40, 57, 63])
+def test_split_products_keep_32_bits(nc):
+    """FP32 storage multiplies in TF32 split in two; one part alone is off by 2^-12.
+
+    With u = 2^-24, a split product drops less than u, rounds once per 8 columns
+    and once per stored operand: (NT + 3) u a product.  A kick of far-from-unit
+    links is three products and four rounded links, its anti-hermitian part
+    1 / sqrt(2) of the whole: 1.5 (3 (NT + 3) + 4) u.  An update with |X| of order
+    one rounds U on the way in and out, its increment (LEVEL products, falling as
+    1 / k!) to 2 (NT + 3) u: (2 (NT + 3) + 4) u."""
+    dims = [3, 2, 2]
+    O, u, _, rng = start(nc, dims, 70 + nc)
+    u = fields.near_identity(nc, u.size // nc ** 2, 2.0 / np.sqrt(nc), rng).reshape(O.shape)
+    pi = np.asarray(fields.momenta(nc, u.size // nc ** 2, 2.0 * nc, rng, O)).reshape(O.shape)
+    nt, unit = (nc + 7) // 8, 2.0 ** -24
+    with ab.Engine(nc, dims, beta=2.0 * nc, dt=0.1, level=8, precision="fp32", reunitarise=False) as e:
+        ab.set_tuning(e, {"path": 4})
+        e.set_links(u)
+        e.set_momenta(np.zeros_like(pi), 0)
+        e.updateE(0.1)
+        assert rel(e.get_momenta(1), O.updateE(u, np.zeros_like(pi), 0.1)) < 1.5 * (3 * (nt + 3) + 4) * unit
+        e.set_momenta(0.5 * pi, 1)
+        e.updateUandcopyDown(0.1)
+        assert rel(e.get_links(), O.updateU(u, 0.5 * pi, 0.1, 8)) < (2 * (nt + 3) + 4) * unit
+
+
 @pytest.mark.parametrize("precision", ["fp64", "fp32"])
 def test_batch_equals_single_chains(precision):
     chains = [dict(nc=nc, dims=d, beta=2.0 * nc, dt=0.02, level=lv, seed=40 + nc)
