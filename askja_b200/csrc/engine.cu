@@ -599,12 +599,14 @@ int askja_create(const askja_params* p, askja_ctx** out) {
   c->lc.pairs = c->partial;
   CKC(cudaMemset(c->sums, 0, SUMS * sizeof(double)));
   c->lc.ticket = reinterpret_cast<unsigned*>(c->sums + SUMS - 1);
-  // untuned default: TF32 tensor cores for FP32 NC = 32 and 64, else thread-per-link for NC <= 4 and the
-  // FP64 MMA above; NC = 16 on the TF32 tensor cores is an explicit path and an autotuner candidate
+  // untuned default: thread-per-link for NC <= 4, warp MMA above; FP32 NC = 64 the tcgen05 path, whose products
+  // are large enough there (us per step, tcgen05 / warp MMA: SU(64) 4x4 57 / 93, 4x8x16 773 / 1383; SU(32) 4x4
+  // 31 / 16, 8^4 1902 / 1687; SU(16) 6^4 278 / 74: a product of two small matrices waits for its operands' way
+  // through shared memory and the accumulator's way back).  All are explicit paths and autotuner candidates.
   c->lc.force_rows = p->kernel_path != 0 ? p->kernel_path
-                     : (p->nc >= 32 && askja::tc_supported(p->nc, p->dim, p->precision == ASKJA_FP64)) ? 2
-                     : askja::m64_supported(p->nc)                                                            ? 4
-                                                                                                              : 0;
+                     : (p->nc == 64 && askja::tc_supported(p->nc, p->dim, p->precision == ASKJA_FP64)) ? 2
+                     : askja::m64_supported(p->nc)                                                     ? 4
+                                                                                                       : 0;
   c->lc.rows_groups = 0;
   c->lc.small_occ =
       p->kernel_path == 0 ? askja::default_occupancy(p->nc, p->precision == ASKJA_FP64, c->split, V) : 0;

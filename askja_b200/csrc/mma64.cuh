@@ -251,7 +251,8 @@ struct Who {
 // 6^3 431 -> 293.  Links after 20 updates are 5.8e-8 from 64 bits at SU(8) 10^4
 // (FP64 MMA 5.4e-8, the FP32 row kernels 2.1e-7), dH 1.4e-3 (3e-4, 1.7e-2).
 // Two row blocks a warp, sharing a right operand's split, gained nothing (SU(16)
-// 73, SU(32) 8^4 2112 against 2041).
+// 73, SU(32) 8^4 1782 against 1684); the next plane's links prefetched to L1
+// cost 3 to 10 %.
 template <int NT, bool CONJ, int KU, typename FA, typename FB>
 __device__ __forceinline__ void prod(Acc (&c)[NT], FA&& fa, FB&& fb) {
 #pragma unroll KU
@@ -419,7 +420,11 @@ __device__ __forceinline__ void update_link(const Job& job, int idx, const Who<N
   using V2 = typename CT::V2;
   using Acc = AccT<R>;
   using Op = OpT<R>;
-  constexpr int KU = NT <= 4 ? NT : 1;  // left operands from memory: the k loop stays rolled for large NC
+  // left operands from memory: the k loop stays rolled for large NC; in TF32, whose
+  // k step is three times the instructions, by two at NT = 4 (unrolled it runs out
+  // of instruction cache: SU(32) 8^4 2040 us a step, by two 1684, by one 1727; SU(24)
+  // 6^3 30.5 unrolled, 32.3 by one; FP64 SU(32) 6^4 720 unrolled, 749 by two)
+  constexpr int KU = NT < 4 ? NT : NT > 4 ? 1 : sizeof(R) == 4 ? 2 : 4;
   const int lane = threadIdx.x & 31;
   const int V = job.V, D = job.D;
   const int x = idx / D, mu = idx - x * D;
