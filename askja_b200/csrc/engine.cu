@@ -255,7 +255,7 @@ int launch_ok(askja_ctx* c, cudaError_t e, const char* what) {
   } while (0)
 
 // whether the fused kick+drift projects each update without pinning the
-// determinant (row-per-thread and FP64-MMA kernels, with rows_ns)
+// determinant (row-per-thread and warp-MMA kernels, with rows_ns)
 bool per_update_ns(const askja_ctx* c) { return c->lc.force_rows == 1 || c->N > 4; }
 
 // whether the force kernels at the two ends of a trajectory also sum the

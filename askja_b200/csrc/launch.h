@@ -63,9 +63,9 @@ struct LaunchCtx {
   cudaStream_t stream;
   int order;        // effective Taylor order
   int reunit;       // reunitarise after each link update
-  int rows_ns;      // row kernels, FP32: project by one Newton-Schulz step per update (the engine
+  int rows_ns;      // row and warp-MMA kernels, FP32: project by one Newton-Schulz step per update (the engine
                     // re-orthonormalises with the determinant phase every few trajectories)
-  int force_rows;   // kernel mapping: 0 automatic (thread-per-link for NC <= 4, FP64 MMA above),
+  int force_rows;   // kernel mapping: 0 automatic (thread-per-link for NC <= 4, warp MMA above),
                     // 1 row-per-thread, 4 warp MMA (NC >= 5: FP64, split TF32 for FP32 storage),
                     // 2 tensor cores (FP32, NC = 16, 32 or 64, DIM >= 2), 3 site pairs in
                     // packed FP32 (NC = 3, even n[DIM-1]; the fused kick+drift then
@@ -82,13 +82,13 @@ struct LaunchCtx {
 
 // Trajectories between two full reunitarisation passes (Gram-Schmidt with the
 // determinant phase) over U, where the per-update projection leaves drift: the
-// tensor-core path and the FP32 row kernels (Newton-Schulz per update).
+// tensor-core path and the other FP32 kernels of NC > 4 (Newton-Schulz per update).
 constexpr int FULL_REUNIT_EVERY = 10;
 
 // whether the tensor-core mapping exists for this shape and precision
 inline bool tc_supported(int N, int D, bool fp64) { return !fp64 && (N == 16 || N == 32 || N == 64) && D >= 2; }
 
-// whether the FP64-MMA mapping exists for this colour number
+// whether the warp-MMA mapping exists for this colour number
 inline bool m64_supported(int N) { return link_major(N); }
 
 // Untuned register budget (LaunchCtx::small_occ) of the thread-per-link kernels,

@@ -92,19 +92,19 @@ __device__ __forceinline__ void publish(const double (&v)[K], double* __restrict
 // ReTr(A B C^dag D^dag) is evaluated as Re sum_ij (AB)_ij conj((DC)_ij).
 template <int NT, typename S2>
 __device__ __forceinline__ void plaq_site(const Lat& L, const S2* __restrict__ U, int s, double (&v)[2]) {
-  const int N = NT > 0 ? NT : L.N;
+  constexpr int N = NT;
   if (s < L.V && counted(L, s)) {
     for (int mu = 0; mu < L.D; mu++) {
       const int xpmu = nb_plus(L, mu, s);
       for (int nu = mu + 1; nu < L.D; nu++) {
         const int xpnu = nb_plus(L, nu, s);
         double tr = 0.0;
-#pragma unroll(NT > 0 ? NT : 1)
+#pragma unroll
         for (int i = 0; i < N; i++)
-#pragma unroll(NT > 0 ? NT : 1)
+#pragma unroll
           for (int j = 0; j < N; j++) {
             cpx<double> ab = czero<double>(), dc = czero<double>();
-#pragma unroll(NT > 0 ? NT : 1)
+#pragma unroll
             for (int k = 0; k < N; k++) {
               cmac(ab, ldc<double>(U + eoffn<NT>(L, mu, i * N + k, s)), ldc<double>(U + eoffn<NT>(L, nu, k * N + j, xpmu)));
               cmac(dc, ldc<double>(U + eoffn<NT>(L, nu, i * N + k, s)), ldc<double>(U + eoffn<NT>(L, mu, k * N + j, xpnu)));
@@ -134,15 +134,15 @@ __global__ void __launch_bounds__(RED_THREADS) k_plaq(Lat L, const S2* __restric
 template <int NT, typename S2>
 __device__ __forceinline__ void link_sums(const Lat& L, const S2* __restrict__ Pa, const S2* __restrict__ Pb,
                                           const S2* __restrict__ U, long t, double (&v)[3]) {
-  const int N = NT > 0 ? NT : L.N;
+  constexpr int N = NT;
   if (t < (long)L.V * L.D && counted(L, (int)(t % L.V))) {
     const int d = (int)(t / L.V);
     const int s = (int)(t - (long)d * L.V);
     if (Pa) {
       double a = 0.0, b = 0.0;
-#pragma unroll(NT > 0 ? NT : 1)
+#pragma unroll
       for (int i = 0; i < N; i++)
-#pragma unroll(NT > 0 ? NT : 1)
+#pragma unroll
         for (int j = 0; j < N; j++) {
           const cpx<double> x = ldc<double>(Pa + eoffn<NT>(L, d, i * N + j, s));
           const cpx<double> y = ldc<double>(Pa + eoffn<NT>(L, d, j * N + i, s));
@@ -160,12 +160,12 @@ __device__ __forceinline__ void link_sums(const Lat& L, const S2* __restrict__ P
     }
     if (U) {
       double c = 0.0;
-#pragma unroll(NT > 0 ? NT : 1)
+#pragma unroll
       for (int i = 0; i < N; i++)
-#pragma unroll(NT > 0 ? NT : 1)
+#pragma unroll
         for (int j = 0; j < N; j++) {
           cpx<double> aij = czero<double>(), aji = czero<double>();
-#pragma unroll(NT > 0 ? NT : 1)
+#pragma unroll
           for (int k = 0; k < N; k++) {
             cmac_nc(aij, ldc<double>(U + eoffn<NT>(L, d, i * N + k, s)), ldc<double>(U + eoffn<NT>(L, d, j * N + k, s)));
             cmac_nc(aji, ldc<double>(U + eoffn<NT>(L, d, j * N + k, s)), ldc<double>(U + eoffn<NT>(L, d, i * N + k, s)));
@@ -592,13 +592,7 @@ static __global__ void k_count_nonfinite(const double* __restrict__ x, long n, u
   if (c) atomicAdd(count, c);
 }
 
-// ---- large colour number (NC >= BIG_NC): one CTA per site or per link ----
-// The thread-per-site / thread-per-link kernels above carry O(NC^3) / O(NC^2)
-// serial work per thread, which leaves a lattice of a few thousand sites with
-// a few thousand threads; these spread one site or link over a CTA.
-
-constexpr int BIG_NC = 16;
-
+// ---- the plaquettes of a site by a whole CTA, any NC (FourierTrafo: a few sites) ----
 // Plaquette sums of one site (same sums as plaq_site): B = U_nu(x+mu) and
 // C = U_mu(x+nu) staged in shared memory as FP64 ([N][N+1]), thread t owns row
 // t / 4 and the columns j = 4q + t % 4 of AB and DC (A = U_mu(x), D = U_nu(x)

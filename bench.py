@@ -43,13 +43,13 @@ CONFIGS = {
     "su3_32": dict(nc=3, dims=[32, 32, 32, 32], beta=6.0, dt=0.02, level=6, nsteps=50),
     "su8_10": dict(nc=8, dims=[10, 10, 10, 10], beta=20.0, dt=0.01, level=8, nsteps=100, ensemble=60),
     "su3_8": dict(nc=3, dims=[8, 8, 8, 8], beta=5.70, dt=0.02, level=8, nsteps=50),
-    # large NC: every complex product of the FP32 path on the tensor cores (split TF32 x 3);
+    # large NC: every complex product of the FP32 path in split TF32 x 3, SU(64) on tcgen05, SU(32)
+    # and SU(16) by warp MMA (both are autotuner candidates);
     # the CPU sample runs the same colour number on a smaller lattice (per-link rates)
     "su32_8": dict(nc=32, dims=[8, 8, 8, 8], beta=2048.0, dt=0.005, level=8, nsteps=20, tensor=True,
                    cpu_dims=[2, 2, 2, 2], ensemble=20),
     "su64_4x16": dict(nc=64, dims=[4, 16, 16], beta=8192.0, dt=0.005, level=8, nsteps=20, tensor=True,
                       cpu_dims=[2, 2, 4], ensemble=20),
-    # NC = 16: the tensor cores on the padded M = 64 shape against the row kernels (the autotuner picks)
     "su16_6": dict(nc=16, dims=[6, 6, 6, 6], beta=512.0, dt=0.005, level=8, nsteps=20, tensor=True,
                    cpu_dims=[2, 2, 2, 2], ensemble=20),
 }
@@ -124,6 +124,13 @@ def tensor_products_per_link(dim, level, reunit=True):
     and two Newton-Schulz products."""
     order = level if 0 <= level <= 8 else 8
     return 4 * (dim - 1) + 1 + max(order - 1, 0) + 1 + (2 if reunit else 0)
+
+
+def mma_products_per_link(dim, order):
+    """Complex products of one fused kick+drift by warp MMA: 4(D-1) staple products, U S, and the
+    exponential by Paterson-Stockmeyer in blocks of three terms with U' = U + (E - 1) U."""
+    blocks = order // 3 - (1 if order % 3 == 0 else 0) if order >= 3 else 0
+    return 4 * (dim - 1) + 1 + 1 + (1 if order >= 3 else 0) + max(blocks, 0) + 1
 
 
 def tensor_flops_per_link(nc, dim, level, reunit=True):
@@ -347,18 +354,29 @@ def run_ours(args):
     bytes_per_lu = link_update_bytes(nc, residual)
     achieved = alg_per_lu * links / (f32["kernel_ms"] / 1e3) / 1e9
     traffic = measured_traffic(args.config)
-    if cfg.get("tensor") and (f32["tuning"]["path"] == 2 or (f32["tuning"]["path"] is None and nc >= 32)):
+    if cfg.get("tensor") and (f32["tuning"]["path"] == 2 or (f32["tuning"]["path"] is None and nc == 64)):
         fpl = tensor_flops_per_link(nc, len(dims), cfg["level"])
         sec = f32["kernel_ms"] / 1e3
         pk, src = tf32_peak()
         tflops = fpl * links / sec / 1e12
-        roofline = {"bound": "tensor", "kernel": f"tensor-core link update (tc::k_link<{nc},1> + per-link copy of U)",
+        roofline = {"bound": "tensor", "kernel": f"tensor-core link update (tc::k_link<{nc},1>)",
                     "achieved": tflops, "peak": pk, "unit": "TFLOP/s", "frac": tflops / pk, "peak_source": src,
                     "traffic": None, "flops_per_launch": fpl * links, "avg_launch_ms": f32["kernel_ms"],
                     "complex_tflops": 8 * nc ** 3 * tensor_products_per_link(len(dims), cfg["level"]) * links
                     / sec / 1e12}
-    elif f32["tuning"]["path"] == 1 or (f32["tuning"]["path"] is None and nc > 4):
-        # row-per-thread kernels (NC >= 5): bound by the FP32 FMA pipe; flops per link =
+    elif nc > 4 and f32["tuning"]["path"] in (4, None):
+        # warp MMA: complex products of the TF32 kernel (the FP64 projection left out), six m16n8k8
+        # MMAs per 8 x 8 x 8 block
+        order = cfg["level"] if 0 <= cfg["level"] <= 8 else 8
+        fpl = 6 * 2 * 16 * 8 * 8 * (-(-nc // 8)) ** 3 * mma_products_per_link(len(dims), order)
+        pk, src = tf32_peak()
+        tflops = fpl * links / (f32["kernel_ms"] / 1e3) / 1e12
+        roofline = {"bound": "tensor", "kernel": f"fused kick+drift (m64::k_link, split TF32 mma.sync, NC = {nc})",
+                    "achieved": tflops, "peak": pk, "unit": "TFLOP/s", "frac": tflops / pk, "peak_source": src,
+                    "traffic": None, "flops_per_launch": fpl * links, "avg_launch_ms": f32["kernel_ms"],
+                    "hbm_achieved_gbs": achieved}
+    elif f32["tuning"]["path"] == 1:
+        # row-per-thread kernels: bound by the FP32 FMA pipe; flops per link =
         # 8 NC^3 x (4(D-1) + 1 force products + LEVEL Horner products), against the FFMA peak
         # measured on this device now
         order = cfg["level"] if 0 <= cfg["level"] <= 8 else 8
@@ -435,7 +453,10 @@ def run_ours(args):
                 "api": "askja_set_links_async (FP64 U-conf from pinned host memory) + askja_trajectory_async "
                        "(outcome to pinned host memory) per trajectory; uploads overlap the previous trajectory"},
         "roofline": roofline,
-        "gpu_launches": f32["K"] * (nsteps + 15) + f64["K"] * (nsteps + 15),
+        # beside the MD steps: FP64 and warp MMA refresh, last kick, energies + Metropolis, accept copy (and the
+        # FP32 projection); otherwise plaquette, kinetic and energy launches at both ends too
+        "gpu_launches": f32["K"] * (nsteps + (12 if residual or f32["tuning"]["path"] in (1, 2) else 5))
+        + f64["K"] * (nsteps + 4),
         "clocks": f32["clocks"],
     }
     if args.config == "su3_32" and not args.no_batch:

@@ -70,12 +70,13 @@ typedef struct {
   int level;           /* LEVEL: Taylor order of exp(i dt P); outside 0..8 acts as 8 (sunmat.h:215-246) */
   int precision;       /* ASKJA_FP64, ASKJA_FP32 or ASKJA_FP32_LEAN */
   int reunitarise;     /* -1 default (on for FP32, off for FP64), 0 off, 1 on.  On: every
-                          link update is projected back onto SU(NC); the FP32 row kernels
-                          (NC > 4) and tensor cores project onto U(NC) per update and
+                          link update is projected back onto SU(NC); the FP32 kernels of
+                          NC > 4 project onto U(NC) per update and
                           askja_trajectory / askja_run_trajectories run the full SU(NC)
                           projection before every 10th trajectory */
   int device;          /* CUDA device ordinal */
-  int kernel_path;     /* 0 automatic; 1 row-per-thread kernels for every NC (testing);
+  int kernel_path;     /* 0 automatic (thread per link for NC <= 4, warp MMA above, tensor
+                          cores for FP32 NC = 64 with DIM >= 2); 1 row-per-thread kernels for every NC (testing);
                           2 tensor cores (FP32 with NC = 16, 32 or 64 and DIM >= 2 only);
                           3 site pairs in packed FP32 (NC = 3, FP32, DIM >= 2 and
                             an even extent N{DIM-1} only) */
@@ -227,10 +228,11 @@ ASKJA_API int askja_md_steps(askja_ctx* ctx, int nsteps, double eps);
  * row-per-thread (NC threads per link, shared-memory tiles) or tensor cores
  * (FP32, NC = 16, 32 or 64: every complex product a split-TF32 MMA) or site pairs
  * (FP32 SU(3): two adjacent sites' links per thread in packed FP32x2
- * arithmetic), the number of sites per CTA of the row kernels, and the
+ * arithmetic) or warp MMA (NC >= 5: products on mma.sync, FP64 or split TF32,
+ * operands in registers), the number of sites per CTA of the row kernels, and the
  * register budget of the thread-per-link kernels. */
 typedef struct {
-  int path;       /* 0 thread-per-link, 1 row-per-thread, 2 tensor cores, 3 site pairs */
+  int path;       /* 0 thread-per-link, 1 row-per-thread, 2 tensor cores, 3 site pairs, 4 warp MMA */
   int groups;     /* row-per-thread: sites per CTA (0 = default) */
   int occupancy;  /* thread-per-link, and row-per-thread FP32 with 5 <= NC <= 8: 0 default registers, 1 and 2
                      tighter budgets / more resident CTAs */
