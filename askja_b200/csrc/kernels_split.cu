@@ -162,25 +162,38 @@ cudaError_t momenta_to_matrix(const LaunchCtx& c, const void* P, const void* PL,
   });
 }
 
-cudaError_t slab(const LaunchCtx& c, bool fp64, void* f, void* lo, long s0, long ns, void* buf, bool to_buf) {
-  const long tot = ns * c.lat.D * c.lat.N * c.lat.N;
-  const unsigned grid = blocks_for(tot, 256);
-  if (fp64) {
-    if (to_buf)
-      split::k_slab_get<double2><<<grid, 256, 0, c.stream>>>(c.lat, (const double2*)f, nullptr, (int)s0, (int)ns,
-                                                             (double2*)buf);
-    else
-      split::k_slab_set<double2><<<grid, 256, 0, c.stream>>>(c.lat, (double2*)f, nullptr, (int)s0, (int)ns,
-                                                             (const double2*)buf);
-  } else {
-    if (to_buf)
-      split::k_slab_get<float2><<<grid, 256, 0, c.stream>>>(c.lat, (const float2*)f, (const uint32_t*)lo, (int)s0,
-                                                            (int)ns, (double2*)buf);
-    else
-      split::k_slab_set<float2><<<grid, 256, 0, c.stream>>>(c.lat, (float2*)f, (uint32_t*)lo, (int)s0, (int)ns,
-                                                            (const double2*)buf);
+namespace {
+
+template <typename S2, bool GET>
+cudaError_t slab_of(const LaunchCtx& c, S2* f, uint32_t* lo, int s0, int ns, double2* buf) {
+  if (link_major(c.lat.N)) {
+    const long tot = (long)ns * c.lat.D * c.lat.N * c.lat.N;
+    split::k_slab_link_major<S2, GET><<<blocks_for(tot, 256), 256, 0, c.stream>>>(c.lat, f, s0, ns, buf);
+    return cudaGetLastError();
   }
-  return cudaGetLastError();
+  return by_nc(c.lat.N, [&](auto n) {
+    constexpr int N = decltype(n)::value;
+    auto k = split::k_slab<N, S2, GET>;
+    const size_t smem = (size_t)32 * ((c.lat.D * N * N) | 1) * sizeof(double2);  // 131 KB at most (SU(4), D = 16)
+    if (smem > 48 * 1024) {
+      const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e != cudaSuccess) return e;
+    }
+    const unsigned grid = (unsigned)(((s0 + ns - 1) >> 5) - (s0 >> 5) + 1);
+    k<<<grid, 256, smem, c.stream>>>(c.lat, f, lo, s0, ns, buf);
+    return cudaGetLastError();
+  });
+}
+
+}  // namespace
+
+cudaError_t slab(const LaunchCtx& c, bool fp64, void* f, void* lo, long s0, long ns, void* buf, bool to_buf) {
+  double2* b = (double2*)buf;
+  if (fp64)
+    return to_buf ? slab_of<double2, true>(c, (double2*)f, nullptr, (int)s0, (int)ns, b)
+                  : slab_of<double2, false>(c, (double2*)f, nullptr, (int)s0, (int)ns, b);
+  return to_buf ? slab_of<float2, true>(c, (float2*)f, (uint32_t*)lo, (int)s0, (int)ns, b)
+                : slab_of<float2, false>(c, (float2*)f, (uint32_t*)lo, (int)s0, (int)ns, b);
 }
 
 }  // namespace splitk

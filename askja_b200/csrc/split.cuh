@@ -857,32 +857,66 @@ __global__ void k_momenta_to_matrix(Lat L, const float* __restrict__ P, const ui
 
 // ---- slabs of sites in the U-conf layout ----------------------------------------
 // Links of the sites [s0, s0 + ns) to / from buf in the U-conf order (FP64,
-// element t = ((s - s0) D + d) NN + e), for any storage: S2 = double2 or float2,
-// with the residual plane `lo` when non-null.  Used for the halo slabs of a
-// domain-decomposed chain.
-template <typename S2>
-__global__ void k_slab_get(Lat L, const S2* __restrict__ f, const uint32_t* __restrict__ lo, int s0, int ns,
-                           double2* __restrict__ buf) {
-  const int NN = L.N * L.N;
-  const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (long)ns * L.D * NN) return;
-  const long lk = t / NN;
-  const int e = (int)(t - lk * NN);
-  const int s = s0 + (int)(lk / L.D);
-  const int d = (int)(lk - (lk / L.D) * L.D);
-  const size_t o = eoff(L, d, e, s);
-  cpx<double> v = ldc<double>(f + o);
-  if (lo) {
-    const uint32_t w = lo[o];
-    v.re += (double)lo_low(w);
-    v.im += (double)lo_high(w);
+// element t = ((s - s0) D + d) NN + e).  Used for the halo slabs of a
+// domain-decomposed chain and for handing the links to a caller's device buffer.
+
+// NC <= 4, any storage: S2 = double2 or float2, with the residual plane `lo` when
+// non-null.  A CTA takes a block of 32 sites with all their directions through
+// shared memory (rows of an odd number of 16-byte units: no bank conflicts), so
+// that the fields are read by 32 sites and buf written in one run of up to 32 D NN
+// elements.  Bound by HBM.  askja_slab of a whole lattice, its copy from the
+// staging buffer included, against a thread per element: SU(3) 32^4 FP64 434 ->
+// 378 us out, 487 -> 380 in, residual planes 490 -> 386 and 662 -> 361, SU(4) 24^4
+// 289 -> 230 and 401 -> 229; 8^4 21 and 21.  Pieces that stay in L2 between the
+// kernel and the copy were slower (16, 32, 64 MB: 566, 426, 454).
+template <int N, typename S2, bool GET>
+__global__ void __launch_bounds__(256) k_slab(Lat L, S2* __restrict__ f, uint32_t* __restrict__ lo, int s0, int ns,
+                                              double2* __restrict__ buf) {
+  extern __shared__ __align__(16) unsigned char slab_smem[];
+  double2* sh = reinterpret_cast<double2*>(slab_smem);
+  constexpr int NN = N * N;
+  const int DN = L.D * NN, row = DN | 1;
+  const int base = ((s0 >> 5) + (int)blockIdx.x) << 5;  // first site of the block
+  const int a = max(s0 - base, 0), b = min(s0 + ns - base, 32);
+  const int lane = threadIdx.x & 31;
+  const long first = (long)(base + a - s0) * DN;
+  const int n = (b - a) * DN;
+  if (!GET) {
+    for (int i = threadIdx.x; i < n; i += 256) sh[(a + i / DN) * row + i % DN] = buf[first + i];
+    __syncthreads();
   }
-  buf[t] = make_double2(v.re, v.im);
+  if (lane >= a && lane < b) {
+    for (int q = threadIdx.x >> 5; q < DN; q += 8) {
+      const size_t o = eoffn<N>(L, q / NN, q % NN, base + lane);
+      double2& v = sh[lane * row + q];
+      if (GET) {
+        const cpx<double> x = ldc<double>(f + o);
+        v = make_double2(x.re, x.im);
+        if (lo) {
+          const uint32_t w = lo[o];
+          v.x += (double)lo_low(w);
+          v.y += (double)lo_high(w);
+        }
+      } else if (lo) {
+        float hr, lr, hi, li;
+        split_of(v.x, hr, lr);
+        split_of(v.y, hi, li);
+        stc(f + o, mkc<float>(hr, hi));
+        lo[o] = lo_pack(lr, li);
+      } else {
+        stc(f + o, mkc<double>(v.x, v.y));
+      }
+    }
+  }
+  if (GET) {
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += 256) buf[first + i] = sh[(a + i / DN) * row + i % DN];
+  }
 }
 
-template <typename S2>
-__global__ void k_slab_set(Lat L, S2* __restrict__ f, uint32_t* __restrict__ lo, int s0, int ns,
-                           const double2* __restrict__ buf) {
+// NC >= 5: matrices are contiguous on both sides
+template <typename S2, bool GET>
+__global__ void k_slab_link_major(Lat L, S2* __restrict__ f, int s0, int ns, double2* __restrict__ buf) {
   const int NN = L.N * L.N;
   const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (long)ns * L.D * NN) return;
@@ -891,14 +925,11 @@ __global__ void k_slab_set(Lat L, S2* __restrict__ f, uint32_t* __restrict__ lo,
   const int s = s0 + (int)(lk / L.D);
   const int d = (int)(lk - (lk / L.D) * L.D);
   const size_t o = eoff(L, d, e, s);
-  const double2 v = buf[t];
-  if (lo) {
-    float hr, lr, hi, li;
-    split_of(v.x, hr, lr);
-    split_of(v.y, hi, li);
-    stc(f + o, mkc<float>(hr, hi));
-    lo[o] = lo_pack(lr, li);
+  if (GET) {
+    const cpx<double> v = ldc<double>(f + o);
+    buf[t] = make_double2(v.re, v.im);
   } else {
+    const double2 v = buf[t];
     stc(f + o, mkc<double>(v.x, v.y));
   }
 }

@@ -144,3 +144,26 @@ def test_two_ranks_match_whole_lattice(precision):
     for _, h0, h1, _ in res:
         assert h0 == pytest.approx(want_h0, rel=1e-12 if precision == "fp64" else 1e-9)
         assert h1 == pytest.approx(want_h1, rel=1e-12 if precision == "fp64" else 1e-9)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32", "fp32-lean"])
+@pytest.mark.parametrize("nc,dims", [(2, [3]), (2, [5, 13]), (3, [3, 5, 7]), (3, [2, 2, 3, 4, 3]), (4, [9, 11]),
+                                     (4, [2, 1, 3, 2, 1, 3]), (4, [1] * 14 + [3, 12]), (3, [1] * 15 + [33])])
+def test_ragged_slabs_are_the_links(nc, dims, precision):
+    """Ranges that begin and end inside a block of 32 sites, extents of 1, up to 16
+    directions: a slab is exactly that part of the links, and writing one back
+    changes nothing outside it."""
+    rng = np.random.default_rng(7 * nc + len(dims))
+    with ab.Engine(nc, dims, beta=2.0, precision=precision) as e, ab.Engine(nc, dims, beta=2.0,
+                                                                            precision=precision) as f:
+        u = fields.haar(nc, e.vol * len(dims), rng).reshape(e.shape)
+        e.set_links(u)
+        u = e.get_links()  # as stored
+        want = f.get_links()  # the identity
+        V = e.vol
+        for s0, n in {(0, V), (0, 1), (V - 1, 1), (V // 3, max(1, V // 2)), (min(31, V - 1), min(2, V - min(31, V - 1)))}:
+            got = e.get_slab(s0, n)
+            np.testing.assert_array_equal(got, u[s0:s0 + n])
+            f.set_slab(s0, got)
+            want[s0:s0 + n] = u[s0:s0 + n]
+            np.testing.assert_array_equal(f.get_links(), want)
