@@ -241,29 +241,30 @@ __device__ __forceinline__ void staple_sum(Mat<N, T>& acc, const S2* __restrict_
       xmnu = xmnu2;
       xpmu_mnu = xpmu_mnu2;
     }
-  }
-  for (int nu = 0; nu < L.D; nu++) {
-    if (nu == mu) continue;
-    const int xpnu = nb_plus(L, nu, x);
-    const int xmnu = nb_minus(L, nu, x);
-    const int xpmu_mnu = nb_minus(L, nu, xpmu);
-    {
-      Mat<N, T> A, B, T1;
-      load(A, U, L, nu, xpmu);
-      load(B, U, L, mu, xpnu);
-      mul_nd<N, T, R2 ? 2 : N>(T1, A, B);
-      if constexpr (R2) su3_third_row(T1);
-      load(A, U, L, nu, x);
-      mac_nd(acc, T1, A);
-    }
-    {
-      Mat<N, T> A, B, T1;
-      load(A, U, L, nu, xpmu_mnu);
-      load(B, U, L, mu, xmnu);
-      mul_dd<N, T, R2 ? 2 : N>(T1, A, B);
-      if constexpr (R2) su3_third_row(T1);
-      load(A, U, L, nu, xmnu);
-      mac_nn(acc, T1, A);
+  } else {
+    for (int nu = 0; nu < L.D; nu++) {
+      if (nu == mu) continue;
+      const int xpnu = nb_plus(L, nu, x);
+      const int xmnu = nb_minus(L, nu, x);
+      const int xpmu_mnu = nb_minus(L, nu, xpmu);
+      {
+        Mat<N, T> A, B, T1;
+        load(A, U, L, nu, xpmu);
+        load(B, U, L, mu, xpnu);
+        mul_nd<N, T, R2 ? 2 : N>(T1, A, B);
+        if constexpr (R2) su3_third_row(T1);
+        load(A, U, L, nu, x);
+        mac_nd(acc, T1, A);
+      }
+      {
+        Mat<N, T> A, B, T1;
+        load(A, U, L, nu, xpmu_mnu);
+        load(B, U, L, mu, xmnu);
+        mul_dd<N, T, R2 ? 2 : N>(T1, A, B);
+        if constexpr (R2) su3_third_row(T1);
+        load(A, U, L, nu, xmnu);
+        mac_nn(acc, T1, A);
+      }
     }
   }
 }
