@@ -85,10 +85,19 @@ struct Cta {
   static constexpr bool KEEP = NT <= (sizeof(R) == 8 ? 2 : 4);
   static constexpr int TILES = KEEP ? 1 : 2;
   static constexpr size_t SMEM = (size_t)LINKS * TILES * TILE * sizeof(V2);
-  // resident CTAs the register budget is set for; float at 6 / 8 and 4 / 5 / 3 CTAs
-  // (NT = 1, 2): SU(8) 10^4 90 / 93 us a step, SU(16) 6^4 74 / 80 / 76
-  static constexpr int MIN_CTAS = sizeof(R) == 8 ? (NT == 1 ? 8 : NT == 2 ? 4 : NT == 3 ? 5 : NT == 4 ? 4 : 1)
-                                                 : (NT == 1 ? 6 : NT == 2 ? 4 : NT == 3 ? 5 : NT == 4 ? 3 : 1);
+  // resident CTAs the register budget is set for, us a step beside the next choice:
+  // float at 6 / 8 and 4 / 5 / 3 CTAs (NT = 1, 2) SU(8) 10^4 90 / 93, SU(16) 6^4 74 /
+  // 80 / 76; 5 / 4 / 6 (NT = 3) SU(24) 6^3 29 / 36 / 31; 3 / 4 / 2 (NT = 4) SU(32) 8^4
+  // 1686 / 1749 / 1880.  NT = 5, 6: one CTA of NT warps a SM (200 to 255 registers)
+  // leaves it idle at every barrier; two (168, spills of 4 to 116 bytes): SU(40) 6^3
+  // FP64 262 -> 207, FP32 206 -> 161, SU(48) 6^3 371 -> 298 and 292 -> 242, SU(45) 5x6x6
+  // 319 -> 262 and 291 -> 221.  A third spills more (SU(40) 6^3 189, 143, but 4x4 38 ->
+  // 42), as a second does at NT = 7 (SU(50) 5^3 FP64 317 -> 339); FP64 NT = 8 has no
+  // shared memory for it.  A lattice of at most a link per SM keeps the whole register
+  // file to one CTA (k_link with TIGHT false; SU(48) 4x4 FP32 45 / 54, 10x10 89 / 73).
+  static constexpr int MIN_CTAS = NT > 4 ? (NT <= 6 ? 2 : 1)
+                                  : sizeof(R) == 8 ? (NT == 1 ? 8 : NT == 2 ? 4 : NT == 3 ? 5 : 4)
+                                                   : (NT == 1 ? 6 : NT == 2 ? 4 : NT == 3 ? 5 : 3);
 };
 
 template <typename R>
@@ -703,8 +712,8 @@ __device__ __forceinline__ void update_link(const Job& job, int idx, const Who<N
   store_rows(static_cast<S2*>(job.U[cur ^ 1]) + own, me, Y);
 }
 
-template <int NT, bool FULL, typename S2, bool SUMS, typename R>
-__global__ void __launch_bounds__(Cta<NT, R>::THREADS, Cta<NT, R>::MIN_CTAS)
+template <int NT, bool FULL, typename S2, bool SUMS, typename R, bool TIGHT>
+__global__ void __launch_bounds__(Cta<NT, R>::THREADS, TIGHT ? Cta<NT, R>::MIN_CTAS : 1)
     k_link(const __grid_constant__ Job one, const Job* __restrict__ table, const int2* __restrict__ items, int cur,
            double kick_scale, int mode) {
   grid_wait();

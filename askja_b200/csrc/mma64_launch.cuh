@@ -11,18 +11,18 @@
 namespace askja {
 namespace m64 {
 
-template <int NT, bool FULL, typename S2>
-cudaError_t launch_link(const Job& one, const Grid& g, int cur, double ks, int mode, cudaStream_t st) {
+template <int NT, bool FULL, typename S2, bool TIGHT>
+cudaError_t launch_link(const Job& one, const Grid& g, int ctas, int cur, double ks, int mode, cudaStream_t st) {
   // FP32 storage: the kicks and fused updates in split TF32, unless the launch
   // also sums the energies (two a trajectory: the sums take FP64 products of the
   // stored links) or only drifts (once a trajectory).  Figures beside prod.
   const bool sums = mode & (SUMS_OLD | SUMS_NEW);
   mode &= 3;
-  auto k = sums ? k_link<NT, FULL, S2, true, double> : k_link<NT, FULL, S2, false, double>;
+  auto k = sums ? k_link<NT, FULL, S2, true, double, TIGHT> : k_link<NT, FULL, S2, false, double, TIGHT>;
   size_t smem = Cta<NT>::SMEM;
   if constexpr (sizeof(S2) == 8) {
     if (!sums && mode != 2) {
-      k = k_link<NT, FULL, S2, false, float>;
+      k = k_link<NT, FULL, S2, false, float, TIGHT>;
       smem = Cta<NT, float>::SMEM;
     }
   }
@@ -30,12 +30,20 @@ cudaError_t launch_link(const Job& one, const Grid& g, int cur, double ks, int m
     const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
-  const int ctas = g.table ? g.ctas : ctas_for((long)one.V * one.D, Cta<NT>::LINKS);
   if (g.table) {  // a batch's launches depend on other streams' work: ordinary order
     k<<<ctas, Cta<NT>::THREADS, smem, st>>>(one, g.table, g.items, cur, ks, mode);
     return cudaGetLastError();
   }
   return launch_overlapped(k, ctas, Cta<NT>::THREADS, smem, st, one, g.table, g.items, cur, ks, mode);
+}
+
+// a CTA per SM at most: the loose register budget (beside Cta::MIN_CTAS)
+template <int NT, bool FULL, typename S2>
+cudaError_t launch_link(const Job& one, const Grid& g, int cur, double ks, int mode, cudaStream_t st) {
+  const int ctas = g.table ? g.ctas : ctas_for((long)one.V * one.D, Cta<NT>::LINKS);
+  if constexpr (NT == 5 || NT == 6)
+    if (ctas <= 148) return launch_link<NT, FULL, S2, false>(one, g, ctas, cur, ks, mode, st);
+  return launch_link<NT, FULL, S2, true>(one, g, ctas, cur, ks, mode, st);
 }
 
 template <int NT, bool FULL, typename S2>

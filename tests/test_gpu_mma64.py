@@ -90,6 +90,22 @@ def test_reunitarise_after_each_update_fp64(nc):
         assert rel(e.get_links(), want) < 1e-11
 
 
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("nc,dims", [(33, [5, 15]), (40, [7, 11]), (45, [75, 1]), (48, [5, 5, 2])])
+def test_more_links_than_processors(nc, dims, precision):
+    """33 <= NC <= 48 above 148 links: two CTAs per SM under the tight register budget."""
+    O, u, pi, _ = start(nc, dims, 300 + nc)
+    tol_u, tol_p = (1e-12, 1e-12) if precision == "fp64" else (1e-5, 5e-5)
+    with ab.Engine(nc, dims, beta=2.0 * nc, dt=0.02, level=8, precision=precision, reunitarise=False) as e:
+        e.set_links(u)
+        e.set_momenta(pi, 0)
+        e.leapfrog(1, 0.02)
+        p = O.updateE(u, pi, 0.01)
+        v = O.updateU(u, p, 0.02, 8)
+        assert rel(e.get_links(), v) < tol_u
+        assert rel(e.get_momenta(0), O.updateE(v, p, 0.01)) < tol_p
+
+
 @pytest.mark.parametrize("nc", [5, 8, 11, 16, 23, 31, 40, 57, 63])
 def test_split_products_keep_32_bits(nc):
     """FP32 storage multiplies in TF32 split in two; one part alone is off by 2^-12.
