@@ -119,7 +119,14 @@ __device__ __forceinline__ void stc(S2* __restrict__ p, const cpx<T>& z) {
 
 // First thing in a kernel launched with launch_overlapped (launch.h): waits
 // until the kernel before it in the stream has finished and its writes are
-// visible.  grid_done: from here on the next kernel's CTAs may be placed (it
+// visible.  What that kernel may have written must then be loaded after the
+// wait, in the compiler's eyes too, and coherently: these CTAs are resident while
+// the fields are still being written, so the promises behind ld.global.nc and
+// __restrict__ do not hold.  Such kernels therefore take no __restrict__ field (a
+// load through one is no access to the wait's "memory" and may move above it),
+// and their loads written in asm are volatile ld.global.  Only tables that stay
+// as they are while an engine lives (neighbours) go through __ldg.
+// grid_done: from here on the next kernel's CTAs may be placed (it
 // still waits for this kernel's end).  It stands before the last stores, not at
 // the start: CTAs placed while every SM still runs one of this kernel double up
 // on some SMs and leave others empty (SU(3) 8^4 FP32 4.5 us a step without

@@ -123,17 +123,34 @@ __device__ __forceinline__ void zero(AccT<R> (&c)[NT]) {
   for (int t = 0; t < NT; t++) c[t].re[0] = c[t].re[1] = c[t].im[0] = c[t].im[1] = R(0);
 }
 
-// two consecutive complex numbers of a row (c even)
+// Loads of fields that the launch does not write, coherent and volatile: k_link
+// is resident while the launch before still writes them, so they must not be
+// ld.global.nc nor move above its grid_wait (common.cuh).  Left free to move with
+// their operands (asm without volatile), the loads of NT = 1 spilt 208 bytes
+// instead of 44 in FP64.
+// Two consecutive complex numbers of a row (c even):
 __device__ __forceinline__ void ld_pair(const double2* p, Op& a, Op& b) {
-  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(a.re), "=d"(a.im), "=d"(b.re), "=d"(b.im) : "l"(p));
+  asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(a.re), "=d"(a.im), "=d"(b.re), "=d"(b.im) : "l"(p));
 }
 template <typename R>
 __device__ __forceinline__ void ld_pair(const float2* p, OpT<R>& a, OpT<R>& b) {
-  const float4 v = __ldg(reinterpret_cast<const float4*>(p));
+  float4 v;
+  asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
   a.re = v.x;
   a.im = v.y;
   b.re = v.z;
   b.im = v.w;
+}
+// one
+__device__ __forceinline__ double2 ld_value(const double2* p) {
+  double2 v;
+  asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float2 ld_value(const float2* p) {
+  float2 v;
+  asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+  return v;
 }
 // the same from memory that this launch may write, and to memory
 __device__ __forceinline__ void ld_pair_rw(const double2* p, Op& a, Op& b) {
@@ -167,7 +184,7 @@ __device__ __forceinline__ float2 pack(const float2*, double re, double im) {
 }
 template <typename R = double, typename S2>
 __device__ __forceinline__ OpT<R> ld_one(const S2* p) {
-  const S2 v = __ldg(p);
+  const S2 v = ld_value(p);
   OpT<R> o;
   o.re = (R)v.x;
   o.im = (R)v.y;
@@ -438,7 +455,7 @@ __device__ __forceinline__ void update_link(const Job& job, int idx, const Who<N
   const int V = job.V, D = job.D;
   const int x = idx / D, mu = idx - x * D;
   const size_t NN = FULL ? (size_t)64 * NT * NT : (size_t)me.n * me.n;
-  const S2* __restrict__ U = static_cast<const S2*>(job.U[cur]);
+  const S2* U = static_cast<const S2*>(job.U[cur]);
   const int* __restrict__ nbr = job.nbr;
   auto link = [&](int d, int s) { return U + ((size_t)d * V + s) * NN; };
   const size_t own = ((size_t)mu * V + x) * NN;

@@ -815,9 +815,8 @@ __device__ __forceinline__ void force_link(const Lat& L, const S2* __restrict__ 
 }
 
 template <int N, typename T, typename S2, int MODE>
-__global__ void __launch_bounds__(128) k_force(Lat L, const S2* __restrict__ U, const S2* Pin,
-                                               S2* Pout, S2* __restrict__ Uout, T eps_k, T eps_d,
-                                               int order, int reunit) {
+__global__ void __launch_bounds__(128) k_force(Lat L, const S2* U, const S2* Pin, S2* Pout, S2* Uout, T eps_k,
+                                               T eps_d, int order, int reunit) {
   grid_wait();
   const int x = blockIdx.x * 32 + (threadIdx.x & 31);
   if (x >= L.V) return;
@@ -833,9 +832,8 @@ __global__ void __launch_bounds__(128) k_force(Lat L, const S2* __restrict__ U, 
 inline bool force_ahead(int N, long V) { return N == 2 || (N == 3 && (V + 31) / 32 <= 2 * 148); }
 
 template <int N, typename T, typename S2, int MODE>
-__global__ void __launch_bounds__(128, 2) k_force_ahead(Lat L, const S2* __restrict__ U, const S2* Pin, S2* Pout,
-                                                        S2* __restrict__ Uout, T eps_k, T eps_d, int order,
-                                                        int reunit) {
+__global__ void __launch_bounds__(128, 2) k_force_ahead(Lat L, const S2* U, const S2* Pin, S2* Pout, S2* Uout, T eps_k,
+                                                        T eps_d, int order, int reunit) {
   grid_wait();
   const int x = blockIdx.x * 32 + (threadIdx.x & 31);
   if (x >= L.V) return;
@@ -861,9 +859,8 @@ __device__ __forceinline__ void force_tile_sums(const Lat& L, const S2* __restri
 }
 
 template <int N, typename T, typename S2, int MODE>
-__global__ void __launch_bounds__(128) k_force_sums(Lat L, const S2* __restrict__ U, const S2* Pin, S2* Pout,
-                                                    S2* __restrict__ Uout, T eps_k, T eps_d, int order, int reunit,
-                                                    double* __restrict__ pairs) {
+__global__ void __launch_bounds__(128) k_force_sums(Lat L, const S2* U, const S2* Pin, S2* Pout, S2* Uout, T eps_k,
+                                                    T eps_d, int order, int reunit, double* pairs) {
   grid_wait();
   force_tile_sums<N, T, S2, MODE>(L, U, Pin, Pout, Uout, eps_k, eps_d, order, reunit, blockIdx.x,
                                   pairs + 2 * (size_t)blockIdx.x);
@@ -874,8 +871,7 @@ __global__ void __launch_bounds__(128) k_force_sums(Lat L, const S2* __restrict_
 // the budget where it is faster.
 template <int N, typename T, typename S2, int MODE, int OCC = 1>
 __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 5 + OCC : 2 + OCC)
-    k_force_occ(Lat L, const S2* __restrict__ U, const S2* Pin, S2* Pout, S2* __restrict__ Uout, T eps_k, T eps_d,
-                int order, int reunit) {
+    k_force_occ(Lat L, const S2* U, const S2* Pin, S2* Pout, S2* Uout, T eps_k, T eps_d, int order, int reunit) {
   grid_wait();
   const int x = blockIdx.x * 32 + (threadIdx.x & 31);
   if (x >= L.V) return;

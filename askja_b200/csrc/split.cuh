@@ -508,9 +508,8 @@ struct Tiles {
 };
 template <int N, int MODE, int OCC>
 __global__ void __launch_bounds__(128 * Tiles<N, OCC>::PER_CTA, Tiles<N, OCC>::MIN_CTAS)
-    k_force(Lat L, const float2* __restrict__ U, const uint32_t* __restrict__ UL, const float* Pin,
-            const uint32_t* PLin, float* Pout, uint32_t* PLout, float2* __restrict__ Uout,
-            uint32_t* __restrict__ ULout, float eps_k, float eps_d, int order) {
+    k_force(Lat L, const float2* U, const uint32_t* UL, const float* Pin, const uint32_t* PLin, float* Pout,
+            uint32_t* PLout, float2* Uout, uint32_t* ULout, float eps_k, float eps_d, int order) {
   grid_wait();
   constexpr int TPC = Tiles<N, OCC>::PER_CTA;
   const int warps = (blockDim.x >> 5) / TPC, w = threadIdx.x >> 5;  // warps per tile
