@@ -383,6 +383,22 @@ __device__ __forceinline__ void link_sync(int slot) {
     asm volatile("bar.sync %0, %1;" ::"r"(slot + 1), "r"(32 * NT) : "memory");
 }
 
+// the same barrier, and whether any thread of the link says so
+template <int NT>
+__device__ __forceinline__ bool link_any(int slot, bool mine) {
+  if constexpr (NT == 1) {
+    return __any_sync(0xffffffffu, mine);
+  } else {
+    uint32_t any;
+    asm volatile(
+        "{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n bar.red.or.pred q, %2, %3, p;\n selp.u32 %0, 1, 0, q;\n}"
+        : "=r"(any)
+        : "r"((uint32_t)mine), "r"(slot + 1), "r"(32 * NT)
+        : "memory");
+    return any != 0;
+  }
+}
+
 // own rows of an accumulator to a field matrix
 template <int NT, bool FULL, typename R, typename S2>
 __device__ __forceinline__ void store_rows(S2* m, const Who<NT, FULL>& me, const AccT<R> (&c)[NT]) {
@@ -436,9 +452,15 @@ __device__ __forceinline__ double inv_factorial(int k, int order) {
 // U included, instead of 8 and 6 by Horner), formed without its identity term:
 // U' = U + (E - 1) U.  P is not assumed Hermitian.
 // FP32 storage with `project`: U' = U + (E - 1 - (U U^dag - 1) / 2) U, the
-// Newton-Schulz step on the links as read; it differs from projecting first by
+// Newton-Schulz step on the links as read; it differs from projecting U' by
 // |E - 1| times the defect that the FP32 store left, which the next update
-// removes in turn.
+// removes in turn.  That is enough while E is unitary to rounding.  Where rows
+// of U' say that it is not (low LEVEL, large steps) or that U was not (uploaded
+// links), U' takes the step itself, U' - (U' U'^dag - 1) U' / 2: one vote a link,
+// SU(8) 10^4 90.3 -> 91.0, SU(32) 6^4 541 -> 546 us a step; left to the next update,
+// links after SU(8) steps of 0.1 at LEVEL 2 were 7e-3 off U(8) instead of 5e-5.
+constexpr float ROW_TOLERANCE = 0x1p-22f;  // of a squared row length; rounding of stored entries: std 3e-8
+
 template <int NT, bool FULL, typename S2, bool SUMS, typename R>
 __device__ __forceinline__ void update_link(const Job& job, int idx, const Who<NT, FULL>& me, int slot, int cur,
                                             double kick_scale, int mode, typename Cta<NT, R>::V2* S, double (&v)[2]) {
@@ -696,13 +718,25 @@ __device__ __forceinline__ void update_link(const Job& job, int idx, const Who<N
     prod<NT, true, KU>(
         M, [&](int kb, OpT<double>(&o)[2]) { me.rows(Ux, me.w, kb, o); },
         [&](int kb, int t, OpT<double>(&o)[2]) { me.rows(Ux, t, kb, o); });
+    float d = 0.f;  // of the squared length of row r from 1
 #pragma unroll
     for (int t = 0; t < NT; t++)
 #pragma unroll
       for (int e = 0; e < 2; e++) {
         const bool diag = r == 8 * t + 2 * me.j + e && (FULL || r < me.n);
-        E[t].re[e] -= (R)(0.5 * (M[t].re[e] - (diag ? 1.0 : 0.0)));
-        E[t].im[e] -= (R)(0.5 * M[t].im[e]);
+        M[t].re[e] -= diag ? 1.0 : 0.0;
+        if (diag) d = (float)M[t].re[e];
+      }
+    d += __shfl_xor_sync(0xffffffffu, d, 1);
+    d += __shfl_xor_sync(0xffffffffu, d, 2);
+    // a row further off is left to the step on U' below
+    const double half = fabsf(d) <= ROW_TOLERANCE ? 0.5 : 0.0;
+#pragma unroll
+    for (int t = 0; t < NT; t++)
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        E[t].re[e] -= (R)(half * M[t].re[e]);
+        E[t].im[e] -= (R)(half * M[t].im[e]);
       }
   }
   // U' = U + (E - 1) U; FP32 sums the small product on its own
@@ -725,6 +759,65 @@ __device__ __forceinline__ void update_link(const Job& job, int idx, const Who<N
       Y, [&](int kb, Op(&o)[2]) { from_acc(E, kb, o); },
       [&](int kb, int t, Op(&o)[2]) { me.cols(Ux, kb, t, o); });
   if constexpr (sizeof(R) == 4) add_u();
+  if (sizeof(S2) == 8 && job.project) {
+    // rows of U' further from length 1 than rounding takes them: a Taylor sum or
+    // links that are not unitary to rounding
+    R n2 = R(0);
+#pragma unroll
+    for (int t = 0; t < NT; t++)
+#pragma unroll
+      for (int e = 0; e < 2; e++) n2 = fma(Y[t].re[e], Y[t].re[e], fma(Y[t].im[e], Y[t].im[e], n2));
+    float n = (float)n2;
+    n += __shfl_xor_sync(0xffffffffu, n, 1);
+    n += __shfl_xor_sync(0xffffffffu, n, 2);
+    const bool off = !(fabsf(n - 1.f) <= ROW_TOLERANCE) && (FULL || r < me.n);
+    if (link_any<NT>(slot, off)) {
+      tile_rows(S, me, Y);
+      link_sync<NT>(slot);
+      AccT<double> M[NT];
+      zero(M);
+      prod<NT, true, 1>(
+          M,
+          [&](int kb, OpT<double>(&o)[2]) {
+            Op a[2];
+            tile_row(S, kb, a);
+#pragma unroll
+            for (int e = 0; e < 2; e++) {
+              o[e].re = a[e].re;
+              o[e].im = a[e].im;
+            }
+          },
+          [&](int kb, int t, OpT<double>(&o)[2]) {
+            const V2* p = S + (8 * t + me.q) * CT::LD + 8 * kb + 2 * me.j;
+#pragma unroll
+            for (int e = 0; e < 2; e++) {
+              const V2 v = p[e];
+              o[e].re = v.x;
+              o[e].im = v.y;
+            }
+          });
+      Acc C[NT];
+      zero(C);
+#pragma unroll
+      for (int t = 0; t < NT; t++)
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+          const bool diag = r == 8 * t + 2 * me.j + e && (FULL || r < me.n);
+          E[t].re[e] = (R)(-0.5 * (M[t].re[e] - (diag ? 1.0 : 0.0)));
+          E[t].im[e] = (R)(-0.5 * M[t].im[e]);
+        }
+      prod<NT, false, NT>(
+          C, [&](int kb, Op(&o)[2]) { from_acc(E, kb, o); },
+          [&](int kb, int t, Op(&o)[2]) { tile_cols(S, me, kb, t, o); });
+#pragma unroll
+      for (int t = 0; t < NT; t++)
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+          Y[t].re[e] += C[t].re[e];
+          Y[t].im[e] += C[t].im[e];
+        }
+    }
+  }
   grid_done();
   store_rows(static_cast<S2*>(job.U[cur ^ 1]) + own, me, Y);
 }
