@@ -3,7 +3,8 @@
 // Many HMC chains of uneven shape (NC, DIM, extents, BETA, DT, LEVEL, seed)
 // advance together: per MD step one force launch per colour number covers
 // every chain of that colour number (work list of 32-site tiles or link
-// groups), the launches of different colour numbers run on forked streams,
+// groups; two launches where FP32 chains of one colour number multiply
+// differently, m64::tf32_force), the launches of different colour numbers run on forked streams,
 // and reductions, refresh, Metropolis and the accept/reject copy are one
 // launch each for all chains.  A whole trajectory of all chains is captured
 // once as a CUDA graph and replayed.
@@ -130,7 +131,10 @@ cudaError_t launch_force(askja_batch* b, const askja_batch::Group& g, cudaStream
     mg.table = b->d_jobs;
     mg.items = (const int2*)g.d_item;
     mg.ctas = g.nitems;
-    return askja::m64::link(g.N, sizeof(T) == 8, askja::m64::Job{}, mg, b->cur, ks, mode, st);
+    askja::m64::Job shape{};
+    shape.N = g.N;
+    shape.D = b->desc[g.chains[0]].lat.D;
+    return askja::m64::link(g.N, sizeof(T) == 8, shape, mg, b->cur, ks, mode, st);
   }
   mode &= 3;
   if (g.N == 2 || g.N == 3 || g.N == 4) {
@@ -459,13 +463,17 @@ int askja_batch_create(const askja_chain_params* chains, int nchains, int precis
     if (cudaMemcpy(b->d_jobs, jobs.data(), jobs.size() * sizeof(jobs[0]), cudaMemcpyHostToDevice) != cudaSuccess)
       return fail(berr(b, ASKJA_ERR_CUDA, "job upload"));
   }
-  // force groups: one per colour number
-  std::map<int, std::vector<int>> by_nc;
-  for (int c = 0; c < nchains; c++) by_nc[chains[c].nc].push_back(c);
+  // force groups: one per colour number (FP32, NC >= 5: and arithmetic of the force)
+  std::map<std::pair<int, bool>, std::vector<int>> by_nc;
+  for (int c = 0; c < nchains; c++) {
+    const int nc = chains[c].nc;
+    by_nc[{nc, precision != ASKJA_FP64 && askja::m64_supported(nc) && askja::m64::tf32_force(nc, chains[c].dim)}]
+        .push_back(c);
+  }
   for (auto& kv : by_nc) {
     askja_batch::Group g;
     g.chains = kv.second;
-    const int N = kv.first;
+    const int N = kv.first.first;
     std::vector<int> start(1, 0);
     std::vector<int> item;
     g.N = N;

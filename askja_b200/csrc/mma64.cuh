@@ -1,7 +1,7 @@
 // Link update, plaquette and kinetic sums for 5 <= NC <= 64 on the FP64 tensor
 // instruction (mma.sync m8n8k4 f64; tcgen05 has no FP64 kind), for FP64 and
-// FP32 storage; the kicks and fused updates of FP32 storage in TF32 split in two
-// (see prod).
+// FP32 storage; the kicks and fused updates of FP32 storage, NC >= 7 or 11, in TF32
+// split in two (see prod).
 //
 // A matrix is cut into 8 x 8 tiles (NT = ceil(NC / 8) of them a side); one warp
 // owns the eight rows 8w .. 8w+7 of every left operand and result, NT warps
@@ -38,6 +38,7 @@
 #include "launch.h"
 #include "lines.cuh"
 #include "misc.cuh"
+#include "mma64.h"
 
 namespace askja {
 namespace m64 {
@@ -86,7 +87,7 @@ struct Cta {
   static constexpr int TILES = KEEP ? 1 : 2;
   static constexpr size_t SMEM = (size_t)LINKS * TILES * TILE * sizeof(V2);
   // resident CTAs the register budget is set for, us a step beside the next choice:
-  // float at 6 / 8 and 4 / 5 / 3 CTAs (NT = 1, 2) SU(8) 10^4 90 / 93, SU(16) 6^4 74 /
+  // float (with FINE 0) at 6 / 8 and 4 / 5 / 3 CTAs (NT = 1, 2) SU(8) 10^4 90 / 93, SU(16) 6^4 74 /
   // 80 / 76; 5 / 4 / 6 (NT = 3) SU(24) 6^3 29 / 36 / 31; 3 / 4 / 2 (NT = 4) SU(32) 8^4
   // 1686 / 1749 / 1880.  NT = 5, 6: one CTA of NT warps a SM (200 to 255 registers)
   // leaves it idle at every barrier; two (168, spills of 4 to 116 bytes): SU(40) 6^3
@@ -271,15 +272,20 @@ struct Who {
 // chained, it would scale the staple sum by 1 - 1e-6), lo hi + hi lo, 2^-11
 // smaller, is chained.  Six MMAs of 2.1 SM cycles per 8 x 8 x 8 complex block
 // against 32 cycles for the eight FP64 ones (measured 276 TFLOP/s TF32, 36.8
-// FP64); what bounds it is the wait for operands and their splitting.  us per
-// fused step, FP64 MMA on FP32 storage -> split TF32: SU(8) 10^4 106 -> 90,
-// SU(5) 17x15x13 25.7 -> 23, SU(16) 6^4 102 -> 74, SU(24) 6^3 44 -> 31, SU(48)
-// 6^3 431 -> 293.  Links after 20 updates are 5.8e-8 from 64 bits at SU(8) 10^4
-// (FP64 MMA 5.4e-8, the FP32 row kernels 2.1e-7), dH 1.4e-3 (3e-4, 1.7e-2).
+// FP64); what bounds it is the wait for operands and their splitting.
+// FINE (products of the force, fine_force in mma64.h): what is left of the error
+// is the truncation of hi hi.  1: the MMAs of Re B and Im B each start from zero
+// and are added in FP32, one truncation less on the sum.  2: and the mean of what
+// truncation takes, 2^-23 / 3 of a result (half a unit in the last place of a
+// mantissa spread over its binade evenly in the logarithm), goes into the cross
+// terms.  us per fused step, FP64 MMA on FP32 storage -> split TF32: SU(8) 10^4
+// 106 -> 98 (FINE 0: 91), SU(12) 6^4 114 -> 92 (85), SU(16) 6^4 102 -> 78 (75),
+// SU(17) 6^3 46 -> 36 (35), SU(24) 6^3 43 -> 31, SU(48) 6^3 431 -> 244; SU(5)
+// 17x15x13 stays on the FP64 MMA, 28.3 against 24.9 with FINE 0 (row kernels 28.7).
 // Two row blocks a warp, sharing a right operand's split, gained nothing (SU(16)
 // 73, SU(32) 8^4 1782 against 1684); the next plane's links prefetched to L1
 // cost 3 to 10 %.
-template <int NT, bool CONJ, int KU, typename FA, typename FB>
+template <int NT, bool CONJ, int KU, int FINE = 0, typename FA, typename FB>
 __device__ __forceinline__ void prod(Acc (&c)[NT], FA&& fa, FB&& fb) {
 #pragma unroll KU
   for (int kb = 0; kb < NT; kb++) {
@@ -313,7 +319,7 @@ __device__ __forceinline__ void split_tf32(float x, uint32_t& hi, uint32_t& lo) 
   lo = __float_as_uint(x - __uint_as_float(hi));
 }
 
-template <int NT, bool CONJ, int KU, typename FA, typename FB>
+template <int NT, bool CONJ, int KU, int FINE = 0, typename FA, typename FB>
 __device__ __forceinline__ void prod(AccT<float> (&c)[NT], FA&& fa, FB&& fb) {
   float cor[NT][4];
 #pragma unroll
@@ -345,7 +351,17 @@ __device__ __forceinline__ void prod(AccT<float> (&c)[NT], FA&& fa, FB&& fb) {
       }
       float m[4] = {0.f, 0.f, 0.f, 0.f};
       tmma(m, h1, rh);
-      tmma(m, h2, ih);
+      if constexpr (FINE > 0) {
+        float m2[4] = {0.f, 0.f, 0.f, 0.f};
+        tmma(m2, h2, ih);
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          m[i] += m2[i];
+          if constexpr (FINE > 1) cor[t][i] = fmaf(m[i], 0x1.555556p-25f, cor[t][i]);
+        }
+      } else {
+        tmma(m, h2, ih);
+      }
       tmma(cor[t], l1, rh);
       tmma(cor[t], l2, ih);
       tmma(cor[t], h1, rl);
@@ -473,6 +489,7 @@ __device__ __forceinline__ void update_link(const Job& job, int idx, const Who<N
   // of instruction cache: SU(32) 8^4 2040 us a step, by two 1684, by one 1727; SU(24)
   // 6^3 30.5 unrolled, 32.3 by one; FP64 SU(32) 6^4 720 unrolled, 749 by two)
   constexpr int KU = NT < 4 ? NT : NT > 4 ? 1 : sizeof(R) == 4 ? 2 : 4;
+  constexpr int FINE = fine_force(NT, FULL);
   const int lane = threadIdx.x & 31;
   const int V = job.V, D = job.D;
   const int x = idx / D, mu = idx - x * D;
@@ -526,17 +543,17 @@ __device__ __forceinline__ void update_link(const Job& job, int idx, const Who<N
       {
         const S2 *a = link(nu, xpmu), *b = link(mu, xpnu), *y = link(nu, x);
         zero(T);
-        prod<NT, true, KU>(
+        prod<NT, true, KU, FINE>(
             T, [&](int kb, Op(&o)[2]) { me.rows(a, me.w, kb, o); },
             [&](int kb, int t, Op(&o)[2]) { me.rows(b, t, kb, o); });
-        prod<NT, true, NT>(
+        prod<NT, true, NT, FINE>(
             W, [&](int kb, Op(&o)[2]) { from_acc(T, kb, o); },
             [&](int kb, int t, Op(&o)[2]) { me.rows(y, t, kb, o); });
       }
       {
         const S2 *a = link(nu, xpmu_mnu), *b = link(mu, xmnu), *y = link(nu, xmnu);
         zero(T);
-        prod<NT, true, KU>(
+        prod<NT, true, KU, FINE>(
             T,
             [&](int kb, Op(&o)[2]) {
               me.cols(a, kb, me.w, o);
@@ -544,7 +561,7 @@ __device__ __forceinline__ void update_link(const Job& job, int idx, const Who<N
               o[1].im = -o[1].im;
             },
             [&](int kb, int t, Op(&o)[2]) { me.rows(b, t, kb, o); });
-        prod<NT, false, NT>(
+        prod<NT, false, NT, FINE>(
             W, [&](int kb, Op(&o)[2]) { from_acc(T, kb, o); },
             [&](int kb, int t, Op(&o)[2]) { me.cols(y, kb, t, o); });
       }
@@ -552,7 +569,7 @@ __device__ __forceinline__ void update_link(const Job& job, int idx, const Who<N
     tile_rows(S, me, W);
     link_sync<NT>(slot);
     zero(W);
-    prod<NT, false, KU>(
+    prod<NT, false, KU, FINE>(
         W, [&](int kb, Op(&o)[2]) { me.rows(Ux, me.w, kb, o); },
         [&](int kb, int t, Op(&o)[2]) { tile_cols(S, me, kb, t, o); });
     link_sync<NT>(slot);

@@ -13,15 +13,16 @@ namespace m64 {
 
 template <int NT, bool FULL, typename S2, bool TIGHT>
 cudaError_t launch_link(const Job& one, const Grid& g, int ctas, int cur, double ks, int mode, cudaStream_t st) {
-  // FP32 storage: the kicks and fused updates in split TF32, unless the launch
-  // also sums the energies (two a trajectory: the sums take FP64 products of the
-  // stored links) or only drifts (once a trajectory).  Figures beside prod.
+  // FP32 storage: the kicks and fused updates in split TF32 where that is as exact
+  // (tf32_force), unless the launch also sums the energies (two a trajectory: the
+  // sums take FP64 products of the stored links) or only drifts (once a trajectory).
+  // Figures beside prod.
   const bool sums = mode & (SUMS_OLD | SUMS_NEW);
   mode &= 3;
   auto k = sums ? k_link<NT, FULL, S2, true, double, TIGHT> : k_link<NT, FULL, S2, false, double, TIGHT>;
   size_t smem = Cta<NT>::SMEM;
   if constexpr (sizeof(S2) == 8) {
-    if (!sums && mode != 2) {
+    if (!sums && mode != 2 && tf32_force(one.N, one.D)) {
       k = k_link<NT, FULL, S2, false, float, TIGHT>;
       smem = Cta<NT, float>::SMEM;
     }
