@@ -203,9 +203,11 @@ cudaError_t drift_launch(askja_ctx* c, double eps) {
   if (c->split)
     return askja::splitk::drift(c->lc, cur_u(c), cur_ul(c), c->P2C, c->P2CL, c->PC, c->PCL, eps);
   if (askja::link_major(c->N) && c->lc.force_rows != 1) {
-    const cudaError_t e = c->ks->force(c->lc, 2, cur_u(c), c->P2, nullptr, c->U[1 - c->cur], 0.0, eps);
+    const bool tensor = c->lc.force_rows == 2;  // leaves the copy to the caller
+    const cudaError_t e =
+        c->ks->force(c->lc, 2, cur_u(c), c->P2, tensor ? nullptr : c->P, c->U[1 - c->cur], 0.0, eps);
     if (e == cudaSuccess) c->cur ^= 1;
-    return e == cudaSuccess ? copy_down(c) : e;
+    return e == cudaSuccess && tensor ? copy_down(c) : e;
   }
   return c->ks->drift(c->lc, cur_u(c), c->P2, c->P, eps);
 }

@@ -151,8 +151,11 @@ cudaError_t m64_link(const LaunchCtx& c, int mode, const void* U, const void* Pi
                      double ed) {
   m64::Job j = m64_job(c.lat);
   j.order = c.order;
-  // FP32 single chains: projected to first order in the kernel (as rows_ns); otherwise in full afterwards
-  const bool ns = sizeof(T) == 4 && c.rows_ns && (mode & 3) == 1;
+  // FP32 single chains: projected in the kernel (as rows_ns); otherwise in full afterwards.  A drift of its own
+  // is projected in full too, but for NC = 32, whose Gram-Schmidt pass takes 510 us for the 49 us of the update
+  // (4^4; 101 us in all when the tensor-core path, which does not pin the determinant either, was the default).
+  const int N = c.lat.N, kind = mode & 3;
+  const bool ns = sizeof(T) == 4 && c.rows_ns && (kind == 1 || (kind == 2 && N == 32));
   j.project = c.reunit && ns;
   j.U[0] = const_cast<void*>(U);
   j.U[1] = Uout;
@@ -162,8 +165,8 @@ cudaError_t m64_link(const LaunchCtx& c, int mode, const void* U, const void* Pi
   j.dt = ed;
   j.pairs = c.pairs;
   j.ctas = sum_ctas(c.lat);
-  cudaError_t e = m64::link(c.lat.N, sizeof(T) == 8, j, m64::Grid{}, 0, 1.0, mode, c.stream);
-  if (e != cudaSuccess || (mode & 3) == 0 || !c.reunit || ns) return e;
+  cudaError_t e = m64::link(N, sizeof(T) == 8, j, m64::Grid{}, 0, 1.0, mode, c.stream);
+  if (e != cudaSuccess || kind == 0 || !c.reunit || ns) return e;
   LaunchCtx full = c;
   full.gate = nullptr;
   return reunit<T>(full, Uout);

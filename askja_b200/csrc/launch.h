@@ -116,7 +116,7 @@ inline bool pair_supported(int N, int D, bool fp64, int n_fast) {
 //   gauss    -> out[0]
 struct KernelSet {
   // mode 0: Pout = Pin - ek F(U); mode 1: also Uout = exp(i ed Pout) U;
-  // mode 2 (FP64 MMA and tensor cores): Uout = exp(i ed Pin) U
+  // mode 2 (NC >= 5): Uout = exp(i ed Pin) U; warp MMA also Pout = Pin
   cudaError_t (*force)(const LaunchCtx&, int mode, const void* U, const void* Pin, void* Pout, void* Uout, double ek,
                        double ed);
   // U = exp(i eps P) U in place and Pcopy = P

@@ -459,7 +459,7 @@ __device__ __forceinline__ double inv_factorial(int k, int order) {
 }
 
 // mode 0: Pout = Pin - kick F(U);  1: the same, and Uout = exp(i dt Pout) U;
-// 2: Uout = exp(i dt Pin) U.  SUMS (mode 0, 1): v += (ReTr W, ReTr P P) of own
+// 2: Uout = exp(i dt Pin) U and Pout = Pin.  SUMS (mode 0, 1): v += (ReTr W, ReTr P P) of own
 // rows, P after a kick alone (the end of a trajectory), before a kick and drift
 // (its start).
 //
@@ -612,11 +612,13 @@ __device__ __forceinline__ void update_link(const Job& job, int idx, const Who<N
     if (mode == 0) return;
   } else {
     const S2* P = static_cast<const S2*>(job.Pin) + own;
+    S2* Po = static_cast<S2*>(job.Pout) + own;
     const R ed = (R)job.dt;
 #pragma unroll
     for (int t = 0; t < NT; t++) {
       Op p[2];
       me.rows(P, me.w, t, p);
+      me.put(Po, t, p);
 #pragma unroll
       for (int e = 0; e < 2; e++) {
         X[t].re[e] = -ed * p[e].im;

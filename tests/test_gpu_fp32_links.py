@@ -1,6 +1,8 @@
 """FP32 storage, NC >= 5 (warp MMA): every fused update projects the new links,
 at any order of the exponential, and a force is no further from 64 bits than
 FP32 FMAs put it."""
+import time
+
 import numpy as np
 import pytest
 
@@ -65,6 +67,35 @@ def test_first_update_of_a_trajectory_is_projected(nc, dims):
             pytest.fail("no trajectory was accepted")
         v = projected_update(O, u, O.updateE(u, pi, eps / 2), eps, level)
         assert rel(e.get_links(), v) < 1e-5
+
+
+@pytest.mark.parametrize("level", [1, 8])
+def test_su32_drift_is_projected_and_cheap(level):
+    """updateUandcopyDown of FP32 SU(32): one Newton-Schulz step in the update's own
+    launch, no Gram-Schmidt pass, which took several times a whole fused step."""
+    nc, dims, eps = 32, [4, 4, 4, 4], 0.02
+    rng = np.random.default_rng(32)
+    O = Oracle(nc, dims)
+    nl = O.vol * O.dim
+    u = fields.haar(nc, nl, rng).reshape(O.shape)
+    pi = np.asarray(fields.momenta(nc, nl, 2.0 * nc, rng, O)).reshape(O.shape)
+    with ab.Engine(nc, dims, beta=2.0 * nc, dt=eps, level=level, precision="fp32") as e:
+        e.set_links(u)
+        e.set_momenta(pi, 1)
+        e.updateUandcopyDown(eps)
+        assert rel(e.get_links(), projected_update(O, u, pi, eps, level)) < 1e-5
+        np.testing.assert_array_equal(e.get_momenta(0), e.get_momenta(1))
+
+        def median(f):
+            t = []
+            for _ in range(21):
+                start = time.perf_counter()
+                f()
+                t.append(time.perf_counter() - start)
+            return sorted(t)[10]
+
+        # one fused update and one kick, against one update alone
+        assert median(lambda: e.updateUandcopyDown(eps)) < median(lambda: e.leapfrog(1, eps))
 
 
 def fma_force(u, dims):
