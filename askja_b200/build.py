@@ -36,7 +36,7 @@ CU_SOURCES = ["kernels_fp64.cu", "kernels_fp32.cu", "kernels_split.cu", "engine.
 PEAK_SRC = "peak.cu"
 PEAK_LIB = os.path.join(HERE, "libaskja_peak.so")
 CPP_SOURCES = ["hostio.cpp"]
-HEADERS = ["common.cuh", "small.cuh", "rows.cuh", "misc.cuh", "kernels.cuh", "launch.h", "batch.cuh", "tc.cuh", "eig.cuh", "pair.cuh", "tab.cuh", "split.cuh", "split.h",
+HEADERS = ["common.cuh", "small.cuh", "rows.cuh", "misc.cuh", "kernels.cuh", "launch.h", "budget.h", "batch.cuh", "tc.cuh", "eig.cuh", "pair.cuh", "tab.cuh", "split.cuh", "split.h",
            "mma64.cuh", "mma64.h", "mma64_launch.cuh", "lines.cuh"]
 
 

@@ -108,7 +108,7 @@ cudaError_t small_force(const LaunchCtx& c, int mode, const void* U, const void*
   }
   if (mode > 1) return cudaErrorInvalidValue;
   if constexpr (sizeof(T) == 8 && N <= 3) {
-    if (c.small_occ == 0 && small::force_ahead(N, c.lat.V)) {
+    if (c.small_occ == 0 && force_ahead(N, c.lat.V)) {
       auto ka = mode == 0 ? small::k_force_ahead<N, T, S2, 0> : small::k_force_ahead<N, T, S2, 1>;
       return launch_overlapped(ka, grid, threads, 0, c.stream, c.lat, u, pi, (S2*)Pout, (S2*)Uout, ek, ed, c.order,
                                c.reunit);

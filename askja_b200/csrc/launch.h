@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "budget.h"
 #include "common.cuh"
 
 namespace askja {
@@ -90,20 +91,6 @@ inline bool tc_supported(int N, int D, bool fp64) { return !fp64 && (N == 16 || 
 
 // whether the warp-MMA mapping exists for this colour number
 inline bool m64_supported(int N) { return link_major(N); }
-
-// Untuned register budget (LaunchCtx::small_occ) of the thread-per-link kernels,
-// by 32-site tiles.  Measured us per step at budget 0 and 2:
-//  FP32 (residual planes), NC = 2, 3: with more tiles than four CTAs per SM
-//   hold, the tight budget's seven CTAs hide more latency (SU(3) 32^4 469 / 443,
-//   SU(2) 16^4 15.5 / 12.9); below, the loose one's extra loads in flight win
-//   (SU(3) 12^4 11.3 / 11.1, 10^4 7.4 / 8.4, 8^4 4.5 / 6.5).  NC = 4 spills at 2.
-//  FP64, NC = 2: the budgets are the other way round (80 and 126 registers):
-//   10^4 6.8 / 5.6, 16^4 19.5 / 19.0, 32^4 308 / 326.  NC = 3: no difference.
-inline int default_occupancy(int N, bool fp64, bool residual, long V) {
-  const long tiles = (V + 31) / 32;
-  if (fp64) return N == 2 && tiles <= 2048 ? 2 : 0;
-  return residual && N <= 3 && tiles > 4 * 148 ? 2 : 0;
-}
 
 // whether the site-pair mapping exists (n_fast: extent of the fastest direction)
 inline bool pair_supported(int N, int D, bool fp64, int n_fast) {

@@ -825,12 +825,7 @@ __global__ void __launch_bounds__(128) k_force(Lat L, const S2* U, const S2* Pin
 }
 
 // FP64 with the links of the next staple in flight: at most two CTAs per SM (234
-// registers for N = 3), which is all a lattice of force_ahead's size has.  us
-// per graph-replayed step, SU(3) 8^4 6.3 -> 5.6, 16^3 5.2 -> 4.3; with three
-// resident CTAs to hide the loads the plain kernel wins (10^4 11.0 / 12.2, 32^4
-// 909 / 954).  N = 2 has the registers at any size (32^4 389 -> 376).
-inline bool force_ahead(int N, long V) { return N == 2 || (N == 3 && (V + 31) / 32 <= 2 * 148); }
-
+// registers for N = 3), which is all a lattice of force_ahead's size (budget.h) has.
 template <int N, typename T, typename S2, int MODE>
 __global__ void __launch_bounds__(128, 2) k_force_ahead(Lat L, const S2* U, const S2* Pin, S2* Pout, S2* Uout, T eps_k,
                                                         T eps_d, int order, int reunit) {
