@@ -30,4 +30,17 @@ inline int default_occupancy(int N, bool fp64, bool residual, long V) {
   return residual && N <= 3 && tiles > 4 * 148 ? 2 : 0;
 }
 
+// A mapping tuned on one lattice serves later ones of the same (NC, DIM,
+// precision); the thread-per-link budget (path 0) is carried only to lattices on
+// the same side of the rules above, others take their own untuned one.
+// Otherwise tuning FP32 SU(3) 8^4 (budget 0) cost every later 32^4 6 %, the reverse
+// every later 8^4 44 %.
+inline int carried_occupancy(int tuned, int path, int N, bool fp64, bool residual, long V_tuned, long V) {
+  if (path != 0) return tuned;
+  const int here = default_occupancy(N, fp64, residual, V);
+  const bool same = here == default_occupancy(N, fp64, residual, V_tuned) &&
+                    (!fp64 || force_ahead(N, V) == force_ahead(N, V_tuned));
+  return same ? tuned : here;
+}
+
 }  // namespace askja

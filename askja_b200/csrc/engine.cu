@@ -51,7 +51,8 @@ static thread_local std::string g_last_error;
 
 // autotuning results of this process, per (NC, DIM, precision)
 static std::mutex g_tune_mutex;
-static std::map<std::tuple<int, int, int>, askja_tuning> g_tune_cache;
+// the choice and the sites of the lattice it was timed on
+static std::map<std::tuple<int, int, int>, std::pair<askja_tuning, long>> g_tune_cache;
 
 // doubles of scalar results in front of the per-line results
 constexpr int SUMS = 8;
@@ -616,10 +617,13 @@ int askja_create(const askja_params* p, askja_ctx** out) {
     std::lock_guard<std::mutex> lock(g_tune_mutex);
     auto it = g_tune_cache.find(std::make_tuple(p->nc, p->dim, p->precision));
     if (it != g_tune_cache.end() &&
-        (it->second.path != 3 || askja::pair_supported(p->nc, p->dim, p->precision == ASKJA_FP64, p->n[p->dim - 1]))) {
-      c->lc.force_rows = it->second.path;
-      c->lc.rows_groups = it->second.groups;
-      c->lc.small_occ = it->second.occupancy;
+        (it->second.first.path != 3 ||
+         askja::pair_supported(p->nc, p->dim, p->precision == ASKJA_FP64, p->n[p->dim - 1]))) {
+      const askja_tuning& t = it->second.first;
+      c->lc.force_rows = t.path;
+      c->lc.rows_groups = t.groups;
+      c->lc.small_occ = askja::carried_occupancy(t.occupancy, t.path, p->nc, p->precision == ASKJA_FP64, c->split,
+                                                 it->second.second, V);
     }
   }
   // cold start by default
@@ -1240,7 +1244,7 @@ int askja_autotune(askja_ctx* c, int reps, askja_tuning* out) {
   if (int rc = askja_set_tuning(c, &res)) return rc;
   {
     std::lock_guard<std::mutex> lock(g_tune_mutex);
-    g_tune_cache[std::make_tuple(c->N, c->D, c->p.precision)] = res;
+    g_tune_cache[std::make_tuple(c->N, c->D, c->p.precision)] = {res, c->V};
   }
   if (out) *out = res;
   return ASKJA_OK;

@@ -245,7 +245,8 @@ typedef struct {
 /* Times every candidate on this context's lattice (reps launches each, on
  * scratch copies of the fields -- u and pi are left unchanged, Pi is
  * overwritten), switches the context to the fastest and remembers it for
- * later contexts with the same (NC, DIM, precision) in this process. */
+ * later contexts with the same (NC, DIM, precision) in this process (the register
+ * budget of the thread-per-link kernels: for those of a similar size). */
 ASKJA_API int askja_autotune(askja_ctx* ctx, int reps, askja_tuning* out);
 /* Applies a previously found mapping (for example read back from a file). */
 ASKJA_API int askja_set_tuning(askja_ctx* ctx, const askja_tuning* t);
