@@ -3,6 +3,7 @@
 #pragma once
 
 #include <algorithm>
+#include <type_traits>
 
 #include "launch.h"
 #include "mma64.cuh"
@@ -329,13 +330,19 @@ cudaError_t plaq(const LaunchCtx& c, const void* U, double* partial, double* out
     return m64::plaq(N, sizeof(T) == 8, j, m64::Grid{}, 0, c.stream);
   }
   const unsigned nb = blocks_for(c.lat.V, misc::RED_THREADS);
+  unsigned* ticket = nullptr;
+  auto go = [&](auto n) {
+    constexpr int NN = decltype(n)::value;
+    ticket = misc::one_launch<misc::k_plaq<NN, S2>>(nb, misc::ticket_waves(sizeof(T) == 8, NN, false), c.ticket);
+    misc::k_plaq<NN, S2><<<nb, misc::RED_THREADS, 0, c.stream>>>(c.lat, (const S2*)U, partial, out, ticket);
+  };
   if (N == 2)
-    misc::k_plaq<2, S2><<<nb, misc::RED_THREADS, 0, c.stream>>>(c.lat, (const S2*)U, partial, out, c.ticket);
+    go(std::integral_constant<int, 2>{});
   else if (N == 3)
-    misc::k_plaq<3, S2><<<nb, misc::RED_THREADS, 0, c.stream>>>(c.lat, (const S2*)U, partial, out, c.ticket);
+    go(std::integral_constant<int, 3>{});
   else
-    misc::k_plaq<4, S2><<<nb, misc::RED_THREADS, 0, c.stream>>>(c.lat, (const S2*)U, partial, out, c.ticket);
-  return cudaGetLastError();
+    go(std::integral_constant<int, 4>{});
+  return misc::total<2>(nb, partial, out, ticket, c.stream);
 }
 
 template <typename T>
@@ -355,16 +362,20 @@ cudaError_t linksums(const LaunchCtx& c, const void* Pa, const void* Pb, const v
     return U ? m64::uviol(N, fp64, j, c.stream) : m64::kinetic(fp64, j, m64::Grid{}, c.stream);
   }
   const unsigned nb = blocks_for(nlinks(c.lat), misc::RED_THREADS);
+  unsigned* ticket = nullptr;
+  auto go = [&](auto n) {
+    constexpr int NN = decltype(n)::value;
+    ticket = misc::one_launch<misc::k_linksums<NN, S2>>(nb, misc::ticket_waves(sizeof(T) == 8, NN, true), c.ticket);
+    misc::k_linksums<NN, S2><<<nb, misc::RED_THREADS, 0, c.stream>>>(c.lat, (const S2*)Pa, (const S2*)Pb,
+                                                                    (const S2*)U, partial, out, ticket);
+  };
   if (N == 2)
-    misc::k_linksums<2, S2><<<nb, misc::RED_THREADS, 0, c.stream>>>(c.lat, (const S2*)Pa, (const S2*)Pb,
-                                                                    (const S2*)U, partial, out, c.ticket);
+    go(std::integral_constant<int, 2>{});
   else if (N == 3)
-    misc::k_linksums<3, S2><<<nb, misc::RED_THREADS, 0, c.stream>>>(c.lat, (const S2*)Pa, (const S2*)Pb,
-                                                                    (const S2*)U, partial, out, c.ticket);
+    go(std::integral_constant<int, 3>{});
   else
-    misc::k_linksums<4, S2><<<nb, misc::RED_THREADS, 0, c.stream>>>(c.lat, (const S2*)Pa, (const S2*)Pb,
-                                                                    (const S2*)U, partial, out, c.ticket);
-  return cudaGetLastError();
+    go(std::integral_constant<int, 4>{});
+  return misc::total<3>(nb, partial, out, ticket, c.stream);
 }
 
 // groups (NC >= 5) or CTAs whose partial matrices the Gauss law sums

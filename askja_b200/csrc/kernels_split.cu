@@ -85,9 +85,10 @@ cudaError_t plaq(const LaunchCtx& c, const void* U, const void* UL, double* part
   const unsigned nb = blocks_for(c.lat.V, misc::RED_THREADS);
   return by_nc(c.lat.N, [&](auto n) {
     constexpr int N = decltype(n)::value;
+    unsigned* ticket = misc::one_launch<split::k_plaq<N>>(nb, misc::ticket_waves(false, N, false), c.ticket);
     split::k_plaq<N><<<nb, misc::RED_THREADS, 0, c.stream>>>(c.lat, (const float2*)U, (const uint32_t*)UL, partial,
-                                                                 out, c.ticket);
-    return cudaGetLastError();
+                                                                 out, ticket);
+    return misc::total<2>(nb, partial, out, ticket, c.stream);
   });
 }
 
@@ -96,10 +97,11 @@ cudaError_t linksums(const LaunchCtx& c, const void* Pa, const void* PLa, const 
   const unsigned nb = blocks_for(nlinks(c.lat), misc::RED_THREADS);
   return by_nc(c.lat.N, [&](auto n) {
     constexpr int N = decltype(n)::value;
+    unsigned* ticket = misc::one_launch<split::k_linksums<N>>(nb, misc::ticket_waves(false, N, true), c.ticket);
     split::k_linksums<N><<<nb, misc::RED_THREADS, 0, c.stream>>>(
         c.lat, (const float*)Pa, (const uint32_t*)PLa, (const float*)Pb, (const uint32_t*)PLb, (const float2*)U,
-        (const uint32_t*)UL, partial, out, c.ticket);
-    return cudaGetLastError();
+        (const uint32_t*)UL, partial, out, ticket);
+    return misc::total<3>(nb, partial, out, ticket, c.stream);
   });
 }
 

@@ -58,7 +58,8 @@ __global__ void k_finish(const double* __restrict__ partial, int nblocks, double
 // Writes this block's K sums (in thread 0) to the partials and lets the last
 // block to do so add them up, in block order whatever the finishing order, into
 // out (not null): no launch of its own for the total.  *ticket counts the
-// blocks, zero before and after.
+// blocks, zero before and after.  Without a ticket k_finish adds the partials up,
+// in the same order (one_launch).
 template <int K>
 __device__ __forceinline__ void publish(const double (&v)[K], double* __restrict__ partial, double* __restrict__ out,
                                         unsigned* ticket) {
@@ -66,9 +67,11 @@ __device__ __forceinline__ void publish(const double (&v)[K], double* __restrict
   if (threadIdx.x == 0) {
 #pragma unroll
     for (int k = 0; k < K; k++) partial[(size_t)blockIdx.x * K + k] = v[k];
+    if (!ticket) return;
     __threadfence();
     last = atomicAdd(ticket, 1u) == gridDim.x - 1;
   }
+  if (!ticket) return;
   __syncthreads();
   if (!last) return;
   __threadfence();
@@ -85,6 +88,34 @@ __device__ __forceinline__ void publish(const double (&v)[K], double* __restrict
     for (int k = 0; k < K; k++) out[k] = s[k];
     *ticket = 0;
   }
+}
+
+// The ticket for a reduction of nb blocks by KERNEL, or none above so many waves of
+// its resident blocks.  A block waits for its fence and its number before it leaves
+// its SM, about 1.2 us of each wave, unless other blocks' loads fill that time; the
+// launch of k_finish takes 1 to 3 us.
+template <auto KERNEL>
+unsigned* one_launch(unsigned nb, unsigned waves, unsigned* ticket) {
+  static const unsigned resident = [] {
+    int n = 0;
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, KERNEL, RED_THREADS, 0) == cudaSuccess ? n : 1;
+  }();
+  return nb <= (size_t)waves * 148 * resident ? ticket : nullptr;
+}
+// The waves, us a call with a ticket / without.  FP64 fields: SU(2) 32^4 kinetic
+// (15 waves) 91 / 96, SU(3) 24^4 57.1 / 58.5, 32^4 plaquettes (14) 263 / 260; SU(4)
+// 16^4 kinetic (3.5) 32.2 / 34.6, 24^4 (17) 90.8 / 81.1.  FP32: plaquettes SU(3) 24^4
+// (4.4) 139.7 / 141.8, 32^4 (14) 373 / 364; kinetic SU(2) 24^4 (4.4) 40.4 / 42.8, 32^4
+// (14) 90 / 80; SU(3) 24^4 (7) 53.0 / 46.1, 32^4 121 / 105; UViol SU(4) 16^4 (2.3) 40.4
+// / 33.1.
+constexpr unsigned ticket_waves(bool fp64, int N, bool links) {
+  return fp64 ? (N <= 3 ? 1u << 20 : 4) : N == 2 || !links ? 5 : 2;
+}
+// The sums of a reduction that had no ticket.
+template <int K>
+cudaError_t total(unsigned nb, const double* partial, double* out, const unsigned* ticket, cudaStream_t st) {
+  if (!ticket) k_finish<K><<<1, RED_THREADS, 0, st>>>(partial, (int)nb, out);
+  return cudaGetLastError();
 }
 
 // Plaquette sums per site (sun.cpp:507-537 EnergyMag; measurements4d.cpp:885-927
