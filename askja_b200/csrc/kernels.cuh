@@ -428,7 +428,11 @@ cudaError_t line_traces(const LaunchCtx& c, const void* U, const LineSet& ls, do
 template <typename T>
 cudaError_t slice_trace(const LaunchCtx& c, const void* U, double* out) {
   using S2 = typename Storage<T>::type;
-  misc::k_slice_trace<S2><<<c.lat.n[0], misc::SLICE_THREADS, 0, c.stream>>>(c.lat, (const S2*)U, out);
+  if (link_major(c.lat.N))
+    misc::k_slice_trace_major<S2><<<c.lat.n[0] * misc::SLICE_CTAS, misc::RED_THREADS, 0, c.stream>>>(
+        c.lat, (const S2*)U, out);
+  else
+    misc::k_slice_trace<S2><<<c.lat.n[0], misc::SLICE_THREADS, 0, c.stream>>>(c.lat, (const S2*)U, out);
   return cudaGetLastError();
 }
 

@@ -8,6 +8,8 @@
 // cases (fully unrolled) and NT = 0 for any NC (runtime loops).
 #pragma once
 
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 
 namespace askja {
@@ -237,21 +239,21 @@ __global__ void __launch_bounds__(RED_THREADS) k_linksums(Lat L, const S2* __res
 }
 
 // Slice averages for measurements4d.cpp:357-408 scalarLoopcorr:
-// out[x0] = mean over the x0-slice of ReTr U_{D-1} / NC.  One CTA per slice, of
-// as many threads as there may be: the slices are few and their loads are all
-// the kernel does (SU(3) 16^4: 22 us with 256 threads).
+// out[x0] = mean over the x0-slice of ReTr U_{D-1} / NC.  Blocked fields: one CTA
+// per slice, of as many threads as there may be: the slices are few and their loads
+// are all the kernel does (SU(3) 16^4: 22 us with 256 threads).
 constexpr int SLICE_THREADS = 1024;
 template <typename S2>
 __global__ void __launch_bounds__(SLICE_THREADS) k_slice_trace(Lat L, const S2* __restrict__ U,
                                                                double* __restrict__ out) {
   __shared__ double sh[SLICE_THREADS / 32];
-  const int N = L.N, es = estride(L);
+  const int N = L.N;
   const int slice = L.stride[0];
   double v = 0.0;
   for (int s = blockIdx.x * slice + threadIdx.x; s < (blockIdx.x + 1) * slice; s += SLICE_THREADS) {
-    const S2* p = U + mbase(L, L.D - 1, s);
+    const S2* p = U + bbase(L, L.D - 1, s);
     double t = 0.0;
-    for (int k = 0; k < N; k++) t += (double)p[(size_t)k * (N + 1) * es].x;
+    for (int k = 0; k < N; k++) t += (double)p[(size_t)k * (N + 1) * 32].x;
     v += t / N;
   }
 #pragma unroll
@@ -264,6 +266,37 @@ __global__ void __launch_bounds__(SLICE_THREADS) k_slice_trace(Lat L, const S2* 
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
     if (threadIdx.x == 0) out[blockIdx.x] = v / slice;
   }
+}
+
+// The same for link-major fields, where a diagonal element lies in a sector of its
+// own: a cluster of CTAs per slice, since one SM fetches sectors too slowly, and a
+// thread per element (us a call, with a CTA per slice and a thread per site / so:
+// SU(12) 8^4 30 / 25.7, SU(32) 6^4 30 / 26, SU(64) 4^4 30 / 23).
+constexpr int SLICE_CTAS = 8;
+template <typename S2>
+__global__ void __cluster_dims__(SLICE_CTAS, 1, 1) __launch_bounds__(RED_THREADS)
+    k_slice_trace_major(Lat L, const S2* __restrict__ U, double* __restrict__ out) {
+  namespace cg = cooperative_groups;
+  const cg::cluster_group cluster = cg::this_cluster();
+  __shared__ double part;
+  const int N = L.N, slice = L.stride[0], x0 = blockIdx.x / SLICE_CTAS;
+  const S2* p = U + mbase(L, L.D - 1, x0 * slice);
+  const long n = (long)slice * N;
+  double v[1] = {0.0};
+#pragma unroll 4
+  for (long q = (long)cluster.block_rank() * RED_THREADS + threadIdx.x; q < n; q += SLICE_CTAS * RED_THREADS) {
+    const long s = q / N;
+    v[0] += (double)p[s * (N * N) + (q - s * N) * (N + 1)].x;
+  }
+  block_sum<1>(v);
+  if (threadIdx.x == 0) part = v[0];
+  cluster.sync();
+  if (cluster.block_rank() == 0 && threadIdx.x == 0) {
+    double t = 0.0;
+    for (int r = 0; r < SLICE_CTAS; r++) t += *cluster.map_shared_rank(&part, r);
+    out[x0] = t / ((double)N * slice);
+  }
+  cluster.sync();  // the others' shared memory stays until it has been read
 }
 
 // Momentum refresh (sun.cpp:209-252 initializeE with the reference's

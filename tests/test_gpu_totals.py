@@ -1,5 +1,6 @@
 """Reductions whose total is added up by the last block or, from a number of
-blocks on, by a launch of its own, against plain torch in 64 bits on the engine's own fields.
+blocks on, by a launch of its own, and the slice averages of link-major fields,
+against plain torch in 64 bits on the engine's own fields.
 
 Tolerance: sums of at most 2e7 terms in FP64, whatever the order, are within
 2e7 * 1.1e-16 of their terms' absolute sum in the worst case, and the terms are
@@ -51,3 +52,14 @@ def test_sums_of_few_and_of_many_blocks(nc, dims, precision):
         e.set_links(1.01 * u)
         viol = torch_sums(e.get_links(), p, dims, nc)[2]
         assert e.UViol() == pytest.approx(viol, rel=1e-8)
+
+
+# slices of fewer elements than threads, of a ragged number, and of several passes
+@pytest.mark.parametrize("nc,dims,precision", [(5, [3, 1], "fp64"), (5, [2, 3, 7], "fp32"), (12, [3, 8, 8, 8], "fp64"),
+                                               (16, [5, 9, 11], "fp32"), (64, [4, 4, 4, 4], "fp64"), (33, [3, 5, 3], "fp64")])
+def test_slice_averages_of_link_major_fields(nc, dims, precision):
+    with ab.Engine(nc, dims, beta=2.0 * nc, precision=precision, seed=5) as e:
+        e.hot_start(3)
+        u = e.get_links().reshape(dims[0], -1, len(dims), nc, nc)[:, :, -1]
+        want = np.trace(u, axis1=-2, axis2=-1).real.mean(1) / nc
+        np.testing.assert_allclose(e.scalarLoopcorr(), want, rtol=0, atol=1e-12)
