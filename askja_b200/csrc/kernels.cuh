@@ -264,6 +264,7 @@ cudaError_t force(const LaunchCtx& c, int mode, const void* U, const void* Pin, 
     if (N == 3) return small_force<3, T>(c, mode, U, Pin, Pout, Uout, ek, ed);
     if (N == 4) return small_force<4, T>(c, mode, U, Pin, Pout, Uout, ek, ed);
   }
+  if (N <= 4) return rows_force<4, T>(c, mode, U, Pin, Pout, Uout, ek, ed);
   if (N <= 8) return rows_force<8, T>(c, mode, U, Pin, Pout, Uout, ek, ed);
   if (N <= 16) return rows_force<16, T>(c, mode, U, Pin, Pout, Uout, ek, ed);
   if (N <= 32) return rows_force<32, T>(c, mode, U, Pin, Pout, Uout, ek, ed);
@@ -281,6 +282,7 @@ cudaError_t drift(const LaunchCtx& c, void* U, const void* P, void* Pcopy, doubl
   }
   const cudaError_t e = cudaMemcpyAsync(Pcopy, P, field_elems(c.lat) * sizeof(cpx<T>), cudaMemcpyDeviceToDevice, c.stream);
   if (e != cudaSuccess) return e;
+  if (N <= 4) return rows_drift<4, T>(c, U, P, eps);
   if (N <= 8) return rows_drift<8, T>(c, U, P, eps);
   if (N <= 16) return rows_drift<16, T>(c, U, P, eps);
   if (N <= 32) return rows_drift<32, T>(c, U, P, eps);

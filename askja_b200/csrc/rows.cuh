@@ -35,10 +35,17 @@ __device__ __forceinline__ cpx<T>* group_tile(unsigned char* smem_raw, int g, in
   return reinterpret_cast<cpx<T>*>(smem_raw) + (size_t)g * group_elems<T>(N);
 }
 
-// whether the fields are link-major (NC <= 4 runs on the kernels of NMAX = 8)
+// whether the fields are link-major (NC <= 4 has kernels of its own, NMAX = 4: the
+// layout chosen at run time cost them and NC = 5..8 up to 12 %)
 template <int NMAX>
-__device__ __forceinline__ bool major(int N) {
-  return NMAX > 8 || link_major(N);
+__host__ __device__ constexpr bool major() {
+  return NMAX > 4;
+}
+
+// offset of element 0 of the link (d, s)
+template <int NMAX>
+__device__ __forceinline__ size_t lbase(const Lat& L, int d, int s) {
+  return major<NMAX>() ? ((size_t)d * L.V + s) * (size_t)(L.N * L.N) : bbase(L, d, s);
 }
 
 // One thread's share q < NC of copying the link (d, s) to its tile, element
@@ -51,31 +58,36 @@ template <int NMAX, typename T, typename S2>
 __device__ __forceinline__ void stage(cpx<T>* tile, int NP, const S2* __restrict__ f, const Lat& L, int d, int s,
                                       int q) {
   const int N = L.N;
-  if (major<NMAX>(N)) {
-    const S2* p = f + ((size_t)d * L.V + s) * (size_t)(N * N) + q;
+  if constexpr (major<NMAX>()) {
+    const S2* p = f + lbase<NMAX>(L, d, s) + q;
     if constexpr (NMAX == 8 && sizeof(T) == 4) {
+      // always true, but a branch that keeps the loads of the next matrices behind this
+      // one's: three in flight cost a resident CTA (136 registers; SU(8) 8^4 kick 66 ->
+      // 107 us)
+      if (N > 4) {
 #pragma unroll
-      for (int c = 0; c < NMAX; c++)
-        if (c < N) tile[c * NP + q] = ldc<T>(p + c * N);
+        for (int c = 0; c < NMAX; c++)
+          if (c < N) tile[c * NP + q] = ldc<T>(p + c * N);
+      }
     } else {
       constexpr int LOADS = NMAX <= 16 ? 4 : 16;  // in flight
 #pragma unroll LOADS
       for (int c = 0; c < N; c++) tile[c * NP + q] = ldc<T>(p + c * N);
     }
     if (NP > N) tile[q * NP + N] = czero<T>();
-    return;
-  }
-  const S2* p = f + bbase(L, d, s) + (size_t)q * N * 32;
+  } else {
+    const S2* p = f + lbase<NMAX>(L, d, s) + (size_t)q * N * 32;
 #pragma unroll
-  for (int c = 0; c < NMAX; c += 2) {
-    if (c >= N) continue;
-    const cpx<T> v0 = ldc<T>(p + c * 32);
-    const cpx<T> v1 = c + 1 < N ? ldc<T>(p + (c + 1) * 32) : czero<T>();
-    if constexpr (sizeof(T) == 4) {
-      *reinterpret_cast<float4*>(tile + q * NP + c) = make_float4(v0.re, v0.im, v1.re, v1.im);
-    } else {
-      tile[q * NP + c] = v0;
-      tile[q * NP + c + 1] = v1;
+    for (int c = 0; c < NMAX; c += 2) {
+      if (c >= N) continue;
+      const cpx<T> v0 = ldc<T>(p + c * 32);
+      const cpx<T> v1 = c + 1 < N ? ldc<T>(p + (c + 1) * 32) : czero<T>();
+      if constexpr (sizeof(T) == 4) {
+        *reinterpret_cast<float4*>(tile + q * NP + c) = make_float4(v0.re, v0.im, v1.re, v1.im);
+      } else {
+        tile[q * NP + c] = v0;
+        tile[q * NP + c + 1] = v1;
+      }
     }
   }
 }
@@ -84,8 +96,8 @@ __device__ __forceinline__ void stage(cpx<T>* tile, int NP, const S2* __restrict
 template <int NMAX, typename T, typename S2>
 __device__ __forceinline__ void unstage(S2* f, const cpx<T>* tile, int LD, const Lat& L, int d, int s, int q) {
   const int N = L.N;
-  const bool m = major<NMAX>(N);
-  S2* p = m ? f + ((size_t)d * L.V + s) * (size_t)(N * N) + q : f + bbase(L, d, s) + (size_t)q * N * 32;
+  constexpr bool m = major<NMAX>();
+  S2* p = f + lbase<NMAX>(L, d, s) + (m ? q : q * N * 32);
   const cpx<T>* t = m ? tile + q : tile + q * LD;
   const int fs = m ? N : 32, ts = m ? LD : 1;
 #pragma unroll 4
@@ -174,8 +186,8 @@ __device__ __forceinline__ void row_times_tile_acc(cpx<T> (&acc)[NMAX], const cp
 template <int NMAX, typename T, typename S2>
 __device__ __forceinline__ void load_row(cpx<T> (&v)[NMAX], const S2* __restrict__ f, const Lat& L, int d, int s,
                                          int r) {
-  const int N = L.N, es = major<NMAX>(N) ? 1 : 32;
-  const S2* p = f + mbase(L, d, s) + (size_t)r * N * es;
+  const int N = L.N, es = major<NMAX>() ? 1 : 32;
+  const S2* p = f + lbase<NMAX>(L, d, s) + (size_t)r * N * es;
 #pragma unroll
   for (int c = 0; c < NMAX; c++)
     if (c < N) v[c] = ldc<T>(p + c * es);
@@ -184,8 +196,8 @@ __device__ __forceinline__ void load_row(cpx<T> (&v)[NMAX], const S2* __restrict
 template <int NMAX, typename T, typename S2>
 __device__ __forceinline__ void store_row(S2* __restrict__ f, const cpx<T> (&v)[NMAX], const Lat& L, int d, int s,
                                           int r) {
-  const int N = L.N, es = major<NMAX>(N) ? 1 : 32;
-  S2* p = f + mbase(L, d, s) + (size_t)r * N * es;
+  const int N = L.N, es = major<NMAX>() ? 1 : 32;
+  S2* p = f + lbase<NMAX>(L, d, s) + (size_t)r * N * es;
 #pragma unroll
   for (int c = 0; c < NMAX; c++)
     if (c < N) stc(p + c * es, v[c]);
@@ -425,7 +437,7 @@ __device__ __forceinline__ void force_rows(const Lat& L, const S2* __restrict__ 
   cpx<T>* T1 = T0 + N * NP;
   cpx<T>* T2 = T1 + N * NP;
   // copy role
-  const bool m = major<NMAX>(N);
+  constexpr bool m = major<NMAX>();
   const int cg = m ? g : tid % GS;
   const int cr = m ? r : tid / GS;
   const int cx = site0 + cg;
@@ -549,8 +561,8 @@ __device__ __forceinline__ void force_rows(const Lat& L, const S2* __restrict__ 
     // FP32, NC <= 8, order >= 5: the same series by Paterson-Stockmeyer (the
     // Horner loop below is then skipped; for larger NC its extra row arrays
     // cost more occupancy than it saves); FP64 keeps the reference's Horner order
-    const bool ps = sizeof(T) == 4 && NMAX == 8 && order >= 5;
-    if constexpr (sizeof(T) == 4 && NMAX == 8)
+    const bool ps = sizeof(T) == 4 && NMAX <= 8 && order >= 5;
+    if constexpr (sizeof(T) == 4 && NMAX <= 8)
       if (ps) drift_ps<NMAX, T>(tm, p, u, T0, T1, T2, N, NP, r, act, order);
     for (int n = ps ? 0 : order; n >= 1; n--) {
       __syncthreads();
