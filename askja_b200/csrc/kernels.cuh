@@ -91,6 +91,16 @@ cudaError_t rows_drift(const LaunchCtx& c, void* U, const void* P, double eps) {
   return cudaGetLastError();
 }
 
+// the thread-per-link kernel of register budget 0
+template <int N, typename T, int MODE>
+constexpr auto default_force() {
+  using S2 = typename Storage<T>::type;
+  if constexpr (sizeof(T) == 4 && small::HELD<N, MODE> != 0)
+    return small::k_force_occ<N, T, S2, MODE, small::HELD<N, MODE>>;
+  else
+    return small::k_force<N, T, S2, MODE>;
+}
+
 template <int N, typename T>
 cudaError_t small_force(const LaunchCtx& c, int mode, const void* U, const void* Pin, void* Pout, void* Uout,
                         double ek, double ed) {
@@ -119,7 +129,7 @@ cudaError_t small_force(const LaunchCtx& c, int mode, const void* U, const void*
                ? (mode == 0 ? small::k_force_occ<N, T, S2, 0, 2> : small::k_force_occ<N, T, S2, 1, 2>)
            : c.small_occ == 1
                ? (mode == 0 ? small::k_force_occ<N, T, S2, 0, 1> : small::k_force_occ<N, T, S2, 1, 1>)
-               : (mode == 0 ? small::k_force<N, T, S2, 0> : small::k_force<N, T, S2, 1>);
+               : (mode == 0 ? default_force<N, T, 0>() : default_force<N, T, 1>());
   return launch_overlapped(k, grid, threads, 0, c.stream, c.lat, u, pi, (S2*)Pout, (S2*)Uout, (T)ek, (T)ed, c.order,
                            c.reunit);
 }

@@ -863,7 +863,20 @@ __global__ void __launch_bounds__(128) k_force_sums(Lat L, const S2* U, const S2
 
 // The same kernel with a tighter register budget for more resident CTAs
 // (OCC = 1: 6 per SM in FP32, 3 in FP64; OCC = 2: 7 / 4); the autotuner picks
-// the budget where it is faster.
+// the budget where it is faster.  Budget 0 in FP32 is held to the CTAs it has where
+// its registers would take a step more: HELD<N>.
+template <int N, int MODE>
+constexpr int HELD = 0;  // k_force
+// us, held / not, of the kick of SU(4) 24^4 204 / 235 (127 and 130 registers)
+template <>
+constexpr int HELD<4, 0> = -1;
+// of SU(3) 24^4 122 / 126 (80, 90)
+template <>
+constexpr int HELD<3, 0> = 1;
+// of the fused step of SU(2) 24^4 57.8 / 61 (56, 62)
+template <>
+constexpr int HELD<2, 1> = 4;
+
 template <int N, typename T, typename S2, int MODE, int OCC = 1>
 __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 5 + OCC : 2 + OCC)
     k_force_occ(Lat L, const S2* U, const S2* Pin, S2* Pout, S2* Uout, T eps_k, T eps_d, int order, int reunit) {
