@@ -178,14 +178,12 @@ __host__ __device__ __forceinline__ size_t eoff(const Lat& L, int d, int e, int 
   return mbase(L, d, s) + (size_t)e * estride(L);
 }
 
-// The same for a colour number known at compile time (NT 2..4: blocked, no
-// choice of layout at run time; NT 0: any).
+// The same for a colour number NT <= 4 known at compile time: blocked, no choice
+// of layout at run time.
 template <int NT>
 __host__ __device__ __forceinline__ size_t eoffn(const Lat& L, int d, int e, int s) {
-  if constexpr (NT > 0 && NT <= 4)
-    return ((size_t)d * L.B + (s >> 5)) * (size_t)(NT * NT * 32) + (s & 31) + (size_t)e * 32;
-  else
-    return eoff(L, d, e, s);
+  static_assert(NT >= 2 && NT <= 4, "blocked layout");
+  return ((size_t)d * L.B + (s >> 5)) * (size_t)(NT * NT * 32) + (s & 31) + (size_t)e * 32;
 }
 
 // Link and matrix element of the t-th complex number of a field; false for padding.

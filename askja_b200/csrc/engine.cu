@@ -508,7 +508,7 @@ int askja_create(const askja_params* p, askja_ctx** out) {
   if (p->kernel_path < 0 || p->kernel_path > 3)
     return set_err(nullptr, ASKJA_ERR_ARG, "unknown kernel path %d", p->kernel_path);
   if (p->kernel_path == 2 && !askja::tc_supported(p->nc, p->dim, p->precision == ASKJA_FP64))
-    return set_err(nullptr, ASKJA_ERR_ARG, "tensor-core path needs FP32, NC = 32 or 64 and DIM >= 2");
+    return set_err(nullptr, ASKJA_ERR_ARG, "tensor-core path needs FP32, NC = 16, 32 or 64 and DIM >= 2");
   if (p->kernel_path == 3 && !askja::pair_supported(p->nc, p->dim, p->precision == ASKJA_FP64, p->n[p->dim - 1]))
     return set_err(nullptr, ASKJA_ERR_ARG, "site-pair path needs FP32, NC = 3, DIM >= 2 and an even N%d",
                    p->dim - 1);
@@ -605,7 +605,8 @@ int askja_create(const askja_params* p, askja_ctx** out) {
   // untuned default: thread-per-link for NC <= 4, warp MMA above; FP32 NC = 64 the tcgen05 path, whose products
   // are large enough there (us per step, tcgen05 / warp MMA: SU(64) 4x4 57 / 93, 4x8x16 773 / 1383; SU(32) 4x4
   // 31 / 16, 8^4 1902 / 1687; SU(16) 6^4 278 / 74: a product of two small matrices waits for its operands' way
-  // through shared memory and the accumulator's way back).  All are explicit paths and autotuner candidates.
+  // through shared memory and the accumulator's way back).  All are autotuner candidates and paths of
+  // askja_set_tuning; kernel_path names the tcgen05 path but not the warp MMA, the default of the other NC >= 5.
   c->lc.force_rows = p->kernel_path != 0 ? p->kernel_path
                      : (p->nc == 64 && askja::tc_supported(p->nc, p->dim, p->precision == ASKJA_FP64)) ? 2
                      : askja::m64_supported(p->nc)                                                     ? 4

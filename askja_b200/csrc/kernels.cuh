@@ -142,7 +142,7 @@ cudaError_t small_drift(const LaunchCtx& c, void* U, const void* P, void* Pcopy,
   return cudaGetLastError();
 }
 
-// FP64-MMA kernels: this lattice's fields as their job
+// Warp-MMA kernels: this lattice's fields as their job
 inline m64::Job m64_job(const Lat& L) {
   m64::Job j{};
   j.nbr = L.nbr;

@@ -12,7 +12,7 @@ size_t partial_doubles(const Lat& L) {
   const size_t links = 3 * ((nl + misc::RED_THREADS - 1) / misc::RED_THREADS);
   // partial matrices of the Gauss law and their sum
   const size_t gauss = 2 * (size_t)L.N * L.N * (detail::gauss_partials(L) + 1);
-  // the FP64-MMA reductions: blocks of sites and of links
+  // the warp-MMA reductions: blocks of sites and of links
   const size_t big = !m64_supported(L.N) ? 0
                                          : std::max(2 * (size_t)m64::ctas_for(L.V, m64::sites_per_cta(L.N)),
                                                     3 * (size_t)m64::ctas_for(nl, m64::sites_per_cta(L.N)));

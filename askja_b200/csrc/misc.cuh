@@ -1,11 +1,12 @@
 // Reductions, measurements, momentum refresh, hot start and the Metropolis
 // step.  Every reduction accumulates in FP64 whatever the storage precision
-// of the links (FP32 links are promoted on load), writes one partial per
-// block, and a single-block pass sums the partials in block order, so results
-// are deterministic run to run.
+// of the links (FP32 links are promoted on load) and writes one partial per
+// block; the last block to do so sums them in block order (publish; a pass of
+// one block, k_finish, in static_plaq.cu), so results are deterministic run to
+// run.
 //
-// The kernels take the colour number as a template parameter NT for the small
-// cases (fully unrolled) and NT = 0 for any NC (runtime loops).
+// The reductions take the colour number, 2 to 4, as a template parameter NT and
+// are fully unrolled; those of NC >= 5 are in mma64.cuh.
 #pragma once
 
 #include <cooperative_groups.h>
@@ -362,10 +363,9 @@ __device__ __forceinline__ void refresh_link(const Lat& L, S2* __restrict__ P, u
   const int N = L.N;
   const int d = (int)(t / L.V);
   const int s = (int)(t - (long)d * L.V);
-  S2* p = P + mbase(L, d, s);
-  const int es = estride(L);
+  S2* p = P + bbase(L, d, s);
   refresh_entries(L, seed, traj, scale, d, s,
-                  [&](int i, int j, const cpx<double>& v) { stc(p + (i * N + j) * es, v); });
+                  [&](int i, int j, const cpx<double>& v) { stc(p + (i * N + j) * 32, v); });
 }
 
 // refresh_link for link-major fields, a thread per Philox block: block b of a

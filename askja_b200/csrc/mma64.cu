@@ -1,4 +1,4 @@
-// Dispatch of the FP64-MMA kernels over storage type and tile count.
+// Dispatch of the warp-MMA kernels over storage type and tile count.
 #include "mma64_launch.cuh"
 
 namespace askja {

@@ -1,6 +1,7 @@
-// Launches of the FP64-MMA kernels (mma64.cuh) for 5 <= NC <= 64: one lattice
-// by value (table null), or the CTAs of many lattices of one colour number
-// through a job table and a per-CTA list of (job, block).
+// Launches of the warp-MMA kernels (mma64.cuh: FP64, and split TF32 for FP32
+// storage) for 5 <= NC <= 64: one lattice by value (table null), or the CTAs of
+// many lattices of one colour number through a job table and a per-CTA list of
+// (job, block).
 #pragma once
 
 #include <cuda_runtime.h>

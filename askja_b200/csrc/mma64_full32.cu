@@ -1,4 +1,4 @@
-// FP64-MMA kernels, FP32 storage, NC a multiple of 8 (a translation unit of its own: build time).
+// Warp-MMA kernels (FP64 and split TF32), FP32 storage, NC a multiple of 8 (a translation unit of its own: build time).
 #include "mma64_launch.cuh"
 
 namespace askja {

@@ -1,4 +1,4 @@
-// FP64-MMA kernels, FP64 storage, NC a multiple of 8 (a translation unit of its own: build time).
+// Warp-MMA kernels (FP64), FP64 storage, NC a multiple of 8 (a translation unit of its own: build time).
 #include "mma64_launch.cuh"
 
 namespace askja {

@@ -1,4 +1,4 @@
-// FP64-MMA kernels, FP64 storage, any other NC (a translation unit of its own: build time).
+// Warp-MMA kernels (FP64), FP64 storage, any other NC (a translation unit of its own: build time).
 #include "mma64_launch.cuh"
 
 namespace askja {
